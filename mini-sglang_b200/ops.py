@@ -6,7 +6,8 @@ tensor that is not on a CUDA device, a missing compiler or an unsupported size r
 Matrix products with more than a few rows are the one exception to "hand-written": `linear` then calls
 the library GEMM that torch binds (cuBLAS), in bfloat16 with float32 accumulation or in true float32
 (TF32 off), as the reference does for every projection (F.linear in mini_sglang/layers/linear.py).  Up to
-SMALL_M_MAX rows go to this engine's weight-streaming kernel.  The reference's own kernels for the
+SMALL_M_MAX rows go to this engine's weight-streaming kernel, and the gated products and output heads of larger decode batches to
+its decode-batch kernel.  The reference's own kernels for the
 other operations come from sgl_kernel / flash-attn (mini_sglang/layers/layernorm.py:39-50,
 mini_sglang/layers/rotary_embedding.py, mini_sglang/layers/attn/fa3_attn_backend.py).
 """
@@ -97,6 +98,8 @@ def _lib():
                                              c_void_p, c_void_p, c_void_p]
         lib.msgl_gemm_tc2_splits.argtypes = [c_int, c_int, c_int, c_int]
         lib.msgl_gemm_tc2_splits.restype = c_int
+        lib.msgl_gemm_rows.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_int, c_float, c_int,
+                                       c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
         lib.msgl_sample.argtypes = [c_void_p, c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_ull, c_void_p,
                                     c_void_p, c_void_p, c_void_p, c_int, c_void_p]
         _common = lib
@@ -663,6 +666,40 @@ def _tc_gemm_mid(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
     return out
 
 
+# The product for a decode batch (csrc/gemm_rows.cu: weights on the tensor core's M dimension, tokens on its N dimension) against
+# the library's, measured on B200 over the Qwen3 widths.  Gated products, [2 n_out, K] weights, library product + activation kernel
+# against this kernel: 16 rows [6144, 1024] 7.2 / 6.0 us, [12288, 2048] 14.1 / 11.4, [24576, 4096] 42.7 / 35.9, [51200, 5120] 99.9 / 82.5;
+# 64 rows 7.2 / 7.3, 14.4 / 13.2, 45.0 / 37.4, 103 / 83; 128 rows 7.6 / 9.5, 14.4 / 17.6, 45.3 / 41.8, 107 / 94; 176 rows behind everywhere.
+# Up to 8 rows the weight-streaming kernel is level (35.0 / 34.7 us at one row of [24576, 4096]) or ahead on small weights.
+# Float32 products with very many columns (output heads, 151,936 columns): K = 4096, 1 / 8 / 24 / 64 / 128 rows 194 / 200 / 214 / 215 / 233
+# (the better of the library and the weight-streaming kernel) against 181 / 184 / 188 / 196 / 227 us, K = 1024, 1 / 64 rows 54 / 64 against
+# 51 / 64; with 32,768 columns the last round of blocks is nearly empty and it is 2 to 18 % behind.  Plain bfloat16 products stay with
+# the library (4096 x 4096 at 48 rows: 9.6 against 10.1 us, 128 rows 9.7 against 12.3).
+ROWS_GLU_MAX, ROWS_GLU_MAX_LARGE, ROWS_LARGE_WEIGHT = 64, 128, 40_000_000      # rows; elements of the weight from which the second bound holds
+ROWS_F32_MAX, ROWS_F32_MIN_OUT = 128, 114_000
+
+
+def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """x @ weight^T (mode 0) or its gated activation (1: SwiGLU, 2: ReGLU; bias [2I]) for at most 256 rows by the decode-batch kernel;
+    None where it cannot run."""
+    if not (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2 and 0 < x.shape[0] <= 256
+            and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))
+            and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.is_contiguous() and weight.data_ptr() % 16 == 0
+            and weight.shape[1] % 8 == 0 and (bias is None or (bias.dtype == torch.bfloat16 and bias.is_contiguous()))):
+        return None
+    M, (N, K) = x.shape[0], weight.shape
+    n_out = N // 2 if mode else N
+    if n_out % 2 or (mode and N % 2) or (mode and out_dtype != torch.bfloat16):
+        return None
+    out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+    code = _lib().msgl_gemm_rows(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, n_out, K, x.stride(0), n_out, mode, int(out_dtype == torch.float32),
+                                 0.0, 0, None, 0, 0, 0, _ptr(_status_tensor(x.device)), _stream())
+    if code == 2:             # no tensor maps on this driver or of this layout
+        return None
+    _check(code, "gemm_rows")
+    return out
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """y = x @ weight^T (+ bias); weight is [out, in] as stored in the checkpoint.
@@ -670,6 +707,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     Up to SMALL_M_MAX bfloat16 rows go through this engine's weight-streaming kernel
     (csrc/gemm_small_m.cu); everything else is the library GEMM."""
     _need_cuda(x, weight, bias)
+    if out_dtype == torch.float32 and weight.shape[0] >= ROWS_F32_MIN_OUT and x.dim() == 2 and x.shape[0] <= ROWS_F32_MAX:
+        y = _gemm_rows(x, weight, bias, 0, torch.float32)
+        if y is not None:
+            return y
     if _small_m_ok(x, weight, bias) and out_dtype in (None, torch.bfloat16, torch.float32):
         M, (N, K) = x.shape[0], weight.shape
         od = out_dtype or torch.bfloat16
@@ -705,6 +746,10 @@ def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tens
             code = _small_m(gate_up, x, bias, out, M, N, K, N // 2, mode, 0)
             _check(code, "gemm_small_m (gated)")
             return out
+        if x.dim() == 2 and x.shape[0] <= (ROWS_GLU_MAX_LARGE if gate_up.numel() >= ROWS_LARGE_WEIGHT else ROWS_GLU_MAX):
+            y = _gemm_rows(x, gate_up, bias, mode, torch.bfloat16)
+            if y is not None:
+                return y
         y = _tc_gemm(x, gate_up, bias, mode) if x.shape[0] >= TC_GEMM_MIN_M else _tc_gemm_mid(x, gate_up, bias, mode)
         if y is not None:
             return y
