@@ -1193,6 +1193,7 @@ def _gated_lib():
         lib.msgl_experts_few.argtypes = [c_void_p, c_ll] + [c_void_p] * 4 + [c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int,
                                                                             c_float, c_void_p, c_void_p, c_void_p]
         lib.msgl_clamped_glu.argtypes = [c_void_p, c_ll, c_int, c_float, c_void_p, c_int, c_int, c_void_p]
+        lib.msgl_expert_rows.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
         lib.msgl_expert_order.argtypes = [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]
         lib.msgl_expert_gather.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p]
         lib.msgl_expert_combine.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_void_p,
@@ -1536,6 +1537,9 @@ def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx:
     assert gate_up.shape == (E, 2, F, H) and down.shape == (E, H, F)
     assert gate_up.is_contiguous() and down.is_contiguous() and gate_up.dtype == down.dtype == h.dtype
     assert idx.dtype == torch.int32 and wts.dtype == torch.float32 and idx.is_contiguous() and wts.is_contiguous()
+    done = _expert_products(h, gate_up, down, idx, limit, torch.float32)
+    if done is not None:
+        return expert_combine(done[0], done[1], wts, scale, extra=extra, extra_gate=extra_gate)
     act = torch.empty((T * top, F), dtype=h.dtype, device=h.device)
     out = torch.empty((T, H), dtype=torch.float32, device=h.device)
     code = _gated_lib().msgl_experts_few(_ptr(h), _rows_view(h, H, "h"), _ptr(gate_up), _ptr(down), _ptr(idx), _ptr(wts), top, H, F,
@@ -1545,6 +1549,70 @@ def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx:
     global LAUNCHES
     LAUNCHES += 1
     return out
+
+
+# The chosen experts' products on the decode-batch kernel (csrc/gemm_rows.cu, grouped: an expert's weights are read once, whatever the
+# number of tokens that chose it) against the others, measured on B200: a feed-forward of 32 experts of [2 x 1536, 2048] + [2048, 1536], four
+# a token, beside a shared one.  Against a warp per row and (token, choice) pair: 1 token 82 -> 66 us, 8 tokens 224 -> 106, 24 tokens
+# 528 -> 132, 128 tokens 2,516 -> 140.  Against the library's grouped product with the activation between: 300 tokens 230 -> 156,
+# 700 tokens 247 -> 184, 1,024 tokens (128 rows an expert) 267 -> 214; with 150 rows an expert its products take 178 us, the library's
+# 145: such tiles leave one block an SM.
+EXPERT_ROWS_MEAN_MAX = 128
+EXPERT_ROWS_MAX_PAIRS = 8192
+
+
+def expert_rows(h: torch.Tensor, idx: torch.Tensor, n_experts: int) -> Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]]:
+    """idx int32 [T, top], numbers below n_experts -> (rows [T * top, H]: every token's row once per expert it uses, in the order of the experts,
+    pairs of one expert in their own order; place int32 [T * top]: row of every pair; ends int32 [n_experts]: running sum of the experts'
+    rows) in one launch; None where the sizes are not the kernel's (see `expert_order`, `expert_gather`)."""
+    _need_cuda(h, idx)
+    T, H = h.shape
+    top = idx.shape[1]
+    V = 16 // h.element_size()
+    if T * top > EXPERT_ROWS_MAX_PAIRS or H % V or h.stride(0) % V or h.stride(1) != 1 or h.data_ptr() % 16 or n_experts > ROUTE_MAX_EXPERTS:
+        return None
+    assert idx.dtype == torch.int32 and idx.is_contiguous() and idx.shape[0] == T
+    rows = torch.empty((T * top, H), dtype=h.dtype, device=h.device)
+    place = torch.empty(T * top, dtype=torch.int32, device=h.device)
+    ends = torch.empty(n_experts, dtype=torch.int32, device=h.device)
+    _check(_gated_lib().msgl_expert_rows(_ptr(h), h.stride(0), _ptr(idx), T * top, top, n_experts, H, _ptr(rows), _ptr(place), _ptr(ends), _dt(h),
+                                         _stream()), "expert_rows")
+    return rows, place, ends
+
+
+def _expert_products(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, limit: float,
+                     out_dtype: torch.dtype) -> Optional[Tuple[torch.Tensor, torch.Tensor]]:
+    """Both products of the chosen experts, gate_up [E, 2, F, H] and down [E, H, F], with the activation of `experts_few` between them, on the
+    decode-batch kernel -> (y [T * top, H] in the order of the experts, place); None where it does not apply."""
+    T, H = h.shape
+    E, _, F, _ = gate_up.shape
+    P = T * idx.shape[1]
+    if h.dtype != torch.bfloat16 or H % 8 or F % 8 or P > EXPERT_ROWS_MEAN_MAX * E or gate_up.data_ptr() % 16 or down.data_ptr() % 16:
+        return None
+    ordered = expert_rows(h, idx, E)
+    if ordered is None:
+        return None
+    rows, place, ends = ordered
+    act = torch.empty((P, F), dtype=h.dtype, device=h.device)
+    y = torch.empty((P, H), dtype=out_dtype, device=h.device)
+    status = _ptr(_status_tensor(h.device))
+    code = _lib().msgl_gemm_rows(_ptr(gate_up), _ptr(rows), None, _ptr(act), P, F, H, H, F, 3 if limit > 0 else 1, 0, float(limit), E, _ptr(ends), T, 0, 0,
+                                 status, _stream())
+    if code == 2:             # no tensor maps on this driver
+        return None
+    _check(code, "gemm_rows (experts)")
+    _check(_lib().msgl_gemm_rows(_ptr(down), _ptr(act), None, _ptr(y), P, H, F, F, H, 0, int(out_dtype == torch.float32), 0.0, E, _ptr(ends), T, 0, 0,
+                                 status, _stream()), "gemm_rows (experts)")
+    return y, place
+
+
+def experts_many(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, scale: float = 1.0,
+                 limit: float = 0.0, extra: Optional[torch.Tensor] = None, extra_gate: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+    """`experts_few` for the tokens of a prompt portion (the experts' outputs are rounded to the activation type before they are
+    summed): None where the decode-batch kernel does not apply or the library's grouped product is ahead."""
+    _need_cuda(h, gate_up, down, idx, wts, extra)
+    done = _expert_products(h, gate_up, down, idx, limit, h.dtype)
+    return None if done is None else expert_combine(done[0], done[1], wts, scale, extra=extra, extra_gate=extra_gate)
 
 
 def expert_order(idx: torch.Tensor, n_experts: int) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:

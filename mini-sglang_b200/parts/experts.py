@@ -75,6 +75,9 @@ class RoutedExperts(FeedForward):
         T = x.shape[0]
         if ctx.uniform_decode or T * self.top <= ops.EXPERTS_FEW_PAIRS:
             return ops.experts_few(x, self.gate_up, self.down, idx, wts, self.out_scale)
+        y = ops.experts_many(x, self.gate_up, self.down, idx, wts, self.out_scale)
+        if y is not None:
+            return y
         counts, ends, place = ops.expert_order(idx, self.n_exp)
         rows = ops.expert_gather(x, place, self.top)
         if x.dtype == torch.bfloat16 and self.H % 8 == 0 and self.F % 8 == 0 and hasattr(torch, "_grouped_mm"):
@@ -164,6 +167,9 @@ class SoftmaxExperts(FeedForward):
         T = x.shape[0]
         if ctx.uniform_decode or T * self.top <= ops.EXPERTS_FEW_PAIRS:
             return ops.experts_few(x, self.gate_up, self.down, idx, wts, limit=self.limit, extra=shared, extra_gate=sgate)
+        y = ops.experts_many(x, self.gate_up, self.down, idx, wts, limit=self.limit, extra=shared, extra_gate=sgate)
+        if y is not None:
+            return y
         counts, ends, place = ops.expert_order(idx, self.n_exp)
         rows = ops.expert_gather(x, place, self.top)
         if x.dtype == torch.bfloat16 and self.H % 8 == 0 and self.F % 8 == 0 and hasattr(torch, "_grouped_mm"):
