@@ -1031,6 +1031,7 @@ struct DeltaParams {
     float2* kq; float4* sc;                      // what delta_prep_kernel leaves
     float* state; const int* q_start; const int* slots; float* out;
     int heads, kv_heads, d, dv, T;
+    int n_min, n_max;                            // the requests that a launch takes: those with n_min <= tokens <= n_max
 };
 
 template <typename T>
@@ -1086,7 +1087,7 @@ __global__ void __launch_bounds__(DR_MANY_WARPS * 32) delta_rule_kernel(const De
     const int part = lane / DR_WCOLS, wc = lane % DR_WCOLS;             // lanes of a part read neighbouring columns
     const int g = h / (p.heads / p.kv_heads);
     const int t0 = p.q_start[r], n = p.q_start[r + 1] - t0;
-    if (n <= 0) return;
+    if (n < p.n_min || n > p.n_max) return;
     const int lcol = warp * DR_WCOLS + wc, col = c0 + lcol;
     const bool col_ok = col < dv;
     const int Ck = p.kv_heads * d, W = 2 * Ck + p.heads * dv;
@@ -1166,15 +1167,402 @@ __global__ void __launch_bounds__(DR_MANY_WARPS * 32) delta_rule_kernel(const De
     }
 }
 
-// floats of scratch memory that msgl_delta_rule wants for T tokens
-MSGL_API long long msgl_delta_rule_scratch(int T_, int heads, int kv_heads, int d) {
-    return (long long)T_ * kv_heads * d * 2 + (long long)T_ * heads * 4;
+// ---------------------------------------------------------------------------------------
+// The same recurrence for a run of tokens in chunks of DC_C (float32 throughout).  With the chunk's start state S0, its decays
+// multiplied up, P_t = g_1 ... g_t and D_ts = g_(s+1) ... g_t:
+//     u_t + sum_{s < t} beta_t D_ts (k_t . k_s) u_s = beta_t v_t - beta_t P_t S0^T k_t
+//     o_t = P_t S0^T q_t + sum_{s <= t} D_ts (q_t . k_s) u_s,      S <- P_C S0 + sum_s D_Cs k_s u_s^T
+// so u = U - W S0 with U and W from two forward substitutions that do not read the state.  delta_chunk_kernel makes U, W and the
+// weights M_ts = D_ts (q_t . k_s) of all chunks side by side; delta_chunk_scan_kernel walks a request's chunks in order with 16 columns
+// of one state a block: three small products a chunk from shared memory, the next chunk's operands on their way.
+// The decays are products of the g themselves, not differences of sums of logarithms, which would lose digits where they are small.
+//
+// Token by token the walk is a chain (a product with the state, two rounds of shuffles, the update) of 0.37 us a token whatever the number of
+// SMs; a chunk of 32 tokens takes the blocks about 1.3 us.  32 and not 64: the work a token grows by a fifth with 64, and the walk gets no shorter.
+// ---------------------------------------------------------------------------------------
+constexpr int DC_C = 32, DC_COLS = 16, DC_THREADS = 256;
+
+struct DeltaChunkParams {
+    const void* qkv; const float2* kq; const float4* sc;
+    float* W;                                    // [T][heads][d]
+    float* U;                                    // [T][heads][dv]
+    float* M;                                    // [T][heads][DC_C]: row t of its chunk's weights, zeros behind the diagonal
+    float2* ps;                                  // [T][heads]: P_t and D_Ct
+    float* K; float* Q;                          // [T][kv_heads][d]
+    float* state; const int* q_start; const int* slots; float* out;
+    int heads, kv_heads, dv, T, B, n_min;
+};
+
+// A block makes one head's chunk.  Latency decides (loads, 32 steps of the decays, the substitution's chain), so four blocks share an SM: with the
+// substitution's factors kept in registers (255 a thread, one block an SM) and the heads of a q/k head in one block it took 116 us
+// for 1,411 tokens of 16 heads.
+template <typename T, int D>
+__global__ void __launch_bounds__(DC_THREADS, 3) delta_chunk_kernel(const DeltaChunkParams p) {
+    constexpr int LD = D + 4;                    // rows 16 bytes apart in the banks
+    extern __shared__ __align__(16) unsigned char dc_smem[];
+    float* Ks = reinterpret_cast<float*>(dc_smem);           // [C][LD]
+    float* Qs = Ks + DC_C * LD;                              // [C][LD]
+    float* KK = Qs + DC_C * LD;                              // [C][C + 1]
+    float* QK = KK + DC_C * (DC_C + 1);                      // [C][C + 1]
+    float* Ls = QK + DC_C * (DC_C + 1);                      // [C][C], 16-byte rows
+    float* Ms = Ls + DC_C * DC_C;                            // [C][C]
+    __shared__ float beta_s[DC_C], g_s[DC_C], pre_s[DC_C], suf_s[DC_C];
+    __shared__ int where_s[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, per = p.heads / p.kv_heads, g = h / per;
+    if (warp == 0) {                             // the blockIdx.x-th chunk of the requests that are taken, 32 requests a look
+        int left = blockIdx.x, at = -1, rest = 0;
+        for (int r0 = 0; r0 < p.B && at < 0; r0 += 32) {
+            const int r = r0 + lane;
+            const int n = r < p.B ? p.q_start[r + 1] - p.q_start[r] : 0;
+            const int c = n >= p.n_min ? (n + DC_C - 1) / DC_C : 0;
+            int sum = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
+            const unsigned hit = __ballot_sync(0xffffffffu, left < sum);
+            if (hit) {
+                const int l = __ffs(hit) - 1;
+                at = r0 + l;
+                rest = left - __shfl_sync(0xffffffffu, sum - c, l);
+            }
+            left -= __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) { where_s[0] = at; where_s[1] = rest; }
+    }
+    __syncthreads();
+    if (where_s[0] < 0) return;
+    const int r = where_s[0], base = p.q_start[r] + where_s[1] * DC_C, nb = min(DC_C, p.q_start[r + 1] - base);
+    const bool first = h == g * per;             // this head's block leaves k and q for the walk
+#pragma unroll 4
+    for (int i = tid; i < DC_C * D / 2; i += DC_THREADS) {
+        const int t = i / (D / 2), e = 2 * (i - t * (D / 2));
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < nb) {
+            const size_t at = ((size_t)(base + t) * p.kv_heads + g) * D + e;
+            v = *reinterpret_cast<const float4*>(p.kq + at);
+            if (first) {
+                *reinterpret_cast<float2*>(p.K + at) = make_float2(v.x, v.z);
+                *reinterpret_cast<float2*>(p.Q + at) = make_float2(v.y, v.w);
+            }
+        }
+        *reinterpret_cast<float2*>(Ks + t * LD + e) = make_float2(v.x, v.z);
+        *reinterpret_cast<float2*>(Qs + t * LD + e) = make_float2(v.y, v.w);
+    }
+    if (tid < DC_C) {
+        const float4 c = tid < nb ? p.sc[(size_t)(base + tid) * p.heads + h] : make_float4(0.f, 1.f, 0.f, 0.f);
+        beta_s[tid] = c.x; g_s[tid] = c.y;
+    }
+    __syncthreads();
+    {   // k_t . k_s and q_t . k_s: rows ti, ti + 16 against columns tj, tj + 16
+        const int ti = tid >> 4, tj = tid & 15;
+        float kk[2][2][4] = {}, qk[2][2][4] = {};            // four partial sums each: less rounding than one over all of D
+#pragma unroll 2
+        for (int e = 0; e < D; e += 4) {
+            float4 kt[2], qt[2], ks[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                kt[i] = *reinterpret_cast<const float4*>(Ks + (ti + 16 * i) * LD + e);
+                qt[i] = *reinterpret_cast<const float4*>(Qs + (ti + 16 * i) * LD + e);
+                ks[i] = *reinterpret_cast<const float4*>(Ks + (tj + 16 * i) * LD + e);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    kk[i][j][0] = fmaf(kt[i].x, ks[j].x, kk[i][j][0]); kk[i][j][1] = fmaf(kt[i].y, ks[j].y, kk[i][j][1]);
+                    kk[i][j][2] = fmaf(kt[i].z, ks[j].z, kk[i][j][2]); kk[i][j][3] = fmaf(kt[i].w, ks[j].w, kk[i][j][3]);
+                    qk[i][j][0] = fmaf(qt[i].x, ks[j].x, qk[i][j][0]); qk[i][j][1] = fmaf(qt[i].y, ks[j].y, qk[i][j][1]);
+                    qk[i][j][2] = fmaf(qt[i].z, ks[j].z, qk[i][j][2]); qk[i][j][3] = fmaf(qt[i].w, ks[j].w, qk[i][j][3]);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int at = (ti + 16 * i) * (DC_C + 1) + tj + 16 * j;
+                KK[at] = (kk[i][j][0] + kk[i][j][1]) + (kk[i][j][2] + kk[i][j][3]);
+                QK[at] = (qk[i][j][0] + qk[i][j][1]) + (qk[i][j][2] + qk[i][j][3]);
+            }
+    }
+    const int Ck = p.kv_heads * D, Wd = 2 * Ck + p.heads * p.dv;
+    const T* qkv = reinterpret_cast<const T*>(p.qkv);
+    __syncthreads();
+    if (tid < DC_C) {                            // column s = tid: the decays from s on
+        const int s = tid;
+        float run = 1.f;
+        for (int t = 0; t < DC_C; ++t) {
+            if (t > s) run *= g_s[t];
+            Ls[t * DC_C + s] = t > s ? beta_s[t] * run * KK[t * (DC_C + 1) + s] : 0.f;
+            Ms[t * DC_C + s] = t >= s ? run * QK[t * (DC_C + 1) + s] : 0.f;
+            if (s == 0) pre_s[t] = g_s[0] * run;
+            if (t == nb - 1) suf_s[s] = run;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < nb * DC_C; i += DC_THREADS) p.M[((size_t)(base + i / DC_C) * p.heads + h) * DC_C + i % DC_C] = Ms[i];
+    if (tid < nb) p.ps[(size_t)(base + tid) * p.heads + h] = make_float2(pre_s[tid], suf_s[tid]);
+    for (int c = tid; c < p.dv + D; c += DC_THREADS) {
+        const bool is_u = c < p.dv;
+        float x[DC_C];
+        if (is_u) {              // all loads under way at once; rows behind the last token repeat it and are not used (their beta is 0)
+            const T* src = qkv + (size_t)base * Wd + 2 * Ck + (size_t)h * p.dv + c;
+            T raw[DC_C];
+#pragma unroll
+            for (int t = 0; t < DC_C; ++t) raw[t] = src[(size_t)min(t, nb - 1) * Wd];
+#pragma unroll
+            for (int t = 0; t < DC_C; ++t) x[t] = to_f32<T>(raw[t]);
+        } else {
+#pragma unroll
+            for (int t = 0; t < DC_C; ++t) x[t] = pre_s[t] * Ks[t * LD + c - p.dv];
+        }
+        float* dst = is_u ? p.U + ((size_t)base * p.heads + h) * p.dv + c : p.W + ((size_t)base * p.heads + h) * D + (c - p.dv);
+        const size_t step = (size_t)p.heads * (is_u ? p.dv : D);
+#pragma unroll
+        for (int t = 0; t < DC_C; ++t) {
+            float a0 = beta_s[t] * x[t], a1 = 0.f;
+#pragma unroll
+            for (int s4 = 0; s4 < t; s4 += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(Ls + t * DC_C + s4);
+                a0 = fmaf(-l.x, x[s4], a0);
+                if (s4 + 1 < t) a1 = fmaf(-l.y, x[s4 + 1], a1);
+                if (s4 + 2 < t) a0 = fmaf(-l.z, x[s4 + 2], a0);
+                if (s4 + 3 < t) a1 = fmaf(-l.w, x[s4 + 3], a1);
+            }
+            x[t] = a0 + a1;
+            if (t < nb) dst[t * step] = x[t];
+            if (t % 4 == 3) asm volatile("" ::: "memory");       // the next rows' factors are read here, not all at the start into 255 registers
+        }
+    }
 }
 
+// Shared memory of a block of the walk, in floats: W, Q and the decays of two chunks (the next one's on their way), K, M and U of the chunk under way
+// (asked for at its start), the state's columns, u.  104 KB: two blocks an SM.
+template <int D> struct DcStage {
+    static constexpr int LD = D + 4, LDM = DC_C + 4;
+    static constexpr int W = 0, Q = W + DC_C * LD, PS = Q + DC_C * LD, SIZE = PS + 2 * DC_C;
+    static constexpr int K = 2 * SIZE, M = K + DC_C * LD, U = M + DC_C * LDM, S = U + DC_C * DC_COLS, US = S + D * DC_COLS + D, UDS = US + DC_C * DC_COLS;
+    static constexpr int TOTAL = UDS + DC_C * DC_COLS;
+    static_assert(DC_C * LD >= 4 * 2 * DC_C * DC_COLS, "the partial sums lie over W");
+};
+
+template <int D>
+__global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_scan_kernel(const DeltaChunkParams p) {
+    static_assert(D == 128, "the update's layout is that of 128 rows");
+    using St = DcStage<D>;
+    constexpr int LD = St::LD, LDM = St::LDM, KS = D / 4;      // KS: a quarter of the state's rows
+    extern __shared__ __align__(16) unsigned char dc_smem[];
+    float* sm = reinterpret_cast<float*>(dc_smem);
+    float* Ss = sm + St::S;                                  // [D][16], four floats more behind every four rows (a quarter-warp writes rows 4 apart)
+    auto s_at = [](int row, int col) { return row * DC_COLS + (row >> 2) * 4 + col; };
+    float* us = sm + St::US;                                 // [C][16] u
+    float* uds = sm + St::UDS;                               // [C][16] u, decayed to the chunk's end
+    const int h = blockIdx.x, c0 = blockIdx.y * DC_COLS, r = blockIdx.z;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int t0 = p.q_start[r], n = p.q_start[r + 1] - t0;
+    if (n < p.n_min) return;
+    const int g = h / (p.heads / p.kv_heads), dv = p.dv;
+    float* S = p.state + ((size_t)p.slots[r] * p.heads + h) * D * dv + c0;
+
+    // the state entries this thread keeps: rows row0 .. row0 + 3, columns col0, col0 + 1
+    const int dl = lane & 7, b3 = (lane >> 3) & 1, b4 = lane >> 4;
+    const int row0 = (warp >> 2) * 64 + b4 * 32 + 4 * dl, col0 = (warp & 3) * 4 + 2 * b3;
+    float s_reg[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        s_reg[i][0] = S[(size_t)(row0 + i) * dv + col0];
+        s_reg[i][1] = S[(size_t)(row0 + i) * dv + col0 + 1];
+        *reinterpret_cast<float2*>(Ss + s_at(row0 + i, col0)) = make_float2(s_reg[i][0], s_reg[i][1]);
+    }
+    auto copy16 = [&](float* dst, const float* src, bool valid) {        // 16 bytes, zeros behind the request's last token
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0));
+    };
+    constexpr int V = D / 4;
+    auto fetch_ahead = [&](int st, int b0) {                 // W, Q and the decays of the chunk at b0
+        float* sp = sm + st * St::SIZE;
+        const int nb = min(DC_C, n - b0);
+        for (int i = tid; i < DC_C * V; i += DC_THREADS) {
+            const int t = i / V, e = (i - t * V) * 4;
+            const bool ok = t < nb;
+            const size_t tok = (size_t)(t0 + b0 + (ok ? t : 0));
+            copy16(sp + St::W + t * LD + e, p.W + (tok * p.heads + h) * D + e, ok);
+            copy16(sp + St::Q + t * LD + e, p.Q + (tok * p.kv_heads + g) * D + e, ok);
+        }
+        if (tid < DC_C) {
+            const bool ok = tid < nb;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(sp + St::PS + 2 * tid)),
+                         "l"(p.ps + (size_t)(t0 + b0 + (ok ? tid : 0)) * p.heads + h), "r"(ok ? 8 : 0));
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    auto fetch_now = [&](int b0) {                           // K, M and U of the chunk at b0
+        const int nb = min(DC_C, n - b0);
+        for (int i = tid; i < DC_C * V; i += DC_THREADS) {
+            const int t = i / V, e = (i - t * V) * 4;
+            const bool ok = t < nb;
+            copy16(sm + St::K + t * LD + e, p.K + ((size_t)(t0 + b0 + (ok ? t : 0)) * p.kv_heads + g) * D + e, ok);
+        }
+        const int t = tid >> 3, e = (tid & 7) * 4;
+        const bool ok = t < nb;
+        const size_t row = (size_t)(t0 + b0 + (ok ? t : 0)) * p.heads + h;
+        copy16(sm + St::M + t * LDM + e, p.M + row * DC_C + e, ok);
+        if (e < DC_COLS) copy16(sm + St::U + t * DC_COLS + e, p.U + row * dv + c0 + e, ok);
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    fetch_ahead(0, 0);
+    for (int b0 = 0, st = 0; b0 < n; b0 += DC_C, st ^= 1) {
+        const int nb = min(DC_C, n - b0);
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        __syncthreads();                         // W, Q and the state's columns are there; the rest of the shared memory is free
+        fetch_now(b0);
+        if (b0 + DC_C < n) fetch_ahead(st ^ 1, b0 + DC_C);
+        else asm volatile("cp.async.commit_group;\n" ::);
+        float* sp = sm + st * St::SIZE;
+        float* part = sp + St::W;                // [4][2 C][16] sums over quarters of the rows: W S, then Q S; over W once it is read
+        {   // W S and Q S: a warp takes one of them over a quarter of the rows, a thread tokens rg + 8 i and columns 4 cg ..
+            const int ks = warp & 3, rg = lane & 7, cg = lane >> 3;
+            const float* A = sp + (warp < 4 ? St::W : St::Q) + rg * LD + ks * KS;
+            const float* Bp = Ss + s_at(ks * KS, cg * 4);
+            float acc[4][4] = {};
+#pragma unroll 2
+            for (int e = 0; e < KS; e += 4) {
+                float4 a[4], b[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    a[i] = *reinterpret_cast<const float4*>(A + 8 * i * LD + e);
+                    b[i] = *reinterpret_cast<const float4*>(Bp + s_at(e + i, 0));
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float av[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        acc[i][0] = fmaf(av[k], b[k].x, acc[i][0]); acc[i][1] = fmaf(av[k], b[k].y, acc[i][1]);
+                        acc[i][2] = fmaf(av[k], b[k].z, acc[i][2]); acc[i][3] = fmaf(av[k], b[k].w, acc[i][3]);
+                    }
+                }
+            }
+            __syncthreads();
+            // the four 16-byte groups of a row turned by the row, so that the eight rows of a quarter-warp fall on different banks
+            float* dst = part + (ks * 2 * DC_C + (warp < 4 ? 0 : DC_C) + rg) * DC_COLS + ((cg + (rg >> 1)) & 3) * 4;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(dst + 8 * i * DC_COLS) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        }
+        asm volatile("cp.async.wait_group 1;\n" ::);
+        __syncthreads();                         // the partial sums, K, M and U
+        const int t = tid >> 3, c = (tid & 7) * 2;
+        float2 ws = make_float2(0.f, 0.f), qs = ws;
+        {
+            const float* src = part + t * DC_COLS + (((c >> 2) + ((t & 7) >> 1)) & 3) * 4 + (c & 3);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float2 a = *reinterpret_cast<const float2*>(src + k * 2 * DC_C * DC_COLS);
+                const float2 b = *reinterpret_cast<const float2*>(src + (k * 2 * DC_C + DC_C) * DC_COLS);
+                ws.x += a.x; ws.y += a.y; qs.x += b.x; qs.y += b.y;
+            }
+        }
+        const float2 ps = *reinterpret_cast<const float2*>(sp + St::PS + 2 * t);
+        {
+            const float2 u0 = *reinterpret_cast<const float2*>(sm + St::U + t * DC_COLS + c);
+            const float ux = u0.x - ws.x, uy = u0.y - ws.y;
+            *reinterpret_cast<float2*>(us + t * DC_COLS + c) = make_float2(ux, uy);
+            *reinterpret_cast<float2*>(uds + t * DC_COLS + c) = make_float2(ps.y * ux, ps.y * uy);
+        }
+        __syncthreads();
+        {   // o: tokens up to t only, so that a later token's infinity stays with it
+            float ox = ps.x * qs.x, oy = ps.x * qs.y, o2x = 0.f, o2y = 0.f;
+            const float* Mr = sm + St::M + t * LDM;
+#pragma unroll
+            for (int s4 = 0; s4 < DC_C; s4 += 4) {
+                if (s4 > t) break;
+                const float4 m4 = *reinterpret_cast<const float4*>(Mr + s4);
+                const float m[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 u = *reinterpret_cast<const float2*>(us + (s4 + k) * DC_COLS + c);
+                    if (s4 + k <= t) {
+                        if (k & 1) { o2x = fmaf(m[k], u.x, o2x); o2y = fmaf(m[k], u.y, o2y); }
+                        else { ox = fmaf(m[k], u.x, ox); oy = fmaf(m[k], u.y, oy); }
+                    }
+                }
+            }
+            if (t < nb) *reinterpret_cast<float2*>(p.out + ((size_t)(t0 + b0 + t) * p.heads + h) * dv + c0 + c) = make_float2(ox + o2x, oy + o2y);
+        }
+        {   // the state at the chunk's end: a thread sums every fourth token for rows 4 dl .. and 32 + 4 dl .. of its warp's 64 and four columns,
+            // the four lanes that share them then hand each other three quarters of their sums
+            const float* Kp = sm + St::K + (lane >> 3) * LD + (warp >> 2) * 64 + 4 * dl;
+            const float* up = uds + (lane >> 3) * DC_COLS + (warp & 3) * 4;
+            float add[2][4][4] = {};
+#pragma unroll 2
+            for (int s = 0; s < DC_C; s += 4) {
+                const float4 u = *reinterpret_cast<const float4*>(up + s * DC_COLS);
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(Kp + s * LD + 32 * m);
+                    const float kv[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        add[m][i][0] = fmaf(kv[i], u.x, add[m][i][0]); add[m][i][1] = fmaf(kv[i], u.y, add[m][i][1]);
+                        add[m][i][2] = fmaf(kv[i], u.z, add[m][i][2]); add[m][i][3] = fmaf(kv[i], u.w, add[m][i][3]);
+                    }
+                }
+            }
+            const float decay = sp[St::PS + 2 * (nb - 1)];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = (b4 ? add[1][i][j] : add[0][i][j]) + __shfl_xor_sync(0xffffffffu, b4 ? add[0][i][j] : add[1][i][j], 16);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float a = (b3 ? v[2 + j] : v[j]) + __shfl_xor_sync(0xffffffffu, b3 ? v[j] : v[2 + j], 8);
+                    s_reg[i][j] = fmaf(decay, s_reg[i][j], a);
+                }
+                *reinterpret_cast<float2*>(Ss + s_at(row0 + i, col0)) = make_float2(s_reg[i][0], s_reg[i][1]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        S[(size_t)(row0 + i) * dv + col0] = s_reg[i][0];
+        S[(size_t)(row0 + i) * dv + col0 + 1] = s_reg[i][1];
+    }
+}
+
+// whether runs of tokens are taken in chunks for these sizes
+static bool delta_chunks_ok(int d, int dv) { return d == 128 && dv % DC_COLS == 0; }
+
+// floats of scratch memory that msgl_delta_rule wants for T tokens; chunks: with runs of tokens taken in chunks
+MSGL_API long long msgl_delta_rule_scratch(int T_, int heads, int kv_heads, int d, int dv, int chunks) {
+    const long long prep = (long long)T_ * kv_heads * d * 2 + (long long)T_ * heads * 4;
+    if (!chunks || !delta_chunks_ok(d, dv)) return prep;
+    return prep + (long long)T_ * heads * (d + dv + DC_C + 2) + (long long)T_ * kv_heads * d * 2 + 16;
+}
+
+template <typename T, int D>
+static int delta_chunk_launch(const DeltaChunkParams& p, int n_chunks, cudaStream_t stream) {
+    constexpr size_t smem1 = (size_t)(2 * DC_C * (D + 4) + 2 * DC_C * (DC_C + 1) + 2 * DC_C * DC_C) * 4;
+    constexpr size_t smem2 = (size_t)DcStage<D>::TOTAL * 4;
+    static MsglOncePerDevice once;
+    if (once.due()) {      // first call on this device, never inside a stream capture
+        if (cudaFuncSetAttribute(delta_chunk_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess ||
+            cudaFuncSetAttribute(delta_chunk_scan_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess ||
+            cudaFuncSetAttribute(delta_chunk_kernel<T, D>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+            cudaFuncSetAttribute(delta_chunk_scan_kernel<D>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+            return msgl_check_launch();
+        once.mark();
+    }
+    delta_chunk_kernel<T, D><<<dim3(n_chunks, p.heads), DC_THREADS, smem1, stream>>>(p);
+    delta_chunk_scan_kernel<D><<<dim3(p.heads, p.dv / DC_COLS, p.B), DC_THREADS, smem2, stream>>>(p);
+    return msgl_check_launch();
+}
+
+// n_chunks, n_min: chunks of DC_C tokens of the requests with n_min tokens or more (host's count), which are taken in chunks; 0: none.
+// n_short: whether requests with fewer tokens are in the step.
 MSGL_API int msgl_delta_rule(const void* qkv, const void* proj, long long proj_stride, int a_off, int b_off, const float* a_log,
                              const float* dt_bias, float* state, const int* q_start, const int* slots, float* out, float* scratch,
-                             int heads, int kv_heads, int d, int dv, int T_, int B, int dtype, cudaStream_t stream) {
+                             int heads, int kv_heads, int d, int dv, int T_, int B, int dtype, int n_chunks, int n_min, int n_short,
+                             cudaStream_t stream) {
     if (B <= 0 || T_ <= 0) return MSGL_OK;
+    if (n_chunks > 0 && (!delta_chunks_ok(d, dv) || n_min < 1 || B > 65535 || heads > 65535)) return MSGL_ERR_SIZE;
     if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || d <= 0 || dv <= 0 || d > DR_PARTS * 64 || scratch == nullptr) return MSGL_ERR_SIZE;
     if (((uintptr_t)scratch & 15) != 0) return MSGL_ERR_ALIGN;
     if (dtype != MSGL_F32 && dtype != MSGL_BF16) return MSGL_ERR_DTYPE;
@@ -1183,11 +1571,25 @@ MSGL_API int msgl_delta_rule(const void* qkv, const void* proj, long long proj_s
     p.sc = reinterpret_cast<float4*>(scratch);                                  // [T][heads] first: 16-byte rows stay aligned
     p.kq = reinterpret_cast<float2*>(scratch + (size_t)T_ * heads * 4);
     p.state = state; p.q_start = q_start; p.slots = slots; p.out = out; p.heads = heads; p.kv_heads = kv_heads; p.d = d; p.dv = dv; p.T = T_;
+    p.n_min = 1; p.n_max = n_chunks > 0 ? n_min - 1 : 0x7fffffff;
     const dim3 g0(T_, (kv_heads + 3) / 4);
     if (dtype == MSGL_F32) delta_prep_kernel<float><<<g0, 128, 0, stream>>>(p);
     else delta_prep_kernel<__nv_bfloat16><<<g0, 128, 0, stream>>>(p);
     int code = msgl_check_launch();
     if (code != MSGL_OK) return code;
+    if (n_chunks > 0) {
+        DeltaChunkParams c;
+        c.qkv = qkv; c.kq = p.kq; c.sc = p.sc; c.state = state; c.q_start = q_start; c.slots = slots; c.out = out;
+        c.heads = heads; c.kv_heads = kv_heads; c.dv = dv; c.T = T_; c.B = B; c.n_min = n_min;
+        const size_t th = (size_t)T_ * heads, tk = (size_t)T_ * kv_heads;
+        // 16-byte rows of d, dv and DC_C floats; the pairs last
+        c.W = scratch + (((size_t)T_ * heads * 4 + tk * d * 2 + 3) & ~(size_t)3);
+        c.U = c.W + th * d; c.M = c.U + th * dv; c.K = c.M + th * DC_C; c.Q = c.K + tk * d;
+        c.ps = reinterpret_cast<float2*>(c.Q + tk * d);
+        if (dtype == MSGL_F32) code = delta_chunk_launch<float, 128>(c, n_chunks, stream);
+        else code = delta_chunk_launch<__nv_bfloat16, 128>(c, n_chunks, stream);
+        if (code != MSGL_OK || !n_short) return code;
+    }
     const int many_cols = DR_MANY_WARPS * DR_WCOLS;
     const long long blocks_many = (long long)heads * B * ((dv + many_cols - 1) / many_cols);
     const int warps = blocks_many >= 2LL * msgl_sm_count() ? DR_MANY_WARPS : DR_FEW_WARPS;

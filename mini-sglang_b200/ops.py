@@ -1677,6 +1677,11 @@ SINK_ATTENTION_ROWS = 8             # (token, head) rows of a block of the atten
 SINK_ATTENTION_MAX_HEAD_DIM = 512
 SINK_ATTENTION_SPLIT_KEYS = 256     # keys of a piece when a one-token step cuts a request's keys over several blocks
 DELTA_RULE_MAX_KEY_DIM = 512
+DELTA_CHUNK, DELTA_CHUNK_KEY_DIMS = 32, (128,)      # tokens of a chunk; key sizes whose runs of tokens are taken in chunks
+# Tokens of a request in one step from which they are taken in chunks; token by token / in chunks, 16 heads of 128 x 128 (us, all kernels): one
+# request of 64 tokens 37 / 44, 96: 49 / 42, 128: 62 / 42, 1,111 and 300: 477 / 182, 8,000: 3,223 / 944; 16 requests of 100: 218 / 229, of 128:
+# 273 / 234, of 300: 632 / 503; 64 of 128: 1,063 / 842
+DELTA_CHUNK_MIN_TOKENS = 128
 
 
 def _delta_lib():
@@ -1691,8 +1696,8 @@ def _delta_lib():
             [c_int] * 12 + [c_float, c_float, c_int, c_void_p, c_ll, c_int, c_void_p]
         lib.msgl_sink_attention_mma.argtypes = [c_void_p] * 6 + [c_int, c_int, c_int, c_void_p, c_void_p, c_ll, c_void_p, c_void_p] + \
             [c_int] * 10 + [c_float, c_float, c_void_p, c_ll, c_int, c_void_p]
-        lib.msgl_delta_rule.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_int] + [c_void_p] * 7 + [c_int] * 7 + [c_void_p]
-        lib.msgl_delta_rule_scratch.argtypes = [c_int] * 4
+        lib.msgl_delta_rule.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_int] + [c_void_p] * 7 + [c_int] * 10 + [c_void_p]
+        lib.msgl_delta_rule_scratch.argtypes = [c_int] * 6
         lib.msgl_delta_rule_scratch.restype = c_ll
         lib.msgl_side_gate_mul.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p]
         _delta = lib
@@ -1871,15 +1876,21 @@ def delta_rule(qkv: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, heads: in
     assert a_log.dtype == torch.float32 and dt_bias.dtype == torch.float32 and a_log.numel() == heads and dt_bias.numel() == heads
     out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=qkv.device)
     B = q_start.numel() - 1
-    # what does not depend on the state (unit q and k, beta, g) is made for all tokens at once by a kernel of its own
-    numel = int(_delta_lib().msgl_delta_rule_scratch(T, heads, kv_heads, key_dim))
+    # runs of tokens go in chunks, single tokens and short runs token by token: a matter of the request's own tokens in this step
+    # and of the sizes, so a request's results do not depend on the requests beside it
+    long_runs = [n for n in q_lens or () if n >= DELTA_CHUNK_MIN_TOKENS] if key_dim in DELTA_CHUNK_KEY_DIMS and value_dim % 16 == 0 else []
+    n_chunks = sum(-(-n // DELTA_CHUNK) for n in long_runs)
+    short = not long_runs or any(0 < n < DELTA_CHUNK_MIN_TOKENS for n in q_lens)
+    # what does not depend on the state (unit q and k, beta, g, and for chunks all that lies within one) is made for all tokens at once
+    numel = int(_delta_lib().msgl_delta_rule_scratch(T, heads, kv_heads, key_dim, value_dim, int(n_chunks > 0)))
     scratch = workspace.get("delta_rule_prep", numel, torch.float32) if workspace is not None else \
         torch.empty(numel, dtype=torch.float32, device=qkv.device)
     code = _delta_lib().msgl_delta_rule(_ptr(qkv), _ptr(a), stride, 0, _col_off(b, a), _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(q_start),
-                                        _ptr(slots), _ptr(out), _ptr(scratch), heads, kv_heads, key_dim, value_dim, T, B, _dt(qkv), _stream())
+                                        _ptr(slots), _ptr(out), _ptr(scratch), heads, kv_heads, key_dim, value_dim, T, B, _dt(qkv), n_chunks,
+                                        DELTA_CHUNK_MIN_TOKENS, int(short), _stream())
     _check(code, f"delta_rule (key size {key_dim})")
     global LAUNCHES
-    LAUNCHES += 1
+    LAUNCHES += 1 + (1 + int(short) if n_chunks else 0)
     return out
 
 
