@@ -746,7 +746,7 @@ def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tens
             code = _small_m(gate_up, x, bias, out, M, N, K, N // 2, mode, 0)
             _check(code, "gemm_small_m (gated)")
             return out
-        if x.dim() == 2 and x.shape[0] <= (ROWS_GLU_MAX_LARGE if gate_up.numel() >= ROWS_LARGE_WEIGHT else ROWS_GLU_MAX):
+        if x.dim() == 2 and not MID_GEMM and x.shape[0] <= (ROWS_GLU_MAX_LARGE if gate_up.numel() >= ROWS_LARGE_WEIGHT else ROWS_GLU_MAX):
             y = _gemm_rows(x, gate_up, bias, mode, torch.bfloat16)
             if y is not None:
                 return y
