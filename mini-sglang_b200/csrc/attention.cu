@@ -26,8 +26,8 @@
 //   attn_decode_even_kernel<D,...> the same arithmetic for a decode step whose keys the host has dealt out evenly over
 //                               a fixed number of blocks per kv head (requests of very different lengths)
 //   attn_decode_kernel<D,...>   the same for head sizes 16 mod 32: heads on the M dimension
-//   attn_simt_kernel<T>         any head size up to 512, float32 arithmetic throughout; this is
-//                               the true 32-bit path and the fallback for odd head sizes
+//   attn_f32_kernel<D>          float32 data, float32 arithmetic: the true 32-bit path at head sizes that are a multiple of 16
+//   attn_simt_kernel<T>         any head size up to 512, float32 arithmetic throughout: the other head sizes of both types
 //   attn_combine_kernel<T>      merge of the kv splits; attn_combine_diff_kernel<T> for heads that are the difference of two maps
 // Scores, softmax and the accumulation are float32 in all of them.  In a step of single tokens the blocks take the
 // requests in the order the step gives (`order`: longest first), the kv heads of one request in adjacent blocks.
@@ -1410,6 +1410,194 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_simt_kernel(const AttnParam
     }
 }
 
+// The same for float32 data at the library's own head size (a multiple of 16): 16 rows a block, key tiles of 32 in two stages (cp.async, 16 bytes a
+// lane, a tile's pages looked up once a warp), both products from registers.  A warp owns four rows: a lane takes four keys of them over a
+// quarter of the head's elements, the four lanes that share the keys then hand each other three quarters of their sums, so that a
+// lane is left with four scores of one row; for the second product it owns four elements of the head.  Weights pass through shared
+// memory within the warp, so the block meets once a key tile.  The kernel above takes 26 us a key tile (4-byte loads with a page
+// lookup each, one score a thread at a time), this one 4: 210 and 37 tokens, 16 heads on 8 of 128, 186 -> 28 us.
+template <int D>
+__global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams p) {
+    constexpr int R = SIMT_R, KT = SIMT_KT, LD = D + 4, LDP = KT + 8, NV = (D + 127) / 128;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float* Qs = reinterpret_cast<float*>(smem_raw);          // [R][LD]
+    float* Ps = Qs + R * LD;                                 // [R][LDP]
+    float* KV = Ps + R * LDP;                                // two stages of K [KT][LD], V [KT][LD]
+    __shared__ int sh_tile[4];
+    const int G = p.n_q / p.n_kv;
+    const int Gc = G <= R ? G : R;
+    const int n_chunks = G <= R ? 1 : (G + R - 1) / R;
+    const int QT = G <= R ? R / G : 1;
+    int tile_idx, by;
+    block_place(p, tile_idx, by);
+    const int kvh = by / n_chunks;
+    const int chunk = by - kvh * n_chunks;
+    TileInfo ti;
+    if (!find_tile(p, QT, ti, sh_tile, tile_idx, (int)gridDim.x)) return;
+    const int ns = p.nsplit ? min(max(p.nsplit[ti.req], 1), p.max_split) : 1;
+    const int split = blockIdx.z;
+    if (split >= ns) return;
+    int p_min, p_max, kt_begin, kt_end;
+    key_tile_range(p, ti, KT, split, ns, p_min, p_max, kt_begin, kt_end);
+    const int k_first = first_key(p, p_min);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float* qg = reinterpret_cast<const float*>(p.q);
+    const float* kc = reinterpret_cast<const float*>(p.k_cache);
+    const float* vc = reinterpret_cast<const float*>(p.v_cache);
+    const int* bt = p.block_table + (size_t)ti.req * p.bt_stride;
+    const float sc = p.scale * 1.4426950408889634f;
+    auto row_valid = [&](int r) { const int tl = r / Gc; return tl < ti.n_tok && tl < QT && chunk * R + (r - tl * Gc) < G; };
+    auto row_token = [&](int r) { return (size_t)(ti.q_base + ti.t0 + r / Gc); };
+    auto row_head = [&](int r) { return kvh * G + chunk * R + r % Gc; };
+
+    auto fetch = [&](int kt, int st) {                       // rows past the last key, before the window or the chunk arrive as zeros
+        float* Ks = KV + st * 2 * KT * LD;
+        const int mine = kt * KT + lane;
+        const int pg_mine = (mine <= p_max && mine >= k_first) ? bt[page_index(p, mine)] : -1;
+#pragma unroll
+        for (int i = 0; i < KT / 4; ++i) {
+            const int kl = warp * (KT / 4) + i, pg = __shfl_sync(0xffffffffu, pg_mine, kl);
+            const size_t off = (((size_t)max(pg, 0) * p.n_kv + kvh) * p.page_size + (pg >= 0 ? page_slot(p, kt * KT + kl) : 0)) * D;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const int e = 4 * (lane + 32 * v);
+                if (e < D) {
+                    cp_async16(Ks + kl * LD + e, kc + off + e, pg >= 0);
+                    cp_async16(Ks + (KT + kl) * LD + e, vc + off + e, pg >= 0);
+                }
+            }
+        }
+    };
+    if (kt_begin < kt_end) fetch(kt_begin, 0);
+    cp_async_commit();
+    for (int idx = tid; idx < R * (D / 4); idx += SIMT_THREADS) {
+        const int r = idx / (D / 4), e = 4 * (idx - r * (D / 4));
+        *reinterpret_cast<float4*>(Qs + r * LD + e) =
+            row_valid(r) ? *reinterpret_cast<const float4*>(qg + (row_token(r) * p.n_q + row_head(r)) * D + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const int kg = lane & 7, b3 = (lane >> 3) & 1, b4 = lane >> 4;
+    const int my_row = 4 * warp + 2 * b3 + b4, my_pos = p_min + my_row / Gc, my_first = first_key(p, my_pos);
+    const bool my_live = my_row / Gc < ti.n_tok;
+    float m_run = -INFINITY, l_run = 0.f;                    // of my_row; l over this lane's keys
+    float o[NV][4][4];
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) o[v][r][0] = o[v][r][1] = o[v][r][2] = o[v][r][3] = 0.f;
+    for (int kt = kt_begin, st = 0; kt < kt_end; ++kt, st ^= 1) {
+        cp_async_wait<0>();
+        __syncthreads();                                     // the tile (and q) lie in shared memory; the other stage is free
+        if (kt + 1 < kt_end) fetch(kt + 1, st ^ 1);
+        cp_async_commit();
+        const float* Ks = KV + st * 2 * KT * LD;
+        const float* Vs = Ks + KT * LD;
+        float s[4];
+        {
+            float acc[4][4] = {};
+            const float* qp = Qs + 4 * warp * LD + 4 * (lane >> 3);
+            const float* kp = Ks + kg * LD + 4 * (lane >> 3);
+#pragma unroll 2
+            for (int e = 0; e < D; e += 16) {
+                float4 q4[4], k4[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    q4[i] = *reinterpret_cast<const float4*>(qp + i * LD + e);
+                    k4[i] = *reinterpret_cast<const float4*>(kp + 8 * i * LD + e);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        acc[i][j] = fmaf(q4[i].x, k4[j].x, acc[i][j]); acc[i][j] = fmaf(q4[i].y, k4[j].y, acc[i][j]);
+                        acc[i][j] = fmaf(q4[i].z, k4[j].z, acc[i][j]); acc[i][j] = fmaf(q4[i].w, k4[j].w, acc[i][j]);
+                    }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float v[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) v[i] = (b3 ? acc[2 + i][j] : acc[i][j]) + __shfl_xor_sync(0xffffffffu, b3 ? acc[i][j] : acc[2 + i][j], 8);
+                s[j] = (b4 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b4 ? v[0] : v[1], 16);
+            }
+        }
+        float mx = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int key = kt * KT + kg + 8 * j;
+            s[j] = my_live && key <= my_pos && key >= my_first ? s[j] * sc : -INFINITY;
+            mx = fmaxf(mx, s[j]);
+        }
+#pragma unroll
+        for (int x = 1; x < 8; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+        const float m_new = fmaxf(m_run, mx), mu = (m_new == -INFINITY) ? 0.f : m_new, alpha = exp2f(m_run - mu);
+        m_run = m_new;
+        l_run *= alpha;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float w = exp2f(s[j] - mu);
+            l_run += w;
+            Ps[my_row * LDP + kg + 8 * j] = w;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float a = __shfl_sync(0xffffffffu, alpha, (r >> 1) * 8 + (r & 1) * 16);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) { o[v][r][0] *= a; o[v][r][1] *= a; o[v][r][2] *= a; o[v][r][3] *= a; }
+        }
+#pragma unroll 2
+        for (int kl = 0; kl < KT; kl += 4) {
+            float w[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(w[r]) = *reinterpret_cast<const float4*>(Ps + (4 * warp + r) * LDP + kl);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const int e = 4 * (lane + 32 * v);
+                if (e < D) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float4 x = *reinterpret_cast<const float4*>(Vs + (kl + k) * LD + e);
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            o[v][r][0] = fmaf(w[r][k], x.x, o[v][r][0]); o[v][r][1] = fmaf(w[r][k], x.y, o[v][r][1]);
+                            o[v][r][2] = fmaf(w[r][k], x.z, o[v][r][2]); o[v][r][3] = fmaf(w[r][k], x.w, o[v][r][3]);
+                        }
+                    }
+                }
+            }
+        }
+        __syncwarp();                                        // the weights are read before the next tile's replace them
+    }
+#pragma unroll
+    for (int x = 1; x < 8; x <<= 1) l_run += __shfl_xor_sync(0xffffffffu, l_run, x);
+    float* og = reinterpret_cast<float*>(p.out);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int src = (r >> 1) * 8 + (r & 1) * 16, row = 4 * warp + r;
+        const float m = __shfl_sync(0xffffffffu, m_run, src);
+        float l = __shfl_sync(0xffffffffu, l_run, src);
+        if (!row_valid(row)) continue;
+        const size_t tok = row_token(row);
+        const int head = row_head(row);
+        const size_t at = ns == 1 ? tok * p.n_q + head : ((size_t)split * p.T + tok) * p.n_q + head;
+        if (ns == 1) l += null_weight(p.null_log2, head, m);
+        else if (lane == 0) { p.part_ml[at * 2] = m; p.part_ml[at * 2 + 1] = l; }
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int e = 4 * (lane + 32 * v);
+            if (e >= D) continue;
+            float y[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                y[k] = ns == 1 ? (l > 0.f ? o[v][r][k] / l : 0.f) * gate_factor<float>(p.gate, p.gate_stride, tok, head * D + e + k) : o[v][r][k];
+            *reinterpret_cast<float4*>((ns == 1 ? og : p.part_o) + at * D + e) = make_float4(y[0], y[1], y[2], y[3]);
+        }
+    }
+}
+template <int D> static size_t f32_smem_bytes() {
+    return sizeof(float) * ((size_t)SIMT_R * (D + 4) + SIMT_R * (SIMT_KT + 8) + (size_t)4 * SIMT_KT * (D + 4));
+}
+
 // ---------------------------------------------------------------------------------------
 // merge of the kv splits, in split order: out = sum_s 2^(m_s - M) o_s / (sum_s 2^(m_s - M) l_s + the term without a key),
 // times sigmoid(gate) where gates are given
@@ -1687,7 +1875,17 @@ static int attention_launch(const void* q, void* out, const void* k_cache, const
         if (smem > 227 * 1024) return MSGL_ERR_SIZE;
         static size_t simt_attr[MSGL_MAX_DEVICES][2] = {};   // largest size already granted per device and element type
         size_t* granted = simt_attr[msgl_device()];
-        if (dtype == MSGL_F32) {
+        constexpr int HD = MSGL_HEAD_DIM;
+        // rows of 16-byte pieces: the head size the library is built for, caches and q as torch allocates them
+        if (dtype == MSGL_F32 && d == HD && HD % 16 == 0 && f32_smem_bytes<HD>() <= 227 * 1024 &&
+            (((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)part_o) & 15) == 0) {
+            static MsglOncePerDevice f32_attr;
+            if (f32_attr.due()) {
+                cudaFuncSetAttribute(attn_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f32_smem_bytes<HD>());
+                f32_attr.mark();
+            }
+            attn_f32_kernel<HD><<<grid, SIMT_THREADS, f32_smem_bytes<HD>(), stream>>>(p);
+        } else if (dtype == MSGL_F32) {
             if (smem > 48 * 1024 && smem > granted[0]) {
                 cudaFuncSetAttribute(attn_simt_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 granted[0] = smem;
