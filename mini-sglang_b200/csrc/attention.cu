@@ -90,6 +90,9 @@ struct AttnParams {
     // runs always leave partial results then, and the merge takes the difference.
     int diff = 0;
     float diff_lam = 0.f, diff_eps = 0.f, diff_scale = 0.f;
+    // prefill tiles whose keys are cut: key tiles a piece should have, and how many pieces every token's tile was cut into (written)
+    int piece_tiles = 0;
+    int* tok_pieces = nullptr;
 };
 
 // weight of the term without a key against the reference m (log2 units) of a row's exponentials
@@ -1605,12 +1608,14 @@ template <int D> static size_t f32_smem_bytes() {
 // A warp takes one head of a run of `run` tokens: it looks the tokens' pieces up together and merges those that have more than one, four
 // elements of the head a lane.  Bound by latency: the piece weights, then the pieces themselves, all of a row's loads under way at once.
 // run = 1 where there are few rows (decode steps: the attention layer of 8 requests of 4,096 keys 58.9 us with a block a row and
-// scalar loads, 57.9 now); 32 in steps with prompt portions, most of whose tokens have nothing to merge and cost one look a run
-// (1,901 tokens x 32 heads of which 3 tokens are cut: 64 us with a block a row, and the attention layer 293.7 -> 236.9 us).
+// scalar loads, 57.9 now); up to 32 in steps with prompt portions, most of whose tokens have nothing to merge and cost one look a
+// run (1,901 tokens x 32 heads of which 3 tokens are cut: 64 us with a block a row, and the attention layer 293.7 -> 236.9 us).
+// A run's tokens are merged one after the other, so runs are no longer than the number of blocks asks for (65 cut
+// tokens among the 1,901: 126 us in runs of 32).
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(128) attn_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                     const int* __restrict__ token_req, const int* __restrict__ nsplit,
-                                    T* __restrict__ out, int T_, int n_q, int d, int max_split, const float* __restrict__ null_log2,
+                                    T* __restrict__ out, int T_, int T_plane, int n_q, int d, int max_split, const float* __restrict__ null_log2,
                                     const void* __restrict__ gate, long long gate_stride, int run) {
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
@@ -1623,7 +1628,7 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(const float* __restri
     if (lane < run && tok0 + lane < T_) my_ns = min(max(nsplit[token_req ? token_req[tok0 + lane] : tok0 + lane], 1), max_split);
     for (unsigned todo = __ballot_sync(0xffffffffu, my_ns > 1); todo != 0u; todo &= todo - 1u) {
         const int i = __ffs(todo) - 1, tok = tok0 + i, ns = __shfl_sync(0xffffffffu, my_ns, i);
-        const size_t row = (size_t)tok * n_q + h, plane = (size_t)T_ * n_q;
+        const size_t row = (size_t)tok * n_q + h, plane = (size_t)T_plane * n_q;
         float M = -INFINITY;
         for (int s = lane; s < ns; s += 32) M = fmaxf(M, part_ml[(s * plane + row) * 2]);
         M = warp_max(M);
@@ -1980,12 +1985,16 @@ static int attention_launch(const void* q, void* out, const void* k_cache, const
 // version 1: 128 query rows per block, two blocks per SM, any page size; version 2: 256 rows per block in
 // ping-pong, TMA page sizes only (MSGL_ERR_SIZE otherwise: the caller then uses version 1).  grid_x counts
 // tiles of 128 / group (version 1) or 256 / group (version 2) tokens.
+// piece_tiles > 0: query tiles with more than 1.5 times as many key tiles are cut into up to `pieces` pieces (version 2 without window, chunks, kept
+// tokens, bias or pairs of maps); their partial results go to part_o [pieces][T][n_q][128], part_ml [pieces][T][n_q][2], the number of pieces to
+// tok_pieces [T] (tokens that the launch does not take are left alone), and msgl_attention_combine merges them.
 MSGL_API int msgl_attention_tc(const void* q, void* out, const void* k_cache, const void* v_cache, const int* q_start,
                                const int* kv_len, const int* block_table, int B, int T_, int n_q, int n_kv, int d,
                                int page_size, int bt_stride, int window, float scale, int qlen_min, int qlen_max,
                                int grid_x, int cache_pages, int version, int* status, int keep_first, const float* bias,
                                int bias_len, const float* null_log2, const void* gate, long long gate_stride, int chunk_keys,
-                               int diff, float diff_lam, float diff_eps, float diff_scale, cudaStream_t stream) {
+                               int diff, float diff_lam, float diff_eps, float diff_scale, int piece_tiles, int pieces, float* part_o,
+                               float* part_ml, int* tok_pieces, cudaStream_t stream) {
 #if MSGL_HEAD_DIM == 128
     if (gate != nullptr && ((gate_stride & 7) || ((uintptr_t)gate & 15))) return MSGL_ERR_ALIGN;
     // kept first tokens under the window and a bias by distance ([n_q][bias_len] float32, log2 units): version 2 only
@@ -2010,6 +2019,13 @@ MSGL_API int msgl_attention_tc(const void* q, void* out, const void* k_cache, co
     p.null_log2 = null_log2; p.gate = gate; p.gate_stride = gate_stride;
     p.diff = diff; p.diff_lam = diff_lam; p.diff_eps = diff_eps; p.diff_scale = diff_scale;
     p.keep_first = window > 0 ? keep_first : 0; p.bias = bias; p.bias_len = bias_len;
+    if (piece_tiles > 0) {
+        if (version != 2 || ext || diff || window > 0 || chunk_keys > 0 || pieces < 2 || pieces > 64 || part_o == nullptr || part_ml == nullptr || tok_pieces == nullptr)
+            return MSGL_ERR_SIZE;
+        if ((long long)grid_x * pieces > 65535) return MSGL_ERR_SIZE;
+        if ((uintptr_t)part_o & 15) return MSGL_ERR_ALIGN;
+        p.piece_tiles = piece_tiles; p.max_split = pieces; p.part_o = part_o; p.part_ml = part_ml; p.tok_pieces = tok_pieces;
+    }
     const int G = n_q / n_kv;
     const int n_chunks = (diff || G <= TC_ROWS) ? 1 : (G + TC_ROWS - 1) / TC_ROWS;
     const size_t smem = (size_t)TC_SMEM_BYTES + 1024;
@@ -2018,7 +2034,8 @@ MSGL_API int msgl_attention_tc(const void* q, void* out, const void* k_cache, co
         if (cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
             cudaFuncSetAttribute(attn_tc2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC2_SMEM_ALLOC) != cudaSuccess ||
             cudaFuncSetAttribute(attn_tc2_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC2_SMEM_ALLOC) != cudaSuccess ||
-            cudaFuncSetAttribute(attn_tc2_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC2_SMEM_ALLOC) != cudaSuccess)
+            cudaFuncSetAttribute(attn_tc2_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC2_SMEM_ALLOC) != cudaSuccess ||
+            cudaFuncSetAttribute(attn_tc2_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC2_SMEM_ALLOC) != cudaSuccess)
             return msgl_check_launch();
         attr_set.mark();
     }
@@ -2035,6 +2052,8 @@ MSGL_API int msgl_attention_tc(const void* q, void* out, const void* k_cache, co
     if (version == 2) {
         if (tma_box == 0) return MSGL_ERR_SIZE;
         if (diff) attn_tc2_kernel<false, true><<<dim3(n_kv, grid_x, 1), TC2_THREADS, TC2_SMEM_ALLOC, stream>>>(p, status, kmap, vmap, tma_box);
+        else if (p.piece_tiles > 0)
+            attn_tc2_kernel<false, false, true><<<dim3(n_kv * n_chunks, grid_x * pieces), TC2_THREADS, TC2_SMEM_ALLOC, stream>>>(p, status, kmap, vmap, tma_box);
         else if (ext) attn_tc2_kernel<true><<<dim3(n_kv * n_chunks, grid_x, 1), TC2_THREADS, TC2_SMEM_ALLOC, stream>>>(p, status, kmap, vmap, tma_box);
         else attn_tc2_kernel<false><<<dim3(n_kv * n_chunks, grid_x, 1), TC2_THREADS, TC2_SMEM_ALLOC, stream>>>(p, status, kmap, vmap, tma_box);
         return msgl_check_launch();
@@ -2046,23 +2065,41 @@ MSGL_API int msgl_attention_tc(const void* q, void* out, const void* k_cache, co
 #endif
 }
 
-MSGL_API int msgl_attention_combine(const float* part_o, const float* part_ml, const int* token_req,
-                                    const int* nsplit, void* out, int T_, int n_q, int d, int max_split, int dtype,
-                                    const float* null_log2, const void* gate, long long gate_stride, cudaStream_t stream) {
+// T_ neighbouring tokens of pieces that were left for T_plane (all pointers at the first of them)
+static int combine_launch(const float* part_o, const float* part_ml, const int* token_req, const int* nsplit, void* out, int T_, int T_plane, int n_q,
+                          int d, int max_split, int dtype, const float* null_log2, const void* gate, long long gate_stride, cudaStream_t stream) {
     if (T_ <= 0 || max_split <= 1) return MSGL_OK;
-    const int run = (long long)T_ * n_q <= 32LL * msgl_sm_count() ? 1 : 32;
+    // tokens a warp looks at: one where the rows give some hundred blocks, more where the launch would have thousands that find nothing
+    const long long rows = (long long)T_ * n_q, few = 32LL * msgl_sm_count();
+    const int run = rows <= few ? 1 : (int)(rows / few + 1 < 32 ? rows / few + 1 : 32);
     const long long items = (long long)((T_ + run - 1) / run) * n_q;
     const dim3 grid((unsigned)((items + 3) / 4));
     const bool vec = d % 4 == 0 && (((uintptr_t)part_o | (uintptr_t)out) & 15) == 0;      // rows of d lie back to back in both
 #define COMBINE(T, VEC) \
-    msgl_launch_pdl(attn_combine_kernel<T, VEC>, grid, dim3(128), 0, stream, part_o, part_ml, token_req, nsplit, (T*)out, T_, n_q, d, max_split, \
-                    null_log2, gate, gate_stride, run)
+    msgl_launch_pdl(attn_combine_kernel<T, VEC>, grid, dim3(128), 0, stream, part_o, part_ml, token_req, nsplit, (T*)out, T_, T_plane, n_q, d, \
+                    max_split, null_log2, gate, gate_stride, run)
     if (dtype == MSGL_F32) { if (vec) COMBINE(float, true); else COMBINE(float, false); }
     else if (dtype == MSGL_BF16) { if (vec) COMBINE(__nv_bfloat16, true); else COMBINE(__nv_bfloat16, false); }
 #undef COMBINE
     else
         return MSGL_ERR_DTYPE;
     return msgl_check_launch();
+}
+
+MSGL_API int msgl_attention_combine(const float* part_o, const float* part_ml, const int* token_req,
+                                    const int* nsplit, void* out, int T_, int n_q, int d, int max_split, int dtype,
+                                    const float* null_log2, const void* gate, long long gate_stride, cudaStream_t stream) {
+    return combine_launch(part_o, part_ml, token_req, nsplit, out, T_, T_, n_q, d, max_split, dtype, null_log2, gate, gate_stride, stream);
+}
+
+// tokens tok0 .. tok0 + n - 1 of T_, pieces [T_]: how many pieces every token has (read for these tokens only)
+MSGL_API int msgl_attention_combine_range(const float* part_o, const float* part_ml, const int* pieces, void* out, int T_, int tok0, int n, int n_q,
+                                          int d, int max_split, int dtype, const float* null_log2, const void* gate, long long gate_stride,
+                                          cudaStream_t stream) {
+    if (tok0 < 0 || n < 0 || tok0 + n > T_ || pieces == nullptr) return MSGL_ERR_SIZE;
+    const size_t row = (size_t)tok0 * n_q, item = dtype == MSGL_F32 ? 4 : 2;
+    return combine_launch(part_o + row * d, part_ml + row * 2, nullptr, pieces + tok0, (char*)out + row * d * item, n, T_, n_q, d, max_split, dtype, null_log2,
+                          gate ? (const char*)gate + (size_t)tok0 * gate_stride * item : nullptr, gate_stride, stream);
 }
 
 // The merge for pairs of maps: out [T, n_q / 2, d]; q_start [B + 1], qlen_max and nsplit tell which requests left partial

@@ -58,7 +58,11 @@ constexpr unsigned TC2_SMEM_ALLOC = TC2_SMEM_BYTES + 256u + 1024u;
 // EXT: the launch has kept first tokens under its window or a bias by distance (AttnParams::keep_first, bias): the key tiles
 // that hold kept tokens before the window's first tile are walked ahead of the window's, and every score gets its table entry.
 // Without EXT none of that is compiled in.
-template <bool EXT, bool DIFF = false>
+// SPLIT: a step whose longest tiles would still run when all others are done (a short portion behind many cached tokens beside a new
+// prompt, or too few tiles to fill the SMs) cuts those tiles' keys into pieces, blocks of their own; their rows go out as float32
+// partial results.  Attention layer at Qwen3-8B's widths, portions of 1500, 333, 65, 1, 1, 1 tokens behind 0, 700, 4000, 2047, 511, 37:
+// this kernel 89 -> 66 us, the layer 238 -> 228 with the merge.  (Pieces along z of the grid, which start after all other tiles: 92 us.)
+template <bool EXT, bool DIFF = false, bool SPLIT = false>
 __global__ void __launch_bounds__(TC2_THREADS, 1) attn_tc2_kernel(const AttnParams p, int* status,
                                                                   const __grid_constant__ CUtensorMap kmap,
                                                                   const __grid_constant__ CUtensorMap vmap, int tma_box) {
@@ -96,21 +100,35 @@ __global__ void __launch_bounds__(TC2_THREADS, 1) attn_tc2_kernel(const AttnPara
     const int chunk = blockIdx.x - kvh * n_chunks;
 
     TileInfo ti;
-    if (!find_tile(p, DIFF ? QH : 2 * QH, ti, sh_tile, (int)blockIdx.y, (int)gridDim.y)) return;
+    // SPLIT: the pieces of a tile are neighbours along y, so that the heaviest tiles' pieces all start first
+    const int y_tile = SPLIT ? (int)blockIdx.y / p.max_split : (int)blockIdx.y, piece = SPLIT ? (int)blockIdx.y - y_tile * p.max_split : 0;
+    if (!find_tile(p, DIFF ? QH : 2 * QH, ti, sh_tile, y_tile, SPLIT ? (int)gridDim.y / p.max_split : (int)gridDim.y)) return;
     // positions of the block's tokens and its key tiles (anchored at absolute positions)
     const int p_min = ti.kv_len - ti.q_len + ti.t0;
     const int p_max = p_min + ti.n_tok - 1;
     const int ntok_a = DIFF ? ti.n_tok : min(ti.n_tok, QH), ntok_b = DIFF ? ti.n_tok : ti.n_tok - ntok_a;
     const int pmax_a = p_min + ntok_a - 1;
     const int k_lo = first_key(p, p_min);                        // the first key any row of the block sees
-    const int kt_begin = k_lo / TC_KT;
+    int kt_begin = k_lo / TC_KT;
     // kept first tokens before the window's first tile: keys [0, sink_hi) in n_sink tiles that come first for both query tiles
     const int sink_hi = (EXT && p.window > 0) ? min(p.keep_first, kt_begin * TC_KT) : 0;
     const int n_sink = (sink_hi + TC_KT - 1) / TC_KT;
     auto tile_of = [&](int j) -> int { return (EXT && j < n_sink) ? j : kt_begin + (j - n_sink); };
-    const int n_a = pmax_a / TC_KT + 1 - kt_begin + n_sink;               // key tiles of tile A
-    const int n_b = ntok_b > 0 ? p_max / TC_KT + 1 - kt_begin + n_sink : 0;  // key tiles of tile B (0: no token there)
-    const int n_tiles = max(n_a, n_b);
+    int n_a = pmax_a / TC_KT + 1 - kt_begin + n_sink;               // key tiles of tile A
+    int n_b = ntok_b > 0 ? p_max / TC_KT + 1 - kt_begin + n_sink : 0;  // key tiles of tile B (0: no token there)
+    int n_tiles = max(n_a, n_b);
+    int pieces = 1;
+    if (SPLIT) {                                                  // this block's share of the key tiles (tile A may have none in the last piece)
+        if (2 * n_tiles > 3 * p.piece_tiles) pieces = min((n_tiles + p.piece_tiles - 1) / p.piece_tiles, p.max_split);
+        if (piece >= pieces) return;
+        const int lo = piece * n_tiles / pieces, hi = (piece + 1) * n_tiles / pieces;
+        if (piece == 0 && blockIdx.x == 0)
+            for (int i = threadIdx.x; i < ti.n_tok; i += TC2_THREADS) p.tok_pieces[ti.q_base + ti.t0 + i] = pieces;
+        kt_begin += lo;
+        n_a = max(min(n_a, hi) - lo, 0);
+        n_b = max(min(n_b, hi) - lo, 0);
+        n_tiles = hi - lo;
+    }
 
     if (tid == 0) {
         for (int x = 0; x < 2; ++x) {
@@ -300,7 +318,7 @@ __global__ void __launch_bounds__(TC2_THREADS, 1) attn_tc2_kernel(const AttnPara
             if (!tc_mbar_wait(bar_s(x), it & 1)) { fail = 1; break; }
             tc_fence_after();
             TC2_MARK(0)
-            if (!DIFF && p.gate != nullptr && it + 1 == n_mine) {
+            if (!DIFF && p.gate != nullptr && it + 1 == n_mine && (!SPLIT || pieces == 1)) {
                 // Q_X has been read for the last time: the rows' gates take its place while the last tile is worked on
                 const unsigned long long mine = reinterpret_cast<unsigned long long>(
                     reinterpret_cast<const __nv_bfloat16*>(p.gate) + my_tok * p.gate_stride + (size_t)my_head * TC_D);
@@ -488,6 +506,26 @@ __global__ void __launch_bounds__(TC2_THREADS, 1) attn_tc2_kernel(const AttnPara
                     const unsigned long long d = __shfl_sync(0xffffffffu, my_dst, r);
                     const uint4 o = ld_stage((warp & 3) * 32 + r, c);
                     if (d != 0ull) *reinterpret_cast<uint4*>(d + x * 128 + c * 16) = o;
+                }
+            }
+        } else if (SPLIT && pieces > 1) {
+            const size_t prow = ((size_t)piece * p.T + my_tok) * p.n_q + my_head;
+            if (my_valid && !fail) { p.part_ml[prow * 2] = m_run; p.part_ml[prow * 2 + 1] = l_run; }
+#pragma unroll 1
+            for (int cb = 0; cb < 4; ++cb) {
+                float v[32];
+                if (n_mine > 0) {
+                    tc_ld32(to + cb * 32, v);                            // every thread of the warp takes part
+                    tc_wait_ld(v);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = 0.f;
+                }
+                if (my_valid && !fail) {
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4)
+                        *reinterpret_cast<float4*>(p.part_o + prow * TC_D + cb * 32 + j) =
+                            make_float4(v[j] * o_scale, v[j + 1] * o_scale, v[j + 2] * o_scale, v[j + 3] * o_scale);
                 }
             }
         } else if (!__any_sync(0xffffffffu, fail) && n_mine > 0) {

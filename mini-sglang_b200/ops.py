@@ -116,8 +116,9 @@ def _attn_lib(head_dim: int):
         lib.msgl_attention_window.argtypes = [c_void_p] * 10 + [c_int] * 9 + [c_float] + [c_int] * 6 + [c_void_p, c_int, c_void_p, c_int, c_void_p]
         lib.msgl_attention_combine.argtypes = [c_void_p] * 5 + [c_int] * 5 + [c_void_p, c_void_p, c_ll, c_void_p]
         lib.msgl_attention_tc.argtypes = [c_void_p] * 7 + [c_int] * 8 + [c_float] + [c_int] * 5 + [c_void_p, c_int, c_void_p, c_int, c_void_p,
-                                         c_void_p, c_ll, c_int, c_int, c_float, c_float, c_float, c_void_p]
+                                         c_void_p, c_ll, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]
         lib.msgl_attention_combine_diff.argtypes = [c_void_p] * 5 + [c_int, c_void_p] + [c_int] * 5 + [c_float, c_float, c_float, c_void_p]
+        lib.msgl_attention_combine_range.argtypes = [c_void_p] * 4 + [c_int] * 7 + [c_void_p, c_void_p, c_ll, c_void_p]
         lib.msgl_attention_head_dim.restype = c_int
         _attn[hd] = lib
     return lib
@@ -378,12 +379,14 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
                  q_start: torch.Tensor, kv_len: torch.Tensor, block_table: torch.Tensor, n_kv: int, page_size: int,
                  window: int, scale: float, qlen_min: int, qlen_max: int, q_lens: Sequence[int], keep_first: int = 0,
                  bias_log2: Optional[torch.Tensor] = None, null_log2: Optional[torch.Tensor] = None,
-                 gate: Optional[torch.Tensor] = None, chunk: int = 0, diff: Optional[Tuple[float, float, float]] = None) -> bool:
+                 gate: Optional[torch.Tensor] = None, chunk: int = 0, diff: Optional[Tuple[float, float, float]] = None,
+                 kv_lens: Optional[Sequence[int]] = None, workspace=None) -> bool:
     """Prefill attention on tcgen05 tensor cores for the requests with q_len in [qlen_min, qlen_max];
     q_lens: the host's copy of every request's number of query tokens (to size the grid).  keep_first, bias_log2: as in
     `attention`; they are taken by the kernel on pairs of query tiles only (TMA page sizes), and the call returns False,
     having launched nothing, where that kernel cannot run.  null_log2, gate, chunk: as in `attention`, taken by both kernels;
-    diff: as there, by the kernel on pairs of query tiles only."""
+    diff: as there, by the kernel on pairs of query tiles only.  With kv_lens (the host's copy of kv_len) and a workspace
+    query tiles with far more keys than the launch's mean are cut into pieces (`plan_tc_pieces`) and merged here."""
     global _tc2_usable
     gate_stride = _attention_extras(q, null_log2, gate)
     _need_cuda(q, out, k_cache, v_cache, q_start, kv_len, block_table)
@@ -409,19 +412,71 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
         rows = TC_ROWS * version
         qt = rows // group if group <= TC_ROWS else version
         grid_x = sum(-(-n // qt) for n in q_lens if qlen_min <= n <= qlen_max)
+        cut = None
+        if version == 2 and kv_lens is not None and workspace is not None and not (window or chunk or ext) and \
+                sum((n // qt + 1) * (kv // 128 + 1) for n, kv in zip(q_lens, kv_lens) if n >= qlen_min) * n_kv >= TC_PIECE_MEAN * sm_count(q.device):
+            cut = plan_tc_pieces(q_lens, kv_lens, qlen_min=qlen_min, qlen_max=qlen_max, tile_tokens=qt, heads=n_kv * (1 if group <= TC_ROWS else -(-group // TC_ROWS)),
+                                 sms=sm_count(q.device), bytes_per_piece=T * n_q * d * 4)
+        part_o = part_ml = tok_pieces = None
+        if cut is not None:
+            part_o = workspace.get("attn_part_o", cut[1] * T * n_q * d, torch.float32)
+            part_ml = workspace.get("attn_part_ml", cut[1] * T * n_q * 2, torch.float32)
+            tok_pieces = workspace.get("attn_tok_pieces", T, torch.int32)
         code = _attn_lib(d).msgl_attention_tc(
             _ptr(q), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(q_start), _ptr(kv_len), _ptr(block_table), B, T, n_q,
             n_kv, d, page_size, block_table.stride(0), window, float(scale), qlen_min, qlen_max, grid_x, pages, version,
             _ptr(status), int(keep_first), _ptr(bias_log2), bias_log2.shape[1] if bias_log2 is not None else 0, _ptr(null_log2), _ptr(gate),
-            gate_stride, int(chunk), int(diff is not None), *(diff or (0.0, 0.0, 0.0)), _stream())
+            gate_stride, int(chunk), int(diff is not None), *(diff or (0.0, 0.0, 0.0)), *(cut[:2] if cut else (0, 0)), _ptr(part_o), _ptr(part_ml), _ptr(tok_pieces),
+            _stream())
         if code == 2 and version == 2:        # no tensor maps here (driver without the encoder, unaligned cache): one-tile kernel
             _tc2_usable = False
             if ext:
                 return False
             continue
         _check(code, "attention_tc")
+        for tok0, n in cut[2] if cut is not None else ():
+            _check(_attn_lib(d).msgl_attention_combine_range(_ptr(part_o), _ptr(part_ml), _ptr(tok_pieces), _ptr(out), T, tok0, n, n_q, d, cut[1], _dt(out),
+                                                             _ptr(null_log2), _ptr(gate), gate_stride, _stream()), "attention_combine_range")
         return True
     return False
+
+
+# The tcgen05 kernel walks a query tile's key tiles (128 keys) one after the other, 2 to 3 us each, one block an SM.  Cutting a tile's keys
+# costs the merge of the pieces (their float32 rows out and in, and a launch a request), so it is done where the longest tile gets
+# shorter by TC_PIECE_GAIN key tiles at least, and only in launches of TC_PIECE_MEAN key tiles an SM or more: the host launches a
+# layer's kernels in 80 to 100 us, which covers smaller ones (attention layer, 4B widths, 100 tokens behind 3,000: 98 us whole, 110 cut; 0.6B,
+# 1,300 and 40 behind 2,900: 94 / 115; 8B, 65 behind 3,000 and 1,500 behind 100: 204 / 195).
+TC_PIECE_MIN, TC_PIECE_MEAN, TC_PIECE_GAIN, TC_PIECE_MAX, TC_PIECE_BYTES = 4, 8, 8, 8, 1 << 28
+
+
+def plan_tc_pieces(q_lens: Sequence[int], kv_lens: Sequence[int], *, qlen_min: int, qlen_max: int, tile_tokens: int, heads: int, sms: int,
+                   bytes_per_piece: int) -> Optional[Tuple[int, int, Tuple[Tuple[int, int], ...]]]:
+    """(key tiles a piece, most pieces of a query tile, (first token, tokens) of every run of tokens whose tiles are cut) of a tcgen05 prefill
+    launch, or None if its tiles stay whole.  A piece gets about the key tiles that every SM would have if they were dealt out
+    evenly; tiles with up to 1.5 times that stay whole.  At most TC_PIECE_BYTES of partial results."""
+    total, tiles, first = 0, [], 0
+    for n, kv in zip(q_lens, kv_lens):
+        if qlen_min <= n <= qlen_max:
+            for t in range(0, n, tile_tokens):
+                m = min(tile_tokens, n - t)
+                k = (kv - n + t + m - 1) // 128 + 1
+                total += k
+                tiles.append((k, first + t, m))
+        first += n
+    if not tiles:
+        return None
+    longest, per = max(t[0] for t in tiles), max(TC_PIECE_MIN, -(-total * heads // sms))
+    pieces = min(-(-longest // per), TC_PIECE_MAX, TC_PIECE_BYTES // max(bytes_per_piece, 1))
+    if total * heads < TC_PIECE_MEAN * sms or 2 * longest <= 3 * per or pieces < 2 or longest - max(-(-longest // pieces), per) < TC_PIECE_GAIN:
+        return None
+    runs = []
+    for k, at, m in tiles:                  # the rule of the kernel: a tile is cut if it has more than 1.5 times `per`
+        if 2 * k > 3 * per:
+            if runs and runs[-1][0] + runs[-1][1] == at:
+                runs[-1][1] += m
+            else:
+                runs.append([at, m])
+    return per, pieces, tuple((a, m) for a, m in runs)
 
 
 def attention_tile_tokens(variant: int, group: int, head_dim: int = 128) -> int:

@@ -162,7 +162,8 @@ def paged_attend(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KV
             if n_row and unsplit and ops.tc_supported(d, q.dtype, G):
                 on_tc = ops.attention_tc(q, out, cache.k, cache.v, q_start=ctx.q_start, kv_len=ctx.kv_len,
                                          block_table=g.block_table, n_kv=n_kv, page_size=cache.page_size, window=window,
-                                         scale=scale, qlen_min=qt_dec + 1, qlen_max=big, q_lens=ctx.host_q_lens, **extra)
+                                         scale=scale, qlen_min=qt_dec + 1, qlen_max=big, q_lens=ctx.host_q_lens, kv_lens=ctx.host_kv_lens,
+                                         workspace=ctx.workspace, **extra)
             if n_row and not on_tc:
                 ops.attention(q, out, cache.k, cache.v, qlen_min=qt_dec + 1, qlen_max=big,
                               variant=ops.VARIANT_MMA_ROWS, grid_x=n_row, **common)
