@@ -440,120 +440,121 @@ __global__ void qknorm_rope_kvwrite_kernel(const T* __restrict__ qkv, int qkv_st
     }
 }
 
-// Fast path for head sizes 32, 64, 128, 256 with full rotation: a lane owns E = d / 32 consecutive
-// elements, so loads and stores are contiguous, and its rotation partner (element + d/2) sits in
-// lane ^ 16 -- no shared memory.  Same arithmetic as the general kernel above.
-// E consecutive elements of T as one access of E * sizeof(T) bytes (2 ... 32 bytes, aligned to that size)
-template <typename T, int E> struct Pack {
-    static constexpr int BYTES = E * (int)sizeof(T);
-    static __device__ __forceinline__ void load(const T* p, float (&v)[E]) {
-        __align__(16) T tmp[E];
-        if constexpr (BYTES == 32) {
-            reinterpret_cast<uint4*>(tmp)[0] = reinterpret_cast<const uint4*>(p)[0];
-            reinterpret_cast<uint4*>(tmp)[1] = reinterpret_cast<const uint4*>(p)[1];
-        } else if constexpr (BYTES == 16) {
-            *reinterpret_cast<uint4*>(tmp) = *reinterpret_cast<const uint4*>(p);
-        } else if constexpr (BYTES == 8) {
-            *reinterpret_cast<uint2*>(tmp) = *reinterpret_cast<const uint2*>(p);
-        } else if constexpr (BYTES == 4) {
-            *reinterpret_cast<unsigned*>(tmp) = *reinterpret_cast<const unsigned*>(p);
-        } else {
+// Head sizes 32, 64, 128 and 256 whose rotation covers the whole head; same arithmetic as the general kernel above.
+// L = d / 16 lanes own one head of TOK consecutive tokens: a lane holds eight elements of the head's lower half and the eight they are rotated
+// with, so that the rotation takes no shuffle, the sum log2(L) and every copy is 16 bytes; a warp's lanes stand on neighbouring heads.  In prompt
+// portions warps in flight decide (two tokens at 64 registers, four blocks an SM; four tokens at 99 registers took 15.3 us where this takes 12.1,
+// and 62 where it takes 47), in decode steps the chain load-sum-rotate-store.  Against a warp a head and four tokens with 8-byte copies and a shuffle for
+// every rotated element, bfloat16, 32 + 8 heads of 128: 64 tokens 3.2 -> 1.7 us, 1,911 tokens (47 MB) 19.0 -> 12.1, 8,000 tokens (197 MB) 76.9 -> 47.4 (4.2 TB/s).
+template <typename T, int N> struct Half {       // eight neighbouring elements as they are in memory
+    uint4 raw[N];
+    __device__ __forceinline__ void load(const T* p) {
 #pragma unroll
-            for (int j = 0; j < E; ++j) tmp[j] = p[j];
-        }
-#pragma unroll
-        for (int j = 0; j < E; ++j) v[j] = to_f32<T>(tmp[j]);
+        for (int i = 0; i < N; ++i) raw[i] = reinterpret_cast<const uint4*>(p)[i];
     }
-    static __device__ __forceinline__ void store(T* p, const float (&v)[E]) {
-        __align__(16) T tmp[E];
+    __device__ __forceinline__ void store(T* p) const {
 #pragma unroll
-        for (int j = 0; j < E; ++j) tmp[j] = from_f32<T>(v[j]);
-        if constexpr (BYTES == 32) {
-            reinterpret_cast<uint4*>(p)[0] = reinterpret_cast<const uint4*>(tmp)[0];
-            reinterpret_cast<uint4*>(p)[1] = reinterpret_cast<const uint4*>(tmp)[1];
-        } else if constexpr (BYTES == 16) {
-            *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(tmp);
-        } else if constexpr (BYTES == 8) {
-            *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(tmp);
-        } else if constexpr (BYTES == 4) {
-            *reinterpret_cast<unsigned*>(p) = *reinterpret_cast<const unsigned*>(tmp);
-        } else {
+        for (int i = 0; i < N; ++i) reinterpret_cast<uint4*>(p)[i] = raw[i];
+    }
+    __device__ __forceinline__ void get(float* v) const {
+        const T* t = reinterpret_cast<const T*>(raw);
 #pragma unroll
-            for (int j = 0; j < E; ++j) p[j] = tmp[j];
-        }
+        for (int j = 0; j < 8; ++j) v[j] = to_f32<T>(t[j]);
+    }
+    __device__ __forceinline__ void set(const float* v) {
+        T* t = reinterpret_cast<T*>(raw);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t[j] = from_f32<T>(v[j]);
     }
 };
 
-// A warp owns one head of QKR_TOK consecutive tokens: their rows are fetched first, then worked on one after the
-// other, so that several loads are in flight per lane (one token a warp leaves the kernel bound by block turnover).
-constexpr int QKR_TOK = 4;
-template <typename T, int E>
-__global__ void qknorm_rope_kvwrite_vec_kernel(const T* __restrict__ qkv, int qkv_stride,
-                                               const int* __restrict__ positions, const int* __restrict__ out_loc,
-                                               const void* __restrict__ qw, const void* __restrict__ kw, int w_is_f32,
-                                               float eps, const float* __restrict__ table, int max_pos,
-                                               T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache,
-                                               int page_size, int n_q, int n_kv, int T_) {
-    constexpr int d = 32 * E;
+constexpr int QKR_THREADS = 256, QKR_TOK = 2;
+template <typename T, int L, int TOK>
+__global__ void __launch_bounds__(QKR_THREADS, TOK > 1 && sizeof(T) == 4 ? 3 : 4) qknorm_rope_kvwrite_vec_kernel(
+    const T* __restrict__ qkv, int qkv_stride, const int* __restrict__ positions, const int* __restrict__ out_loc,
+    const void* __restrict__ qw, const void* __restrict__ kw, int w_is_f32, float eps, const float* __restrict__ table, int max_pos,
+    T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache, int page_size, int n_q, int n_kv, int T_) {
+    constexpr int d = 16 * L, half = 8 * L;
+    using H8 = Half<T, sizeof(T) / 2>;
     pdl_launch_dependents();
-    const int t0 = blockIdx.x * QKR_TOK;
-    const int warps = blockDim.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const int head = blockIdx.y * warps + (threadIdx.x >> 5);
+    const int l8 = (threadIdx.x & (L - 1)) * 8;
     const int n_heads = n_q + 2 * n_kv;
-    if (head >= n_heads) return;
-    const bool is_q = head < n_q;
-    const bool is_k = !is_q && head < n_q + n_kv;
+    const long long row = (long long)blockIdx.x * (QKR_THREADS / L) + threadIdx.x / L;
+    const int run = (int)(row / n_heads), head = (int)(row - (long long)run * n_heads), t0 = run * TOK;
+    const bool is_q = head < n_q, is_k = !is_q && head < n_q + n_kv;
     const bool writes_cache = (k_cache != nullptr) && (out_loc != nullptr);
-    if (!is_q && !writes_cache) return;
+    const bool active = t0 < T_ && (is_q || writes_cache);      // the others stay for the shuffles
+    const bool rotates = active && table != nullptr && (is_q || is_k);
 
     // positions, cache slots and norm weights are nobody's output: fetched while the kernel before this one finishes
-    float v[QKR_TOK][E];
-    int pos[QKR_TOK], slot[QKR_TOK];
+    int pos[TOK], slot[TOK];
 #pragma unroll
-    for (int i = 0; i < QKR_TOK; ++i) {
+    for (int i = 0; i < TOK; ++i) {
         const int t = t0 + i < T_ ? t0 + i : T_ - 1;                     // past the end: the last token again, not stored
-        pos[i] = (table != nullptr && (is_q || is_k)) ? positions[t] : 0;
-        slot[i] = is_q ? 0 : out_loc[t];
+        pos[i] = rotates ? positions[t] : 0;
+        slot[i] = active && !is_q ? out_loc[t] : 0;
     }
     const void* nw = is_q ? qw : (is_k ? kw : nullptr);
-    float w[E];
+    float w[16];
     if (nw != nullptr) {
 #pragma unroll
-        for (int j = 0; j < E; ++j) w[j] = load_weight(nw, lane * E + j, w_is_f32);
+        for (int j = 0; j < 16; ++j) w[j] = load_weight(nw, (j < 8 ? 0 : half - 8) + l8 + j, w_is_f32);
     }
+    constexpr bool AHEAD = TOK == 1;             // the angles too where the registers allow it
+    float4 tab[4];
+    auto angles = [&](int i, float4* to) {
+        const int ps = pos[i] < 0 ? 0 : (pos[i] >= max_pos ? max_pos - 1 : pos[i]);
+        const float4* at = reinterpret_cast<const float4*>(table + (size_t)ps * d + l8);
+        to[0] = at[0]; to[1] = at[1]; to[2] = at[half / 4]; to[3] = at[half / 4 + 1];
+    };
+    if (AHEAD && rotates) angles(0, tab);
     pdl_wait();
     pdl_after_wait();
     pdl_small();
+    H8 lo[TOK], hi[TOK];
 #pragma unroll
-    for (int i = 0; i < QKR_TOK; ++i) {
+    for (int i = 0; i < TOK; ++i) {
         const int t = t0 + i < T_ ? t0 + i : T_ - 1;
-        Pack<T, E>::load(qkv + (size_t)t * qkv_stride + (size_t)head * d + lane * E, v[i]);
+        const T* src = qkv + (size_t)t * qkv_stride + (size_t)head * d + l8;
+        lo[i].load(src);
+        hi[i].load(src + half);
     }
 #pragma unroll
-    for (int i = 0; i < QKR_TOK; ++i) {
-        if (t0 + i >= T_) break;
-        if (nw != nullptr) {
-            float ss = 0.f;
+    for (int i = 0; i < TOK; ++i) {
+        if (is_q || is_k) {
+            float x[8], y[8];
+            lo[i].get(x);
+            hi[i].get(y);
+            if (nw != nullptr) {
+                float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-            for (int j = 0; j < E; ++j) ss += v[i][j] * v[i][j];
-            ss = warp_sum(ss);
-            const float inv = rsqrtf(ss / (float)d + eps);
+                for (int j = 0; j < 8; ++j) { s0 += x[j] * x[j]; s1 += y[j] * y[j]; }
+                float ss = s0 + s1;
+                const unsigned group = (unsigned)(((1ull << L) - 1) << (threadIdx.x & 31 & ~(L - 1)));
 #pragma unroll
-            for (int j = 0; j < E; ++j) v[i][j] = v[i][j] * inv * w[j];
-        }
-        if (table != nullptr && (is_q || is_k)) {
-            const int ps = pos[i] < 0 ? 0 : (pos[i] >= max_pos ? max_pos - 1 : pos[i]);
-            const float* cs = table + (size_t)ps * d;
-            const int pi = (lane & 15) * E;           // index of the pair within the half
-            const bool upper = lane >= 16;
+                for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(group, ss, o);
+                const float inv = rsqrtf(ss / (float)d + eps);
 #pragma unroll
-            for (int j = 0; j < E; ++j) {
-                const float other = __shfl_xor_sync(0xffffffffu, v[i][j], 16);
-                const float c = cs[pi + j], sn = cs[d / 2 + pi + j];
-                v[i][j] = upper ? (other * sn + v[i][j] * c) : (v[i][j] * c - other * sn);
+                for (int j = 0; j < 8; ++j) { x[j] = x[j] * inv * w[j]; y[j] = y[j] * inv * w[8 + j]; }
             }
+            if (rotates) {
+                if (!AHEAD) angles(i, tab);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float4 c4 = tab[q], s4 = tab[2 + q];
+                    const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float u = x[4 * q + j], v = y[4 * q + j];
+                        x[4 * q + j] = u * c[j] - v * s[j];
+                        y[4 * q + j] = u * s[j] + v * c[j];
+                    }
+                }
+            }
+            lo[i].set(x);
+            hi[i].set(y);
         }
+        if (!active || t0 + i >= T_) continue;
         T* dst;
         if (is_q) {
             dst = q_out + ((size_t)(t0 + i) * n_q + head) * d;
@@ -563,7 +564,8 @@ __global__ void qknorm_rope_kvwrite_vec_kernel(const T* __restrict__ qkv, int qk
             T* base = is_k ? k_cache : v_cache;
             dst = base + (((size_t)page * n_kv + kvh) * page_size + off) * d;
         }
-        Pack<T, E>::store(dst + lane * E, v[i]);
+        lo[i].store(dst + l8);
+        hi[i].store(dst + half + l8);
     }
 }
 
@@ -578,21 +580,30 @@ MSGL_API int msgl_qknorm_rope_kvwrite(const void* qkv, int qkv_stride, const int
     const int warps = n_heads < 8 ? n_heads : 8;
     dim3 grid(T_, (n_heads + warps - 1) / warps);
     const size_t smem = table ? (size_t)warps * d * sizeof(float) : 0;
-    const bool aligned = (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 31) == 0 &&
-                         (qkv_stride % (d / 32 > 0 ? d / 32 : 1)) == 0;
+    // 16-byte copies of the rows and of the table; the library's head sizes whose rotation covers the whole head
+    const size_t esize = dtype == MSGL_F32 ? 4 : 2;
+    const bool aligned = (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)table) & 15) == 0 &&
+                         (qkv_stride * esize) % 16 == 0;
     if (aligned && (d == 32 || d == 64 || d == 128 || d == 256) && (table == nullptr || (rot == d && !interleaved)) &&
         (dtype == MSGL_F32 || dtype == MSGL_BF16)) {
-#define QKR_VEC(TT, EE)                                                                                              \
-    msgl_launch_pdl(qknorm_rope_kvwrite_vec_kernel<TT, EE>, dim3((T_ + QKR_TOK - 1) / QKR_TOK, grid.y), dim3(warps * 32), 0, stream, \
+        // One token a lane up to three blocks an SM, all resident at once (384 blocks: 2.8 us against 3.5 with QKR_TOK), then QKR_TOK, whose copies are
+        // under way together (512 blocks: 3.75 us against 4.27).
+        const int L = d / 16;
+        const bool few = (long long)T_ * n_heads * L <= (long long)msgl_sm_count() * 3 * QKR_THREADS;
+        const long long rows = (long long)(few ? T_ : (T_ + QKR_TOK - 1) / QKR_TOK) * n_heads;
+        const dim3 vgrid((unsigned)((rows * L + QKR_THREADS - 1) / QKR_THREADS));
+#define QKR_RUN(TT, LL, TOK)                                                                                         \
+    msgl_launch_pdl(qknorm_rope_kvwrite_vec_kernel<TT, LL, TOK>, vgrid, dim3(QKR_THREADS), 0, stream,                \
         (const TT*)qkv, qkv_stride, positions, out_loc, qw, kw, w_is_f32, eps, table, max_pos, (TT*)q_out,           \
         (TT*)k_cache, (TT*)v_cache, page_size, n_q, n_kv, T_)
-        const int E = d / 32;
+#define QKR_VEC(TT, LL) do { if (few) QKR_RUN(TT, LL, 1); else QKR_RUN(TT, LL, QKR_TOK); } while (0)
         if (dtype == MSGL_F32) {
-            if (E == 1) QKR_VEC(float, 1); else if (E == 2) QKR_VEC(float, 2); else if (E == 4) QKR_VEC(float, 4); else QKR_VEC(float, 8);
+            if (L == 2) QKR_VEC(float, 2); else if (L == 4) QKR_VEC(float, 4); else if (L == 8) QKR_VEC(float, 8); else QKR_VEC(float, 16);
         } else {
-            if (E == 1) QKR_VEC(__nv_bfloat16, 1); else if (E == 2) QKR_VEC(__nv_bfloat16, 2);
-            else if (E == 4) QKR_VEC(__nv_bfloat16, 4); else QKR_VEC(__nv_bfloat16, 8);
+            if (L == 2) QKR_VEC(__nv_bfloat16, 2); else if (L == 4) QKR_VEC(__nv_bfloat16, 4);
+            else if (L == 8) QKR_VEC(__nv_bfloat16, 8); else QKR_VEC(__nv_bfloat16, 16);
         }
+#undef QKR_RUN
 #undef QKR_VEC
         return msgl_check_launch();
     }

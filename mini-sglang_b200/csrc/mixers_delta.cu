@@ -1178,7 +1178,8 @@ __global__ void __launch_bounds__(DR_MANY_WARPS * 32) delta_rule_kernel(const De
 // The decays are products of the g themselves, not differences of sums of logarithms, which would lose digits where they are small.
 //
 // Token by token the walk is a chain (a product with the state, two rounds of shuffles, the update) of 0.37 us a token whatever the number of
-// SMs; a chunk of 32 tokens takes the blocks about 1.3 us.  32 and not 64: the work a token grows by a fifth with 64, and the walk gets no shorter.
+// SMs; a chunk of 32 tokens takes the blocks 2.8 us (8,000 tokens: 697 us).  32 tokens: a row of the weights is a warp's width, the substitution's
+// rows stay in a thread's registers and two blocks' stages fit an SM.
 // ---------------------------------------------------------------------------------------
 constexpr int DC_C = 32, DC_COLS = 16, DC_THREADS = 256;
 
@@ -1193,7 +1194,7 @@ struct DeltaChunkParams {
     int heads, kv_heads, dv, T, B, n_min;
 };
 
-// A block makes one head's chunk.  Latency decides (loads, 32 steps of the decays, the substitution's chain), so four blocks share an SM: with the
+// A block makes one head's chunk.  Latency decides (loads, 32 steps of the decays, the substitution's chain), so three blocks share an SM: with the
 // substitution's factors kept in registers (255 a thread, one block an SM) and the heads of a q/k head in one block it took 116 us
 // for 1,411 tokens of 16 heads.
 template <typename T, int D>
