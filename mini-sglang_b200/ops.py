@@ -59,7 +59,8 @@ def _need_cuda(*tensors: Optional[torch.Tensor]) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the handle alone: the Stream object costs a microsecond a launch, which prompt steps of a few tokens wait for
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -413,12 +414,15 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
         qt = rows // group if group <= TC_ROWS else version
         grid_x = sum(-(-n // qt) for n in q_lens if qlen_min <= n <= qlen_max)
         cut = None
+        # the plan is made in Python: two bounds on the key tiles, the cheap one first, keep it out of launches that the rule leaves whole
         if version == 2 and kv_lens is not None and workspace is not None and not (window or chunk or ext) and \
-                sum((n // qt + 1) * (kv // 128 + 1) for n, kv in zip(q_lens, kv_lens) if n >= qlen_min) * n_kv >= TC_PIECE_MEAN * sm_count(q.device):
+                (longest := max(kv_lens)) > 128 * (TC_PIECE_MIN + TC_PIECE_GAIN - 1) and \
+                (T // qt + B) * (longest // 128 + 1) * n_kv >= (enough := TC_PIECE_MEAN * sm_count(q.device)) and \
+                sum((n // qt + 1) * (kv // 128 + 1) for n, kv in zip(q_lens, kv_lens) if n >= qlen_min) * n_kv >= enough:
             cut = plan_tc_pieces(q_lens, kv_lens, qlen_min=qlen_min, qlen_max=qlen_max, tile_tokens=qt, heads=n_kv * (1 if group <= TC_ROWS else -(-group // TC_ROWS)),
                                  sms=sm_count(q.device), bytes_per_piece=T * n_q * d * 4)
         part_o = part_ml = tok_pieces = None
-        if cut is not None:
+        if cut is not None:                   # the decode requests' pieces may wait in the same buffer: [piece][token], their tokens are others
             part_o = workspace.get("attn_part_o", cut[1] * T * n_q * d, torch.float32)
             part_ml = workspace.get("attn_part_ml", cut[1] * T * n_q * 2, torch.float32)
             tok_pieces = workspace.get("attn_tok_pieces", T, torch.int32)
