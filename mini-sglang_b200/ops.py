@@ -636,11 +636,19 @@ def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32) -> int:
     return _lib().msgl_gemm_small_m(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), ldo, mode, out_f32, _stream())
 
 
+def _product_ok(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> bool:
+    """Whether x [M, K] . weight [N, K]^T + bias [N] is a bfloat16 product whose operands lie as the kernels read them: rows of x one behind
+    the other on 16-byte pitches, packed weights and bias, one device.  The kernels get addresses and sizes only, so whatever
+    does not fit goes to the library, which takes it or refuses it."""
+    return (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2 and weight.dim() == 2 and x.shape[1] == weight.shape[1]
+            and x.stride(1) == 1 and x.stride(0) % 8 == 0 and weight.is_contiguous() and x.get_device() == weight.get_device()
+            and (bias is None or (bias.dtype == torch.bfloat16 and bias.dim() == 1 and bias.shape[0] == weight.shape[0] and bias.is_contiguous()
+                                  and bias.get_device() == weight.get_device())))
+
+
 def _small_m_ok(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> bool:
-    return (USE_SMALL_M and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2
-            and 0 < x.shape[0] <= SMALL_M_MAX and x.stride(1) == 1 and x.stride(0) % 8 == 0 and weight.is_contiguous()
-            and weight.shape[1] % 32 == 0 and weight.shape[0] % 16 == 0
-            and (bias is None or bias.dtype == torch.bfloat16))
+    return (USE_SMALL_M and 0 < x.shape[0] <= SMALL_M_MAX and _product_ok(x, weight, bias)
+            and weight.shape[1] % 32 == 0 and weight.shape[0] % 16 == 0)
 
 
 # This engine's tcgen05 GEMM (csrc/gemm_tc.cu) against the library's, measured on B200 at Qwen3-8B's sizes.  With SwiGLU in
@@ -659,9 +667,8 @@ def _tc_gemm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]
     """x @ weight^T (mode 0) or its gated activation (mode 1: SwiGLU, 2: ReGLU; bias [2I]) by the tcgen05 kernel; None where it
     does not apply."""
     global _tc_gemm_usable
-    if not ((TC_GEMM == "all" or (TC_GEMM == "swiglu" and mode != 0)) and _tc_gemm_usable and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2
-            and x.shape[0] >= TC_GEMM_MIN_M and x.stride(1) == 1 and x.stride(0) % 8 == 0 and weight.is_contiguous()
-            and weight.shape[1] % 8 == 0 and (bias is None or bias.dtype == torch.bfloat16)):
+    if not ((TC_GEMM == "all" or (TC_GEMM == "swiglu" and mode != 0)) and _tc_gemm_usable and x.shape[0] >= TC_GEMM_MIN_M
+            and _product_ok(x, weight, bias) and weight.shape[1] % 8 == 0):
         return None
     M, (N, K) = x.shape[0], weight.shape
     n_out = N // 2 if mode else N
@@ -692,10 +699,8 @@ def _tc_gemm_mid(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
     """x @ weight^T (mode 0) or its gated activation (modes 1, 2) for a middling number of rows by the split-K tcgen05 kernel; None where
     it does not apply."""
     global _tc_gemm_usable
-    if not (MID_GEMM and TC_GEMM != "0" and TC_GEMM_CTAS == 2 and _tc_gemm_usable and x.dtype == torch.bfloat16
-            and weight.dtype == torch.bfloat16 and x.dim() == 2 and SMALL_M_MAX < x.shape[0] < TC_GEMM_MIN_M and x.stride(1) == 1
-            and x.stride(0) % 8 == 0 and weight.is_contiguous() and weight.shape[1] % 8 == 0 and weight.shape[0] % 8 == 0
-            and weight.shape[1] >= 512 and (bias is None or bias.dtype == torch.bfloat16)):
+    if not (MID_GEMM and TC_GEMM != "0" and TC_GEMM_CTAS == 2 and _tc_gemm_usable and SMALL_M_MAX < x.shape[0] < TC_GEMM_MIN_M
+            and _product_ok(x, weight, bias) and weight.shape[1] % 8 == 0 and weight.shape[0] % 8 == 0 and weight.shape[1] >= 512):
         return None
     M, (N, K) = x.shape[0], weight.shape
     n_out = N // 2 if mode else N
@@ -741,10 +746,9 @@ ROWS_F32_MAX, ROWS_F32_MIN_OUT = 128, 114_000
 def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
     """x @ weight^T (mode 0) or its gated activation (1: SwiGLU, 2: ReGLU; bias [2I]) for at most 256 rows by the decode-batch kernel;
     None where it cannot run."""
-    if not (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2 and 0 < x.shape[0] <= 256
-            and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))
-            and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.is_contiguous() and weight.data_ptr() % 16 == 0
-            and weight.shape[1] % 8 == 0 and (bias is None or (bias.dtype == torch.bfloat16 and bias.is_contiguous()))):
+    if not (0 < x.shape[0] <= 256 and _product_ok(x, weight, bias)
+            and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
+            and (x.stride(0) >= x.shape[1] or x.shape[0] == 1) and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and weight.shape[1] % 8 == 0):
         return None
     M, (N, K) = x.shape[0], weight.shape
     n_out = N // 2 if mode else N
