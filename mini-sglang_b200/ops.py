@@ -1582,6 +1582,26 @@ def expert_combine_self(y: torch.Tensor, place: torch.Tensor, wts: torch.Tensor,
     return out
 
 
+def _expert_operands(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor,
+                     extra: Optional[torch.Tensor], extra_gate: Optional[torch.Tensor]) -> Tuple[torch.Tensor, torch.Tensor]:
+    """What every kernel of the routed experts is told by addresses and sizes alone has to lie as they read it: raises, or returns idx and wts of h's tokens,
+    both [T, top]."""
+    _need_cuda(h, gate_up, down, idx, wts, extra, extra_gate)
+    if extra is not None:
+        assert extra.dtype == torch.float32 and extra.is_contiguous() and tuple(extra.shape) == tuple(h.shape)
+        assert extra_gate is None or (extra_gate.dtype == torch.float32 and extra_gate.numel() == h.shape[0])
+    T, H = h.shape
+    E, _, F, _ = gate_up.shape
+    assert gate_up.shape == (E, 2, F, H) and down.shape == (E, H, F)
+    assert gate_up.is_contiguous() and down.is_contiguous() and gate_up.dtype == down.dtype == h.dtype
+    assert idx.dtype == torch.int32 and wts.dtype == torch.float32 and idx.is_contiguous() and wts.is_contiguous()
+    if idx.shape[0] != T or wts.shape != idx.shape:           # more rows than tokens, weights in one row: the first numbers count
+        top = idx.shape[1]
+        assert idx.shape[0] >= T and wts.numel() >= T * top
+        idx, wts = idx[:T], wts.view(-1)[:T * top].view(T, top)
+    return idx, wts
+
+
 def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor,
                 scale: float = 1.0, limit: float = 0.0, extra: Optional[torch.Tensor] = None,
                 extra_gate: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -1590,16 +1610,9 @@ def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx:
     for a few tokens.  limit > 0: the activation is g * sigmoid(1.702 g) * (u + 1) with g = min(gate, limit) and
     u = clamp(up, -limit, limit).  extra float32 [T, H] (a shared expert's output) is added inside the sum, times
     extra_gate float32 [T] where given."""
-    _need_cuda(h, gate_up, down, idx, wts, extra, extra_gate)
-    if extra is not None:
-        assert extra.dtype == torch.float32 and extra.is_contiguous() and tuple(extra.shape) == tuple(h.shape)
-        assert extra_gate is None or (extra_gate.dtype == torch.float32 and extra_gate.numel() == h.shape[0])
+    idx, wts = _expert_operands(h, gate_up, down, idx, wts, extra, extra_gate)
     T, H = h.shape
-    E, _, F, _ = gate_up.shape
-    top = idx.shape[1]
-    assert gate_up.shape == (E, 2, F, H) and down.shape == (E, H, F)
-    assert gate_up.is_contiguous() and down.is_contiguous() and gate_up.dtype == down.dtype == h.dtype
-    assert idx.dtype == torch.int32 and wts.dtype == torch.float32 and idx.is_contiguous() and wts.is_contiguous()
+    F, top = gate_up.shape[2], idx.shape[1]
     done = _expert_products(h, gate_up, down, idx, limit, torch.float32)
     if done is not None:
         return expert_combine(done[0], done[1], wts, scale, extra=extra, extra_gate=extra_gate)
@@ -1673,7 +1686,7 @@ def experts_many(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx
                  limit: float = 0.0, extra: Optional[torch.Tensor] = None, extra_gate: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """`experts_few` for the tokens of a prompt portion (the experts' outputs are rounded to the activation type before they are
     summed): None where the decode-batch kernel does not apply or the library's grouped product is ahead."""
-    _need_cuda(h, gate_up, down, idx, wts, extra)
+    idx, wts = _expert_operands(h, gate_up, down, idx, wts, extra, extra_gate)
     done = _expert_products(h, gate_up, down, idx, limit, h.dtype)
     return None if done is None else expert_combine(done[0], done[1], wts, scale, extra=extra, extra_gate=extra_gate)
 
