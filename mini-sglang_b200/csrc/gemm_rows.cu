@@ -13,7 +13,8 @@
 //     warp 1    one lane issues four tcgen05.mma 128 x tokens x 16 a slab and commits the stage back to the loader
 //     warps 2-5 accumulator -> shared memory, [token][weight row] float32
 //     all       the blocks of a tile's ranges form a cluster: each sums its share of the tokens over the cluster's shared
-//               memories in range order (the result does not depend on timing), then bias / activation and one rounding
+//               memories (in the order of one tree whatever the block, so the result depends on neither timing nor the row's place),
+//               then bias / activation and one rounding
 //
 // The ranges' sums never touch global memory, so the kernel needs no scratch.  Two blocks share an SM where the stages allow it:
 // one streams while the other starts or drains.  Every wait is bounded; a block that gives up sets status[2] and frees its
@@ -70,9 +71,11 @@ __device__ __forceinline__ void gr_store(float* p, float a) { *p = a; }
 __device__ __forceinline__ void gr_store(__nv_bfloat16* p, float a) { *p = __float2bfloat16_rn(a); }
 
 // Block `range` of a tile's SP blocks: tokens range, range + SP, ... of the pass, summed over the blocks' accumulators in shared
-// memory in an order that only depends on the token, then bias / activation and the store.  A thread takes two output columns of a token, four tokens at a
-// time: the loads from the other blocks take a few hundred cycles each and have to be under way together (one after the other
-// they made the product of 128 rows of 24,576 x 4,096 44 us long).
+// memory as a balanced tree over the ranges, ((0 + 1) + (2 + 3)) + ..., then bias / activation and the store.  Every block starts at its own
+// accumulator (they do not all read one) and goes on by the tree: its neighbour's, the neighbouring pair's ...  Only the two sides of an
+// addition change places with the block, so a row's result does not depend on where in the batch it stands.  A thread takes two output
+// columns of a token, four tokens at a time: the loads from the other blocks take a few hundred cycles each and have to be under way together
+// (one after the other they made the product of 128 rows of 24,576 x 4,096 44 us long).
 template <int MODE, typename OutT, int SP>
 __device__ __forceinline__ void gr_reduce(const GemmRowsParams& p, unsigned sums, int range, int tok0, int n_tok, int col0) {
     constexpr bool GLU = MODE != GR_PLAIN;
@@ -91,28 +94,39 @@ __device__ __forceinline__ void gr_reduce(const GemmRowsParams& p, unsigned sums
     }
     unsigned peer[SP];
 #pragma unroll
-    for (int r = 0; r < SP; ++r) peer[r] = gr_peer(sums + (unsigned)j * 8u, (unsigned)((range + r) % SP));      // its own first: the blocks do not all read one
+    for (int r = 0; r < SP; ++r) peer[r] = gr_peer(sums + (unsigned)j * 8u, (unsigned)(range ^ r));
     OutT* out = reinterpret_cast<OutT*>(p.out) + col;
     for (int n0 = range + (int)(threadIdx.x / PER) * SP; n0 < n_tok; n0 += U * SLOTS * SP) {
-        float2 a[U], u[U];
-#pragma unroll
-        for (int i = 0; i < U; ++i) a[i] = u[i] = make_float2(0.f, 0.f);
+        // the tree's open sums, one a level: after r + 1 ranges those of the set bits of r + 1 are waiting for their right-hand sides
+        constexpr int LEVELS = SP >= 8 ? 4 : SP >= 4 ? 3 : SP >= 2 ? 2 : 1;
+        float2 a[LEVELS][U], u[LEVELS][U];
 #pragma unroll
         for (int r = 0; r < SP; ++r)
 #pragma unroll
             for (int i = 0; i < U; ++i) {
                 const int n = n0 + i * SLOTS * SP;
-                if (n >= n_tok) continue;
-                const float2 v = gr_peer_load(peer[r] + (unsigned)n * 512u);
-                a[i].x += v.x; a[i].y += v.y;
-                if (GLU) { const float2 w = gr_peer_load(peer[r] + (unsigned)n * 512u + 256u); u[i].x += w.x; u[i].y += w.y; }
+                float2 v = make_float2(0.f, 0.f), w = v;
+                if (n < n_tok) {
+                    v = gr_peer_load(peer[r] + (unsigned)n * 512u);
+                    if (GLU) w = gr_peer_load(peer[r] + (unsigned)n * 512u + 256u);
+                }
+                int level = 0;
+#pragma unroll
+                for (int bit = 1; bit < SP; bit <<= 1) {
+                    if (!(r & bit)) break;
+                    v.x += a[level][i].x; v.y += a[level][i].y;
+                    if (GLU) { w.x += u[level][i].x; w.y += u[level][i].y; }
+                    ++level;
+                }
+                a[level][i] = v;
+                if (GLU) u[level][i] = w;
             }
 #pragma unroll
         for (int i = 0; i < U; ++i) {
             const int n = n0 + i * SLOTS * SP;
             if (n >= n_tok) continue;
-            float x = a[i].x + ba.x, y = a[i].y + ba.y;
-            if (GLU) { x = gr_act<MODE>(x, u[i].x + bu.x, p.limit); y = gr_act<MODE>(y, u[i].y + bu.y, p.limit); }
+            float x = a[LEVELS - 1][i].x + ba.x, y = a[LEVELS - 1][i].y + ba.y;
+            if (GLU) { x = gr_act<MODE>(x, u[LEVELS - 1][i].x + bu.x, p.limit); y = gr_act<MODE>(y, u[LEVELS - 1][i].y + bu.y, p.limit); }
             OutT* dst = out + (size_t)(tok0 + n) * p.ldo;
             if (two) gr_store2(dst, x, y);              // ldo and col are even, the base 16-byte aligned
             else gr_store(dst, x);

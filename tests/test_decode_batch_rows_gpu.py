@@ -1,0 +1,35 @@
+"""A row's product does not depend on where in the decode batch it stands or on how many rows stand beside it (csrc/gemm_rows.cu)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def product(x, w, b, mode, f32, splits=0, experts=0, ends=None, tokens=0):
+    from mini_sglang_b200 import ops
+    n_out, K = w.shape[-2] // (2 if mode and not experts else 1), w.shape[-1]
+    out = torch.empty((x.shape[0], n_out), dtype=torch.float32 if f32 else torch.bfloat16, device=DEV)
+    code = ops._lib().msgl_gemm_rows(ops._ptr(w), ops._ptr(x), ops._ptr(b), ops._ptr(out), x.shape[0], n_out, K, x.stride(0), n_out, mode, int(f32), 7.0,
+                                     experts, ops._ptr(ends), tokens, splits, 0, ops._ptr(ops._status_tensor(x.device)), ops._stream())
+    assert code == 0
+    return out
+
+
+@pytest.mark.parametrize("mode,f32", [(0, True), (1, False), (3, False)])
+@pytest.mark.parametrize("splits", [0, 1, 2, 4, 8])
+def test_equal_rows_give_equal_results(mode, f32, splits):
+    from mini_sglang_b200 import ops
+    K, N = 2048 + 72, 2 * 130
+    g = torch.Generator(device=DEV).manual_seed(splits)
+    row = torch.randn((1, K), generator=g, device=DEV).bfloat16()
+    w = (torch.randn((N, K), generator=g, device=DEV) * K ** -0.5).bfloat16()
+    b = torch.randn(N, generator=g, device=DEV).bfloat16()
+    alone = product(row, w, b, mode, f32, splits)
+    for M in (7, 16, 53, 128):
+        many = product(row.expand(M, K).contiguous(), w, b, mode, f32, splits)
+        assert torch.equal(many, alone.expand(M, -1)), M
+        among = torch.randn((M, K), generator=g, device=DEV).bfloat16()
+        among[M // 2] = row
+        assert torch.equal(product(among, w, b, mode, f32, splits)[M // 2], alone[0]), M
+    ops.check_kernel_status()
