@@ -9,7 +9,7 @@ step's tokens are written, so its first new token sits at position kv_len[r] - q
 from __future__ import annotations
 
 import dataclasses
-from typing import Any, Sequence, Dict, List, Optional, Tuple
+from typing import Any, Sequence, Dict, List, Optional, Set, Tuple
 
 import torch
 
@@ -53,21 +53,32 @@ class StepContext:
 
 
 class Workspace:
-    """Scratch tensors by name, grown on demand and kept, so that steady-state steps allocate
-    nothing and captured graphs keep their addresses."""
+    """Scratch tensors by name, grown on demand and kept, so that steady-state steps allocate nothing and captured graphs keep
+    their addresses.  An outgrown buffer that a stream capture has seen stays alive for its graph; any other goes back to the
+    allocator, so prompt steps of growing sizes hold the largest one's scratch and not the sum of all."""
 
     def __init__(self, device):
-        self.device = device
+        self.device = torch.device(device)
         self._bufs: Dict[str, torch.Tensor] = {}
-        self._retired: List[torch.Tensor] = []      # outgrown buffers stay alive: captured graphs point at them
+        self._captured: Set[str] = set()            # names whose present buffer was handed out inside a stream capture
+        self._retired: List[torch.Tensor] = []      # outgrown buffers that captured graphs point at
+
+    def _capturing(self) -> bool:
+        return self.device.type == "cuda" and torch.cuda.is_current_stream_capturing()
 
     def get(self, name: str, numel: int, dtype: torch.dtype) -> torch.Tensor:
         buf = self._bufs.get(name)
         if buf is None or buf.numel() < numel or buf.dtype != dtype:
-            if buf is not None:
+            if name in self._captured or (buf is not None and self._capturing()):
                 self._retired.append(buf)
+                self._captured.discard(name)
+            elif buf is not None and buf.is_cuda:
+                # whoever shares a workspace between streams orders them, so what used this buffer lies ahead of the present stream's next work
+                buf.record_stream(torch.cuda.current_stream(buf.device))
             buf = torch.empty(max(numel, 1), dtype=dtype, device=self.device)
             self._bufs[name] = buf
+        if name not in self._captured and self._capturing():
+            self._captured.add(name)
         return buf[:numel]
 
 
