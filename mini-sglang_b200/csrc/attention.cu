@@ -90,8 +90,9 @@ struct AttnParams {
     // runs always leave partial results then, and the merge takes the difference.
     int diff = 0;
     float diff_lam = 0.f, diff_eps = 0.f, diff_scale = 0.f;
-    // prefill tiles whose keys are cut: key tiles a piece should have, and how many pieces every token's tile was cut into (written)
-    int piece_tiles = 0;
+    // prefill tiles whose keys are cut: key tiles a piece should have, how many pieces every token's tile was cut into (written), and the
+    // tokens that part_o and part_ml have rows for: piece_plane of them from piece_tok0 on, every cut one among them
+    int piece_tiles = 0, piece_tok0 = 0, piece_plane = 0;
     int* tok_pieces = nullptr;
 };
 
@@ -1986,15 +1987,16 @@ static int attention_launch(const void* q, void* out, const void* k_cache, const
 // ping-pong, TMA page sizes only (MSGL_ERR_SIZE otherwise: the caller then uses version 1).  grid_x counts
 // tiles of 128 / group (version 1) or 256 / group (version 2) tokens.
 // piece_tiles > 0: query tiles with more than 1.5 times as many key tiles are cut into up to `pieces` pieces (version 2 without window, chunks, kept
-// tokens, bias or pairs of maps); their partial results go to part_o [pieces][T][n_q][128], part_ml [pieces][T][n_q][2], the number of pieces to
-// tok_pieces [T] (tokens that the launch does not take are left alone), and msgl_attention_combine merges them.
+// tokens, bias or pairs of maps); their partial results go to part_o [pieces][piece_plane][n_q][128], part_ml [pieces][piece_plane][n_q][2] with a row
+// for each of the piece_plane tokens from piece_tok0 on, which have to hold every token of a cut tile; the number of pieces goes to
+// tok_pieces [T] (tokens that the launch does not take are left alone), and msgl_attention_combine_range merges them.
 MSGL_API int msgl_attention_tc(const void* q, void* out, const void* k_cache, const void* v_cache, const int* q_start,
                                const int* kv_len, const int* block_table, int B, int T_, int n_q, int n_kv, int d,
                                int page_size, int bt_stride, int window, float scale, int qlen_min, int qlen_max,
                                int grid_x, int cache_pages, int version, int* status, int keep_first, const float* bias,
                                int bias_len, const float* null_log2, const void* gate, long long gate_stride, int chunk_keys,
-                               int diff, float diff_lam, float diff_eps, float diff_scale, int piece_tiles, int pieces, float* part_o,
-                               float* part_ml, int* tok_pieces, cudaStream_t stream) {
+                               int diff, float diff_lam, float diff_eps, float diff_scale, int piece_tiles, int pieces, int piece_tok0,
+                               int piece_plane, float* part_o, float* part_ml, int* tok_pieces, cudaStream_t stream) {
 #if MSGL_HEAD_DIM == 128
     if (gate != nullptr && ((gate_stride & 7) || ((uintptr_t)gate & 15))) return MSGL_ERR_ALIGN;
     // kept first tokens under the window and a bias by distance ([n_q][bias_len] float32, log2 units): version 2 only
@@ -2022,9 +2024,10 @@ MSGL_API int msgl_attention_tc(const void* q, void* out, const void* k_cache, co
     if (piece_tiles > 0) {
         if (version != 2 || ext || diff || window > 0 || chunk_keys > 0 || pieces < 2 || pieces > 64 || part_o == nullptr || part_ml == nullptr || tok_pieces == nullptr)
             return MSGL_ERR_SIZE;
-        if ((long long)grid_x * pieces > 65535) return MSGL_ERR_SIZE;
+        if ((long long)grid_x * pieces > 65535 || piece_tok0 < 0 || piece_plane <= 0 || piece_tok0 + piece_plane > T_) return MSGL_ERR_SIZE;
         if ((uintptr_t)part_o & 15) return MSGL_ERR_ALIGN;
         p.piece_tiles = piece_tiles; p.max_split = pieces; p.part_o = part_o; p.part_ml = part_ml; p.tok_pieces = tok_pieces;
+        p.piece_tok0 = piece_tok0; p.piece_plane = piece_plane;
     }
     const int G = n_q / n_kv;
     const int n_chunks = (diff || G <= TC_ROWS) ? 1 : (G + TC_ROWS - 1) / TC_ROWS;
@@ -2092,14 +2095,15 @@ MSGL_API int msgl_attention_combine(const float* part_o, const float* part_ml, c
     return combine_launch(part_o, part_ml, token_req, nsplit, out, T_, T_, n_q, d, max_split, dtype, null_log2, gate, gate_stride, stream);
 }
 
-// tokens tok0 .. tok0 + n - 1 of T_, pieces [T_]: how many pieces every token has (read for these tokens only)
-MSGL_API int msgl_attention_combine_range(const float* part_o, const float* part_ml, const int* pieces, void* out, int T_, int tok0, int n, int n_q,
-                                          int d, int max_split, int dtype, const float* null_log2, const void* gate, long long gate_stride,
-                                          cudaStream_t stream) {
-    if (tok0 < 0 || n < 0 || tok0 + n > T_ || pieces == nullptr) return MSGL_ERR_SIZE;
-    const size_t row = (size_t)tok0 * n_q, item = dtype == MSGL_F32 ? 4 : 2;
-    return combine_launch(part_o + row * d, part_ml + row * 2, nullptr, pieces + tok0, (char*)out + row * d * item, n, T_, n_q, d, max_split, dtype, null_log2,
-                          gate ? (const char*)gate + (size_t)tok0 * gate_stride * item : nullptr, gate_stride, stream);
+// Tokens tok0 .. tok0 + n - 1 of T_, pieces [T_]: how many pieces every token has (read for these tokens only); part_o, part_ml: rows for the
+// piece_plane tokens from piece_tok0 on.
+MSGL_API int msgl_attention_combine_range(const float* part_o, const float* part_ml, const int* pieces, void* out, int T_, int piece_tok0, int piece_plane,
+                                          int tok0, int n, int n_q, int d, int max_split, int dtype, const float* null_log2, const void* gate,
+                                          long long gate_stride, cudaStream_t stream) {
+    if (n < 0 || tok0 < piece_tok0 || tok0 + n > piece_tok0 + piece_plane || piece_tok0 < 0 || piece_tok0 + piece_plane > T_ || pieces == nullptr) return MSGL_ERR_SIZE;
+    const size_t row = (size_t)tok0 * n_q, prow = (size_t)(tok0 - piece_tok0) * n_q, item = dtype == MSGL_F32 ? 4 : 2;
+    return combine_launch(part_o + prow * d, part_ml + prow * 2, nullptr, pieces + tok0, (char*)out + row * d * item, n, piece_plane, n_q, d, max_split, dtype,
+                          null_log2, gate ? (const char*)gate + (size_t)tok0 * gate_stride * item : nullptr, gate_stride, stream);
 }
 
 // The merge for pairs of maps: out [T, n_q / 2, d]; q_start [B + 1], qlen_max and nsplit tell which requests left partial

@@ -509,8 +509,11 @@ __global__ void __launch_bounds__(TC2_THREADS, 1) attn_tc2_kernel(const AttnPara
                 }
             }
         } else if (SPLIT && pieces > 1) {
-            const size_t prow = ((size_t)piece * p.T + my_tok) * p.n_q + my_head;
-            if (my_valid && !fail) { p.part_ml[prow * 2] = m_run; p.part_ml[prow * 2 + 1] = l_run; }
+            // (a token that the host's copy of the lengths, which sized the plane, did not see cut has no row)
+            const int prow_tok = (int)my_tok - p.piece_tok0;
+            const bool stored = my_valid && !fail && prow_tok >= 0 && prow_tok < p.piece_plane;
+            const size_t prow = stored ? ((size_t)piece * p.piece_plane + prow_tok) * p.n_q + my_head : 0;
+            if (stored) { p.part_ml[prow * 2] = m_run; p.part_ml[prow * 2 + 1] = l_run; }
 #pragma unroll 1
             for (int cb = 0; cb < 4; ++cb) {
                 float v[32];
@@ -521,7 +524,7 @@ __global__ void __launch_bounds__(TC2_THREADS, 1) attn_tc2_kernel(const AttnPara
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = 0.f;
                 }
-                if (my_valid && !fail) {
+                if (stored) {
 #pragma unroll
                     for (int j = 0; j < 32; j += 4)
                         *reinterpret_cast<float4*>(p.part_o + prow * TC_D + cb * 32 + j) =

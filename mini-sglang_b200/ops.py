@@ -117,9 +117,9 @@ def _attn_lib(head_dim: int):
         lib.msgl_attention_window.argtypes = [c_void_p] * 10 + [c_int] * 9 + [c_float] + [c_int] * 6 + [c_void_p, c_int, c_void_p, c_int, c_void_p]
         lib.msgl_attention_combine.argtypes = [c_void_p] * 5 + [c_int] * 5 + [c_void_p, c_void_p, c_ll, c_void_p]
         lib.msgl_attention_tc.argtypes = [c_void_p] * 7 + [c_int] * 8 + [c_float] + [c_int] * 5 + [c_void_p, c_int, c_void_p, c_int, c_void_p,
-                                         c_void_p, c_ll, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]
+                                         c_void_p, c_ll, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]
         lib.msgl_attention_combine_diff.argtypes = [c_void_p] * 5 + [c_int, c_void_p] + [c_int] * 5 + [c_float, c_float, c_float, c_void_p]
-        lib.msgl_attention_combine_range.argtypes = [c_void_p] * 4 + [c_int] * 7 + [c_void_p, c_void_p, c_ll, c_void_p]
+        lib.msgl_attention_combine_range.argtypes = [c_void_p] * 4 + [c_int] * 9 + [c_void_p, c_void_p, c_ll, c_void_p]
         lib.msgl_attention_head_dim.restype = c_int
         _attn[hd] = lib
     return lib
@@ -422,16 +422,18 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
             cut = plan_tc_pieces(q_lens, kv_lens, qlen_min=qlen_min, qlen_max=qlen_max, tile_tokens=qt, heads=n_kv * (1 if group <= TC_ROWS else -(-group // TC_ROWS)),
                                  sms=sm_count(q.device), bytes_per_piece=T * n_q * d * 4)
         part_o = part_ml = tok_pieces = None
-        if cut is not None:                   # the decode requests' pieces may wait in the same buffer: [piece][token], their tokens are others
-            part_o = workspace.get("attn_part_o", cut[1] * T * n_q * d, torch.float32)
-            part_ml = workspace.get("attn_part_ml", cut[1] * T * n_q * 2, torch.float32)
+        lo = plane = 0
+        if cut is not None:                   # rows for the tokens from the first cut one to the last, in buffers that no decode graph knows
+            lo, plane = cut[2][0][0], cut[2][-1][0] + cut[2][-1][1] - cut[2][0][0]
+            part_o = workspace.get("attn_piece_o", cut[1] * plane * n_q * d, torch.float32)
+            part_ml = workspace.get("attn_piece_ml", cut[1] * plane * n_q * 2, torch.float32)
             tok_pieces = workspace.get("attn_tok_pieces", T, torch.int32)
         code = _attn_lib(d).msgl_attention_tc(
             _ptr(q), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(q_start), _ptr(kv_len), _ptr(block_table), B, T, n_q,
             n_kv, d, page_size, block_table.stride(0), window, float(scale), qlen_min, qlen_max, grid_x, pages, version,
             _ptr(status), int(keep_first), _ptr(bias_log2), bias_log2.shape[1] if bias_log2 is not None else 0, _ptr(null_log2), _ptr(gate),
-            gate_stride, int(chunk), int(diff is not None), *(diff or (0.0, 0.0, 0.0)), *(cut[:2] if cut else (0, 0)), _ptr(part_o), _ptr(part_ml), _ptr(tok_pieces),
-            _stream())
+            gate_stride, int(chunk), int(diff is not None), *(diff or (0.0, 0.0, 0.0)), *(cut[:2] if cut else (0, 0)), lo, plane, _ptr(part_o),
+            _ptr(part_ml), _ptr(tok_pieces), _stream())
         if code == 2 and version == 2:        # no tensor maps here (driver without the encoder, unaligned cache): one-tile kernel
             _tc2_usable = False
             if ext:
@@ -439,8 +441,8 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
             continue
         _check(code, "attention_tc")
         for tok0, n in cut[2] if cut is not None else ():
-            _check(_attn_lib(d).msgl_attention_combine_range(_ptr(part_o), _ptr(part_ml), _ptr(tok_pieces), _ptr(out), T, tok0, n, n_q, d, cut[1], _dt(out),
-                                                             _ptr(null_log2), _ptr(gate), gate_stride, _stream()), "attention_combine_range")
+            _check(_attn_lib(d).msgl_attention_combine_range(_ptr(part_o), _ptr(part_ml), _ptr(tok_pieces), _ptr(out), T, lo, plane, tok0, n, n_q, d, cut[1],
+                                                             _dt(out), _ptr(null_log2), _ptr(gate), gate_stride, _stream()), "attention_combine_range")
         return True
     return False
 
@@ -457,7 +459,7 @@ def plan_tc_pieces(q_lens: Sequence[int], kv_lens: Sequence[int], *, qlen_min: i
                    bytes_per_piece: int) -> Optional[Tuple[int, int, Tuple[Tuple[int, int], ...]]]:
     """(key tiles a piece, most pieces of a query tile, (first token, tokens) of every run of tokens whose tiles are cut) of a tcgen05 prefill
     launch, or None if its tiles stay whole.  A piece gets about the key tiles that every SM would have if they were dealt out
-    evenly; tiles with up to 1.5 times that stay whole.  At most TC_PIECE_BYTES of partial results."""
+    evenly; tiles with up to 1.5 times that stay whole.  At most TC_PIECE_BYTES of partial results if all tokens were cut."""
     total, tiles, first = 0, [], 0
     for n, kv in zip(q_lens, kv_lens):
         if qlen_min <= n <= qlen_max:
