@@ -37,7 +37,8 @@ struct GemmRowsParams {
     int up_off;                    // gated: how many rows of W an up row lies behind its gate row
     int expert_rows;               // grouped: rows of W an expert has
     const int* ends;               // grouped: [experts] running sum of the experts' rows in x
-    int bn, stages, splits;        // tokens a pass (a multiple of 16), ring depth, ranges of K
+    int bn, stages, splits;        // tokens a pass (a multiple of 16), ring depth, blocks that share a tile's K
+    int halves;                    // 2: a block has two ranges of K (splits is 1 then), an accumulator each
     unsigned tmem_cols;
     float limit;                   // GR_CLAMPED
     int* status;
@@ -161,7 +162,8 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
     }
     const int slabs_all = (p.K + 63) / 64;
     const int k_begin = (int)((long long)range * slabs_all / splits), k_end = (int)((long long)(range + 1) * slabs_all / splits);
-    const int n_slabs = k_end - k_begin;
+    const int n_slabs = k_end - k_begin, n_first = p.halves == 2 ? slabs_all / 2 : n_slabs;        // slabs of the block's first accumulator
+    const unsigned half_cols = p.tmem_cols / 2;
     const int col0 = tile * (GLU ? 64 : 128);
     const int w_row = expert * p.expert_rows + col0;
 
@@ -233,9 +235,10 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
                     if (!tc_mbar_wait(bar_full(st), (g / S) & 1)) { fail = 1; break; }
                     tc_fence_after();
                     const unsigned long long da = da0 + (unsigned long long)st * step, db = db0 + (unsigned long long)st * step;
+                    const unsigned acc = i < n_first ? tmem : tmem + half_cols;
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        tc_mma(tmem, da + (unsigned long long)(2 * kk), db + (unsigned long long)(2 * kk), idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                        tc_mma(acc, da + (unsigned long long)(2 * kk), db + (unsigned long long)(2 * kk), idesc, ((i > 0 && i != n_first) || kk > 0) ? 1u : 0u);
                     tc_commit(bar_empty(st));
                 }
                 if (!fail) tc_commit(bar_acc);
@@ -251,6 +254,13 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
                     unsigned v[16];
                     tc_ld16(src + (unsigned)c, v);
                     tc_wait_ld16(v);
+                    if (p.halves == 2) {                // the sum that two blocks would make of their accumulators
+                        unsigned w[16];
+                        tc_ld16(src + half_cols + (unsigned)c, w);
+                        tc_wait_ld16(w);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+                    }
 #pragma unroll
                     for (int j = 0; j < 16; ++j) asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(dst + (unsigned)(c + j) * 512u), "r"(v[j]) : "memory");
                 }
@@ -304,13 +314,13 @@ static int gr_launch(const CUtensorMap& xm, const CUtensorMap& wm, const GemmRow
 // gated, 48 rows: 1 range 38.7-41.0 us, 2 ranges 36.5, 4 ranges 43.0; [6,144 x 1,024] gated, 16 rows: 7.9 / 5.9 / 5.7 us.
 // Blocks an SM: three where the shared memory allows it, two where they fill their last round better (32 experts of
 // [2,048 x 1,536], 700 tokens, four experts each: 512 blocks, two an SM 46.5 us, three 52.5; [3,072 x 2,048]: 768 blocks, 85.3 / 79.0).
-static void gr_plan(long long tiles, int slabs, int bn, bool grouped, int& splits, int& stages, int want_splits, int want_per_sm) {
+static void gr_plan(long long tiles, int slabs, int bn, int& splits, int& stages, int want_splits, int want_per_sm) {
     const unsigned stage_bytes = GR_A_BYTES + (unsigned)bn * 128u;
     const int sms = msgl_sm_count();
     splits = 1;
     if (want_splits > 0) splits = want_splits;
     else
-        while (splits < (grouped ? 2 : GR_MAX_SPLITS) && tiles * splits < 2 * sms && slabs >= splits * 2 * 4) splits *= 2;
+        while (splits < GR_MAX_SPLITS && tiles * splits < 2 * sms && slabs >= splits * 2 * 4) splits *= 2;
     while (splits > slabs) splits /= 2;
     auto fill = [&](int per_sm) {              // how full the rounds of blocks are
         const long long slots = (long long)sms * per_sm, rounds = (tiles * splits + slots - 1) / slots;
@@ -327,10 +337,18 @@ static void gr_plan(long long tiles, int slabs, int bn, bool grouped, int& split
     if (stages > most && (unsigned)most * stage_bytes >= (unsigned)bn * 512u) stages = most;
 }
 
+// Grouped products: a tile's K is one range or two, added at the end, and which of them follows from the sizes alone, so that a token's results do not
+// depend on how many tokens stand beside it.  Two where `experts` experts, the fewest that a step uses, give fewer than two blocks an SM (as
+// above).  How two ranges are worked on does follow the tokens and changes no bit: by the two blocks of a cluster where the experts in use give too few blocks, else
+// by one block with an accumulator each (up to 64 tokens: beyond, the accumulators of three blocks are more than an SM's tensor memory).
+static int gr_ranges(long long tiles, long long experts, int slabs) { return tiles * experts < 2 * msgl_sm_count() && slabs >= 8 ? 2 : 1; }
+
 // mode 0: out[M, n_out] = x . W^T (+ bias); 1, 2: act(gate) * up with act = silu, relu, W = [gate; up] (n_out rows each); 3: the
 // clamped form min(g, limit) * sigmoid(1.702 min(g, limit)) * (clamp(u, -limit, limit) + 1).
 // experts > 0: W is [experts][n_out or 2 n_out][K], x holds M rows in the order of their experts, ends [experts] their running sum on
-// the device; tokens: how many tokens brought the rows.  Else M is at most 256.  splits, per_sm: 0 = chosen by gr_plan.
+// the device; tokens: how many tokens brought the rows, M / tokens experts each.  Else M is at most 256.
+// splits: ranges of K; 0 = chosen from the sizes, grouped: for steps that use all experts; -1 = grouped, for steps down to a single token.
+// per_sm: 0 = chosen by gr_plan.
 // bfloat16 operands; out bfloat16 or (mode 0) float32.  K, ldx multiples of 8, ldo even, bases 16-byte aligned.
 MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void* out, int M, int n_out, int K, long long ldx, long long ldo,
                             int mode, int out_f32, float limit, int experts, const int* ends, int tokens, int splits, int per_sm,
@@ -338,7 +356,7 @@ MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void
     if (M <= 0) return MSGL_OK;
     const bool glu = mode != GR_PLAIN, grouped = experts > 0;
     if (mode < 0 || mode > 3 || n_out <= 0 || K <= 0 || (K & 7) || (ldx & 7) || (ldo & 1) || status == nullptr || experts < 0 || experts > 65535 ||
-        splits < 0 || splits > GR_MAX_SPLITS || (splits & (splits - 1)) || per_sm < 0 || per_sm > 3)
+        splits < -1 || (splits == -1 && !grouped) || splits > GR_MAX_SPLITS || (splits > 0 && (splits & (splits - 1))) || per_sm < 0 || per_sm > 3)
         return MSGL_ERR_SIZE;
     if (grouped ? (ends == nullptr || bias != nullptr || tokens <= 0) : M > 256) return MSGL_ERR_SIZE;
     if (((uintptr_t)W | (uintptr_t)X | (uintptr_t)out) & 15) return MSGL_ERR_ALIGN;
@@ -363,9 +381,16 @@ MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void
     p.bias = (const __nv_bfloat16*)bias; p.out = out; p.ldo = ldo; p.M = M; p.n_valid = n_out; p.K = K;
     p.up_off = n_out; p.expert_rows = grouped ? (glu ? 2 * n_out : n_out) : 0; p.ends = ends; p.bn = bn; p.limit = limit; p.status = (int*)status;
     const int tiles = (n_out + (glu ? 63 : 127)) / (glu ? 64 : 128);
-    gr_plan((long long)(tiles * live), (K + 63) / 64, bn, grouped, p.splits, p.stages, splits, per_sm);
+    const int slabs = (K + 63) / 64;
+    p.halves = 1;
+    if (grouped) {
+        if (splits <= 0) splits = gr_ranges(tiles, splits < 0 ? (M + tokens - 1) / tokens : experts, slabs);
+        if (splits == 2 && slabs >= 2 && bn <= 64 && tiles * live >= 2.0 * msgl_sm_count()) { p.halves = 2; splits = 1; }
+    }
+    gr_plan((long long)(tiles * live), slabs, bn, p.splits, p.stages, splits, per_sm);
     p.tmem_cols = 32;
     while (p.tmem_cols < (unsigned)bn) p.tmem_cols *= 2;
+    if (p.halves == 2) p.tmem_cols *= 2;
     const size_t smem = (size_t)p.stages * (GR_A_BYTES + (unsigned)bn * 128u) + GR_HEAD_BYTES + 1024u;
 #define GR_GO(MODE, T) (grouped ? gr_launch<MODE, T, true>(xm, wm, p, tiles, experts, smem, stream) : gr_launch<MODE, T, false>(xm, wm, p, tiles, 1, smem, stream))
     if (out_f32) return mode == GR_PLAIN ? GR_GO(GR_PLAIN, float) : MSGL_ERR_DTYPE;

@@ -1661,7 +1661,9 @@ def expert_rows(h: torch.Tensor, idx: torch.Tensor, n_experts: int) -> Optional[
 def _expert_products(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, limit: float,
                      out_dtype: torch.dtype) -> Optional[Tuple[torch.Tensor, torch.Tensor]]:
     """Both products of the chosen experts, gate_up [E, 2, F, H] and down [E, H, F], with the activation of `experts_few` between them, on the
-    decode-batch kernel -> (y [T * top, H] in the order of the experts, place); None where it does not apply."""
+    decode-batch kernel -> (y [T * top, H] in the order of the experts, place); None where it does not apply.  The ranges of K, and with them the
+    order of the sums, follow from the sizes: float32 results (decode steps) take those of a single token's step, so that a request's
+    tokens are the same in every batch, rounded ones those of a step that uses all experts."""
     T, H = h.shape
     E, _, F, _ = gate_up.shape
     P = T * idx.shape[1]
@@ -1673,14 +1675,14 @@ def _expert_products(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor,
     rows, place, ends = ordered
     act = torch.empty((P, F), dtype=h.dtype, device=h.device)
     y = torch.empty((P, H), dtype=out_dtype, device=h.device)
-    status = _ptr(_status_tensor(h.device))
-    code = _lib().msgl_gemm_rows(_ptr(gate_up), _ptr(rows), None, _ptr(act), P, F, H, H, F, 3 if limit > 0 else 1, 0, float(limit), E, _ptr(ends), T, 0, 0,
+    status, ranges = _ptr(_status_tensor(h.device)), -1 if out_dtype == torch.float32 else 0
+    code = _lib().msgl_gemm_rows(_ptr(gate_up), _ptr(rows), None, _ptr(act), P, F, H, H, F, 3 if limit > 0 else 1, 0, float(limit), E, _ptr(ends), T, ranges, 0,
                                  status, _stream())
     if code == 2:             # no tensor maps on this driver
         return None
     _check(code, "gemm_rows (experts)")
-    _check(_lib().msgl_gemm_rows(_ptr(down), _ptr(act), None, _ptr(y), P, H, F, F, H, 0, int(out_dtype == torch.float32), 0.0, E, _ptr(ends), T, 0, 0,
-                                 status, _stream()), "gemm_rows (experts)")
+    _check(_lib().msgl_gemm_rows(_ptr(down), _ptr(act), None, _ptr(y), P, H, F, F, H, 0, int(out_dtype == torch.float32), 0.0, E, _ptr(ends), T, ranges,
+                                 0, status, _stream()), "gemm_rows (experts)")
     return y, place
 
 

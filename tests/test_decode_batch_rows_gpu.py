@@ -33,3 +33,27 @@ def test_equal_rows_give_equal_results(mode, f32, splits):
         among[M // 2] = row
         assert torch.equal(product(among, w, b, mode, f32, splits)[M // 2], alone[0]), M
     ops.check_kernel_status()
+
+
+@pytest.mark.parametrize("E,H,F,top,sizes", [(16, 2560, 1536, 2, (1, 2, 9, 33, 128, 700)), (64, 512, 520, 3, (1, 5, 40, 130)), (6, 264, 136, 2, (1, 17, 129))])
+@pytest.mark.parametrize("limit", [0.0, 7.0])
+def test_routed_tokens_are_the_same_in_every_batch(E, H, F, top, sizes, limit):
+    """One range of K and two, two taken by the blocks of a cluster and by one block with two accumulators, tokens of an expert that many chose."""
+    from mini_sglang_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(E)
+    T = max(sizes)
+    h = torch.randn((T, H), generator=g, device=DEV).bfloat16()
+    gu, dn = ((torch.randn(s, generator=g, device=DEV) * s[-1] ** -0.5).bfloat16() for s in ((E, 2, F, H), (E, H, F)))
+    idx = torch.rand((T, E), generator=g, device=DEV).argsort(-1)[:, :top].int().contiguous()
+    idx[T // 3: T // 2] = idx[0]                                  # a crowd at one token's experts
+    wts = torch.rand((T, top), generator=g, device=DEV)
+    for call, least in ((ops.experts_few, 1), (ops.experts_many, 17)):
+        whole = call(h, gu, dn, idx, wts, limit=limit)
+        assert whole is not None and torch.isfinite(whole).all()
+        for n in sizes:
+            if n < least:
+                continue
+            for at in {0, T // 2 - n // 2, T - n}:
+                some = slice(at, at + n)
+                assert torch.equal(call(h[some], gu, dn, idx[some], wts[some], limit=limit), whole[some]), (call, n, at)
+    ops.check_kernel_status()
