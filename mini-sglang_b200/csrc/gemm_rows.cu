@@ -75,12 +75,13 @@ __device__ __forceinline__ void gr_store(__nv_bfloat16* p, float a) { *p = __flo
 // memory as a balanced tree over the ranges, ((0 + 1) + (2 + 3)) + ..., then bias / activation and the store.  Every block starts at its own
 // accumulator (they do not all read one) and goes on by the tree: its neighbour's, the neighbouring pair's ...  Only the two sides of an
 // addition change places with the block, so a row's result does not depend on where in the batch it stands.  A thread takes two output
-// columns of a token, four tokens at a time: the loads from the other blocks take a few hundred cycles each and have to be under way together
-// (one after the other they made the product of 128 rows of 24,576 x 4,096 44 us long).
+// columns of a token, four tokens at a time (two with eight ranges): the loads from the other blocks take a few hundred cycles each and have to be
+// under way together, ahead of all additions (one token after the other they made the product of 128 rows of 24,576 x 4,096 44 us long; additions
+// between the loads of eight ranges made that of 16 rows of 2,048 x 4,096 9.0 us long instead of 7.3).
 template <int MODE, typename OutT, int SP>
 __device__ __forceinline__ void gr_reduce(const GemmRowsParams& p, unsigned sums, int range, int tok0, int n_tok, int col0) {
     constexpr bool GLU = MODE != GR_PLAIN;
-    constexpr int PER = GLU ? 32 : 64, SLOTS = GR_THREADS / PER, U = 4;
+    constexpr int PER = GLU ? 32 : 64, SLOTS = GR_THREADS / PER, U = SP >= 8 ? 2 : 4;
     const int j = threadIdx.x % PER, col = col0 + 2 * j;
     if (col >= p.n_valid) return;
     const bool two = col + 1 < p.n_valid;
@@ -98,36 +99,32 @@ __device__ __forceinline__ void gr_reduce(const GemmRowsParams& p, unsigned sums
     for (int r = 0; r < SP; ++r) peer[r] = gr_peer(sums + (unsigned)j * 8u, (unsigned)(range ^ r));
     OutT* out = reinterpret_cast<OutT*>(p.out) + col;
     for (int n0 = range + (int)(threadIdx.x / PER) * SP; n0 < n_tok; n0 += U * SLOTS * SP) {
-        // the tree's open sums, one a level: after r + 1 ranges those of the set bits of r + 1 are waiting for their right-hand sides
-        constexpr int LEVELS = SP >= 8 ? 4 : SP >= 4 ? 3 : SP >= 2 ? 2 : 1;
-        float2 a[LEVELS][U], u[LEVELS][U];
+        float2 a[SP][U], u[SP][U];
 #pragma unroll
         for (int r = 0; r < SP; ++r)
 #pragma unroll
             for (int i = 0; i < U; ++i) {
                 const int n = n0 + i * SLOTS * SP;
-                float2 v = make_float2(0.f, 0.f), w = v;
-                if (n < n_tok) {
-                    v = gr_peer_load(peer[r] + (unsigned)n * 512u);
-                    if (GLU) w = gr_peer_load(peer[r] + (unsigned)n * 512u + 256u);
-                }
-                int level = 0;
-#pragma unroll
-                for (int bit = 1; bit < SP; bit <<= 1) {
-                    if (!(r & bit)) break;
-                    v.x += a[level][i].x; v.y += a[level][i].y;
-                    if (GLU) { w.x += u[level][i].x; w.y += u[level][i].y; }
-                    ++level;
-                }
-                a[level][i] = v;
-                if (GLU) u[level][i] = w;
+                a[r][i] = u[r][i] = make_float2(0.f, 0.f);
+                if (n >= n_tok) continue;
+                a[r][i] = gr_peer_load(peer[r] + (unsigned)n * 512u);
+                if (GLU) u[r][i] = gr_peer_load(peer[r] + (unsigned)n * 512u + 256u);
             }
+#pragma unroll
+        for (int step = 1; step < SP; step *= 2)
+#pragma unroll
+            for (int r = 0; r < SP; r += 2 * step)
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    a[r][i].x += a[r + step][i].x; a[r][i].y += a[r + step][i].y;
+                    if (GLU) { u[r][i].x += u[r + step][i].x; u[r][i].y += u[r + step][i].y; }
+                }
 #pragma unroll
         for (int i = 0; i < U; ++i) {
             const int n = n0 + i * SLOTS * SP;
             if (n >= n_tok) continue;
-            float x = a[LEVELS - 1][i].x + ba.x, y = a[LEVELS - 1][i].y + ba.y;
-            if (GLU) { x = gr_act<MODE>(x, u[LEVELS - 1][i].x + bu.x, p.limit); y = gr_act<MODE>(y, u[LEVELS - 1][i].y + bu.y, p.limit); }
+            float x = a[0][i].x + ba.x, y = a[0][i].y + ba.y;
+            if (GLU) { x = gr_act<MODE>(x, u[0][i].x + bu.x, p.limit); y = gr_act<MODE>(y, u[0][i].y + bu.y, p.limit); }
             OutT* dst = out + (size_t)(tok0 + n) * p.ldo;
             if (two) gr_store2(dst, x, y);              // ldo and col are even, the base 16-byte aligned
             else gr_store(dst, x);
