@@ -35,7 +35,7 @@ struct GemmRowsParams {
     long long ldo;
     int M, n_valid, K;             // tokens (grouped: rows of x), output columns, inner size
     int up_off;                    // gated: how many rows of W an up row lies behind its gate row
-    int expert_rows;               // grouped: rows of W an expert has
+    int expert_rows, experts;      // grouped: rows of W an expert has, how many there are
     const int* ends;               // grouped: [experts] running sum of the experts' rows in x
     int bn, stages, splits;        // tokens a pass (a multiple of 16), ring depth, blocks that share a tile's K
     int halves;                    // 2: a block has two ranges of K (splits is 1 then), an accumulator each
@@ -146,23 +146,60 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = p.stages, splits = p.splits;
     const unsigned stage_bytes = GR_A_BYTES + (unsigned)p.bn * 128u;
-    const int tile = blockIdx.x / splits, range = blockIdx.x - tile * splits, expert = GROUPED ? blockIdx.y : 0;
+    const int tile = blockIdx.x / splits, range = blockIdx.x - tile * splits;
 
-    // the rows of x that this block multiplies: all of them, or its expert's.  Grouped: the blocks of a cluster share the expert,
-    // so they leave together.
-    int row0 = 0, rows = p.M;
-    if (GROUPED) {
-        pdl_wait();                                   // `ends` comes from the kernel before this one
-        row0 = expert > 0 ? p.ends[expert - 1] : 0;
-        rows = p.ends[expert] - row0;
-        if (rows <= 0) return;
-    }
     const int slabs_all = (p.K + 63) / 64;
     const int k_begin = (int)((long long)range * slabs_all / splits), k_end = (int)((long long)(range + 1) * slabs_all / splits);
     const int n_slabs = k_end - k_begin, n_first = p.halves == 2 ? slabs_all / 2 : n_slabs;        // slabs of the block's first accumulator
     const unsigned half_cols = p.tmem_cols / 2;
     const int col0 = tile * (GLU ? 64 : 128);
-    const int w_row = expert * p.expert_rows + col0;
+
+    // The tokens that this block multiplies: all of them, or (grouped) runs of up to bn rows of an expert, counted over the experts in order, from
+    // the blockIdx.y-th on in steps of gridDim.y.  So a crowd at a few experts, whose rows a router may send there together, is worked on side by side.
+    // 32 experts are looked at together, four looks' loads under way at once.  The blocks of a cluster share their runs.
+    int expert = 0, tok0 = 0, n_tok = p.M, run = blockIdx.y, n_runs = 1;
+    auto find_run = [&]() -> bool {
+        int counted = 0;
+        bool found = false;
+        for (int e0 = 0; e0 < p.experts; e0 += 128) {
+            int begin[4], end[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int e = min(e0 + 32 * i + lane, p.experts - 1);
+                end[i] = p.ends[e];
+                begin[i] = e > 0 ? p.ends[e - 1] : 0;
+                if (e0 + 32 * i + lane >= p.experts) begin[i] = end[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (e0 + 32 * i >= p.experts) break;
+                const int rows = end[i] - begin[i];
+                int runs = rows > 0 ? 1 : 0;
+                if (__any_sync(0xffffffffu, rows > p.bn)) runs = (rows + p.bn - 1) / p.bn;
+                const int total = __reduce_add_sync(0xffffffffu, runs);
+                if (!found && run < counted + total) {           // this look's
+                    int sum = runs;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
+                    const int l = __ffs(__ballot_sync(0xffffffffu, run < counted + sum)) - 1;
+                    expert = e0 + 32 * i + l;
+                    tok0 = __shfl_sync(0xffffffffu, begin[i], l) + (run - counted - __shfl_sync(0xffffffffu, sum - runs, l)) * p.bn;
+                    n_tok = min(p.bn, __shfl_sync(0xffffffffu, end[i], l) - tok0);
+                    found = true;
+                }
+                counted += total;
+            }
+        }
+        n_runs = counted;
+        return found;
+    };
+    // the set-up goes on while the kernel before this one finishes, which `ends` comes from, but for blocks that a random choice of experts
+    // leaves without a run
+    const bool ahead = GROUPED && (int)blockIdx.y >= p.experts;
+    if (ahead) {
+        pdl_wait();
+        if (!find_run()) return;
+    }
 
     if (tid == 0) {
         for (int s = 0; s < S; ++s) { tc_mbar_init(bar_full(s), 1); tc_mbar_init(bar_empty(s), 1); }
@@ -177,14 +214,19 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = tmem_base_s;
-    int fail = 0;
 
-    const int n_pass = (rows + p.bn - 1) / p.bn;      // dense: one
-    int g0 = 0;                                        // slabs that went through the ring before this pass
-    for (int pass = 0; pass < n_pass; ++pass, g0 += n_slabs) {
-        const int tok0 = row0 + pass * p.bn, n_tok = min(p.bn, rows - pass * p.bn);
-        const int n16 = (n_tok + 15) & ~15;            // tokens that are multiplied
+    if (GROUPED && !ahead) {
+        pdl_wait();
+        if (!find_run()) {
+            if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(p.tmem_cols) : "memory");
+            return;
+        }
+    }
+    int fail = 0, g0 = 0, pass = 0;                    // g0: slabs that went through the ring before this run
+    for (;;) {
+        const int w_row = expert * p.expert_rows + col0, n16 = (n_tok + 15) & ~15;      // n16: tokens that are multiplied
         const unsigned x_bytes = (GROUPED ? (unsigned)n16 : (unsigned)p.bn) * 128u;
+        const bool last = !GROUPED || run + (int)gridDim.y >= n_runs;
         if (warp == 0) {
             if (lane == 0) {
                 auto load_w = [&](int k, unsigned a_s, unsigned bar) {
@@ -220,7 +262,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
                     load_w(k_begin + i, a_s, bar_full(st));
                     load_x(k_begin + i, a_s + GR_A_BYTES, bar_full(st));
                 }
-                if (pass == n_pass - 1) pdl_late();    // everything is asked for, and tensor memory is allocated: the next kernel may set itself up
+                if (last) pdl_late();                  // everything is asked for, and tensor memory is allocated: the next kernel may set itself up
             }
         } else if (warp == 1) {
             if (lane == 0) {
@@ -251,7 +293,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
                     unsigned v[16];
                     tc_ld16(src + (unsigned)c, v);
                     tc_wait_ld16(v);
-                    if (p.halves == 2) {                // the sum that two blocks would make of their accumulators
+                    if (p.halves == 2) {               // the sum that two blocks would make of their accumulators
                         unsigned w[16];
                         tc_ld16(src + half_cols + (unsigned)c, w);
                         tc_wait_ld16(w);
@@ -272,10 +314,15 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
         else if (splits == 2) gr_reduce<MODE, OutT, 2>(p, ring, range, tok0, n_tok, col0);
         else if (splits == 4) gr_reduce<MODE, OutT, 4>(p, ring, range, tok0, n_tok, col0);
         else gr_reduce<MODE, OutT, 8>(p, ring, range, tok0, n_tok, col0);
-        tc_fence_async_smem();                          // the next pass's copies may overwrite what was read here
+        if (!last) tc_fence_async_smem();               // the next run's copies may overwrite what was read here
         __syncwarp();
         if (splits > 1) gr_cluster_sync();              // ... and the cluster's other blocks have read this block's sums
-        else __syncthreads();
+        else if (!last) __syncthreads();
+        if (last) break;
+        g0 += n_slabs;
+        ++pass;
+        run += (int)gridDim.y;
+        find_run();
     }
     const bool failed = __syncthreads_or(fail) != 0;
     if (failed && p.status != nullptr && tid == 0) atomicExch(p.status + 2, 1);
@@ -283,7 +330,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
 }
 
 template <int MODE, typename OutT, bool GROUPED>
-static int gr_launch(const CUtensorMap& xm, const CUtensorMap& wm, const GemmRowsParams& p, int tiles, int experts, size_t smem, cudaStream_t stream) {
+static int gr_launch(const CUtensorMap& xm, const CUtensorMap& wm, const GemmRowsParams& p, int tiles, int runs, size_t smem, cudaStream_t stream) {
     auto* kernel = gemm_rows_kernel<MODE, OutT, GROUPED>;
     static MsglOncePerDevice attr_set;
     if (attr_set.due()) {      // first call on this device, never inside a stream capture
@@ -296,7 +343,7 @@ static int gr_launch(const CUtensorMap& xm, const CUtensorMap& wm, const GemmRow
     attr[0].val.clusterDim.x = p.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3((unsigned)(tiles * p.splits), (unsigned)experts);
+    cfg.gridDim = dim3((unsigned)(tiles * p.splits), (unsigned)runs);
     cfg.blockDim = dim3(GR_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream; cfg.attrs = attr;
     cfg.numAttrs = msgl_pdl_enabled() ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xm, wm, p);
@@ -361,11 +408,12 @@ MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void
     int bn = (M + 15) & ~15;
     double live = 1.0;
     if (grouped) {
-        // Room for the rows of an expert that the tokens favour: a little over what a random choice gives.  An expert with more
-        // takes several passes over its weights; the room costs shared memory (700 tokens, 88 rows an expert in the mean: 112 rows 79 us,
-        // 160 rows 85 us, 96 rows and two passes for some 100 us).
+        // Room for the rows of an expert that the tokens favour: a little over what a random choice gives, and from 32 to 64 all of 64 (only
+        // rows that are there are copied and multiplied, and three blocks an SM have three stages at 32 as at 64).  An expert with more has
+        // its weights read by several blocks side by side; more room costs shared memory (700 tokens, 88 rows an expert in the mean: 112 rows 79 us,
+        // 160 rows 85 us).
         const double mean = (double)M / experts, room = mean + 4.0 * sqrt(mean) + 2.0;
-        bn = room >= 160.0 ? 160 : ((int)room + 15) & ~15;
+        bn = room >= 160.0 ? 160 : room > 16.0 && room <= 64.0 ? 64 : ((int)room + 15) & ~15;
         const int most = (tokens + 15) & ~15;
         if (bn > most) bn = most;
         live = experts * (1.0 - pow(1.0 - fmin(1.0, (double)M / tokens / experts), (double)tokens));       // experts that some token uses, in the mean
@@ -376,7 +424,7 @@ MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void
     if (!tc_matrix_map(X, M, K, ldx * 2, grouped ? 16 : bn, &xm) || !tc_matrix_map(W, w_rows, K, (long long)K * 2, glu ? 64 : 128, &wm)) return MSGL_ERR_SIZE;
     GemmRowsParams p;
     p.bias = (const __nv_bfloat16*)bias; p.out = out; p.ldo = ldo; p.M = M; p.n_valid = n_out; p.K = K;
-    p.up_off = n_out; p.expert_rows = grouped ? (glu ? 2 * n_out : n_out) : 0; p.ends = ends; p.bn = bn; p.limit = limit; p.status = (int*)status;
+    p.up_off = n_out; p.expert_rows = grouped ? (glu ? 2 * n_out : n_out) : 0; p.experts = experts; p.ends = ends; p.bn = bn; p.limit = limit; p.status = (int*)status;
     const int tiles = (n_out + (glu ? 63 : 127)) / (glu ? 64 : 128);
     const int slabs = (K + 63) / 64;
     p.halves = 1;
@@ -384,12 +432,16 @@ MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void
         if (splits <= 0) splits = gr_ranges(tiles, splits < 0 ? (M + tokens - 1) / tokens : experts, slabs);
         if (splits == 2 && slabs >= 2 && bn <= 64 && tiles * live >= 2.0 * msgl_sm_count()) { p.halves = 2; splits = 1; }
     }
+    // Blocks along y: no more than the runs of up to bn rows that the experts can have, and not many more than a random choice gives (one an
+    // expert): blocks without a run are not free (128 experts, 8,192 rows: 73 rows of them added 12 us to 265).
+    const long long most_runs = (long long)(M < experts ? M : experts) + M / bn, usual = experts + (experts > 128 ? experts / 16 : 8);
+    const long long runs = !grouped ? 1 : most_runs < usual ? most_runs : usual < 65535 ? usual : 65535;
     gr_plan((long long)(tiles * live), slabs, bn, p.splits, p.stages, splits, per_sm);
     p.tmem_cols = 32;
     while (p.tmem_cols < (unsigned)bn) p.tmem_cols *= 2;
     if (p.halves == 2) p.tmem_cols *= 2;
     const size_t smem = (size_t)p.stages * (GR_A_BYTES + (unsigned)bn * 128u) + GR_HEAD_BYTES + 1024u;
-#define GR_GO(MODE, T) (grouped ? gr_launch<MODE, T, true>(xm, wm, p, tiles, experts, smem, stream) : gr_launch<MODE, T, false>(xm, wm, p, tiles, 1, smem, stream))
+#define GR_GO(MODE, T) (grouped ? gr_launch<MODE, T, true>(xm, wm, p, tiles, (int)runs, smem, stream) : gr_launch<MODE, T, false>(xm, wm, p, tiles, 1, smem, stream))
     if (out_f32) return mode == GR_PLAIN ? GR_GO(GR_PLAIN, float) : MSGL_ERR_DTYPE;
     switch (mode) {
         case GR_PLAIN: return GR_GO(GR_PLAIN, __nv_bfloat16);

@@ -8,7 +8,7 @@ DEV = "cuda"
 
 def product(x, w, b, mode, f32, splits=0, experts=0, ends=None, tokens=0):
     from mini_sglang_b200 import ops
-    n_out, K = w.shape[-2] // (2 if mode and not experts else 1), w.shape[-1]
+    n_out, K = w.shape[-2] // (2 if mode else 1), w.shape[-1]        # (grouped: an expert's rows)
     out = torch.empty((x.shape[0], n_out), dtype=torch.float32 if f32 else torch.bfloat16, device=DEV)
     code = ops._lib().msgl_gemm_rows(ops._ptr(w), ops._ptr(x), ops._ptr(b), ops._ptr(out), x.shape[0], n_out, K, x.stride(0), n_out, mode, int(f32), 7.0,
                                      experts, ops._ptr(ends), tokens, splits, 0, ops._ptr(ops._status_tensor(x.device)), ops._stream())
@@ -56,4 +56,37 @@ def test_routed_tokens_are_the_same_in_every_batch(E, H, F, top, sizes, limit):
             for at in {0, T // 2 - n // 2, T - n}:
                 some = slice(at, at + n)
                 assert torch.equal(call(h[some], gu, dn, idx[some], wts[some], limit=limit), whole[some]), (call, n, at)
+    ops.check_kernel_status()
+
+
+@pytest.mark.parametrize("E,n_out,K,mode", [(70, 130, 200, 0), (33, 64, 520, 3), (32, 2 * 64 + 2, 1032, 1), (1, 258, 64, 0)])
+@pytest.mark.parametrize("crowd", [0, 1, 300, 1500])
+def test_runs_of_crowded_experts(E, n_out, K, mode, crowd):
+    """An expert's rows in runs side by side: none, some and a crowd at one expert of each look of 32, at the first and at the last."""
+    from mini_sglang_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(E + crowd)
+    counts = torch.randint(0, 4, (E,), generator=torch.Generator().manual_seed(E)) * 9
+    for e in {0, E // 2, E - 1}:
+        counts[e] = crowd
+    M = int(counts.sum())
+    if M == 0:
+        return
+    x = torch.randn((M, K), generator=g, device=DEV).bfloat16()
+    w = (torch.randn((E, n_out * (2 if mode else 1), K), generator=g, device=DEV) * K ** -0.5).bfloat16()
+    ends = counts.cumsum(0).int().to(DEV)
+    want, at = torch.empty((M, n_out), dtype=torch.float64, device=DEV), 0
+    for e, n in enumerate(counts.tolist()):
+        y = x[at:at + n].double() @ w[e].double().t()
+        if mode:
+            gate, up = y.chunk(2, -1)
+            if mode == 3:
+                gate, up = gate.clamp(max=7.0), up.clamp(-7.0, 7.0)
+            y = gate * torch.sigmoid(1.702 * gate) * (up + 1) if mode == 3 else torch.nn.functional.silu(gate) * up
+        want[at:at + n] = y
+        at += n
+    for tokens in (M, (M + 3) // 4):
+        for ranges in (-1, 0, 2):
+            got = product(x, w, None, mode, False, ranges, E, ends, tokens)
+            # float32 sums of K products of size K^-1/2 (a few 1e-6) and one rounding of 2^-9
+            assert bool(((got.double() - want).abs() <= 2e-5 * (1 + want.abs()) + 2.0 ** -8 * want.abs()).all()), (tokens, ranges)
     ops.check_kernel_status()
