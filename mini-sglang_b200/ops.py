@@ -1615,7 +1615,7 @@ def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx:
     idx, wts = _expert_operands(h, gate_up, down, idx, wts, extra, extra_gate)
     T, H = h.shape
     F, top = gate_up.shape[2], idx.shape[1]
-    done = _expert_products(h, gate_up, down, idx, limit, torch.float32)
+    done = _expert_products(h, gate_up, down, idx, limit, torch.float32) if _experts_grouped(T * top, F * H) else None
     if done is not None:
         return expert_combine(done[0], done[1], wts, scale, extra=extra, extra_gate=extra_gate)
     act = torch.empty((T * top, F), dtype=h.dtype, device=h.device)
@@ -1637,6 +1637,14 @@ def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx:
 # 145: such tiles leave one block an SM.
 EXPERT_ROWS_MEAN_MAX = 128
 EXPERT_ROWS_MAX_PAIRS = 8192
+# Very small experts in decode steps: the two launches per pair are ahead of the grouped product's four until the pairs' weights add up.  Experts
+# of 512 x 128, two of eight a token, cold: 1 token 6.4 / 12.3 us, 32 tokens 12.3 / 13.4, 64 tokens 19.8 / 14.0; 1,024 x 256, six of 64: 1 token 18.1 /
+# 16.4, 8 tokens 38 / 26; 2,048 x 512, two of eight: 1 token 29 / 20 (all weights in L2 already: 14.5 / 16 and 15.5 / 17.5 us at one token).
+EXPERT_ROWS_MIN_WEIGHTS, EXPERT_ROWS_MIN_WORK = 200_000, 5_000_000      # elements of one matrix of an expert; the same times pairs
+
+
+def _experts_grouped(pairs: int, weights: int) -> bool:
+    return weights >= EXPERT_ROWS_MIN_WEIGHTS or pairs * weights >= EXPERT_ROWS_MIN_WORK
 
 
 def expert_rows(h: torch.Tensor, idx: torch.Tensor, n_experts: int) -> Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor]]:

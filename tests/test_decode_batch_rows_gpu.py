@@ -37,9 +37,10 @@ def test_equal_rows_give_equal_results(mode, f32, splits):
 
 @pytest.mark.parametrize("E,H,F,top,sizes", [(16, 2560, 1536, 2, (1, 2, 9, 33, 128, 700)), (64, 512, 520, 3, (1, 5, 40, 130)), (6, 264, 136, 2, (1, 17, 129))])
 @pytest.mark.parametrize("limit", [0.0, 7.0])
-def test_routed_tokens_are_the_same_in_every_batch(E, H, F, top, sizes, limit):
+def test_routed_tokens_are_the_same_in_every_batch(E, H, F, top, sizes, limit, monkeypatch):
     """One range of K and two, two taken by the blocks of a cluster and by one block with two accumulators, tokens of an expert that many chose."""
     from mini_sglang_b200 import ops
+    monkeypatch.setattr(ops, "EXPERT_ROWS_MIN_WEIGHTS", 0)        # the grouped product for every batch
     g = torch.Generator(device=DEV).manual_seed(E)
     T = max(sizes)
     h = torch.randn((T, H), generator=g, device=DEV).bfloat16()
