@@ -735,14 +735,20 @@ def _tc_gemm_mid(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
 # The product for a decode batch (csrc/gemm_rows.cu: weights on the tensor core's M dimension, tokens on its N dimension) against
 # the library's, measured on B200 over the Qwen3 widths.  Gated products, [2 n_out, K] weights, library product + activation kernel
 # against this kernel: 16 rows [6144, 1024] 7.2 / 6.0 us, [12288, 2048] 14.1 / 11.4, [24576, 4096] 42.7 / 35.9, [51200, 5120] 99.9 / 82.5;
-# 64 rows 7.2 / 7.3, 14.4 / 13.2, 45.0 / 37.4, 103 / 83; 128 rows 7.6 / 9.5, 14.4 / 17.6, 45.3 / 41.8, 107 / 94; 176 rows behind everywhere.
+# 64 rows 7.2 / 7.3, 14.4 / 13.2, 45.0 / 37.4, 103 / 83; 128 rows 7.6 / 9.5, 14.4 / 17.6, 45.3 / 41.8, 107 / 94; 176 rows behind everywhere.  Small
+# weights: [512, 256] 48 rows 4.5 / 4.5, 64 rows 4.6 / 5.2, [1536, 512] 5.0 / 4.8 and 5.0 / 5.4, [2048, 1024] 64 rows 6.0 / 5.2.
 # Up to 8 rows the weight-streaming kernel is level (35.0 / 34.7 us at one row of [24576, 4096]) or ahead on small weights.
 # Float32 products with very many columns (output heads, 151,936 columns): K = 4096, 1 / 8 / 24 / 64 / 128 rows 194 / 200 / 214 / 215 / 233
 # (the better of the library and the weight-streaming kernel) against 181 / 184 / 188 / 196 / 227 us, K = 1024, 1 / 64 rows 54 / 64 against
 # 51 / 64; with 32,768 columns the last round of blocks is nearly empty and it is 2 to 18 % behind.  Plain bfloat16 products stay with
 # the library (4096 x 4096 at 48 rows: 9.6 against 10.1 us, 128 rows 9.7 against 12.3).
-ROWS_GLU_MAX, ROWS_GLU_MAX_LARGE, ROWS_LARGE_WEIGHT = 64, 128, 40_000_000      # rows; elements of the weight from which the second bound holds
-ROWS_F32_MAX, ROWS_F32_MIN_OUT = 128, 114_000
+ROWS_GLU_MAX_SMALL, ROWS_GLU_MAX, ROWS_GLU_MAX_LARGE = 48, 64, 128             # rows
+ROWS_SMALL_WEIGHT, ROWS_LARGE_WEIGHT = 1_500_000, 40_000_000                    # elements of the weight up to and from which the outer bounds hold
+ROWS_F32_MAX, ROWS_F32_MIN_OUT = 128, 114_000                                   # rows; columns
+
+
+def _rows_glu_max(weights: int) -> int:
+    return ROWS_GLU_MAX_LARGE if weights >= ROWS_LARGE_WEIGHT else ROWS_GLU_MAX if weights >= ROWS_SMALL_WEIGHT else ROWS_GLU_MAX_SMALL
 
 
 def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
@@ -811,7 +817,7 @@ def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tens
             code = _small_m(gate_up, x, bias, out, M, N, K, N // 2, mode, 0)
             _check(code, "gemm_small_m (gated)")
             return out
-        if x.dim() == 2 and not MID_GEMM and x.shape[0] <= (ROWS_GLU_MAX_LARGE if gate_up.numel() >= ROWS_LARGE_WEIGHT else ROWS_GLU_MAX):
+        if x.dim() == 2 and not MID_GEMM and x.shape[0] <= _rows_glu_max(gate_up.numel()):
             y = _gemm_rows(x, gate_up, bias, mode, torch.bfloat16)
             if y is not None:
                 return y

@@ -5,3 +5,9 @@ def test_rule_of_the_routed_experts():
     from mini_sglang_b200 import ops
     grouped = ops._experts_grouped
     assert grouped(1, 1024 * 256) and not grouped(64, 512 * 128) and grouped(80, 512 * 128) and not grouped(2, 199_999)
+
+
+def test_rule_of_the_gated_products():
+    from mini_sglang_b200 import ops
+    most = ops._rows_glu_max
+    assert most(2 * 256 * 256) == most(1_499_999) == 48 and most(1_500_000) == most(39_999_999) == 64 and most(40_000_000) == 128
