@@ -740,15 +740,27 @@ def _tc_gemm_mid(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
 # Up to 8 rows the weight-streaming kernel is level (35.0 / 34.7 us at one row of [24576, 4096]) or ahead on small weights.
 # Float32 products with very many columns (output heads, 151,936 columns): K = 4096, 1 / 8 / 24 / 64 / 128 rows 194 / 200 / 214 / 215 / 233
 # (the better of the library and the weight-streaming kernel) against 181 / 184 / 188 / 196 / 227 us, K = 1024, 1 / 64 rows 54 / 64 against
-# 51 / 64; with 32,768 columns the last round of blocks is nearly empty and it is 2 to 18 % behind.  Plain bfloat16 products stay with
+# 51 / 64.  The gain is lost where the last round of blocks (three an SM) is nearly empty, so the rule asks how full the rounds are: 2.67 rounds
+# of 3 (151,936 columns) and 2.88 (163,840) are ahead but for up to 3 % at 65 to 80 rows; 2.01 (114,048) and 2.13 (120,832) are 4 to 17 % behind
+# at 9 to 16 rows; 2.26 (128,256) and 2.31 (131,072) up to 13 % behind for K <= 2560 and 0 to 14 % ahead from K = 4096 on.  Heads of fewer
+# columns stay where they were: with 32,768 columns it is 2 to 18 % behind.  Plain bfloat16 products stay with
 # the library (4096 x 4096 at 48 rows: 9.6 against 10.1 us, 128 rows 9.7 against 12.3).
 ROWS_GLU_MAX_SMALL, ROWS_GLU_MAX, ROWS_GLU_MAX_LARGE = 48, 64, 128             # rows
 ROWS_SMALL_WEIGHT, ROWS_LARGE_WEIGHT = 1_500_000, 40_000_000                    # elements of the weight up to and from which the outer bounds hold
 ROWS_F32_MAX, ROWS_F32_MIN_OUT = 128, 114_000                                   # rows; columns
+ROWS_F32_FILL, ROWS_F32_FILL_LONG, ROWS_F32_LONG = 0.85, 0.75, 4096             # how full the rounds of blocks have to be, and from which K the second holds
 
 
 def _rows_glu_max(weights: int) -> int:
     return ROWS_GLU_MAX_LARGE if weights >= ROWS_LARGE_WEIGHT else ROWS_GLU_MAX if weights >= ROWS_SMALL_WEIGHT else ROWS_GLU_MAX_SMALL
+
+
+def _rows_f32(rows: int, n_out: int, K: int, device) -> bool:
+    """Whether a float32 product goes to the decode-batch kernel (figures above)."""
+    if n_out < ROWS_F32_MIN_OUT or rows > ROWS_F32_MAX:
+        return False
+    tiles, slots = -(-n_out // 128), 3 * sm_count(device)
+    return tiles >= (ROWS_F32_FILL_LONG if K >= ROWS_F32_LONG else ROWS_F32_FILL) * slots * -(-tiles // slots)
 
 
 def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
@@ -778,7 +790,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     Up to SMALL_M_MAX bfloat16 rows go through this engine's weight-streaming kernel
     (csrc/gemm_small_m.cu); everything else is the library GEMM."""
     _need_cuda(x, weight, bias)
-    if out_dtype == torch.float32 and weight.shape[0] >= ROWS_F32_MIN_OUT and x.dim() == 2 and x.shape[0] <= ROWS_F32_MAX:
+    if out_dtype == torch.float32 and x.dim() == 2 and _rows_f32(x.shape[0], weight.shape[0], x.shape[1], x.device):
         y = _gemm_rows(x, weight, bias, 0, torch.float32)
         if y is not None:
             return y

@@ -40,7 +40,7 @@ def test_operands_that_do_not_fit_are_not_the_kernels(M, monkeypatch):
 @pytest.mark.parametrize("M", ROWS)
 def test_calls_that_do_not_fit_raise(M, monkeypatch):
     from mini_sglang_b200 import ops
-    monkeypatch.setattr(ops, "ROWS_F32_MIN_OUT", 16)            # a small weight through the rule of the output heads
+    monkeypatch.setattr(ops, "_rows_f32", lambda rows, *a: rows <= 128)            # a small weight by the way of the output heads
     for what, (x, w, b) in bad_calls(M, "cuda").items():
         for call in (lambda: ops.linear(x, w, b), lambda: ops.linear(x, w, b, out_dtype=torch.float32), lambda: ops.linear_glu(x, w, b), lambda: ops.linear_glu(x, w, b, 4)):
             with pytest.raises(RuntimeError):
