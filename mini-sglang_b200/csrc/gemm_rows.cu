@@ -387,6 +387,9 @@ static void gr_plan(long long tiles, int slabs, int bn, int& splits, int& stages
 // by one block with an accumulator each (up to 64 tokens: beyond, the accumulators of three blocks are more than an SM's tensor memory).
 static int gr_ranges(long long tiles, long long experts, int slabs) { return tiles * experts < 2 * msgl_sm_count() && slabs >= 8 ? 2 : 1; }
 
+// Whether the driver makes tensor maps, without which no product of this file runs.
+MSGL_API int msgl_tensor_maps() { return tc_encoder() != nullptr; }
+
 // mode 0: out[M, n_out] = x . W^T (+ bias); 1, 2: act(gate) * up with act = silu, relu, W = [gate; up] (n_out rows each); 3: the
 // clamped form min(g, limit) * sigmoid(1.702 min(g, limit)) * (clamp(u, -limit, limit) + 1).
 // experts > 0: W is [experts][n_out or 2 n_out][K], x holds M rows in the order of their experts, ends [experts] their running sum on

@@ -133,21 +133,22 @@ __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sy
 typedef CUresult (*tc_encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static tc_encode_fn tc_encoder() {              // the driver's, asked for once; null where it has none
+    static const tc_encode_fn encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult qr;
+        const bool found = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr) == cudaSuccess && qr == cudaDriverEntryPointSuccess;
+        return found ? (tc_encode_fn)fn : (tc_encode_fn) nullptr;
+    }();
+    return encode;
+}
+
 static bool tc_matrix_map(const void* base, long long rows, long long cols, long long pitch_bytes, int box_rows, CUtensorMap* out) {
     static std::mutex mu;
     static std::map<std::tuple<const void*, long long, long long, long long, int>, CUtensorMap> maps;
-    static tc_encode_fn encode = nullptr;
-    static bool looked = false;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!looked) {
-        looked = true;
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr) == cudaSuccess &&
-            qr == cudaDriverEntryPointSuccess)
-            encode = (tc_encode_fn)fn;
-    }
+    const tc_encode_fn encode = tc_encoder();
     if (encode == nullptr) return false;
+    std::lock_guard<std::mutex> lock(mu);
     const auto key = std::make_tuple(base, rows, cols, pitch_bytes, box_rows);
     auto it = maps.find(key);
     if (it != maps.end()) { *out = it->second; return true; }

@@ -101,6 +101,8 @@ def _lib():
         lib.msgl_gemm_tc2_splits.restype = c_int
         lib.msgl_gemm_rows.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_int, c_float, c_int,
                                        c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
+        lib.msgl_tensor_maps.argtypes = []
+        lib.msgl_tensor_maps.restype = c_int
         lib.msgl_sample.argtypes = [c_void_p, c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_ull, c_void_p,
                                     c_void_p, c_void_p, c_void_p, c_int, c_void_p]
         _common = lib
@@ -763,6 +765,17 @@ def _rows_f32(rows: int, n_out: int, K: int, device) -> bool:
     return tiles >= (ROWS_F32_FILL_LONG if K >= ROWS_F32_LONG else ROWS_F32_FILL) * slots * -(-tiles // slots)
 
 
+_tensor_maps = None
+
+
+def tensor_maps() -> bool:
+    """Whether the driver makes the tensor maps that the decode-batch product loads by (asked once)."""
+    global _tensor_maps
+    if _tensor_maps is None:
+        _tensor_maps = bool(_lib().msgl_tensor_maps())
+    return _tensor_maps
+
+
 def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
     """x @ weight^T (mode 0) or its gated activation (1: SwiGLU, 2: ReGLU; bias [2I]) for at most 256 rows by the decode-batch kernel;
     None where it cannot run."""
@@ -772,12 +785,12 @@ def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
         return None
     M, (N, K) = x.shape[0], weight.shape
     n_out = N // 2 if mode else N
-    if n_out % 2 or (mode and N % 2) or (mode and out_dtype != torch.bfloat16):
+    if n_out % 2 or (mode and N % 2) or (mode and out_dtype != torch.bfloat16) or not tensor_maps():
         return None
     out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
     code = _lib().msgl_gemm_rows(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, n_out, K, x.stride(0), n_out, mode, int(out_dtype == torch.float32),
                                  0.0, 0, None, 0, 0, 0, _ptr(_status_tensor(x.device)), _stream())
-    if code == 2:             # no tensor maps on this driver or of this layout
+    if code == 2:             # no tensor map of this layout
         return None
     _check(code, "gemm_rows")
     return out
@@ -1693,7 +1706,7 @@ def _expert_products(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor,
     T, H = h.shape
     E, _, F, _ = gate_up.shape
     P = T * idx.shape[1]
-    if h.dtype != torch.bfloat16 or H % 8 or F % 8 or P > EXPERT_ROWS_MEAN_MAX * E or gate_up.data_ptr() % 16 or down.data_ptr() % 16:
+    if h.dtype != torch.bfloat16 or H % 8 or F % 8 or P > EXPERT_ROWS_MEAN_MAX * E or gate_up.data_ptr() % 16 or down.data_ptr() % 16 or not tensor_maps():
         return None
     ordered = expert_rows(h, idx, E)
     if ordered is None:
@@ -1704,7 +1717,7 @@ def _expert_products(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor,
     status, ranges = _ptr(_status_tensor(h.device)), -1 if out_dtype == torch.float32 else 0
     code = _lib().msgl_gemm_rows(_ptr(gate_up), _ptr(rows), None, _ptr(act), P, F, H, H, F, 3 if limit > 0 else 1, 0, float(limit), E, _ptr(ends), T, ranges, 0,
                                  status, _stream())
-    if code == 2:             # no tensor maps on this driver
+    if code == 2:             # no tensor map of this layout
         return None
     _check(code, "gemm_rows (experts)")
     _check(_lib().msgl_gemm_rows(_ptr(down), _ptr(act), None, _ptr(y), P, H, F, F, H, 0, int(out_dtype == torch.float32), 0.0, E, _ptr(ends), T, ranges,
