@@ -449,12 +449,16 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
     return False
 
 
-# The tcgen05 kernel walks a query tile's key tiles (128 keys) one after the other, 2 to 3 us each, one block an SM.  Cutting a tile's keys
-# costs the merge of the pieces (their float32 rows out and in, and a launch a request), so it is done where the longest tile gets
-# shorter by TC_PIECE_GAIN key tiles at least, and only in launches of TC_PIECE_MEAN key tiles an SM or more: the host launches a
-# layer's kernels in 80 to 100 us, which covers smaller ones (attention layer, 4B widths, 100 tokens behind 3,000: 98 us whole, 110 cut; 0.6B,
-# 1,300 and 40 behind 2,900: 94 / 115; 8B, 65 behind 3,000 and 1,500 behind 100: 204 / 195).
+# The tcgen05 kernel walks a query tile's key tiles (128 keys) one after the other, about 2.6 us each, one block an SM.  Cutting a tile's keys
+# costs some 7.5 us (three key tiles: the merge's launches and the pieces' starts) and 2.1 us a megabyte of partial results (their float32 rows out
+# and in), so a launch is cut where its longest tile gets shorter by more key tiles than that, and by TC_PIECE_GAIN at least.  Fitted to
+# attention layers at 8B widths, us whole / cut: 65 + 1,500 tokens behind 3,000 + 100 keys (11 tiles, 2 MB) 190 / 173; six portions of 100, three of them behind
+# 4,000 (16 tiles, 15 MB) 138 / 121; 600 + 64 + 64 behind 0 + 9,000 + 9,000 (57 tiles, 17 MB) 238 / 119; 300 x 4 behind 100, 2,000, 3,000, 10 (8 tiles,
+# 10 MB) 152 / 160: not cut.  Launches of fewer than TC_PIECE_MEAN key tiles an SM stay whole whatever that says: a cautious bound from when small prompt steps
+# waited for the host's launches.  Cut, 64 tokens behind 8,192 take 70 us and not 189, 100 behind 3,000 64 and not 95, 700 + 65 behind 100 + 3,000
+# 99 and not 124.
 TC_PIECE_MIN, TC_PIECE_MEAN, TC_PIECE_GAIN, TC_PIECE_MAX, TC_PIECE_BYTES = 4, 8, 8, 8, 1 << 28
+TC_PIECE_COST, TC_PIECE_TILE_BYTES = 3, 1_250_000          # key tiles that a cut launch costs, and how many bytes of partial results cost another
 
 
 def plan_tc_pieces(q_lens: Sequence[int], kv_lens: Sequence[int], *, qlen_min: int, qlen_max: int, tile_tokens: int, heads: int, sms: int,
@@ -475,15 +479,21 @@ def plan_tc_pieces(q_lens: Sequence[int], kv_lens: Sequence[int], *, qlen_min: i
         return None
     longest, per = max(t[0] for t in tiles), max(TC_PIECE_MIN, -(-total * heads // sms))
     pieces = min(-(-longest // per), TC_PIECE_MAX, TC_PIECE_BYTES // max(bytes_per_piece, 1))
-    if total * heads < TC_PIECE_MEAN * sms or 2 * longest <= 3 * per or pieces < 2 or longest - max(-(-longest // pieces), per) < TC_PIECE_GAIN:
+    if total * heads < TC_PIECE_MEAN * sms or 2 * longest <= 3 * per or pieces < 2:
         return None
-    runs = []
+    runs, cut, whole = [], 0, 0
     for k, at, m in tiles:                  # the rule of the kernel: a tile is cut if it has more than 1.5 times `per`
         if 2 * k > 3 * per:
+            cut += m
             if runs and runs[-1][0] + runs[-1][1] == at:
                 runs[-1][1] += m
             else:
                 runs.append([at, m])
+        else:
+            whole = max(whole, k)
+    saved = longest - max(-(-longest // pieces), per, whole)
+    if saved < TC_PIECE_GAIN or saved < TC_PIECE_COST + bytes_per_piece * pieces * cut / first / TC_PIECE_TILE_BYTES:
+        return None
     return per, pieces, tuple((a, m) for a, m in runs)
 
 
