@@ -6,7 +6,7 @@
 // The weight rows sit on the M dimension of tcgen05.mma (128 of them a tile) and the tokens on its N dimension (16 to 256, in
 // steps of 16), so nothing is computed for padding beyond the last 16 tokens and a tile's weights pass through shared memory
 // once.  A block owns one tile (128 output columns; gated: 64, with their 64 gate and 64 up rows) and one of `splits` equal
-// ranges of K:
+// ranges of K (grouped: or both of two, with an accumulator each):
 //
 //     warp 0    TMA: W tile [128 x 64] and x tile [tokens x 64] of a slab of K into a ring of stages; the first stages' weights
 //               are asked for before the kernel before this one has finished (programmatic dependent launch), x after it
@@ -16,9 +16,10 @@
 //               memories (in the order of one tree whatever the block, so the result depends on neither timing nor the row's place),
 //               then bias / activation and one rounding
 //
-// The ranges' sums never touch global memory, so the kernel needs no scratch.  Two blocks share an SM where the stages allow it:
-// one streams while the other starts or drains.  Every wait is bounded; a block that gives up sets status[2] and frees its
-// tensor memory (results are then invalid and the host raises).
+// The ranges' sums never touch global memory, so the kernel needs no scratch.  Two or three blocks share an SM where the stages
+// allow it: one streams while another starts or drains.  Every wait for a copy or a product is bounded; a block that gives up
+// sets status[2], meets the others all the same and frees its tensor memory (results are then invalid and the host raises).  The
+// cluster's barriers and the allocation of tensor memory are not: they wait for blocks that always get there.
 #include "common.cuh"
 #include "tc_common.cuh"
 #include <math.h>
@@ -353,8 +354,8 @@ static int gr_launch(const CUtensorMap& xm, const CUtensorMap& wm, const GemmRow
 
 // How a product of `tiles` tiles of `slabs` slabs with bn tokens a pass is cut: ranges of K, blocks an SM, ring depth.
 //
-// Ranges: a block alone on an SM streams 45-75 GB/s (its stages are fetched, multiplied and drained one behind the other), so the
-// launch should have two blocks an SM or more; ranges of fewer than four slabs cost more in their sum than they bring.  [24,576 x 4,096]
+// Ranges: a block alone on an SM leaves the memory waiting (its stages are fetched, multiplied and drained one behind the other, and it starts and
+// ends alone), so the launch should have two blocks an SM or more; ranges of fewer than four slabs cost more in their sum than they bring.  [24,576 x 4,096]
 // gated, 48 rows: 1 range 38.7-41.0 us, 2 ranges 36.5, 4 ranges 43.0; [6,144 x 1,024] gated, 16 rows: 7.9 / 5.9 / 5.7 us.
 // Blocks an SM: three where the shared memory allows it, two where they fill their last round better (32 experts of
 // [2,048 x 1,536], 700 tokens, four experts each: 512 blocks, two an SM 46.5 us, three 52.5; [3,072 x 2,048]: 768 blocks, 85.3 / 79.0).
@@ -449,7 +450,7 @@ MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void
     switch (mode) {
         case GR_PLAIN: return GR_GO(GR_PLAIN, __nv_bfloat16);
         case GR_SILU: return GR_GO(GR_SILU, __nv_bfloat16);
-        case GR_RELU: return GR_GO(GR_RELU, __nv_bfloat16);
+        case GR_RELU: return grouped ? MSGL_ERR_SIZE : gr_launch<GR_RELU, __nv_bfloat16, false>(xm, wm, p, tiles, 1, smem, stream);      // no experts with it
         default: return GR_GO(GR_CLAMPED, __nv_bfloat16);
     }
 #undef GR_GO

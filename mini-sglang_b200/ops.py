@@ -810,8 +810,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """y = x @ weight^T (+ bias); weight is [out, in] as stored in the checkpoint.
 
-    Up to SMALL_M_MAX bfloat16 rows go through this engine's weight-streaming kernel
-    (csrc/gemm_small_m.cu); everything else is the library GEMM."""
+    Up to SMALL_M_MAX bfloat16 rows go through this engine's weight-streaming kernel (csrc/gemm_small_m.cu), float32 results of
+    very many columns for a decode batch through its decode-batch kernel (csrc/gemm_rows.cu, `_rows_f32`); everything else is the
+    library GEMM unless MSGL_TC_GEMM or MSGL_TC_MID ask for the tiled kernels."""
     _need_cuda(x, weight, bias)
     if out_dtype == torch.float32 and x.dim() == 2 and _rows_f32(x.shape[0], weight.shape[0], x.shape[1], x.device):
         y = _gemm_rows(x, weight, bias, 0, torch.float32)
@@ -1650,7 +1651,8 @@ def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx:
                 extra_gate: Optional[torch.Tensor] = None) -> torch.Tensor:
     """-> float32 [T, H] = scale * sum_k wts[t, k] * down[e] (silu(gate[e] h_t) * (up[e] h_t)), e = idx[t, k], with the chosen
     experts' rows read straight from the stacked weights gate_up [E, 2, F, H] (an expert's gate, then its up) and down [E, H, F]:
-    for a few tokens.  limit > 0: the activation is g * sigmoid(1.702 g) * (u + 1) with g = min(gate, limit) and
+    for decode steps and a few tokens, in bfloat16 by the grouped decode-batch product but for very small experts
+    (`_experts_grouped`).  limit > 0: the activation is g * sigmoid(1.702 g) * (u + 1) with g = min(gate, limit) and
     u = clamp(up, -limit, limit).  extra float32 [T, H] (a shared expert's output) is added inside the sum, times
     extra_gate float32 [T] where given."""
     idx, wts = _expert_operands(h, gate_up, down, idx, wts, extra, extra_gate)
@@ -1675,7 +1677,8 @@ def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx:
 # a token, beside a shared one.  Against a warp per row and (token, choice) pair: 1 token 82 -> 66 us, 8 tokens 224 -> 106, 24 tokens
 # 528 -> 132, 128 tokens 2,516 -> 140.  Against the library's grouped product with the activation between: 300 tokens 230 -> 156,
 # 700 tokens 247 -> 184, 1,024 tokens (128 rows an expert) 267 -> 214; with 150 rows an expert its products take 178 us, the library's
-# 145: such tiles leave one block an SM.
+# 145: such tiles leave one block an SM.  Those are random choices; without the shared expert and the router, library / this kernel: 700
+# tokens, Zipf-distributed choices (exponent 1.2) 181 / 157, all tokens at the same four experts 92 / 107; 1,024 tokens 209 / 177 and 111 / 139.
 EXPERT_ROWS_MEAN_MAX = 128
 EXPERT_ROWS_MAX_PAIRS = 8192
 # Very small experts in decode steps: the two launches per pair are ahead of the grouped product's four until the pairs' weights add up.  Experts

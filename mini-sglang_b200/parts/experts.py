@@ -20,12 +20,14 @@ class RoutedExperts(FeedForward):
     weights are their s over the sum of those (+ 1e-20).  Expert: down_e (silu(gate_e x) * (up_e x)), no biases.  The output is
     the weighted sum of the chosen experts' outputs, in float32, times `out_scale`.
 
-    A few (token, choice) pairs - and every step that a CUDA graph replays - read the chosen experts' rows straight from the
-    stacked weights (two launches whatever the choice).  Many tokens are put in the order of their experts on the device; in
-    bfloat16 the library's grouped matrix product then runs every expert's gate/up rows in one launch and every down product in
-    another, with the experts' row ranges read on the device (rows of bfloat16, summed in float32); in float32, or where the
-    sizes are no multiples of 8, the host reads the experts' counts (one small copy) and runs one gate/up product with its
-    activation and one down product per expert that has tokens.  One kernel sums every token's rows with their weights.
+    In bfloat16 the tokens are put in the order of their experts on the device (one launch), and the decode-batch kernel runs
+    every expert's gate/up product with its activation in one launch and every down product in another: decode steps and a few
+    (token, choice) pairs with float32 results (`ops.experts_few`), prompt portions of up to 128 rows an expert in the mean with
+    rounded ones (`ops.experts_many`).  Larger portions go through the library's grouped matrix product, with the experts' row
+    ranges read on the device too (rows of bfloat16, summed in float32).  Very small experts in decode steps, float32, and sizes that
+    are no multiples of 8: a few pairs read the chosen experts' rows straight from the stacked weights (two launches whatever the
+    choice); for many the host reads the experts' counts (one small copy) and runs one gate/up product with its activation and
+    one down product per expert that has tokens.  One kernel sums every token's rows with their weights.
 
     params: hidden_size, intermediate_size, num_experts, top, groups, keep_groups, out_scale,
             names (router, correction, expert (with {e} for the expert's number), gate, up, down).
@@ -105,8 +107,8 @@ class SoftmaxExperts(FeedForward):
     experts' outputs in float32.  With `shared_size` > 0 a shared expert of the same form (sizes and limit of its own) runs
     for every token and is added, times sigmoid(wsg . x), one number per token that the router kernel makes beside its logits.
 
-    The launches are those of `routed_experts`: a few (token, choice) pairs and every CUDA-graph step stream the chosen
-    experts' rows; many tokens are put in the order of their experts for one grouped product each way.
+    The launches are those of `routed_experts`: in bfloat16 one grouped product each way for the tokens in the order of their
+    experts, else the chosen experts' rows for a few (token, choice) pairs and a loop over the experts for many.
 
     params: hidden_size, intermediate_size, limit, num_experts, top, shared_size, shared_limit,
             names (router, expert (with {e}), gate, up, down, shared, shared_gate).

@@ -91,3 +91,23 @@ def test_runs_of_crowded_experts(E, n_out, K, mode, crowd):
             # float32 sums of K products of size K^-1/2 (a few 1e-6) and one rounding of 2^-9
             assert bool(((got.double() - want).abs() <= 2e-5 * (1 + want.abs()) + 2.0 ** -8 * want.abs()).all()), (tokens, ranges)
     ops.check_kernel_status()
+
+
+@pytest.mark.parametrize("M", [9, 48, 49, 64, 65])
+@pytest.mark.parametrize("N,K,most", [(2 * 328, 136, 48), (2 * 1024, 1024, 64)])
+def test_gated_products_take_the_kernel_up_to_their_bound(M, N, K, most, monkeypatch):
+    """... and with it lose the rounding of gate and up: one rounding of the result is all that is left."""
+    from mini_sglang_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, b = torch.randn((M, K), generator=g, device=DEV).bfloat16(), torch.randn(N, generator=g, device=DEV).bfloat16()
+    w = (torch.randn((N, K), generator=g, device=DEV) * K ** -0.5).bfloat16()
+    taken, rows = [], ops._gemm_rows
+    monkeypatch.setattr(ops, "_gemm_rows", lambda *a: taken.append(rows(*a)) or taken[-1])
+    got = ops.linear_glu(x, w, b)
+    assert bool(taken) == (M <= most) and (not taken or got is taken[0])
+    if taken:
+        gate, up = (x.double() @ w.double().t() + b.double()).chunk(2, -1)
+        want = torch.nn.functional.silu(gate) * up
+        # float32 sums of K products of size K^-1/2 (a few 1e-6), times the other factor, and one rounding of 2^-9
+        assert bool(((got.double() - want).abs() <= 2e-5 * (1 + want.abs()) + 2.0 ** -8 * want.abs()).all())
+    ops.check_kernel_status()
