@@ -786,11 +786,23 @@ def tensor_maps() -> bool:
     return _tensor_maps
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def _observed(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether something looks on that a kernel called by address would slip past: tracing, a dispatch mode, vmap and its like, forward-mode
+    derivatives, a tensor of another class."""
+    return (type(x) not in _PLAIN or type(weight) not in _PLAIN or torch._C._len_torch_dispatch_stack() > 0
+            or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0
+            or torch._C._get_tracing_state() is not None)
+
+
 def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
     """x @ weight^T (mode 0) or its gated activation (1: SwiGLU, 2: ReGLU; bias [2I]) for at most 256 rows by the decode-batch kernel;
     None where it cannot run."""
     if not (0 < x.shape[0] <= 256 and _product_ok(x, weight, bias)
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
+            and not _observed(x, weight)
             and (x.stride(0) >= x.shape[1] or x.shape[0] == 1) and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and weight.shape[1] % 8 == 0):
         return None
     M, (N, K) = x.shape[0], weight.shape

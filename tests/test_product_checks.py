@@ -46,3 +46,29 @@ def test_calls_that_do_not_fit_raise(M, monkeypatch):
             with pytest.raises(RuntimeError):
                 call()
     ops.check_kernel_status()
+
+
+def test_calls_that_are_traced_mapped_or_differentiated_stay_with_the_library():
+    """The library product was traced and mapped over, and refused what it has no derivative for; a kernel called by address would slip past."""
+    import torch.autograd.forward_ad as forward_ad
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils.flop_counter import FlopCounterMode
+
+    from mini_sglang_b200 import ops
+    x, w = torch.zeros((16, 64), dtype=torch.bfloat16), torch.zeros((64, 64), dtype=torch.bfloat16)
+    seen = []
+
+    def call(t):
+        seen.append(ops._gemm_rows(t, w, None, 0, torch.float32))
+        return t + 1
+
+    torch.func.vmap(call)(x.expand(2, 16, 64).contiguous())
+    torch.func.jvp(call, (x,), (x,))
+    make_fx(call)(x)
+    torch.jit.trace(call, x, check_trace=False)
+    with forward_ad.dual_level():
+        call(forward_ad.make_dual(x, x))
+    with FlopCounterMode(display=False):
+        call(x)
+    assert seen == [None] * 6
+    assert not ops._observed(x, w) and not ops._observed(x, torch.nn.Parameter(w))
