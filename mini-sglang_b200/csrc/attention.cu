@@ -1607,7 +1607,9 @@ template <int D> static size_t f32_smem_bytes() {
 // times sigmoid(gate) where gates are given
 // ---------------------------------------------------------------------------------------
 // A warp takes one head of a run of `run` tokens: it looks the tokens' pieces up together and merges those that have more than one, four
-// elements of the head a lane.  Bound by latency: the piece weights, then the pieces themselves, all of a row's loads under way at once.
+// elements of the head a lane.  Bound by latency: the piece weights, then the pieces themselves, eight loads under way at once (what is left
+// of eight goes one by one: 32 heads, one token, 4 / 8 / 32 pieces 2.9 / 2.6 / 3.6 us, a block a row 2.1 / 2.9 / 5.9; groups of four and two
+// behind those of eight take 168 registers, 2.4 us for 4 pieces but 4.7 and not 3.7 for 64 tokens).
 // run = 1 where there are few rows (decode steps: the attention layer of 8 requests of 4,096 keys 58.9 us with a block a row and
 // scalar loads, 57.9 now); up to 32 in steps with prompt portions, most of whose tokens have nothing to merge and cost one look a
 // run (1,901 tokens x 32 heads of which 3 tokens are cut: 64 us with a block a row, and the attention layer 293.7 -> 236.9 us).
