@@ -1670,9 +1670,9 @@ def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx:
     idx, wts = _expert_operands(h, gate_up, down, idx, wts, extra, extra_gate)
     T, H = h.shape
     F, top = gate_up.shape[2], idx.shape[1]
-    done = _expert_products(h, gate_up, down, idx, limit, torch.float32) if _experts_grouped(T * top, F * H) else None
-    if done is not None:
-        return expert_combine(done[0], done[1], wts, scale, extra=extra, extra_gate=extra_gate)
+    out = _experts_by_rows(h, gate_up, down, idx, wts, scale, limit, extra, extra_gate, torch.float32) if _experts_grouped(T * top, F * H) else None
+    if out is not None:
+        return out
     act = torch.empty((T * top, F), dtype=h.dtype, device=h.device)
     out = torch.empty((T, H), dtype=torch.float32, device=h.device)
     code = _gated_lib().msgl_experts_few(_ptr(h), _rows_view(h, H, "h"), _ptr(gate_up), _ptr(down), _ptr(idx), _ptr(wts), top, H, F,
@@ -1722,32 +1722,36 @@ def expert_rows(h: torch.Tensor, idx: torch.Tensor, n_experts: int) -> Optional[
     return rows, place, ends
 
 
-def _expert_products(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, limit: float,
-                     out_dtype: torch.dtype) -> Optional[Tuple[torch.Tensor, torch.Tensor]]:
-    """Both products of the chosen experts, gate_up [E, 2, F, H] and down [E, H, F], with the activation of `experts_few` between them, on the
-    decode-batch kernel -> (y [T * top, H] in the order of the experts, place); None where it does not apply.  The ranges of K, and with them the
-    order of the sums, follow from the sizes: float32 results (decode steps) take those of a single token's step, so that a request's
-    tokens are the same in every batch, rounded ones those of a step that uses all experts."""
+def _experts_by_rows(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, scale: float, limit: float,
+                     extra: Optional[torch.Tensor], extra_gate: Optional[torch.Tensor], y_dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """The chosen experts, gate_up [E, 2, F, H] and down [E, H, F], on the decode-batch kernel: `expert_rows`, both products with the activation
+    between them, `expert_combine`; None where that does not apply.  The operands have been through `_expert_operands`.  The ranges of K, and
+    with them the order of the sums, follow from the sizes: float32 outputs of the experts (decode steps) take those of a single token's
+    step, so that a request's tokens are the same in every batch, rounded ones those of a step that uses all experts.  (One
+    function and three scratch tensors for the four launches: small eager steps wait for the host.)"""
     T, H = h.shape
     E, _, F, _ = gate_up.shape
-    P = T * idx.shape[1]
-    if h.dtype != torch.bfloat16 or H % 8 or F % 8 or P > EXPERT_ROWS_MEAN_MAX * E or gate_up.data_ptr() % 16 or down.data_ptr() % 16 or not tensor_maps():
+    top = idx.shape[1]
+    P = T * top
+    if h.dtype != torch.bfloat16 or H % 8 or F % 8 or P > EXPERT_ROWS_MEAN_MAX * E or P > EXPERT_ROWS_MAX_PAIRS or E > ROUTE_MAX_EXPERTS or \
+            h.stride(1) != 1 or h.stride(0) % 8 or (h.data_ptr() | gate_up.data_ptr() | down.data_ptr()) % 16 or not tensor_maps():
         return None
-    ordered = expert_rows(h, idx, E)
-    if ordered is None:
-        return None
-    rows, place, ends = ordered
-    act = torch.empty((P, F), dtype=h.dtype, device=h.device)
-    y = torch.empty((P, H), dtype=out_dtype, device=h.device)
-    status, ranges = _ptr(_status_tensor(h.device)), -1 if out_dtype == torch.float32 else 0
-    code = _lib().msgl_gemm_rows(_ptr(gate_up), _ptr(rows), None, _ptr(act), P, F, H, H, F, 3 if limit > 0 else 1, 0, float(limit), E, _ptr(ends), T, ranges, 0,
-                                 status, _stream())
+    dev = h.device
+    numbers, buf = torch.empty(P + E, dtype=torch.int32, device=dev), torch.empty(P * (H + F), dtype=torch.bfloat16, device=dev)
+    y, out = torch.empty(P * H, dtype=y_dtype, device=dev), torch.empty((T, H), dtype=torch.float32, device=dev)
+    place, rows, yp = numbers.data_ptr(), buf.data_ptr(), y.data_ptr()
+    ends, act = place + 4 * P, rows + 2 * P * H
+    f32, status, stream, lib, gated = int(y_dtype == torch.float32), _status_tensor(dev).data_ptr(), _stream(), _lib(), _gated_lib()
+    ranges = -1 if f32 else 0
+    _check(gated.msgl_expert_rows(h.data_ptr(), h.stride(0), idx.data_ptr(), P, top, E, H, rows, place, ends, _DT[torch.bfloat16], stream), "expert_rows")
+    code = lib.msgl_gemm_rows(gate_up.data_ptr(), rows, None, act, P, F, H, H, F, 3 if limit > 0 else 1, 0, float(limit), E, ends, T, ranges, 0, status, stream)
     if code == 2:             # no tensor map of this layout
         return None
     _check(code, "gemm_rows (experts)")
-    _check(_lib().msgl_gemm_rows(_ptr(down), _ptr(act), None, _ptr(y), P, H, F, F, H, 0, int(out_dtype == torch.float32), 0.0, E, _ptr(ends), T, ranges,
-                                 0, status, _stream()), "gemm_rows (experts)")
-    return y, place
+    _check(lib.msgl_gemm_rows(down.data_ptr(), act, None, yp, P, H, F, F, H, 0, f32, 0.0, E, ends, T, ranges, 0, status, stream), "gemm_rows (experts)")
+    _check(gated.msgl_expert_combine(yp, f32, place, wts.data_ptr(), top, H, float(scale), out.data_ptr(), T, _ptr(extra),
+                                     _ptr(extra_gate) if extra is not None else None, stream), "expert_combine")
+    return out
 
 
 def experts_many(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, scale: float = 1.0,
@@ -1755,8 +1759,7 @@ def experts_many(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx
     """`experts_few` for the tokens of a prompt portion (the experts' outputs are rounded to the activation type before they are
     summed): None where the decode-batch kernel does not apply or the library's grouped product is ahead."""
     idx, wts = _expert_operands(h, gate_up, down, idx, wts, extra, extra_gate)
-    done = _expert_products(h, gate_up, down, idx, limit, h.dtype)
-    return None if done is None else expert_combine(done[0], done[1], wts, scale, extra=extra, extra_gate=extra_gate)
+    return _experts_by_rows(h, gate_up, down, idx, wts, scale, limit, extra, extra_gate, h.dtype)
 
 
 def expert_order(idx: torch.Tensor, n_experts: int) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
