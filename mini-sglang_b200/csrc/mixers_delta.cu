@@ -18,12 +18,14 @@
 //                              (max, sum, weighted values) are joined, in the order of the pieces, with the sink
 //   delta_prep_kernel          unit-length q and k, beta and g of the gated delta rule from their projections, all tokens
 //   delta_rule_kernel          S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q per head, token by token
+//   delta_chunk_kernel, delta_chunk_scan_kernel   the same for runs of tokens, in chunks of 32
 //   side_gate_mul_kernel       gelu_tanh(gate) times a slice of a per-token table's row
 //
 // Scores, weights, norms, angles, decays, states and everything that enters the recurrence are float32 (angles: double);
 // T is the type of the activations between kernels (float or bfloat16).  Key chunks and pieces are anchored at absolute
 // positions, so the order of a position's sums does not depend on how the tokens were cut into steps.
 #include "common.cuh"
+#include "tc_common.cuh"
 #include <math.h>
 
 namespace {
@@ -1168,102 +1170,234 @@ __global__ void __launch_bounds__(DR_MANY_WARPS * 32) delta_rule_kernel(const De
 }
 
 // ---------------------------------------------------------------------------------------
-// The same recurrence for a run of tokens in chunks of DC_C (float32 throughout).  With the chunk's start state S0, its decays
-// multiplied up, P_t = g_1 ... g_t and D_ts = g_(s+1) ... g_t:
-//     u_t + sum_{s < t} beta_t D_ts (k_t . k_s) u_s = beta_t v_t - beta_t P_t S0^T k_t
-//     o_t = P_t S0^T q_t + sum_{s <= t} D_ts (q_t . k_s) u_s,      S <- P_C S0 + sum_s D_Cs k_s u_s^T
-// so u = U - W S0 with U and W from two forward substitutions that do not read the state.  delta_chunk_kernel makes U, W and the
-// weights M_ts = D_ts (q_t . k_s) of all chunks side by side; delta_chunk_scan_kernel walks a request's chunks in order with 16 columns
-// of one state a block: three small products a chunk from shared memory, the next chunk's operands on their way.
+// The same recurrence for a run of tokens in chunks of DC_C.  With the chunk's start state S0, its decays multiplied up, P_t = g_1 ... g_t and
+// D_ts = g_(s+1) ... g_t:
+//     x_t = beta_t (v_t - P_t S0^T k_t),     u_t + sum_{s < t} beta_t D_ts (k_t . k_s) u_s = x_t,     that is u = R x with R = (1 + L)^-1
+//     o_t = P_t S0^T q_t + sum_{s <= t} D_ts (q_t . k_s) u_s = P_t S0^T q_t + (M R x)_t
+//     S <- P_C S0 + sum_s D_Cs k_s u_s^T
+// R and M R [C][C] and the factors of a token do not read the state: delta_chunk_kernel makes them for all chunks side by side.
+// delta_chunk_scan_kernel walks a request's chunks in order with 16 columns of one state a block: S0^T k and S0^T q, then x, u and the new state.
 // The decays are products of the g themselves, not differences of sums of logarithms, which would lose digits where they are small.
 //
 // Token by token the walk is a chain (a product with the state, two rounds of shuffles, the update) of 0.37 us a token whatever the number of
-// SMs; a chunk of 32 tokens takes the blocks 2.8 us (8,000 tokens: 697 us).  32 tokens: a row of the weights is a warp's width, the substitution's
-// rows stay in a thread's registers and two blocks' stages fit an SM.
+// SMs.  32 tokens: a row of the weights is a warp's width, and two blocks of the walk fit an SM.
+//
+// The walk's products go to the tensor cores, every float32 operand as the sum of three bfloat16 parts, which hold all of its 24 bits.  Keys and queries
+// of bfloat16 activations need no parts: their rows go in as they came (one part, exactly) and the factors that make them unit vectors go to the other
+// operand or the sum, as in the Gram products of the first kernel; float32 activations come as three parts of the unit rows.
+// What the first kernel leaves is laid out chunk by chunk, rows at the pitch that the walk's shared memory has, tokens behind the request's
+// last one as zeros: a stage of the walk is a straight copy.
 // ---------------------------------------------------------------------------------------
 constexpr int DC_C = 32, DC_COLS = 16, DC_THREADS = 256;
-
-struct DeltaChunkParams {
-    const void* qkv; const float2* kq; const float4* sc;
-    float* W;                                    // [T][heads][d]
-    float* U;                                    // [T][heads][dv]
-    float* M;                                    // [T][heads][DC_C]: row t of its chunk's weights, zeros behind the diagonal
-    float2* ps;                                  // [T][heads]: P_t and D_Ct
-    float* K; float* Q;                          // [T][kv_heads][d]
-    float* state; const int* q_start; const int* slots; float* out;
-    int heads, kv_heads, dv, T, B, n_min;
+constexpr int DC_LDM = DC_C + 4;                 // pitch of the rows of R, M R and x
+template <typename T, int D> struct DcSizes {
+    static constexpr int PARTS = sizeof(T) == 2 ? 1 : 3;         // bfloat16 parts of a key or query row
+    static constexpr int LDK = D + 8;            // pitch of such a row: ldmatrix's eight rows fall on different banks
+    static constexpr int KQ = PARTS * DC_C * LDK * 2, M = DC_C * DC_LDM * 4;         // bytes of a chunk's keys (queries) and of R (M R)
 };
 
-// A block makes one head's chunk.  Latency decides (loads, 32 steps of the decays, the substitution's chain), so three blocks share an SM: with the
-// substitution's factors kept in registers (255 a thread, one block an SM) and the heads of a q/k head in one block it took 116 us
-// for 1,411 tokens of 16 heads.
+struct DeltaChunkParams {
+    const void* qkv; const void* proj; long long proj_stride; int a_off, b_off;
+    const float* a_log; const float* dt_bias;
+    unsigned char* K; unsigned char* Q;          // [chunk][kv_heads]: keys, queries [PARTS][C][LDK] bfloat16
+    // [chunk][heads]: R, M R [C][LDM] float32, zeros behind the diagonal.  Behind row t of R: beta_t, beta_t P_t |k_t|^-1, D_Ct |k_t|^-1, P_t |q_t|^-1 d^-1/2 (the
+    // norms of rows that are not unit rows yet); behind the first row of M R: P of the chunk's last token
+    unsigned char* R; unsigned char* M;
+    float* state; const int* q_start; const int* slots; float* out;
+    int* status;                                 // word 1: a copy did not arrive
+    int heads, kv_heads, dv, B, n_min;
+};
+
+namespace {
+__device__ __forceinline__ void dc_ldmatrix4(unsigned (&r)[4], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void dc_ldmatrix4t(unsigned (&r)[4], const void* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void dc_mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// the next bfloat16 part of two floats, taken off them: cut off or (ROUND) rounded; three parts hold all 24 bits either way, rounded ones fall off faster
+template <bool ROUND> __device__ __forceinline__ unsigned dc_part(float& x, float& y) {
+    if (!ROUND) {
+        const unsigned a = __float_as_uint(x), b = __float_as_uint(y);
+        x -= __uint_as_float(a & 0xffff0000u); y -= __uint_as_float(b & 0xffff0000u);
+        return __byte_perm(a, b, 0x7632);
+    }
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    const unsigned u = *reinterpret_cast<const unsigned*>(&h);
+    x -= __uint_as_float(u << 16); y -= __uint_as_float(u & 0xffff0000u);
+    return u;
+}
+// 8 elements of a row
+__device__ __forceinline__ void dc_load8(const float* p, float* o) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+}
+__device__ __forceinline__ void dc_load8(const __nv_bfloat16* p, float* o) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    const unsigned u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { o[2 * i] = __uint_as_float(u[i] << 16); o[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
+}
+__device__ __forceinline__ float4 dc_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 dc_load4(const __nv_bfloat16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
+// the request and the place in it of the `left`-th chunk of the requests with n_min tokens or more (one warp); at < 0: there is none
+__device__ __forceinline__ void dc_find(const int* q_start, int B, int n_min, int left, int& at, int& rest) {
+    const int lane = threadIdx.x & 31;
+    at = -1; rest = 0;
+    for (int r0 = 0; r0 < B && at < 0; r0 += 32) {
+        const int r = r0 + lane;
+        const int n = r < B ? q_start[r + 1] - q_start[r] : 0;
+        const int c = n >= n_min ? (n + DC_C - 1) / DC_C : 0;
+        int sum = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
+        const unsigned hit = __ballot_sync(0xffffffffu, left < sum);
+        if (hit) {
+            const int l = __ffs(hit) - 1;
+            at = r0 + l;
+            rest = left - __shfl_sync(0xffffffffu, sum - c, l);
+        }
+        left -= __shfl_sync(0xffffffffu, sum, 31);
+    }
+}
+}  // namespace
+
+template <typename T, int D> struct DcPrep {     // shared memory of delta_chunk_kernel, in bytes
+    using Z = DcSizes<T, D>;
+    static constexpr int LDF = D + 4;            // pitch of float32 rows: 16 bytes apart in the banks
+    static constexpr int KS = 0, QS = KS + (Z::PARTS == 1 ? DC_C * Z::LDK * 2 : DC_C * LDF * 4), KK = 2 * QS, QK = KK + DC_C * (DC_C + 1) * 4,
+                         LS = QK + DC_C * (DC_C + 1) * 4, RS = LS + DC_C * DC_LDM * 4, TMP = RS + DC_C * DC_LDM * 4, TOTAL = TMP + 16 * 17 * 4;
+};
+
+// A block makes one head's chunk.  Latency decides, so several blocks share an SM.  R by halves: its two diagonal blocks of 16 rows by substitution, a lane a column of
+// one of them, then R_21 = -R_22 L_21 R_11.  1,411 tokens of 16 heads: 15 us; with unit rows from a launch ahead (7.5 us), Gram products in multiply-adds and a
+// substitution of all of beta v and beta P K (256 columns a head) it took 43.
 template <typename T, int D>
-__global__ void __launch_bounds__(DC_THREADS, 3) delta_chunk_kernel(const DeltaChunkParams p) {
-    constexpr int LD = D + 4;                    // rows 16 bytes apart in the banks
+__global__ void __launch_bounds__(DC_THREADS, 4) delta_chunk_kernel(const DeltaChunkParams p) {
+    using Z = DcSizes<T, D>;
+    using Sm = DcPrep<T, D>;
+    constexpr int LDK = Z::LDK, LDF = Sm::LDF;
+    constexpr bool RAW = Z::PARTS == 1;
+    static_assert(D == 128 && DC_C == 32, "eight threads a row, two halves of 16");
     extern __shared__ __align__(16) unsigned char dc_smem[];
-    float* Ks = reinterpret_cast<float*>(dc_smem);           // [C][LD]
-    float* Qs = Ks + DC_C * LD;                              // [C][LD]
-    float* KK = Qs + DC_C * LD;                              // [C][C + 1]
-    float* QK = KK + DC_C * (DC_C + 1);                      // [C][C + 1]
-    float* Ls = QK + DC_C * (DC_C + 1);                      // [C][C], 16-byte rows
-    float* Ms = Ls + DC_C * DC_C;                            // [C][C]
-    __shared__ float beta_s[DC_C], g_s[DC_C], pre_s[DC_C], suf_s[DC_C];
+    float* Ks = reinterpret_cast<float*>(dc_smem + Sm::KS);              // float32: [C][LDF] unit keys, queries
+    float* Qs = reinterpret_cast<float*>(dc_smem + Sm::QS);
+    __nv_bfloat16* Kr = reinterpret_cast<__nv_bfloat16*>(dc_smem + Sm::KS);      // bfloat16: [2 C][LDK] rows as they came, keys then queries
+    float* KK = reinterpret_cast<float*>(dc_smem + Sm::KK);              // [C][C + 1]
+    float* QK = reinterpret_cast<float*>(dc_smem + Sm::QK);              // then M, in place
+    float* Ls = reinterpret_cast<float*>(dc_smem + Sm::LS);              // [C][LDM]
+    float* Rs = reinterpret_cast<float*>(dc_smem + Sm::RS);              // [C][LDM]
+    float* tmp = reinterpret_cast<float*>(dc_smem + Sm::TMP);            // [16][17]
+    __shared__ float beta_s[DC_C], g_s[DC_C], pre_s[DC_C], suf_s[DC_C], rk_s[DC_C], rq_s[DC_C];
     __shared__ int where_s[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, per = p.heads / p.kv_heads, g = h / per;
-    if (warp == 0) {                             // the blockIdx.x-th chunk of the requests that are taken, 32 requests a look
-        int left = blockIdx.x, at = -1, rest = 0;
-        for (int r0 = 0; r0 < p.B && at < 0; r0 += 32) {
-            const int r = r0 + lane;
-            const int n = r < p.B ? p.q_start[r + 1] - p.q_start[r] : 0;
-            const int c = n >= p.n_min ? (n + DC_C - 1) / DC_C : 0;
-            int sum = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
-            const unsigned hit = __ballot_sync(0xffffffffu, left < sum);
-            if (hit) {
-                const int l = __ffs(hit) - 1;
-                at = r0 + l;
-                rest = left - __shfl_sync(0xffffffffu, sum - c, l);
-            }
-            left -= __shfl_sync(0xffffffffu, sum, 31);
-        }
+    if (warp == 0) {
+        int at, rest;
+        dc_find(p.q_start, p.B, p.n_min, blockIdx.x, at, rest);
         if (lane == 0) { where_s[0] = at; where_s[1] = rest; }
     }
     __syncthreads();
     if (where_s[0] < 0) return;
     const int r = where_s[0], base = p.q_start[r] + where_s[1] * DC_C, nb = min(DC_C, p.q_start[r + 1] - base);
-    const bool first = h == g * per;             // this head's block leaves k and q for the walk
-#pragma unroll 4
-    for (int i = tid; i < DC_C * D / 2; i += DC_THREADS) {
-        const int t = i / (D / 2), e = 2 * (i - t * (D / 2));
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool first = h == g * per;             // this head's block leaves keys and queries for the walk
+    const int Ck = p.kv_heads * D, Wd = 2 * Ck + p.heads * p.dv;
+    const T* qkv = reinterpret_cast<const T*>(p.qkv) + (size_t)base * Wd;
+    const size_t chunk_h = (size_t)blockIdx.x * p.heads + h, chunk_g = (size_t)blockIdx.x * p.kv_heads + g;
+    {   // a row's eight threads take elements 8 j .. and 64 + 8 j ..
+        const int t = tid >> 3, j = tid & 7;
+        float k[16] = {}, q[16] = {};
         if (t < nb) {
-            const size_t at = ((size_t)(base + t) * p.kv_heads + g) * D + e;
-            v = *reinterpret_cast<const float4*>(p.kq + at);
-            if (first) {
-                *reinterpret_cast<float2*>(p.K + at) = make_float2(v.x, v.z);
-                *reinterpret_cast<float2*>(p.Q + at) = make_float2(v.y, v.w);
+            const T* rowq = qkv + (size_t)t * Wd + (size_t)g * D + 8 * j;
+            dc_load8(rowq, q); dc_load8(rowq + 64, q + 8); dc_load8(rowq + Ck, k); dc_load8(rowq + Ck + 64, k + 8);
+        }
+        if (tid < DC_C) {
+            float beta = 0.f, gt = 1.f;
+            if (tid < nb) {
+                const T* proj = reinterpret_cast<const T*>(p.proj) + (size_t)(base + tid) * p.proj_stride;
+                beta = sigmoidf_(to_f32<T>(proj[p.b_off + h]));
+                gt = expf(-expf(p.a_log[h]) * softplusf_(to_f32<T>(proj[p.a_off + h]) + p.dt_bias[h]));
+            }
+            beta_s[tid] = beta; g_s[tid] = gt;
+        }
+        float sq = 0.f, sk = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { sq = fmaf(q[i], q[i], sq); sk = fmaf(k[i], k[i], sk); }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) { sq += __shfl_xor_sync(0xffffffffu, sq, o); sk += __shfl_xor_sync(0xffffffffu, sk, o); }
+        const float rq = (1.f / sqrtf((float)D)) / sqrtf(sq + 1e-6f), rk = 1.f / sqrtf(sk + 1e-6f);
+        if (j == 0) { rk_s[t] = rk; rq_s[t] = rq; }
+        unsigned char* kq[2] = {p.K + chunk_g * Z::KQ, p.Q + chunk_g * Z::KQ};
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+            float* v = which ? q : k;
+            const float unit = which ? rq : rk;
+            if (!RAW || unit == 0.f) {           // a norm beyond float32: zeros either way (an infinity: not a number)
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] *= unit;
+            }
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int e = 64 * half + 8 * j;
+                if (!RAW) {
+                    float* dst = (which ? Qs : Ks) + t * LDF + e;
+                    *reinterpret_cast<float4*>(dst) = make_float4(v[8 * half], v[8 * half + 1], v[8 * half + 2], v[8 * half + 3]);
+                    *reinterpret_cast<float4*>(dst + 4) = make_float4(v[8 * half + 4], v[8 * half + 5], v[8 * half + 6], v[8 * half + 7]);
+                }
+#pragma unroll
+                for (int part = 0; part < Z::PARTS; ++part) {
+                    unsigned u[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) u[i] = dc_part<true>(v[8 * half + 2 * i], v[8 * half + 2 * i + 1]);
+                    const uint4 w = make_uint4(u[0], u[1], u[2], u[3]);
+                    if (RAW) *reinterpret_cast<uint4*>(Kr + (which * DC_C + t) * LDK + e) = w;
+                    if (first) *reinterpret_cast<uint4*>(kq[which] + ((part * DC_C + t) * LDK + e) * 2) = w;
+                }
             }
         }
-        *reinterpret_cast<float2*>(Ks + t * LD + e) = make_float2(v.x, v.z);
-        *reinterpret_cast<float2*>(Qs + t * LD + e) = make_float2(v.y, v.w);
-    }
-    if (tid < DC_C) {
-        const float4 c = tid < nb ? p.sc[(size_t)(base + tid) * p.heads + h] : make_float4(0.f, 1.f, 0.f, 0.f);
-        beta_s[tid] = c.x; g_s[tid] = c.y;
     }
     __syncthreads();
-    {   // k_t . k_s and q_t . k_s: rows ti, ti + 16 against columns tj, tj + 16
+    if constexpr (RAW) {                         // warp: 16 rows (of k or q) against 16 keys
+        float acc[4][2][4] = {};                 // four sums each: less rounding than one over all of D
+        const int m0 = (warp >> 1) * 16, n0 = (warp & 1) * 16;
+        const __nv_bfloat16* ap = Kr + (m0 + (lane & 15)) * LDK + (lane >> 4) * 8;
+        const __nv_bfloat16* bp = Kr + (n0 + (lane & 7) + (lane >> 4) * 8) * LDK + ((lane >> 3) & 1) * 8;
+#pragma unroll
+        for (int e = 0; e < D; e += 16) {
+            unsigned a[4], b[4];
+            dc_ldmatrix4(a, ap + e);
+            dc_ldmatrix4(b, bp + e);
+            dc_mma(acc[e / 16 % 4][0], a, b[0], b[1]);
+            dc_mma(acc[e / 16 % 4][1], a, b[2], b[3]);
+        }
+        float* dst = warp < 4 ? KK : QK;
+        const float* rr = warp < 4 ? rk_s : rq_s;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int row = (m0 & 16) + (lane >> 2) + ((i >> 1) & 1) * 8, col = n0 + (i >> 2) * 8 + (lane & 3) * 2 + (i & 1);
+            const float sum = (acc[0][i >> 2][i & 3] + acc[1][i >> 2][i & 3]) + (acc[2][i >> 2][i & 3] + acc[3][i >> 2][i & 3]);
+            dst[row * (DC_C + 1) + col] = sum * rr[row] * rk_s[col];
+        }
+    } else {
+        // k_t . k_s and q_t . k_s: rows ti, ti + 16 against columns tj, tj + 16
         const int ti = tid >> 4, tj = tid & 15;
         float kk[2][2][4] = {}, qk[2][2][4] = {};            // four partial sums each: less rounding than one over all of D
-#pragma unroll 2
+#pragma unroll 1
         for (int e = 0; e < D; e += 4) {
             float4 kt[2], qt[2], ks[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                kt[i] = *reinterpret_cast<const float4*>(Ks + (ti + 16 * i) * LD + e);
-                qt[i] = *reinterpret_cast<const float4*>(Qs + (ti + 16 * i) * LD + e);
-                ks[i] = *reinterpret_cast<const float4*>(Ks + (tj + 16 * i) * LD + e);
+                kt[i] = *reinterpret_cast<const float4*>(Ks + (ti + 16 * i) * LDF + e);
+                qt[i] = *reinterpret_cast<const float4*>(Qs + (ti + 16 * i) * LDF + e);
+                ks[i] = *reinterpret_cast<const float4*>(Ks + (tj + 16 * i) * LDF + e);
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i)
@@ -1284,275 +1418,378 @@ __global__ void __launch_bounds__(DC_THREADS, 3) delta_chunk_kernel(const DeltaC
                 QK[at] = (qk[i][j][0] + qk[i][j][1]) + (qk[i][j][2] + qk[i][j][3]);
             }
     }
-    const int Ck = p.kv_heads * D, Wd = 2 * Ck + p.heads * p.dv;
-    const T* qkv = reinterpret_cast<const T*>(p.qkv);
     __syncthreads();
-    if (tid < DC_C) {                            // column s = tid: the decays from s on
-        const int s = tid;
+    {   // column s = lane: the decays from s on; a warp takes four rows
+        const int s = lane, t_first = 4 * warp;
         float run = 1.f;
-        for (int t = 0; t < DC_C; ++t) {
+        for (int t = 1; t < t_first; ++t) run *= t > s ? g_s[t] : 1.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = t_first + i, at = t * (DC_C + 1) + s;
             if (t > s) run *= g_s[t];
-            Ls[t * DC_C + s] = t > s ? beta_s[t] * run * KK[t * (DC_C + 1) + s] : 0.f;
-            Ms[t * DC_C + s] = t >= s ? run * QK[t * (DC_C + 1) + s] : 0.f;
+            Ls[t * DC_LDM + s] = t > s ? beta_s[t] * run * KK[at] : 0.f;
+            QK[at] = t >= s ? run * QK[at] : 0.f;
             if (s == 0) pre_s[t] = g_s[0] * run;
             if (t == nb - 1) suf_s[s] = run;
         }
     }
     __syncthreads();
-    for (int i = tid; i < nb * DC_C; i += DC_THREADS) p.M[((size_t)(base + i / DC_C) * p.heads + h) * DC_C + i % DC_C] = Ms[i];
-    if (tid < nb) p.ps[(size_t)(base + tid) * p.heads + h] = make_float2(pre_s[tid], suf_s[tid]);
-    for (int c = tid; c < p.dv + D; c += DC_THREADS) {
-        const bool is_u = c < p.dv;
-        float x[DC_C];
-        if (is_u) {              // all loads under way at once; rows behind the last token repeat it and are not used (their beta is 0)
-            const T* src = qkv + (size_t)base * Wd + 2 * Ck + (size_t)h * p.dv + c;
-            T raw[DC_C];
+    if (warp == 0) {                             // R_11 and R_22: half-warp b, column j of the block at b0; rows one after the other
+        const int b0 = lane & 16, j = lane & 15;
+        float x[16];
 #pragma unroll
-            for (int t = 0; t < DC_C; ++t) raw[t] = src[(size_t)min(t, nb - 1) * Wd];
+        for (int i = 0; i < 16; ++i) {
+            float a = i == j ? 1.f : 0.f, a1 = 0.f;
 #pragma unroll
-            for (int t = 0; t < DC_C; ++t) x[t] = to_f32<T>(raw[t]);
-        } else {
-#pragma unroll
-            for (int t = 0; t < DC_C; ++t) x[t] = pre_s[t] * Ks[t * LD + c - p.dv];
-        }
-        float* dst = is_u ? p.U + ((size_t)base * p.heads + h) * p.dv + c : p.W + ((size_t)base * p.heads + h) * D + (c - p.dv);
-        const size_t step = (size_t)p.heads * (is_u ? p.dv : D);
-#pragma unroll
-        for (int t = 0; t < DC_C; ++t) {
-            float a0 = beta_s[t] * x[t], a1 = 0.f;
-#pragma unroll
-            for (int s4 = 0; s4 < t; s4 += 4) {
-                const float4 l = *reinterpret_cast<const float4*>(Ls + t * DC_C + s4);
-                a0 = fmaf(-l.x, x[s4], a0);
-                if (s4 + 1 < t) a1 = fmaf(-l.y, x[s4 + 1], a1);
-                if (s4 + 2 < t) a0 = fmaf(-l.z, x[s4 + 2], a0);
-                if (s4 + 3 < t) a1 = fmaf(-l.w, x[s4 + 3], a1);
+            for (int s = 0; s < i; ++s) {
+                const float l = Ls[(b0 + i) * DC_LDM + b0 + s];
+                if (s & 1) a1 = fmaf(-l, x[s], a1); else a = fmaf(-l, x[s], a);
             }
-            x[t] = a0 + a1;
-            if (t < nb) dst[t * step] = x[t];
-            if (t % 4 == 3) asm volatile("" ::: "memory");       // the next rows' factors are read here, not all at the start into 255 registers
+            x[i] = a + a1;
+            Rs[(b0 + i) * DC_LDM + b0 + j] = x[i];
         }
+    } else if (warp == 1) {                      // the factors of the tokens
+        const int t = lane;
+        const float rk = RAW ? rk_s[t] : 1.f, rq = RAW ? rq_s[t] : 1.f, beta = beta_s[t];
+        const bool in = t < nb;
+        *reinterpret_cast<float4*>(p.R + chunk_h * Z::M + (t * DC_LDM + DC_C) * 4) =
+            in ? make_float4(beta, beta * pre_s[t] * rk, suf_s[t] * rk, pre_s[t] * rq) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t == 0) *reinterpret_cast<float*>(p.M + chunk_h * Z::M + DC_C * 4) = pre_s[nb - 1];
+    } else if (tid >= 128) {
+        const int i = (tid - 128) >> 3, j = (tid & 7) * 2;                   // R_12 = 0
+        *reinterpret_cast<float2*>(Rs + i * DC_LDM + 16 + j) = make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    const int ri = tid >> 4, rj = tid & 15;
+    {   // L_21 R_11 (columns of R_11 begin at its diagonal)
+        float a = 0.f, a1 = 0.f;
+#pragma unroll
+        for (int s = 0; s < 16; s += 2) {
+            a = fmaf(Ls[(16 + ri) * DC_LDM + s], s >= rj ? Rs[s * DC_LDM + rj] : 0.f, a);
+            a1 = fmaf(Ls[(16 + ri) * DC_LDM + s + 1], s + 1 >= rj ? Rs[(s + 1) * DC_LDM + rj] : 0.f, a1);
+        }
+        tmp[ri * 17 + rj] = a + a1;
+    }
+    __syncthreads();
+    {
+        float a = 0.f, a1 = 0.f;
+#pragma unroll
+        for (int s = 0; s < 16; s += 2) {
+            a = fmaf(s <= ri ? Rs[(16 + ri) * DC_LDM + 16 + s] : 0.f, tmp[s * 17 + rj], a);
+            a1 = fmaf(s + 1 <= ri ? Rs[(16 + ri) * DC_LDM + 17 + s] : 0.f, tmp[(s + 1) * 17 + rj], a1);
+        }
+        Rs[(16 + ri) * DC_LDM + rj] = -(a + a1);
+    }
+    __syncthreads();
+    float* Rg = reinterpret_cast<float*>(p.R + chunk_h * Z::M);
+    float* Mg = reinterpret_cast<float*>(p.M + chunk_h * Z::M);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {                // M R, row 8 i + warp, column lane
+        const int t = 8 * i + warp;
+        float a = 0.f, a1 = 0.f;
+#pragma unroll 8
+        for (int s = 0; s <= t; s += 2) {        // (behind the diagonal both are zeros)
+            a = fmaf(QK[t * (DC_C + 1) + s], Rs[s * DC_LDM + lane], a);
+            a1 = fmaf(QK[t * (DC_C + 1) + s + 1], Rs[(s + 1) * DC_LDM + lane], a1);
+        }
+        Mg[t * DC_LDM + lane] = a + a1;
+        Rg[t * DC_LDM + lane] = Rs[t * DC_LDM + lane];
     }
 }
 
-// Shared memory of a block of the walk, in floats: W, Q and the decays of two chunks (the next one's on their way), K, M and U of the chunk under way
-// (asked for at its start), the state's columns, u.  104 KB: two blocks an SM.
-template <int D> struct DcStage {
-    static constexpr int LD = D + 4, LDM = DC_C + 4;
-    static constexpr int W = 0, Q = W + DC_C * LD, PS = Q + DC_C * LD, SIZE = PS + 2 * DC_C;
-    static constexpr int K = 2 * SIZE, M = K + DC_C * LD, U = M + DC_C * LDM, S = U + DC_C * DC_COLS, US = S + D * DC_COLS + D, UDS = US + DC_C * DC_COLS;
-    static constexpr int TOTAL = UDS + DC_C * DC_COLS;
-    static_assert(DC_C * LD >= 4 * 2 * DC_C * DC_COLS, "the partial sums lie over W");
+// Shared memory of a block of the walk, in bytes: keys, queries and R of two chunks (the next one's on their way), M R of three (read last), the walkers'
+// partial sums of K S and Q S, x, u in three bfloat16 parts.  100 KB for bfloat16 activations: two blocks an SM.
+template <typename T, int D> struct DcStage {
+    using Z = DcSizes<T, D>;
+    static constexpr int K = 0, Q = K + Z::KQ, R = Q + Z::KQ, SIZE = R + Z::M;
+    static constexpr int LDP = D + 8, LDU = DC_COLS + 8, PLANE = DC_C * LDU;
+    static constexpr int M = 2 * SIZE, PK = M + 3 * Z::M, PQ = PK + DC_C * LDP * 4, XS = PQ + DC_C * LDP * 4, UP = XS + DC_COLS * DC_LDM * 4,
+                         BAR = UP + 3 * PLANE * 2, TOTAL = BAR + 16;
 };
+constexpr int DC_WALKERS = 256, DC_READERS = 128;
 
-template <int D>
-__global__ void __launch_bounds__(DC_THREADS, 2) delta_chunk_scan_kernel(const DeltaChunkParams p) {
-    static_assert(D == 128, "the update's layout is that of 128 rows");
-    using St = DcStage<D>;
-    constexpr int LD = St::LD, LDM = St::LDM, KS = D / 4;      // KS: a quarter of the state's rows
+// Two groups of warps.  The eight walkers carry the state from chunk to chunk, 16 of its rows each, in registers: partial sums of K S and Q S over their rows,
+// then S <- P_C S + K^T (D u).  The four readers add the partial sums up, make x and u for the walkers and, while those go on, the outputs.
+//
+// The state lies in the accumulators' layout with its columns as rows, which is the layout of the other operand of K S and Q S, so it never goes through shared
+// memory.  R x and M R x stay float32 multiply-adds over the tokens up to t only: a later token's infinity must not reach back (0 times infinity).
+//
+// Bound by the chain of a chunk (split, products, sums, R x, split, products): 1.7 us a chunk with one block an SM, 68 us for 1,111 + 300 tokens of 16 heads.  All
+// products in multiply-adds were bound by their reads of shared memory (16 columns a block leave no room for more than 4 x 4 results a thread), 2.8-3.4 us
+// a chunk, 121 us; tensor cores with W = R (beta P K) and U = R (beta v) from the first kernel in place of R, three times the copies and twice the
+// products, took 85.  Errors against 64 bits there: outputs 2.0e-7 (multiply-adds 2.4e-7), states 1.8e-7 (2.0e-7).
+//
+// Named barriers (each side meets the other once a chunk, in turn): 1 the first chunk, 3 partial sums of K S, 4 u, 5 partial sums of Q S, 6 Q S read.
+template <typename T, int D>
+__global__ void __launch_bounds__(DC_WALKERS + DC_READERS, DcSizes<T, D>::PARTS == 1 ? 2 : 1) delta_chunk_scan_kernel(const DeltaChunkParams p) {
+    static_assert(D == 128 && DC_C == 32 && DC_COLS == 16, "eight walkers of 16 rows");
+    using St = DcStage<T, D>;
+    using Z = DcSizes<T, D>;
+    constexpr int LDK = Z::LDK, LDP = St::LDP, LDU = St::LDU, PARTS = Z::PARTS;
     extern __shared__ __align__(16) unsigned char dc_smem[];
-    float* sm = reinterpret_cast<float*>(dc_smem);
-    float* Ss = sm + St::S;                                  // [D][16], four floats more behind every four rows (a quarter-warp writes rows 4 apart)
-    auto s_at = [](int row, int col) { return row * DC_COLS + (row >> 2) * 4 + col; };
-    float* us = sm + St::US;                                 // [C][16] u
-    float* uds = sm + St::UDS;                               // [C][16] u, decayed to the chunk's end
+    float* PK = reinterpret_cast<float*>(dc_smem + St::PK);                         // [C][LDP]: walker w's sums at 16 w
+    float* PQ = reinterpret_cast<float*>(dc_smem + St::PQ);
+    __nv_bfloat16* up = reinterpret_cast<__nv_bfloat16*>(dc_smem + St::UP);         // [3][C][LDU]
+    __shared__ int first_s;
     const int h = blockIdx.x, c0 = blockIdx.y * DC_COLS, r = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int t0 = p.q_start[r], n = p.q_start[r + 1] - t0;
     if (n < p.n_min) return;
-    const int g = h / (p.heads / p.kv_heads), dv = p.dv;
-    float* S = p.state + ((size_t)p.slots[r] * p.heads + h) * D * dv + c0;
-
-    // the state entries this thread keeps: rows row0 .. row0 + 3, columns col0, col0 + 1
-    const int dl = lane & 7, b3 = (lane >> 3) & 1, b4 = lane >> 4;
-    const int row0 = (warp >> 2) * 64 + b4 * 32 + 4 * dl, col0 = (warp & 3) * 4 + 2 * b3;
-    float s_reg[4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        s_reg[i][0] = S[(size_t)(row0 + i) * dv + col0];
-        s_reg[i][1] = S[(size_t)(row0 + i) * dv + col0 + 1];
-        *reinterpret_cast<float2*>(Ss + s_at(row0 + i, col0)) = make_float2(s_reg[i][0], s_reg[i][1]);
+    const int g = h / (p.heads / p.kv_heads), dv = p.dv, n_chunks = (n + DC_C - 1) / DC_C;
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(dc_smem + St::BAR);     // a barrier a stage
+    if (warp == 0) {                                         // chunks of the requests before this one
+        int sum = 0;
+        for (int i = lane; i < r; i += 32) {
+            const int m = p.q_start[i + 1] - p.q_start[i];
+            sum += m >= p.n_min ? (m + DC_C - 1) / DC_C : 0;
+        }
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0) {
+            first_s = sum;
+            tc_mbar_init(bar, 1); tc_mbar_init(bar + 8u, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        }
     }
-    auto copy16 = [&](float* dst, const float* src, bool valid) {        // 16 bytes, zeros behind the request's last token
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0));
+    __syncthreads();
+    const size_t first = (size_t)first_s;
+    auto wait = [&](int c) {                                 // for the operands of chunk c: one thread, the others meet it at a barrier
+        if (!tc_mbar_wait(bar + 8u * (c & 1), (unsigned)(c >> 1) & 1u)) atomicExch(p.status + 1, 1);
     };
-    constexpr int V = D / 4;
-    auto fetch_ahead = [&](int st, int b0) {                 // W, Q and the decays of the chunk at b0
-        float* sp = sm + st * St::SIZE;
-        const int nb = min(DC_C, n - b0);
-        for (int i = tid; i < DC_C * V; i += DC_THREADS) {
-            const int t = i / V, e = (i - t * V) * 4;
-            const bool ok = t < nb;
-            const size_t tok = (size_t)(t0 + b0 + (ok ? t : 0));
-            copy16(sp + St::W + t * LD + e, p.W + (tok * p.heads + h) * D + e, ok);
-            copy16(sp + St::Q + t * LD + e, p.Q + (tok * p.kv_heads + g) * D + e, ok);
+
+    if (tid < DC_WALKERS) {
+        const int gr = lane >> 2, gt = 2 * (lane & 3), k0 = 16 * warp;
+        // s[j]: rows k0 + 8 j + gt and the next, columns gr (entries 0, 1) and gr + 8 (2, 3)
+        float* S = p.state + ((size_t)p.slots[r] * p.heads + h) * D * dv + c0;
+        auto copy = [&](int dst, const unsigned char* src, int bytes, unsigned b) {
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                         ::"r"((unsigned)__cvta_generic_to_shared(dc_smem + dst)), "l"(src), "r"(bytes), "r"(b) : "memory");
+        };
+        auto fetch = [&](int c) {
+            const int st = (c & 1) * St::SIZE;
+            const unsigned b = bar + 8u * (c & 1);
+            const size_t ch = (first + c) * p.heads + h, cg = (first + c) * p.kv_heads + g;
+            tc_mbar_expect_tx(b, 2 * Z::KQ + 2 * Z::M);
+            copy(st + St::K, p.K + cg * Z::KQ, Z::KQ, b);
+            copy(st + St::Q, p.Q + cg * Z::KQ, Z::KQ, b);
+            copy(st + St::R, p.R + ch * Z::M, Z::M, b);
+            copy(St::M + (c % 3) * Z::M, p.M + ch * Z::M, Z::M, b);
+        };
+        if (tid == 0) {
+            fetch(0);
+            if (n_chunks > 1) fetch(1);
+            wait(0);
         }
-        if (tid < DC_C) {
-            const bool ok = tid < nb;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(sp + St::PS + 2 * tid)),
-                         "l"(p.ps + (size_t)(t0 + b0 + (ok ? tid : 0)) * p.heads + h), "r"(ok ? 8 : 0));
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-    };
-    auto fetch_now = [&](int b0) {                           // K, M and U of the chunk at b0
-        const int nb = min(DC_C, n - b0);
-        for (int i = tid; i < DC_C * V; i += DC_THREADS) {
-            const int t = i / V, e = (i - t * V) * 4;
-            const bool ok = t < nb;
-            copy16(sm + St::K + t * LD + e, p.K + ((size_t)(t0 + b0 + (ok ? t : 0)) * p.kv_heads + g) * D + e, ok);
-        }
-        const int t = tid >> 3, e = (tid & 7) * 4;
-        const bool ok = t < nb;
-        const size_t row = (size_t)(t0 + b0 + (ok ? t : 0)) * p.heads + h;
-        copy16(sm + St::M + t * LDM + e, p.M + row * DC_C + e, ok);
-        if (e < DC_COLS) copy16(sm + St::U + t * DC_COLS + e, p.U + row * dv + c0 + e, ok);
-        asm volatile("cp.async.commit_group;\n" ::);
-    };
-    fetch_ahead(0, 0);
-    for (int b0 = 0, st = 0; b0 < n; b0 += DC_C, st ^= 1) {
-        const int nb = min(DC_C, n - b0);
-        asm volatile("cp.async.wait_group 0;\n" ::);
-        __syncthreads();                         // W, Q and the state's columns are there; the rest of the shared memory is free
-        fetch_now(b0);
-        if (b0 + DC_C < n) fetch_ahead(st ^ 1, b0 + DC_C);
-        else asm volatile("cp.async.commit_group;\n" ::);
-        float* sp = sm + st * St::SIZE;
-        float* part = sp + St::W;                // [4][2 C][16] sums over quarters of the rows: W S, then Q S; over W once it is read
-        {   // W S and Q S: a warp takes one of them over a quarter of the rows, a thread tokens rg + 8 i and columns 4 cg ..
-            const int ks = warp & 3, rg = lane & 7, cg = lane >> 3;
-            const float* A = sp + (warp < 4 ? St::W : St::Q) + rg * LD + ks * KS;
-            const float* Bp = Ss + s_at(ks * KS, cg * 4);
-            float acc[4][4] = {};
-#pragma unroll 2
-            for (int e = 0; e < KS; e += 4) {
-                float4 a[4], b[4];
+        float s[2][4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    a[i] = *reinterpret_cast<const float4*>(A + 8 * i * LD + e);
-                    b[i] = *reinterpret_cast<const float4*>(Bp + s_at(e + i, 0));
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[j][i] = S[(size_t)(k0 + 8 * j + gt + (i & 1)) * dv + gr + 8 * (i >> 1)];
+        // products of one to three parts of a and three of b, to float32's precision: all but those below 2^-24 of the product, the small ones in a sum of
+        // their own; two b side by side, so that one's latency passes beside the other's
+        auto mma3 = [](float (&big)[2][4], float (&rest)[2][4], const unsigned (&a)[3][4], const unsigned (&b)[2][3][2], bool a_parts, bool b_parts) {
+            constexpr int A[5] = {2, 0, 1, 1, 0}, B[5] = {0, 2, 1, 0, 1};
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+                if ((A[i] == 0 || a_parts) && (B[i] == 0 || b_parts)) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) dc_mma(rest[j], a[A[i]], b[j][B[i]][0], b[j][B[i]][1]);
                 }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float av[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+            for (int j = 0; j < 2; ++j) dc_mma(big[j], a[0], b[j][0][0], b[j][0][1]);
+        };
+        // this warp's share of A [C][D] times the state; groups of four columns change places in every second four rows, for the readers
+        auto with_state = [&](int A, const unsigned (&b)[2][3][2], float* P) {
+            const __nv_bfloat16* Ap = reinterpret_cast<const __nv_bfloat16*>(dc_smem + A) + (lane & 15) * LDK + k0 + (lane >> 4) * 8;
+            float* dst = P + gr * LDP + k0 + (gt ^ (gr & 4));
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        acc[i][0] = fmaf(av[k], b[k].x, acc[i][0]); acc[i][1] = fmaf(av[k], b[k].y, acc[i][1]);
-                        acc[i][2] = fmaf(av[k], b[k].z, acc[i][2]); acc[i][3] = fmaf(av[k], b[k].w, acc[i][3]);
-                    }
-                }
-            }
-            __syncthreads();
-            // the four 16-byte groups of a row turned by the row, so that the eight rows of a quarter-warp fall on different banks
-            float* dst = part + (ks * 2 * DC_C + (warp < 4 ? 0 : DC_C) + rg) * DC_COLS + ((cg + (rg >> 1)) & 3) * 4;
+            for (int m = 0; m < 2; ++m) {
+                unsigned a[3][4];
+                float big[2][4] = {}, rest[2][4] = {};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(dst + 8 * i * DC_COLS) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        }
-        asm volatile("cp.async.wait_group 1;\n" ::);
-        __syncthreads();                         // the partial sums, K, M and U
-        const int t = tid >> 3, c = (tid & 7) * 2;
-        float2 ws = make_float2(0.f, 0.f), qs = ws;
-        {
-            const float* src = part + t * DC_COLS + (((c >> 2) + ((t & 7) >> 1)) & 3) * 4 + (c & 3);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float2 a = *reinterpret_cast<const float2*>(src + k * 2 * DC_C * DC_COLS);
-                const float2 b = *reinterpret_cast<const float2*>(src + (k * 2 * DC_C + DC_C) * DC_COLS);
-                ws.x += a.x; ws.y += a.y; qs.x += b.x; qs.y += b.y;
-            }
-        }
-        const float2 ps = *reinterpret_cast<const float2*>(sp + St::PS + 2 * t);
-        {
-            const float2 u0 = *reinterpret_cast<const float2*>(sm + St::U + t * DC_COLS + c);
-            const float ux = u0.x - ws.x, uy = u0.y - ws.y;
-            *reinterpret_cast<float2*>(us + t * DC_COLS + c) = make_float2(ux, uy);
-            *reinterpret_cast<float2*>(uds + t * DC_COLS + c) = make_float2(ps.y * ux, ps.y * uy);
-        }
-        __syncthreads();
-        {   // o: tokens up to t only, so that a later token's infinity stays with it
-            float ox = ps.x * qs.x, oy = ps.x * qs.y, o2x = 0.f, o2y = 0.f;
-            const float* Mr = sm + St::M + t * LDM;
-#pragma unroll
-            for (int s4 = 0; s4 < DC_C; s4 += 4) {
-                if (s4 > t) break;
-                const float4 m4 = *reinterpret_cast<const float4*>(Mr + s4);
-                const float m[4] = {m4.x, m4.y, m4.z, m4.w};
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float2 u = *reinterpret_cast<const float2*>(us + (s4 + k) * DC_COLS + c);
-                    if (s4 + k <= t) {
-                        if (k & 1) { o2x = fmaf(m[k], u.x, o2x); o2y = fmaf(m[k], u.y, o2y); }
-                        else { ox = fmaf(m[k], u.x, ox); oy = fmaf(m[k], u.y, oy); }
-                    }
-                }
-            }
-            if (t < nb) *reinterpret_cast<float2*>(p.out + ((size_t)(t0 + b0 + t) * p.heads + h) * dv + c0 + c) = make_float2(ox + o2x, oy + o2y);
-        }
-        {   // the state at the chunk's end: a thread sums every fourth token for rows 4 dl .. and 32 + 4 dl .. of its warp's 64 and four columns,
-            // the four lanes that share them then hand each other three quarters of their sums
-            const float* Kp = sm + St::K + (lane >> 3) * LD + (warp >> 2) * 64 + 4 * dl;
-            const float* up = uds + (lane >> 3) * DC_COLS + (warp & 3) * 4;
-            float add[2][4][4] = {};
-#pragma unroll 2
-            for (int s = 0; s < DC_C; s += 4) {
-                const float4 u = *reinterpret_cast<const float4*>(up + s * DC_COLS);
-#pragma unroll
-                for (int m = 0; m < 2; ++m) {
-                    const float4 k4 = *reinterpret_cast<const float4*>(Kp + s * LD + 32 * m);
-                    const float kv[4] = {k4.x, k4.y, k4.z, k4.w};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        add[m][i][0] = fmaf(kv[i], u.x, add[m][i][0]); add[m][i][1] = fmaf(kv[i], u.y, add[m][i][1]);
-                        add[m][i][2] = fmaf(kv[i], u.z, add[m][i][2]); add[m][i][3] = fmaf(kv[i], u.w, add[m][i][3]);
-                    }
-                }
-            }
-            const float decay = sp[St::PS + 2 * (nb - 1)];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                float v[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] = (b4 ? add[1][i][j] : add[0][i][j]) + __shfl_xor_sync(0xffffffffu, b4 ? add[0][i][j] : add[1][i][j], 16);
+                for (int i = 0; i < PARTS; ++i) dc_ldmatrix4(a[i], Ap + (i * DC_C + 16 * m) * LDK);
+                mma3(big, rest, a, b, PARTS > 1, true);
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    const float a = (b3 ? v[2 + j] : v[j]) + __shfl_xor_sync(0xffffffffu, b3 ? v[j] : v[2 + j], 8);
-                    s_reg[i][j] = fmaf(decay, s_reg[i][j], a);
+                    *reinterpret_cast<float2*>(dst + 16 * m * LDP + 8 * j) = make_float2(big[j][0] + rest[j][0], big[j][1] + rest[j][1]);
+                    *reinterpret_cast<float2*>(dst + (16 * m + 8) * LDP + 8 * j) = make_float2(big[j][2] + rest[j][2], big[j][3] + rest[j][3]);
                 }
-                *reinterpret_cast<float2*>(Ss + s_at(row0 + i, col0)) = make_float2(s_reg[i][0], s_reg[i][1]);
             }
-        }
-    }
+        };
+        asm volatile("bar.sync 1, 256;\n" ::: "memory");
+        for (int c = 0; c < n_chunks; ++c) {
+            const int st = (c & 1) * St::SIZE;
+            {
+                unsigned b[2][3][2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        S[(size_t)(row0 + i) * dv + col0] = s_reg[i][0];
-        S[(size_t)(row0 + i) * dv + col0 + 1] = s_reg[i][1];
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        float x = s[k][2 * j], y = s[k][2 * j + 1];
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) b[j][i][k] = dc_part<(PARTS > 1)>(x, y);
+                    }
+                with_state(st + St::K, b, PK);
+                asm volatile("bar.arrive 3, 384;\n" ::: "memory");
+                with_state(st + St::Q, b, PQ);
+                asm volatile("bar.arrive 5, 384;\n" ::: "memory");
+            }
+            const float decay = *reinterpret_cast<const float*>(dc_smem + St::M + (c % 3) * Z::M + DC_C * 4);
+            // keys as [token][row]: turned on the way, both halves of the rows
+            unsigned kb[2][2][3][2];
+            {
+                const __nv_bfloat16* Kp = reinterpret_cast<const __nv_bfloat16*>(dc_smem + st + St::K) + (lane & 15) * LDK + k0 + (lane >> 4) * 8;
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+#pragma unroll
+                    for (int i = 0; i < PARTS; ++i) {
+                        unsigned v[4];
+                        dc_ldmatrix4t(v, Kp + (i * DC_C + 16 * k) * LDK);
+                        kb[k][0][i][0] = v[0]; kb[k][0][i][1] = v[1]; kb[k][1][i][0] = v[2]; kb[k][1][i][1] = v[3];
+                    }
+            }
+            asm volatile("bar.sync 4, 384;\n" ::: "memory");         // u
+            float big[2][2][4] = {}, rest[2][4] = {};
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {                            // 16 tokens
+                unsigned ua[3][4];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) dc_ldmatrix4t(ua[i], up + i * St::PLANE + (16 * k + (lane & 7) + (lane >> 4) * 8) * LDU + ((lane >> 3) & 1) * 8);
+                mma3(big[k], rest, ua, kb[k], true, PARTS > 1);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[j][i] = fmaf(decay, s[j][i], (big[0][j][i] + big[1][j][i]) + rest[j][i]);
+            asm volatile("bar.sync 6, 384;\n" ::: "memory");         // Q S is read, and the stage by every walker; the next chunk is there
+            if (tid == 0 && c + 2 < n_chunks) fetch(c + 2);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) S[(size_t)(k0 + 8 * j + gt + (i & 1)) * dv + gr + 8 * (i >> 1)] = s[j][i];
+    } else {
+        const int w = warp - DC_WALKERS / 32, t = lane, cc = 4 * w;          // token t and columns cc .. cc + 3
+        float* xs = reinterpret_cast<float*>(dc_smem + St::XS);      // [16][LDM]; a warp's columns are its own
+        auto sums = [&](const float* P) {                            // of the eight walkers' shares, as a tree
+            float4 v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = *reinterpret_cast<const float4*>(P + t * LDP + 16 * k + (cc ^ (t & 4)));
+#pragma unroll
+            for (int o = 1; o < 8; o *= 2)
+#pragma unroll
+                for (int k = 0; k < 8; k += 2 * o) { v[k].x += v[k + o].x; v[k].y += v[k + o].y; v[k].z += v[k + o].z; v[k].w += v[k + o].w; }
+            return v[0];
+        };
+        // row t of A [C][LDM] times x for this warp's columns: a thread sums four tokens over every fourth group of four tokens s, then the four lanes that share
+        // them hand each other three quarters.  Tokens up to t only.
+        auto below = [&](int A, float (&out)[4]) {
+            float o[4][4] = {};
+            const int ts = lane & ~3;
+            const float* Ap = reinterpret_cast<const float*>(dc_smem + A) + ts * DC_LDM;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int s4 = 16 * i + 4 * (lane & 3);
+                if (s4 > ts) continue;
+                float4 x[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) x[j] = *reinterpret_cast<const float4*>(xs + (cc + j) * DC_LDM + s4);
+                const bool diag = s4 == ts;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float4 m = *reinterpret_cast<const float4*>(Ap + k * DC_LDM + s4);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        o[k][j] = fmaf(m.x, x[j].x, o[k][j]);
+                        if (k >= 1 || !diag) o[k][j] = fmaf(m.y, x[j].y, o[k][j]);
+                        if (k >= 2 || !diag) o[k][j] = fmaf(m.z, x[j].z, o[k][j]);
+                        if (k >= 3 || !diag) o[k][j] = fmaf(m.w, x[j].w, o[k][j]);
+                    }
+                }
+            }
+            __syncwarp();
+            const bool b0 = lane & 1, b1 = lane & 2;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float y0 = (b1 ? o[2][j] : o[0][j]) + __shfl_xor_sync(0xffffffffu, b1 ? o[0][j] : o[2][j], 2);
+                const float y1 = (b1 ? o[3][j] : o[1][j]) + __shfl_xor_sync(0xffffffffu, b1 ? o[1][j] : o[3][j], 2);
+                out[j] = (b0 ? y1 : y0) + __shfl_xor_sync(0xffffffffu, b0 ? y0 : y1, 1);
+            }
+        };
+        const int Wd = 2 * p.kv_heads * D + p.heads * dv;
+        const T* vp = reinterpret_cast<const T*>(p.qkv) + (size_t)t0 * Wd + 2 * p.kv_heads * D + (size_t)h * dv + c0 + cc;
+        auto value = [&](int c) { return c * DC_C + t < n ? dc_load4(vp + (size_t)(c * DC_C + t) * Wd) : make_float4(0.f, 0.f, 0.f, 0.f); };
+        float4 v = value(0);
+        for (int c = 0; c < n_chunks; ++c) {
+            asm volatile("bar.sync 3, 384;\n" ::: "memory");         // K S
+            const float4 f = *reinterpret_cast<const float4*>(dc_smem + (c & 1) * St::SIZE + St::R + (t * DC_LDM + DC_C) * 4);
+            {
+                const float4 ks = sums(PK);
+                xs[cc * DC_LDM + t] = fmaf(f.x, v.x, -f.y * ks.x); xs[(cc + 1) * DC_LDM + t] = fmaf(f.x, v.y, -f.y * ks.y);
+                xs[(cc + 2) * DC_LDM + t] = fmaf(f.x, v.z, -f.y * ks.z); xs[(cc + 3) * DC_LDM + t] = fmaf(f.x, v.w, -f.y * ks.w);
+            }
+            __syncwarp();
+            float u[4];
+            below((c & 1) * St::SIZE + St::R, u);
+            {
+                float x0 = f.z * u[0], y0 = f.z * u[1], x1 = f.z * u[2], y1 = f.z * u[3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const unsigned lo = dc_part<(PARTS > 1)>(x0, y0), hi = dc_part<(PARTS > 1)>(x1, y1);
+                    *reinterpret_cast<uint2*>(up + i * St::PLANE + t * LDU + cc) = make_uint2(lo, hi);
+                }
+            }
+            asm volatile("bar.arrive 4, 384;\n" ::: "memory");
+            if (c + 1 < n_chunks) v = value(c + 1);
+            asm volatile("bar.sync 5, 384;\n" ::: "memory");         // Q S
+            const float4 qs = sums(PQ);
+            if (tid == DC_WALKERS && c + 1 < n_chunks) wait(c + 1);
+            __syncwarp();
+            asm volatile("bar.arrive 6, 384;\n" ::: "memory");
+            float o[4];
+            below(St::M + (c % 3) * Z::M, o);
+            if (c * DC_C + t < n)
+                *reinterpret_cast<float4*>(p.out + ((size_t)(t0 + c * DC_C + t) * p.heads + h) * dv + c0 + cc) =
+                    make_float4(fmaf(f.w, qs.x, o[0]), fmaf(f.w, qs.y, o[1]), fmaf(f.w, qs.z, o[2]), fmaf(f.w, qs.w, o[3]));
+        }
     }
 }
 
 // whether runs of tokens are taken in chunks for these sizes
 static bool delta_chunks_ok(int d, int dv) { return d == 128 && dv % DC_COLS == 0; }
+static long long delta_prep_floats(int T_, int heads, int kv_heads, int d) {
+    return ((long long)T_ * kv_heads * d * 2 + (long long)T_ * heads * 4 + 3) & ~3LL;
+}
+// bytes that the chunks' parts take; every part is a whole number of 16 bytes
+static long long delta_chunk_bytes(long long n_chunks, int heads, int kv_heads, int dtype) {
+    const long long kq = dtype == MSGL_F32 ? DcSizes<float, 128>::KQ : DcSizes<__nv_bfloat16, 128>::KQ;
+    return n_chunks * (2 * kq * kv_heads + heads * (2LL * DcSizes<float, 128>::M));
+}
 
-// floats of scratch memory that msgl_delta_rule wants for T tokens; chunks: with runs of tokens taken in chunks
-MSGL_API long long msgl_delta_rule_scratch(int T_, int heads, int kv_heads, int d, int dv, int chunks) {
-    const long long prep = (long long)T_ * kv_heads * d * 2 + (long long)T_ * heads * 4;
-    if (!chunks || !delta_chunks_ok(d, dv)) return prep;
-    return prep + (long long)T_ * heads * (d + dv + DC_C + 2) + (long long)T_ * kv_heads * d * 2 + 16;
+// floats of scratch memory that msgl_delta_rule wants for T tokens; n_chunks: chunks of the runs that are taken in chunks, n_short: whether there are
+// requests that are not
+MSGL_API long long msgl_delta_rule_scratch(int T_, int heads, int kv_heads, int d, int dv, int n_chunks, int n_short, int dtype) {
+    if (n_chunks <= 0 || !delta_chunks_ok(d, dv)) return delta_prep_floats(T_, heads, kv_heads, d);
+    return (n_short ? delta_prep_floats(T_, heads, kv_heads, d) : 0) + delta_chunk_bytes(n_chunks, heads, kv_heads, dtype) / 4;
 }
 
 template <typename T, int D>
-static int delta_chunk_launch(const DeltaChunkParams& p, int n_chunks, cudaStream_t stream) {
-    constexpr size_t smem1 = (size_t)(2 * DC_C * (D + 4) + 2 * DC_C * (DC_C + 1) + 2 * DC_C * DC_C) * 4;
-    constexpr size_t smem2 = (size_t)DcStage<D>::TOTAL * 4;
+static int delta_chunk_launch(DeltaChunkParams& p, unsigned char* scratch, int n_chunks, cudaStream_t stream) {
+    using Z = DcSizes<T, D>;
+    constexpr int smem1 = DcPrep<T, D>::TOTAL, smem2 = DcStage<T, D>::TOTAL;
+    static_assert(Z::PARTS > 1 || 2 * (smem2 + 1024 + 64) <= 228 * 1024, "two blocks of the walk an SM");
     static MsglOncePerDevice once;
     if (once.due()) {      // first call on this device, never inside a stream capture
-        if (cudaFuncSetAttribute(delta_chunk_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess ||
-            cudaFuncSetAttribute(delta_chunk_scan_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess ||
+        if (cudaFuncSetAttribute(delta_chunk_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1) != cudaSuccess ||
+            cudaFuncSetAttribute(delta_chunk_scan_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) != cudaSuccess ||
             cudaFuncSetAttribute(delta_chunk_kernel<T, D>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-            cudaFuncSetAttribute(delta_chunk_scan_kernel<D>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+            cudaFuncSetAttribute(delta_chunk_scan_kernel<T, D>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
             return msgl_check_launch();
         once.mark();
     }
+    const size_t ch = (size_t)n_chunks * p.heads, cg = (size_t)n_chunks * p.kv_heads;
+    p.K = scratch; p.Q = p.K + cg * Z::KQ; p.R = p.Q + cg * Z::KQ; p.M = p.R + ch * Z::M;
     delta_chunk_kernel<T, D><<<dim3(n_chunks, p.heads), DC_THREADS, smem1, stream>>>(p);
-    delta_chunk_scan_kernel<D><<<dim3(p.heads, p.dv / DC_COLS, p.B), DC_THREADS, smem2, stream>>>(p);
+    delta_chunk_scan_kernel<T, D><<<dim3(p.heads, p.dv / DC_COLS, p.B), DC_WALKERS + DC_READERS, smem2, stream>>>(p);
     return msgl_check_launch();
 }
 
@@ -1561,9 +1798,10 @@ static int delta_chunk_launch(const DeltaChunkParams& p, int n_chunks, cudaStrea
 MSGL_API int msgl_delta_rule(const void* qkv, const void* proj, long long proj_stride, int a_off, int b_off, const float* a_log,
                              const float* dt_bias, float* state, const int* q_start, const int* slots, float* out, float* scratch,
                              int heads, int kv_heads, int d, int dv, int T_, int B, int dtype, int n_chunks, int n_min, int n_short,
-                             cudaStream_t stream) {
+                             void* status, cudaStream_t stream) {
     if (B <= 0 || T_ <= 0) return MSGL_OK;
-    if (n_chunks > 0 && (!delta_chunks_ok(d, dv) || n_min < 1 || B > 65535 || heads > 65535)) return MSGL_ERR_SIZE;
+    if (n_chunks > 0 && (!delta_chunks_ok(d, dv) || n_min < 1 || B > 65535 || heads > 65535 || dv / DC_COLS > 65535)) return MSGL_ERR_SIZE;
+    if (n_chunks > 0 && (((uintptr_t)qkv & 15) != 0 || status == nullptr)) return MSGL_ERR_ALIGN;
     if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || d <= 0 || dv <= 0 || d > DR_PARTS * 64 || scratch == nullptr) return MSGL_ERR_SIZE;
     if (((uintptr_t)scratch & 15) != 0) return MSGL_ERR_ALIGN;
     if (dtype != MSGL_F32 && dtype != MSGL_BF16) return MSGL_ERR_DTYPE;
@@ -1573,22 +1811,22 @@ MSGL_API int msgl_delta_rule(const void* qkv, const void* proj, long long proj_s
     p.kq = reinterpret_cast<float2*>(scratch + (size_t)T_ * heads * 4);
     p.state = state; p.q_start = q_start; p.slots = slots; p.out = out; p.heads = heads; p.kv_heads = kv_heads; p.d = d; p.dv = dv; p.T = T_;
     p.n_min = 1; p.n_max = n_chunks > 0 ? n_min - 1 : 0x7fffffff;
-    const dim3 g0(T_, (kv_heads + 3) / 4);
-    if (dtype == MSGL_F32) delta_prep_kernel<float><<<g0, 128, 0, stream>>>(p);
-    else delta_prep_kernel<__nv_bfloat16><<<g0, 128, 0, stream>>>(p);
-    int code = msgl_check_launch();
-    if (code != MSGL_OK) return code;
+    int code;
+    if (n_chunks <= 0 || n_short) {
+        const dim3 g0(T_, (kv_heads + 3) / 4);
+        if (dtype == MSGL_F32) delta_prep_kernel<float><<<g0, 128, 0, stream>>>(p);
+        else delta_prep_kernel<__nv_bfloat16><<<g0, 128, 0, stream>>>(p);
+        code = msgl_check_launch();
+        if (code != MSGL_OK) return code;
+    }
     if (n_chunks > 0) {
         DeltaChunkParams c;
-        c.qkv = qkv; c.kq = p.kq; c.sc = p.sc; c.state = state; c.q_start = q_start; c.slots = slots; c.out = out;
-        c.heads = heads; c.kv_heads = kv_heads; c.dv = dv; c.T = T_; c.B = B; c.n_min = n_min;
-        const size_t th = (size_t)T_ * heads, tk = (size_t)T_ * kv_heads;
-        // 16-byte rows of d, dv and DC_C floats; the pairs last
-        c.W = scratch + (((size_t)T_ * heads * 4 + tk * d * 2 + 3) & ~(size_t)3);
-        c.U = c.W + th * d; c.M = c.U + th * dv; c.K = c.M + th * DC_C; c.Q = c.K + tk * d;
-        c.ps = reinterpret_cast<float2*>(c.Q + tk * d);
-        if (dtype == MSGL_F32) code = delta_chunk_launch<float, 128>(c, n_chunks, stream);
-        else code = delta_chunk_launch<__nv_bfloat16, 128>(c, n_chunks, stream);
+        c.qkv = qkv; c.proj = proj; c.proj_stride = proj_stride; c.a_off = a_off; c.b_off = b_off; c.a_log = a_log; c.dt_bias = dt_bias;
+        c.state = state; c.q_start = q_start; c.slots = slots; c.out = out; c.status = (int*)status;
+        c.heads = heads; c.kv_heads = kv_heads; c.dv = dv; c.B = B; c.n_min = n_min;
+        unsigned char* rest = reinterpret_cast<unsigned char*>(scratch + (n_short ? delta_prep_floats(T_, heads, kv_heads, d) : 0));
+        if (dtype == MSGL_F32) code = delta_chunk_launch<float, 128>(c, rest, n_chunks, stream);
+        else code = delta_chunk_launch<__nv_bfloat16, 128>(c, rest, n_chunks, stream);
         if (code != MSGL_OK || !n_short) return code;
     }
     const int many_cols = DR_MANY_WARPS * DR_WCOLS;

@@ -324,7 +324,7 @@ def sample(logits: torch.Tensor, temperatures: Optional[torch.Tensor], row_keys:
 VARIANT_SIMT, VARIANT_MMA_ROWS, VARIANT_MMA_DECODE, VARIANT_TC = 0, 1, 2, 3
 TC_ROWS = 128                     # query rows per block of the tcgen05 prefill kernel
 USE_TC_ATTENTION = os.environ.get("MSGL_NO_TC_ATTENTION", "") == ""
-_status = None                    # device int32[64]: word 0 tcgen05 attention, word 2 tcgen05 GEMM, word 3 decode-step kernel; words 4..: debug counters
+_status = None                    # device int32[64]: word 0 tcgen05 attention, word 1 delta rule in chunks, word 2 tcgen05 GEMM, word 3 decode-step kernel; words 4..: debug counters
 _status_host = None               # its pinned mirror, refreshed by poll_status()
 _status_event = None
 
@@ -357,6 +357,8 @@ def raise_if_failed(wait: bool = False) -> None:
         return
     if int(_status_host[0]) != 0:
         raise KernelError("tcgen05 attention: a block timed out waiting for the tensor core; results are invalid")
+    if int(_status_host[1]) != 0:
+        raise KernelError("delta rule: a block timed out waiting for a chunk's operands; results are invalid")
     if int(_status_host[2]) != 0:
         raise KernelError("tcgen05 GEMM: a block timed out waiting for its pipeline; results are invalid")
     if int(_status_host[3]) != 0:
@@ -1825,10 +1827,10 @@ SINK_ATTENTION_MAX_HEAD_DIM = 512
 SINK_ATTENTION_SPLIT_KEYS = 256     # keys of a piece when a one-token step cuts a request's keys over several blocks
 DELTA_RULE_MAX_KEY_DIM = 512
 DELTA_CHUNK, DELTA_CHUNK_KEY_DIMS = 32, (128,)      # tokens of a chunk; key sizes whose runs of tokens are taken in chunks
-# Tokens of a request in one step from which they are taken in chunks; token by token / in chunks, 16 heads of 128 x 128 (us, all kernels): one
-# request of 64 tokens 37 / 44, 96: 49 / 42, 128: 62 / 42, 1,111 and 300: 477 / 182, 8,000: 3,223 / 944; 16 requests of 100: 218 / 229, of 128:
-# 273 / 234, of 300: 632 / 503; 64 of 128: 1,063 / 842
-DELTA_CHUNK_MIN_TOKENS = 128
+# Tokens of a request in one step from which they are taken in chunks; token by token / in chunks, 16 heads of 128 x 128 bfloat16 (us, all kernels): one
+# request of 16 tokens 11.0 / 10.9, 24: 14.5 / 10.9, 64: 28.8 / 13.2, 100: 42.7 / 16.0; 16 requests of 16: 45 / 42, of 24: 61 / 43, of 100: 208 / 101;
+# 64 of 16: 162 / 158, of 24: 228 / 159
+DELTA_CHUNK_MIN_TOKENS = 24
 
 
 def _delta_lib():
@@ -1843,8 +1845,8 @@ def _delta_lib():
             [c_int] * 12 + [c_float, c_float, c_int, c_void_p, c_ll, c_int, c_void_p]
         lib.msgl_sink_attention_mma.argtypes = [c_void_p] * 6 + [c_int, c_int, c_int, c_void_p, c_void_p, c_ll, c_void_p, c_void_p] + \
             [c_int] * 10 + [c_float, c_float, c_void_p, c_ll, c_int, c_void_p]
-        lib.msgl_delta_rule.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_int] + [c_void_p] * 7 + [c_int] * 10 + [c_void_p]
-        lib.msgl_delta_rule_scratch.argtypes = [c_int] * 6
+        lib.msgl_delta_rule.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_int] + [c_void_p] * 7 + [c_int] * 10 + [c_void_p] * 2
+        lib.msgl_delta_rule_scratch.argtypes = [c_int] * 8
         lib.msgl_delta_rule_scratch.restype = c_ll
         lib.msgl_side_gate_mul.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p]
         _delta = lib
@@ -2028,16 +2030,18 @@ def delta_rule(qkv: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, heads: in
     long_runs = [n for n in q_lens or () if n >= DELTA_CHUNK_MIN_TOKENS] if key_dim in DELTA_CHUNK_KEY_DIMS and value_dim % 16 == 0 else []
     n_chunks = sum(-(-n // DELTA_CHUNK) for n in long_runs)
     short = not long_runs or any(0 < n < DELTA_CHUNK_MIN_TOKENS for n in q_lens)
+    if n_chunks and qkv.data_ptr() % 16:
+        qkv = qkv.clone()            # the chunks' rows are read by 16 bytes
     # what does not depend on the state (unit q and k, beta, g, and for chunks all that lies within one) is made for all tokens at once
-    numel = int(_delta_lib().msgl_delta_rule_scratch(T, heads, kv_heads, key_dim, value_dim, int(n_chunks > 0)))
+    numel = int(_delta_lib().msgl_delta_rule_scratch(T, heads, kv_heads, key_dim, value_dim, n_chunks, int(short), _dt(qkv)))
     scratch = workspace.get("delta_rule_prep", numel, torch.float32) if workspace is not None else \
         torch.empty(numel, dtype=torch.float32, device=qkv.device)
     code = _delta_lib().msgl_delta_rule(_ptr(qkv), _ptr(a), stride, 0, _col_off(b, a), _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(q_start),
                                         _ptr(slots), _ptr(out), _ptr(scratch), heads, kv_heads, key_dim, value_dim, T, B, _dt(qkv), n_chunks,
-                                        DELTA_CHUNK_MIN_TOKENS, int(short), _stream())
+                                        DELTA_CHUNK_MIN_TOKENS, int(short), _ptr(_status_tensor(qkv.device)) if n_chunks else None, _stream())
     _check(code, f"delta_rule (key size {key_dim})")
     global LAUNCHES
-    LAUNCHES += 1 + (1 + int(short) if n_chunks else 0)
+    LAUNCHES += 1 + 2 * int(short and n_chunks > 0)
     return out
 
 

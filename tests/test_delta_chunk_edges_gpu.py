@@ -1,0 +1,50 @@
+"""What the chunked delta rule adds to the sizes of test_delta_chunks_gpu: values of more than 128 columns, rows that do not start on 16 bytes, norms
+beyond float32, and the sizes at which a step's short and long requests part."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def call(qkv, ab, a_log, dt, state, lens, H, G, dv):
+    from mini_sglang_b200 import ops
+    start = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    slots = torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    s = state.clone()
+    o = ops.delta_rule(qkv, ab[:, :H], ab[:, H:], heads=H, kv_heads=G, key_dim=128, value_dim=dv, a_log=a_log, dt_bias=dt, state=s, q_start=start,
+                       slots=slots, q_lens=lens)
+    return o, s
+
+
+def inputs(lens, H, G, dv, dtype, off=0):
+    g = torch.Generator(device=DEV).manual_seed(sum(lens) + dv)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)      # noqa: E731
+    T, W = sum(lens), 2 * G * 128 + H * dv
+    flat = rnd(T * W + off).to(dtype)
+    return [flat[off:].view(T, W), rnd(T, 2 * H).to(dtype), torch.log(1 + 15 * torch.rand(H, generator=g, device=DEV)), rnd(H) - 3, 0.1 * rnd(len(lens), H, 128, dv)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens,H,G,dv,off", [([23, 24, 25], 2, 1, 16, 0), ([96, 1, 127], 4, 2, 272, 0), ([65], 2, 2, 128, 3), ([24] * 33, 1, 1, 32, 0)])
+def test_against_the_token_by_token_kernel(dtype, lens, H, G, dv, off, monkeypatch):
+    from mini_sglang_b200 import ops
+    x = inputs(lens, H, G, dv, dtype, off)
+    o, s = call(*x, lens, H, G, dv)
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", 1 << 30)
+    o1, s1 = call(*x, lens, H, G, dv)
+    # both sum 128 products and a run's decayed updates in float32: a few 1e-7 of the largest terms, which are of the order of one
+    assert (o - o1).abs().max() < 1e-5 and (s - s1).abs().max() < 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_norm_beyond_float32_makes_a_row_of_zeros(dtype, monkeypatch):
+    from mini_sglang_b200 import ops
+    lens, H, G, dv = [40], 2, 1, 16
+    x = inputs(lens, H, G, dv, dtype)
+    x[0][7, :128] = 1e30                                       # a query, a key
+    x[0][33, 128:256] = -1e30
+    o, s = call(*x, lens, H, G, dv)
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", 1 << 30)
+    o1, s1 = call(*x, lens, H, G, dv)
+    assert torch.isfinite(o).all() and (o - o1).abs().max() < 1e-5 and (s - s1).abs().max() < 1e-5
