@@ -1535,6 +1535,52 @@ __global__ void group_rms_gate_kernel(const float* __restrict__ x, int heads, in
     }
 }
 
+// The same for heads of up to 128 elements in fours: a lane takes four neighbouring ones, 16 bytes of x and of w, and a warp R rows, whose loads
+// are all under way together.  Bound by the bytes: an element a lane and load took 12.2 us for 22,576 rows of 128 (23 MB), this 8.0.
+template <typename T> __device__ __forceinline__ void grg_load4(const T* p, float (&o)[4]);
+template <> __device__ __forceinline__ void grg_load4<float>(const float* p, float (&o)[4]) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+}
+template <> __device__ __forceinline__ void grg_load4<__nv_bfloat16>(const __nv_bfloat16* p, float (&o)[4]) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    o[0] = __uint_as_float(v.x << 16); o[1] = __uint_as_float(v.x & 0xffff0000u);
+    o[2] = __uint_as_float(v.y << 16); o[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+__device__ __forceinline__ void grg_store4(float* p, const float (&o)[4]) { *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]); }
+__device__ __forceinline__ void grg_store4(__nv_bfloat16* p, const float (&o)[4]) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(o[0], o[1]), b = __floats2bfloat162_rn(o[2], o[3]);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+}
+template <typename T, int R>
+__global__ void __launch_bounds__(128, 12) group_rms_gate_vec_kernel(const float* __restrict__ x, int heads, int d, const float* __restrict__ w, float eps,
+                                                                 const T* __restrict__ gate, long long gate_stride, T* __restrict__ out,
+                                                                 long long out_stride, float c, int act, int n_rows) {
+    const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R, lane = threadIdx.x & 31, e = 4 * lane;
+    const bool ok = e < d;
+    int t = row0 / heads, h = row0 - t * heads;
+    float xv[R][4] = {}, gv[R][4] = {}, wv[4] = {};
+    T* dst[R];
+    if (ok) grg_load4<float>(w + e, wv);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        dst[i] = out + t * out_stride + h * d + e;
+        if (row0 + i < n_rows && ok) {
+            grg_load4<float>(x + (size_t)(row0 + i) * d + e, xv[i]);
+            if (gate) grg_load4<T>(gate + t * gate_stride + h * d + e, gv[i]);
+        }
+        if (++h == heads) { h = 0; ++t; }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const float rs = 1.f / sqrtf(warp_sum((xv[i][0] * xv[i][0] + xv[i][1] * xv[i][1]) + (xv[i][2] * xv[i][2] + xv[i][3] * xv[i][3])) / (float)d + eps);
+        float o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = xv[i][j] * rs * wv[j] * (gate ? c * (act == 2 ? sigmoidf_(gv[i][j]) : siluf_(gv[i][j])) : c);
+        if (row0 + i < n_rows && ok) grg_store4(dst[i], o);
+    }
+}
+
 MSGL_API int msgl_group_rms_gate(const float* x, int heads, int d, const float* w, float eps, const void* gate,
                                  long long gate_stride, void* out, long long out_stride, float c, int act, int T_, int dtype,
                                  cudaStream_t stream) {
@@ -1544,6 +1590,16 @@ MSGL_API int msgl_group_rms_gate(const float* x, int heads, int d, const float* 
     const int warps = 4;
     const unsigned blocks = (unsigned)((n_rows + warps - 1) / warps);
     if (dtype != MSGL_F32 && dtype != MSGL_BF16) return MSGL_ERR_DTYPE;
+    if (d <= 128 && d % 4 == 0 && n_rows < (1LL << 30) && gate_stride % 4 == 0 && out_stride % 4 == 0 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out) & 15) == 0) {
+        // two rows a warp once that still leaves every SM four blocks or more
+        const bool two = n_rows >= 2LL * 4 * warps * msgl_sm_count();
+        const unsigned g = (unsigned)((n_rows + (two ? 2 : 1) * warps - 1) / ((two ? 2 : 1) * warps));
+#define GRG_VEC(T, R) group_rms_gate_vec_kernel<T, R><<<g, warps * 32, 0, stream>>>(x, heads, d, w, eps, (const T*)gate, gate_stride, (T*)out, out_stride, c, act, (int)n_rows)
+        if (dtype == MSGL_F32) { if (two) GRG_VEC(float, 2); else GRG_VEC(float, 1); }
+        else { if (two) GRG_VEC(__nv_bfloat16, 2); else GRG_VEC(__nv_bfloat16, 1); }
+#undef GRG_VEC
+        return msgl_check_launch();
+    }
 #define GRG_LAUNCH(N)                                                                                                          \
     do {                                                                                                                       \
         if (dtype == MSGL_F32)                                                                                                 \
