@@ -19,7 +19,7 @@
 //   gate_group_norm_kernel     (y * silu(z)) RMS-normed in equal parts of the row, times a weight
 //   unary_act_kernel           relu(x)^2 (and the other activations), times a constant
 //   route_kernel               router logits in float32, sigmoid or softmax scores, correction, limitation to the best groups,
-//                              the top experts and their weights: one block per token
+//                              the top experts and their weights: a block one, two or four tokens
 //                              (or the largest logits and the softmax over the chosen ones; a further row's sigmoid per token
 //                              beside them)
 //   expert_gate_up_kernel, expert_down_kernel      the chosen experts' products for a few tokens, straight from the experts'
@@ -1600,7 +1600,7 @@ MSGL_API int msgl_unary_act(const void* x, long long x_stride, void* out, long l
 }
 
 // ---------------------------------------------------------------------------------------
-// Router of a mixture of experts: one block per token
+// Router of a mixture of experts: a block a token or two or four
 //
 //   z = W h (float32 sums); s = sigmoid(z) (score 0) or softmax(z) over all experts (score 2); choice = s + correction
 //   the experts form `n_groups` equal groups of neighbours; a group's score is the sum of its two largest choice scores, or the
@@ -1611,55 +1611,118 @@ MSGL_API int msgl_unary_act(const void* x, long long x_stride, void* out, long l
 // ---------------------------------------------------------------------------------------
 #define RT_MAX_EXPERTS 1024
 #define RT_MAX_GROUPS 64
-// A few tokens (a decode step): a block a token has up to 32 warps, so that a warp has one or two router rows to multiply; many tokens
-// fill the SMs with blocks of 8 warps.  The sums of a logit are the same in all (one lane's elements in turn, then over the lanes), so the
-// choice does not depend on the batch.  One warp then chooses.  33 rows of 2,048, 8 warps -> 32 warps: 8 tokens 15.4 -> 10.8 us with
-// cold weights, 9.9 -> 6.4 with warm ones.
-template <typename T>
-__global__ void __launch_bounds__(1024) route_kernel(const T* __restrict__ h, long long h_stride, const T* __restrict__ W,
+// A few tokens (a decode step): a block a token, a warp two router rows.  Many tokens: a block has TOK of them and a warp four rows, so that a row is read
+// and unpacked once for TOK tokens; two blocks fit an SM.  The sums of a logit are the
+// same in all (one lane's elements in turn, then over the lanes), so the choice does not depend on the batch.  A warp a token then chooses.
+// Against a warp a row at a time and a token a block (us, warm): 33 bfloat16 rows of 2,048, 8 tokens 6.2 -> 4.9, 296: 8.2 -> 5.9, 700: 12.6 -> 10.3, 2,000:
+// 29.1 -> 19.2; 257 of 7,168, 8 tokens 50.8 -> 36.9, 700: 237 -> 155; 65 float32 rows of 2,048, 700 tokens 30.4 -> 17.5.
+template <typename T, int ROWS, int TOK>
+__device__ __forceinline__ void route_rows(const T* __restrict__ h, long long h_stride, int t0, int T_, const T* __restrict__ W, int H, int E, int rows,
+                                           const T* __restrict__ gate_row, float (&sum)[ROWS * TOK], int r0) {
+    constexpr int V = VecOf<T>::N, STEP = 32 * V;
+    const int lane = threadIdx.x & 31;
+    const T* wr[ROWS];
+    const T* hr[TOK];
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) { const int e = min(r0 + j, rows - 1); wr[j] = (e < E ? W + (size_t)e * H : gate_row) + lane * V; }
+#pragma unroll
+    for (int k = 0; k < TOK; ++k) hr[k] = h + (size_t)min(t0 + k, T_ - 1) * h_stride + lane * V;
+    float acc[ROWS][TOK];
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j)
+#pragma unroll
+        for (int k = 0; k < TOK; ++k) acc[j][k] = 0.f;
+    auto add = [&](const uint4 (&wv)[ROWS], const uint4 (&hv)[TOK]) {
+        float b[TOK][V];
+#pragma unroll
+        for (int k = 0; k < TOK; ++k) VecOf<T>::unpack(hv[k], b[k]);
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            float a[V];
+            VecOf<T>::unpack(wv[j], a);
+#pragma unroll
+            for (int k = 0; k < TOK; ++k)
+#pragma unroll
+                for (int i = 0; i < V; ++i) acc[j][k] = fmaf(a[i], b[k][i], acc[j][k]);
+        }
+    };
+#pragma unroll (TOK > 1 ? 2 : 4)
+    for (int at = 0; at + lane * V < H; at += STEP) {
+        uint4 wv[ROWS], hv[TOK];
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) wv[j] = *reinterpret_cast<const uint4*>(wr[j] + at);
+#pragma unroll
+        for (int k = 0; k < TOK; ++k) hv[k] = *reinterpret_cast<const uint4*>(hr[k] + at);
+        add(wv, hv);
+    }
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j)
+#pragma unroll
+        for (int k = 0; k < TOK; ++k) sum[j * TOK + k] = acc[j][k];
+}
+
+template <typename T, int ROWS /* 0: any sizes and places, an element at a time */, int TOK>
+__global__ void __launch_bounds__(TOK > 1 ? 320 : 1024, TOK > 1 ? 2 : 1) route_kernel(const T* __restrict__ h, long long h_stride, const T* __restrict__ W,
                                                     const float* __restrict__ correction, int H, int E, int n_groups, int keep,
-                                                    int top, int* __restrict__ idx, float* __restrict__ wts, int vec, int score,
+                                                    int top, int* __restrict__ idx, float* __restrict__ wts, int T_, int score,
                                                     int group_max, int renorm, const T* __restrict__ gate_row,
                                                     float* __restrict__ gate_out) {
-    __shared__ float s_sh[RT_MAX_EXPERTS], c_sh[RT_MAX_EXPERTS], g_sh[RT_MAX_GROUPS];
+    __shared__ float s_all[TOK][RT_MAX_EXPERTS], c_all[TOK][RT_MAX_EXPERTS], g_all[TOK][RT_MAX_GROUPS];
     const bool softmax = score == 1;
-    const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-    const T* hr = h + (size_t)t * h_stride;
-    pdl_wait();
-    pdl_small();
+    const int t0 = blockIdx.x * TOK, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     // row E, if there is one, is no expert: the sigmoid of its product with the token is handed out beside the choice
-    for (int e = warp; e < E + (gate_row ? 1 : 0); e += nw) {
-        const T* wr = e < E ? W + (size_t)e * H : gate_row;
-        float acc = 0.f;
-        if (vec) {                                       // 16 bytes of the row a lane and turn
-            constexpr int V = VecOf<T>::N;
-#pragma unroll 4
-            for (int i = lane * V; i < H; i += 32 * V) {
-                float a[V], b[V];
-                VecOf<T>::load(wr + i, a);
-                VecOf<T>::load(hr + i, b);
-#pragma unroll
-                for (int k = 0; k < V; ++k) acc = fmaf(a[k], b[k], acc);
-            }
+    const int rows = E + (gate_row ? 1 : 0);
+    auto put = [&](int e, int k, float z) {
+        if (e >= rows || t0 + k >= T_) return;
+        if (e >= E) {
+            gate_out[t0 + k] = sigmoidf_(z);
+        } else if (score) {                              // the logits themselves (1: are chosen by and weighted)
+            s_all[k][e] = z;
+            c_all[k][e] = z;
         } else {
-            for (int i = lane; i < H; i += 32) acc = fmaf(to_f32<T>(wr[i]), to_f32<T>(hr[i]), acc);
+            const float v = sigmoidf_(z);
+            s_all[k][e] = v;
+            c_all[k][e] = v + (correction ? correction[e] : 0.f);
         }
-        acc = warp_sum(acc);
-        if (lane == 0) {
-            if (e >= E) {
-                gate_out[t] = sigmoidf_(acc);
-            } else if (score) {                          // the logits themselves (1: are chosen by and weighted)
-                s_sh[e] = acc;
-                c_sh[e] = acc;
-            } else {
-                const float s = sigmoidf_(acc);
-                s_sh[e] = s;
-                c_sh[e] = s + (correction ? correction[e] : 0.f);
+    };
+    if constexpr (ROWS == 0) {
+        pdl_wait();
+        pdl_small();
+        const T* hr = h + (size_t)t0 * h_stride;
+        for (int e = warp; e < rows; e += nw) {
+            const T* wr = e < E ? W + (size_t)e * H : gate_row;
+            float acc = 0.f;
+            for (int i = lane; i < H; i += 32) acc = fmaf(to_f32<T>(wr[i]), to_f32<T>(hr[i]), acc);
+            acc = warp_sum(acc);
+            if (lane == 0) put(e, 0, acc);
+        }
+    } else {
+        constexpr int N = ROWS * TOK;
+        pdl_wait();
+        pdl_small();
+        for (int r0 = warp * ROWS; r0 < rows; r0 += nw * ROWS) {
+            float sum[N];
+            route_rows<T, ROWS, TOK>(h, h_stride, t0, T_, W, H, E, rows, gate_row, sum, r0);
+            // sums over the lanes, 16 of them first: each step hands half of the values to the other lane, so a value's additions are those of warp_sum
+            int o = 16;
+#pragma unroll
+            for (int n = N; n > 1; n /= 2, o /= 2) {
+                const bool up = lane & o;
+#pragma unroll
+                for (int i = 0; i < N / 2; ++i)
+                    if (i < n / 2) sum[i] = (up ? sum[i + n / 2] : sum[i]) + __shfl_xor_sync(0xffffffffu, up ? sum[i] : sum[i + n / 2], o);
             }
+            for (; o > 0; o /= 2) sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
+            constexpr int LANES = 32 / N;                // that share a value
+            if (lane % LANES == 0) { const int v = lane / LANES; put(r0 + v / TOK, v % TOK, sum[0]); }
         }
     }
     __syncthreads();
-    if (warp != 0) return;
+    if (warp >= TOK || t0 + warp >= T_) return;
+    const int t = t0 + warp;
+    float* s_sh = s_all[warp];
+    float* c_sh = c_all[warp];
+    float* g_sh = g_all[warp];
     if (score == 2) {                                    // softmax over all of them
         float m = -INFINITY, part = 0.f;
         for (int e = lane; e < E; e += 32) m = fmaxf(m, s_sh[e]);
@@ -1740,24 +1803,33 @@ MSGL_API int msgl_route(const void* h, long long h_stride, const void* W, const 
     const int vec = H % V == 0 && h_stride % V == 0 && ((uintptr_t)h % 16) == 0 && ((uintptr_t)W % 16) == 0 &&
                     ((uintptr_t)gate_row % 16) == 0;
     if (gate_row && !gate_out) return MSGL_ERR_SIZE;
-    const int rows = E + (gate_row ? 1 : 0);
-    const int sms = msgl_sm_count();             // warm, us: 128 tokens 32 warps 6.6, 16: 7.6, 8: 10.1;  296 tokens 12.1, 8.0, 10.5;  700 tokens 25.9, 20.5, 20.9
-    const int most = T_ <= sms ? 32 : T_ <= 2 * sms ? 16 : 8;
-    const int threads = 32 * (rows < 4 ? 4 : rows < most ? rows : most);
+    const int rows = E + (gate_row ? 1 : 0), sms = msgl_sm_count();
+    const int tok = !vec || T_ <= sms ? 1 : T_ <= 2 * sms ? 2 : 4;
+    const int each = !vec ? 1 : tok == 1 ? 2 : 4, most = tok == 1 ? 32 : 10;             // rows a warp takes at a time, warps
+    const int warps = (rows + each - 1) / each < 4 ? 4 : (rows + each - 1) / each < most ? (rows + each - 1) / each : most;
+    const int blocks = (T_ + tok - 1) / tok;
     // Up to a block an SM the blocks are set up while the kernel before this one finishes.  More of them would pile up on the SMs whose share of that
     // kernel ends first (behind a norm, 32 rows of 2,048: 300 tokens 22.2 us against 16.0, 256 rows of 7,168: 500 tokens 366 against 221).
+#define ROUTE_GO(T, ROWS, TOK) \
+    do { \
+        if (blocks <= sms) \
+            msgl_launch_pdl(route_kernel<T, ROWS, TOK>, dim3(blocks), dim3(32 * warps), 0, stream, (const T*)h, h_stride, (const T*)W, correction, H, E, n_groups, keep, top, \
+                            idx, wts, T_, score, group_max, renorm, (const T*)gate_row, gate_out); \
+        else \
+            route_kernel<T, ROWS, TOK><<<blocks, 32 * warps, 0, stream>>>((const T*)h, h_stride, (const T*)W, correction, H, E, n_groups, keep, top, idx, wts, T_, score, \
+                                                                          group_max, renorm, (const T*)gate_row, gate_out); \
+    } while (0)
 #define ROUTE(T) \
     do { \
-        if (T_ <= sms) \
-            msgl_launch_pdl(route_kernel<T>, dim3(T_), dim3(threads), 0, stream, (const T*)h, h_stride, (const T*)W, correction, H, E, n_groups, keep, top, idx, \
-                            wts, vec, score, group_max, renorm, (const T*)gate_row, gate_out); \
-        else \
-            route_kernel<T><<<T_, threads, 0, stream>>>((const T*)h, h_stride, (const T*)W, correction, H, E, n_groups, keep, top, idx, wts, vec, score, \
-                                                        group_max, renorm, (const T*)gate_row, gate_out); \
+        if (!vec) ROUTE_GO(T, 0, 1); \
+        else if (tok == 1) ROUTE_GO(T, 2, 1); \
+        else if (tok == 2) ROUTE_GO(T, 4, 2); \
+        else ROUTE_GO(T, 4, 4); \
     } while (0)
     if (dtype == MSGL_F32) ROUTE(float);
     else ROUTE(__nv_bfloat16);
 #undef ROUTE
+#undef ROUTE_GO
     return msgl_check_launch();
 }
 
