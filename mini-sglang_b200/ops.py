@@ -5,7 +5,8 @@ stream of torch and returns torch tensors.  There is no other implementation beh
 tensor that is not on a CUDA device, a missing compiler or an unsupported size raises.
 Matrix products with more than a few rows are the one exception to "hand-written": `linear` then calls
 the library GEMM that torch binds (cuBLAS), in bfloat16 with float32 accumulation or in true float32
-(TF32 off), as the reference does for every projection (F.linear in mini_sglang/layers/linear.py).  Up to
+(TF32 off), as the reference does for every projection (F.linear in mini_sglang/layers/linear.py).  Float32 products of more than a few rows and
+of weights that are not small go to this engine's float32 kernel on the tensor cores.  Up to
 SMALL_M_MAX rows go to this engine's weight-streaming kernel, and the gated products and output heads of larger decode batches to
 its decode-batch kernel.  The reference's own kernels for the
 other operations come from sgl_kernel / flash-attn (mini_sglang/layers/layernorm.py:39-50,
@@ -101,6 +102,7 @@ def _lib():
         lib.msgl_gemm_tc2_splits.restype = c_int
         lib.msgl_gemm_rows.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_int, c_float, c_int,
                                        c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
+        lib.msgl_gemm_f32.argtypes = [c_void_p] * 4 + [c_int] * 3 + [c_ll, c_ll, c_int, c_void_p, c_void_p]
         lib.msgl_tensor_maps.argtypes = []
         lib.msgl_tensor_maps.restype = c_int
         lib.msgl_sample.argtypes = [c_void_p, c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_ull, c_void_p,
@@ -820,12 +822,40 @@ def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     return out
 
 
+# Float32 products on the tensor cores against the library's, us, library / kernel.  [4096, 1024] at 4 rows 13.7 / 10.1, 1: 5.7 / 9.9, 9: 27.0 / 10.1, 64: 27.4 / 12.7,
+# 247: 45.1 / 24.6, 600: 122.7 / 67.5; [1024, 2048] at 9: 19.5 / 8.9, 247: 46.8 / 16.6; [12288, 2048] at 600: 574 / 268; [512, 1024] at 9: 8.6 / 8.0; [2048, 512] at
+# 16: 10.7 / 8.6, 64: 11.0 / 11.3; [1024, 512] at 16: 7.1 / 8.6, 64: 10.9 / 11.3.  Errors against 64 bits, relative: 0.9e-7 to 1.3e-7, the library's 1.9e-7 to 1e-6.
+F32_MIN_ROWS, F32_MIN_INNER, F32_LONG_INNER, F32_MIN_WEIGHT, F32_MIN_WEIGHT_LONG = 9, 512, 1024, 1_000_000, 500_000
+
+
+def _f32_rule(rows: int, n_out: int, K: int) -> bool:
+    return rows >= F32_MIN_ROWS and K >= F32_MIN_INNER and n_out * K >= (F32_MIN_WEIGHT_LONG if K >= F32_LONG_INNER else F32_MIN_WEIGHT)
+
+
+def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """x @ weight^T + bias in float32 on the tensor cores (csrc/gemm_f32.cu); None where the library's float32 product is to be called: few rows or
+    small weights, operands that do not lie as the kernel reads them, and whatever a kernel called by address would slip past."""
+    if not (x.dtype == torch.float32 and weight.dtype == torch.float32 and x.dim() == 2 and weight.dim() == 2
+            and _f32_rule(x.shape[0], weight.shape[0], weight.shape[1]) and x.shape[1] == weight.shape[1] and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1]
+            and weight.is_contiguous() and weight.shape[1] % 8 == 0 and x.get_device() == weight.get_device() and (x.data_ptr() | weight.data_ptr()) % 16 == 0
+            and (bias is None or (bias.dtype == torch.float32 and bias.dim() == 1 and bias.shape[0] == weight.shape[0] and bias.is_contiguous()
+                                  and bias.get_device() == weight.get_device()))
+            and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
+            and not _observed(x, weight)):
+        return None
+    M, (N, K) = x.shape[0], weight.shape
+    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    _check(_lib().msgl_gemm_f32(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), N, 0, _ptr(_status_tensor(x.device)), _stream()), "gemm_f32")
+    return out
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """y = x @ weight^T (+ bias); weight is [out, in] as stored in the checkpoint.
 
     Up to SMALL_M_MAX bfloat16 rows go through this engine's weight-streaming kernel (csrc/gemm_small_m.cu), float32 results of
-    very many columns for a decode batch through its decode-batch kernel (csrc/gemm_rows.cu, `_rows_f32`); everything else is the
+    very many columns for a decode batch through its decode-batch kernel (csrc/gemm_rows.cu, `_rows_f32`), float32 operands through the float32
+    kernel of the tensor cores (csrc/gemm_f32.cu, `_f32_rule`); everything else is the
     library GEMM unless MSGL_TC_GEMM or MSGL_TC_MID ask for the tiled kernels."""
     _need_cuda(x, weight, bias)
     if out_dtype == torch.float32 and x.dim() == 2 and _rows_f32(x.shape[0], weight.shape[0], x.shape[1], x.device):
@@ -841,6 +871,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         return out
     if out_dtype in (None, torch.bfloat16):
         y = _tc_gemm(x, weight, bias, 0) if x.shape[0] >= TC_GEMM_MIN_M else _tc_gemm_mid(x, weight, bias, 0)
+        if y is not None:
+            return y
+    if out_dtype in (None, torch.float32):
+        y = _gemm_f32(x, weight, bias)
         if y is not None:
             return y
     if out_dtype is not None and out_dtype != x.dtype:

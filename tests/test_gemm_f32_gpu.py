@@ -1,0 +1,65 @@
+"""The float32 product on the tensor cores (csrc/gemm_f32.cu) against float64: edges of its tiles of weight rows and tokens, ranges of K, remainders of a slab, rows on a
+pitch, a bias, numbers that its bfloat16 parts do not hold, and the calls that stay with the library."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def operands(M, N, K, pad=0):
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x = torch.randn((M, K + pad), generator=g, device=DEV)[:, :K]
+    return x, torch.randn((N, K), generator=g, device=DEV), torch.randn(N, generator=g, device=DEV)
+
+
+@pytest.mark.parametrize("M,N,K,pad,bias", [(9, 4096, 128, 0, False), (16, 129, 3904, 4, True), (17, 1000, 504, 0, False), (64, 128, 4096, 0, True), (65, 2048, 264, 8, False),
+                                            (128, 127, 8192, 0, False), (129, 512, 1032, 0, True), (250, 1024, 2048, 0, False), (600, 4096, 136, 12, False)])
+def test_product(M, N, K, pad, bias, monkeypatch):
+    from mini_sglang_b200 import ops
+    ops.set_true_fp32()
+    monkeypatch.setattr(ops, "_f32_rule", lambda rows, n, k: True)
+    x, w, b = operands(M, N, K, pad)
+    b = b if bias else None
+    y = ops._gemm_f32(x, w, b)
+    assert y is not None and torch.equal(y, ops.linear(x, w, b))
+    want = x.double() @ w.double().t() + (b.double() if bias else 0.0)
+    # every term exact to 2^-24, sums of 64 by the tensor core, those added in float32: some 2^-23 of the terms' root mean square sum
+    err = (y.double() - want).abs().max().item()
+    assert err < 2.0 ** -20 * K ** 0.5, err
+    lib = torch.nn.functional.linear(x, w, b)
+    assert (y.double() - want).norm() <= 1.05 * (lib.double() - want).norm()
+    ops.check_kernel_status()
+
+
+def test_numbers_that_three_parts_do_not_hold(monkeypatch):
+    from mini_sglang_b200 import ops
+    ops.set_true_fp32()
+    monkeypatch.setattr(ops, "_f32_rule", lambda rows, n, k: True)
+    for put in (lambda x, w: (x[3].fill_(float("inf")), w[9].clamp_(min=0.5)), lambda x, w: x[60, 1:2].fill_(float("nan")),
+                lambda x, w: (x[3, 7:8].fill_(3.4e38), w[:, 7].mul_(1e-3)), lambda x, w: x.mul_(2.0 ** -120), lambda x, w: x.mul_(2.0 ** -108)):
+        x, w, _ = operands(70, 1024, 512)
+        put(x, w)
+        y, lib = ops._gemm_f32(x, w, None), torch.nn.functional.linear(x, w)
+        assert torch.equal(torch.isnan(y), torch.isnan(lib)) and torch.equal(y == float("inf"), lib == float("inf")) and torch.equal(y == -float("inf"), lib == -float("inf"))
+        ok = torch.isfinite(lib)
+        want = (x.double() @ w.double().t())[ok]
+        assert (y[ok].double() - want).norm() <= 1.05 * (lib[ok].double() - want).norm()
+    ops.check_kernel_status()
+
+
+def test_calls_that_stay_with_the_library():
+    from mini_sglang_b200 import ops
+    x, w, b = operands(32, 1024, 512)
+    w, b = torch.cat((w, w)), torch.cat((b, b))
+    odd = {"few rows": (x[:8], w, None), "a small weight": (x, w[:900], None), "an odd width": (x[:, :508], torch.cat((w, w))[:, :508].contiguous(), None), "columns apart": (x.t().contiguous().t(), w, None),
+           "weight rows apart": (x, w.t().contiguous().t(), None), "off 16 bytes": (torch.randn(32 * 512 + 1, device=DEV)[1:].view(32, 512), w, None),
+           "rows that overlap": (torch.randn(32 * 4 + 512, device=DEV).as_strided((32, 512), (4, 1)), w, None), "a short bias": (x, w, b[:10]),
+           "a gradient": (x.clone().requires_grad_(), w, None), "mixed types": (x, w.bfloat16(), None)}
+    for what, call in odd.items():
+        assert ops._gemm_f32(*call) is None, what
+    for what in ("a short bias", "mixed types"):
+        with pytest.raises(RuntimeError):
+            ops.linear(*odd[what])
+    assert ops.linear(*odd["a gradient"]).requires_grad
+    assert ops._gemm_f32(x, w, b) is not None
