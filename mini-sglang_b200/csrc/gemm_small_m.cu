@@ -32,6 +32,8 @@
 #endif
 constexpr int GS_WARPS = MSGL_GS_WARPS;
 constexpr int GS_PF = MSGL_GS_PF;      // chunks in flight per warp (ring depth)
+constexpr unsigned GS_AHEAD_PIECE = 256u;
+constexpr long long GS_AHEAD_MAX = 8 << 20;
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
                                           unsigned b0, unsigned b1) {
@@ -67,7 +69,7 @@ __device__ __forceinline__ void cp_async16_a(void* smem, const void* gmem) {    
 template <int NB, int GLU, typename OutT>
 __global__ void __launch_bounds__(GS_WARPS * 32) gemm_small_m_kernel(
     const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ bias,
-    OutT* __restrict__ out, int M, int N, int K, long long ldx, long long ldo, int I) {
+    OutT* __restrict__ out, int M, int N, int K, long long ldx, long long ldo, int I, const unsigned char* ahead, unsigned ahead_bytes) {
     // ring[warp][stage][2 + NB][lane] of 16-byte slots; reused for the reduction at the end
     extern __shared__ __align__(16) unsigned char gs_smem[];
     constexpr int SLOTS = 2 + NB;
@@ -143,6 +145,11 @@ __global__ void __launch_bounds__(GS_WARPS * 32) gemm_small_m_kernel(
         }
     }
     pdl_late();         // the stream is read: the next kernel may set itself up beside the reduction
+    if (GLU) {          // this block's share of the weights that the next product reads
+        const unsigned at = (blockIdx.x * (GS_WARPS * 32) + threadIdx.x) * GS_AHEAD_PIECE;
+        for (unsigned i = at; i < ahead_bytes; i += gridDim.x * (GS_WARPS * 32) * GS_AHEAD_PIECE)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(ahead + i), "r"(min(GS_AHEAD_PIECE, ahead_bytes - i)) : "memory");
+    }
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();                      // every warp is done with the ring: reuse it for the sums
     float (*red)[16][8 * NB + 1] = reinterpret_cast<float (*)[16][8 * NB + 1]>(gs_smem);
@@ -183,9 +190,12 @@ __global__ void __launch_bounds__(GS_WARPS * 32) gemm_small_m_kernel(
     }
 }
 
+// ahead: the weights of the product that comes next (gated modes; or null), which the blocks ask into L2 as they end, so that the memory has work while the last of them and
+// the next launch leave it idle.  Only where all blocks run at once and the weights are a few megabytes: feed-forward of 1,024 x 3,072 (384 blocks), 1 token, five in a
+// row 43.3 -> 40.4 us; with more blocks the first ones' requests are in the way of the others' streams (2,048 x 6,144, 768 blocks: 20.6 -> 22.4; 4,096 x 12,288: 53.9 -> 57.5).
 // mode: 0 = plain (out [M, N]), 1 / 2 = SwiGLU / ReGLU (W [2I, K], bias [2I], out [M, I], N = 2I).  out_f32: output type.
 MSGL_API int msgl_gemm_small_m(const void* W, const void* X, const void* bias, void* out, int M, int N, int K,
-                               long long ldx, long long ldo, int mode, int out_f32, cudaStream_t stream) {
+                               long long ldx, long long ldo, int mode, int out_f32, const void* ahead, long long ahead_bytes, cudaStream_t stream) {
     if (M <= 0) return MSGL_OK;
     if (M > 16 || K <= 0 || (K & 31) || N <= 0) return MSGL_ERR_SIZE;
     if (((uintptr_t)W | (uintptr_t)X) & 15) return MSGL_ERR_ALIGN;
@@ -214,8 +224,9 @@ MSGL_API int msgl_gemm_small_m(const void* W, const void* X, const void* bias, v
         if (I & 7) return MSGL_ERR_SIZE;
         const int grid = I / 8;
         if (out_f32) return MSGL_ERR_DTYPE;
+        if (ahead_bytes < 0 || ahead_bytes > GS_AHEAD_MAX || ((ahead_bytes | (long long)(uintptr_t)ahead) & 15) || ahead == nullptr || grid > 3 * msgl_sm_count()) ahead_bytes = 0;
 #define SMALL_M_GLU(NB, GLU, SMEM) \
-    msgl_launch_pdl(gemm_small_m_kernel<NB, GLU, __nv_bfloat16>, dim3(grid), dim3(threads), SMEM, stream, w, x, b, (__nv_bfloat16*)out, M, N, K, ldx, ldo, I)
+    msgl_launch_pdl(gemm_small_m_kernel<NB, GLU, __nv_bfloat16>, dim3(grid), dim3(threads), SMEM, stream, w, x, b, (__nv_bfloat16*)out, M, N, K, ldx, ldo, I, (const unsigned char*)ahead, (unsigned)ahead_bytes)
         if (mode == MSGL_GLU_SILU) { if (M <= 8) SMALL_M_GLU(1, 1, smem1); else SMALL_M_GLU(2, 1, smem2); }
         else { if (M <= 8) SMALL_M_GLU(1, 2, smem1); else SMALL_M_GLU(2, 2, smem2); }
 #undef SMALL_M_GLU
@@ -224,11 +235,11 @@ MSGL_API int msgl_gemm_small_m(const void* W, const void* X, const void* bias, v
     if (N & 15) return MSGL_ERR_SIZE;
     const int grid = N / 16;
     if (out_f32) {
-        if (M <= 8) msgl_launch_pdl(gemm_small_m_kernel<1, 0, float>, dim3(grid), dim3(threads), smem1, stream, w, x, b, (float*)out, M, N, K, ldx, ldo, 0);
-        else msgl_launch_pdl(gemm_small_m_kernel<2, 0, float>, dim3(grid), dim3(threads), smem2, stream, w, x, b, (float*)out, M, N, K, ldx, ldo, 0);
+        if (M <= 8) msgl_launch_pdl(gemm_small_m_kernel<1, 0, float>, dim3(grid), dim3(threads), smem1, stream, w, x, b, (float*)out, M, N, K, ldx, ldo, 0, nullptr, 0u);
+        else msgl_launch_pdl(gemm_small_m_kernel<2, 0, float>, dim3(grid), dim3(threads), smem2, stream, w, x, b, (float*)out, M, N, K, ldx, ldo, 0, nullptr, 0u);
     } else {
-        if (M <= 8) msgl_launch_pdl(gemm_small_m_kernel<1, 0, __nv_bfloat16>, dim3(grid), dim3(threads), smem1, stream, w, x, b, (__nv_bfloat16*)out, M, N, K, ldx, ldo, 0);
-        else msgl_launch_pdl(gemm_small_m_kernel<2, 0, __nv_bfloat16>, dim3(grid), dim3(threads), smem2, stream, w, x, b, (__nv_bfloat16*)out, M, N, K, ldx, ldo, 0);
+        if (M <= 8) msgl_launch_pdl(gemm_small_m_kernel<1, 0, __nv_bfloat16>, dim3(grid), dim3(threads), smem1, stream, w, x, b, (__nv_bfloat16*)out, M, N, K, ldx, ldo, 0, nullptr, 0u);
+        else msgl_launch_pdl(gemm_small_m_kernel<2, 0, __nv_bfloat16>, dim3(grid), dim3(threads), smem2, stream, w, x, b, (__nv_bfloat16*)out, M, N, K, ldx, ldo, 0, nullptr, 0u);
     }
     return msgl_check_launch();
 }

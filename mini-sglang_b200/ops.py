@@ -92,7 +92,7 @@ def _lib():
         lib.msgl_swiglu.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
         lib.msgl_cast_from_f32.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_void_p]
         lib.msgl_gemm_small_m.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int,
-                                          c_int, c_void_p]
+                                          c_int, c_void_p, c_ll, c_void_p]
         lib.msgl_gemm_tc.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_void_p,
                                      c_void_p]
         lib.msgl_gemm_tc2.argtypes = lib.msgl_gemm_tc.argtypes
@@ -650,8 +650,11 @@ SMALL_M_MAX = int(os.environ.get("MSGL_SMALL_M_MAX", "8"))      # tokens up to w
 USE_SMALL_M = os.environ.get("MSGL_NO_SMALL_M", "") == ""
 
 
-def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32) -> int:
-    return _lib().msgl_gemm_small_m(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), ldo, mode, out_f32, _stream())
+def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> int:
+    """ahead: a weight that gated products are to ask into L2 for the product behind them (or None; one that lies elsewhere or in pieces is left alone)."""
+    if ahead is not None and (not ahead.is_contiguous() or ahead.get_device() != x.get_device()):
+        ahead = None
+    return _lib().msgl_gemm_small_m(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), ldo, mode, out_f32, _ptr(ahead), ahead.numel() * ahead.element_size() if ahead is not None else 0, _stream())
 
 
 def _product_ok(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> bool:
@@ -888,17 +891,19 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
 GLU_MODES = {0: 1, 4: 2}          # the ACT_ numbers whose gated products have fused kernels (silu, relu) -> the kernels' mode
 
 
-def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = 0) -> torch.Tensor:
+def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = 0,
+               ahead: Optional[torch.Tensor] = None) -> torch.Tensor:
     """act(x @ gate^T + bg) * (x @ up^T + bu) with gate_up = [gate; up] packed row-wise ([2I, H]) and bias = [bg; bu] or None;
     act: one of the ACT_ numbers.  Where a kernel with the activation in its epilogue applies (silu and relu; a few rows, or
-    many rows in bfloat16) the [T, 2I] intermediate never exists."""
+    many rows in bfloat16) the [T, 2I] intermediate never exists.  ahead: the weight of the product that takes the result, which the kernel for a few rows
+    asks into L2 as it ends."""
     _need_cuda(x, gate_up, bias)
     mode = GLU_MODES.get(act)
     if mode is not None:
         if _small_m_ok(x, gate_up, bias) and (gate_up.shape[0] // 2) % 8 == 0:
             M, (N, K) = x.shape[0], gate_up.shape
             out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
-            code = _small_m(gate_up, x, bias, out, M, N, K, N // 2, mode, 0)
+            code = _small_m(gate_up, x, bias, out, M, N, K, N // 2, mode, 0, ahead)
             _check(code, "gemm_small_m (gated)")
             return out
         if x.dim() == 2 and not MID_GEMM and x.shape[0] <= _rows_glu_max(gate_up.numel()):
@@ -917,9 +922,9 @@ def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tens
     return out
 
 
-def linear_swiglu(x: torch.Tensor, gate_up: torch.Tensor) -> torch.Tensor:
+def linear_swiglu(x: torch.Tensor, gate_up: torch.Tensor, ahead: Optional[torch.Tensor] = None) -> torch.Tensor:
     """silu(x @ gate^T) * (x @ up^T): `linear_glu` without biases."""
-    return linear_glu(x, gate_up)
+    return linear_glu(x, gate_up, ahead=ahead)
 
 
 # ---------------------------------------------------------------------------------------

@@ -32,7 +32,7 @@ class SwiGLUMLP(FeedForward):
         self.down = src.fetch(self.name("down_proj.weight")).contiguous()
 
     def forward(self, x, ctx):
-        return ops.linear(ops.linear_swiglu(x, self.gate_up), self.down)
+        return ops.linear(ops.linear_swiglu(x, self.gate_up, self.down), self.down)
 
     def fused_decode_fields(self):
         return {"kind": "swiglu_mlp", "gate_up": self.gate_up, "down": self.down, "H": self.H, "I": self.I}
@@ -94,7 +94,7 @@ class GatedMLP(FeedForward, Projected):
 
     def forward(self, x, ctx):
         # product and activation in one kernel where the engine has it (few rows; many rows in bfloat16)
-        return ops.linear(ops.linear_glu(x, self.gate_up, self.gate_up_b, self.act), self.down, self.down_b)
+        return ops.linear(ops.linear_glu(x, self.gate_up, self.gate_up_b, self.act, self.down), self.down, self.down_b)
 
 
 UNARY_ACTIVATIONS = {"silu": ops.ACT_SILU, "gelu_tanh": ops.ACT_GELU_TANH, "relu2": ops.ACT_RELU2, "relu": ops.ACT_RELU}
