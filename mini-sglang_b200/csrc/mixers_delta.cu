@@ -1205,7 +1205,7 @@ struct DeltaChunkParams {
     unsigned char* R; unsigned char* M;
     float* state; const int* q_start; const int* slots; float* out;
     int* status;                                 // word 1: a copy did not arrive
-    int heads, kv_heads, dv, B, n_min;
+    int heads, kv_heads, dv, B, n_min, n_chunks;
 };
 
 namespace {
@@ -1535,7 +1535,7 @@ __global__ void __launch_bounds__(DC_WALKERS + DC_READERS, DcSizes<T, D>::PARTS 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int t0 = p.q_start[r], n = p.q_start[r + 1] - t0;
     if (n < p.n_min) return;
-    const int g = h / (p.heads / p.kv_heads), dv = p.dv, n_chunks = (n + DC_C - 1) / DC_C;
+    const int g = h / (p.heads / p.kv_heads), dv = p.dv;
     const unsigned bar = (unsigned)__cvta_generic_to_shared(dc_smem + St::BAR);     // a barrier a stage
     if (warp == 0) {                                         // chunks of the requests before this one
         int sum = 0;
@@ -1552,6 +1552,8 @@ __global__ void __launch_bounds__(DC_WALKERS + DC_READERS, DcSizes<T, D>::PARTS 
     }
     __syncthreads();
     const size_t first = (size_t)first_s;
+    const int n_chunks = min((n + DC_C - 1) / DC_C, p.n_chunks - first_s);         // (no more than the host's count has room for)
+    if (n_chunks <= 0) return;
     auto wait = [&](int c) {                                 // for the operands of chunk c: one thread, the others meet it at a barrier
         if (!tc_mbar_wait(bar + 8u * (c & 1), (unsigned)(c >> 1) & 1u)) atomicExch(p.status + 1, 1);
     };
@@ -1787,6 +1789,7 @@ static int delta_chunk_launch(DeltaChunkParams& p, unsigned char* scratch, int n
         once.mark();
     }
     const size_t ch = (size_t)n_chunks * p.heads, cg = (size_t)n_chunks * p.kv_heads;
+    p.n_chunks = n_chunks;
     p.K = scratch; p.Q = p.K + cg * Z::KQ; p.R = p.Q + cg * Z::KQ; p.M = p.R + ch * Z::M;
     delta_chunk_kernel<T, D><<<dim3(n_chunks, p.heads), DC_THREADS, smem1, stream>>>(p);
     delta_chunk_scan_kernel<T, D><<<dim3(p.heads, p.dv / DC_COLS, p.B), DC_WALKERS + DC_READERS, smem2, stream>>>(p);
