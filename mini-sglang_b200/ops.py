@@ -876,7 +876,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         y = _tc_gemm(x, weight, bias, 0) if x.shape[0] >= TC_GEMM_MIN_M else _tc_gemm_mid(x, weight, bias, 0)
         if y is not None:
             return y
-    if out_dtype in (None, torch.float32):
+    if x.dtype == torch.float32 and out_dtype in (None, torch.float32):
         y = _gemm_f32(x, weight, bias)
         if y is not None:
             return y
@@ -2072,12 +2072,14 @@ def delta_rule(qkv: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, heads: in
     if n_chunks and qkv.data_ptr() % 16:
         qkv = qkv.clone()            # the chunks' rows are read by 16 bytes
     # what does not depend on the state (unit q and k, beta, g, and for chunks all that lies within one) is made for all tokens at once
-    numel = int(_delta_lib().msgl_delta_rule_scratch(T, heads, kv_heads, key_dim, value_dim, n_chunks, int(short), _dt(qkv)))
+    lib, dt = _delta_lib(), _dt(qkv)
+    numel = lib.msgl_delta_rule_scratch(T, heads, kv_heads, key_dim, value_dim, n_chunks, short, dt)
     scratch = workspace.get("delta_rule_prep", numel, torch.float32) if workspace is not None else \
         torch.empty(numel, dtype=torch.float32, device=qkv.device)
-    code = _delta_lib().msgl_delta_rule(_ptr(qkv), _ptr(a), stride, 0, _col_off(b, a), _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(q_start),
-                                        _ptr(slots), _ptr(out), _ptr(scratch), heads, kv_heads, key_dim, value_dim, T, B, _dt(qkv), n_chunks,
-                                        DELTA_CHUNK_MIN_TOKENS, int(short), _ptr(_status_tensor(qkv.device)) if n_chunks else None, _stream())
+    status = (_status if _status is not None else _status_tensor(qkv.device)).data_ptr() if n_chunks else None
+    code = lib.msgl_delta_rule(qkv.data_ptr(), a.data_ptr(), stride, 0, _col_off(b, a), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), q_start.data_ptr(),
+                               slots.data_ptr(), out.data_ptr(), scratch.data_ptr(), heads, kv_heads, key_dim, value_dim, T, B, dt, n_chunks,
+                               DELTA_CHUNK_MIN_TOKENS, short, status, _stream())
     _check(code, f"delta_rule (key size {key_dim})")
     global LAUNCHES
     LAUNCHES += 1 + 2 * int(short and n_chunks > 0)
