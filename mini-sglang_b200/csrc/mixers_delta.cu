@@ -1281,6 +1281,8 @@ template <typename T, int D> struct DcPrep {     // shared memory of delta_chunk
 // A block makes one head's chunk.  Latency decides, so several blocks share an SM.  R by halves: its two diagonal blocks of 16 rows by substitution, a lane a column of
 // one of them, then R_21 = -R_22 L_21 R_11.  1,411 tokens of 16 heads: 15 us; with unit rows from a launch ahead (7.5 us), Gram products in multiply-adds and a
 // substitution of all of beta v and beta P K (256 columns a head) it took 43.
+// A sum takes rows of tokens up to its own only: a later token's row may be no number, and 0 times that is none either.  (What stands behind the diagonal of a row
+// belongs to that row's token or earlier ones, and nobody reads it.)
 template <typename T, int D>
 __global__ void __launch_bounds__(DC_THREADS, 4) delta_chunk_kernel(const DeltaChunkParams p) {
     using Z = DcSizes<T, D>;
@@ -1474,9 +1476,9 @@ __global__ void __launch_bounds__(DC_THREADS, 4) delta_chunk_kernel(const DeltaC
     {
         float a = 0.f, a1 = 0.f;
 #pragma unroll
-        for (int s = 0; s < 16; s += 2) {
-            a = fmaf(s <= ri ? Rs[(16 + ri) * DC_LDM + 16 + s] : 0.f, tmp[s * 17 + rj], a);
-            a1 = fmaf(s + 1 <= ri ? Rs[(16 + ri) * DC_LDM + 17 + s] : 0.f, tmp[(s + 1) * 17 + rj], a1);
+        for (int s = 0; s < 16; s += 2) {        // rows behind ri are left out, not multiplied by zero: they may be no numbers
+            if (s <= ri) a = fmaf(Rs[(16 + ri) * DC_LDM + 16 + s], tmp[s * 17 + rj], a);
+            if (s + 1 <= ri) a1 = fmaf(Rs[(16 + ri) * DC_LDM + 17 + s], tmp[(s + 1) * 17 + rj], a1);
         }
         Rs[(16 + ri) * DC_LDM + rj] = -(a + a1);
     }
@@ -1488,9 +1490,9 @@ __global__ void __launch_bounds__(DC_THREADS, 4) delta_chunk_kernel(const DeltaC
         const int t = 8 * i + warp;
         float a = 0.f, a1 = 0.f;
 #pragma unroll 8
-        for (int s = 0; s <= t; s += 2) {        // (behind the diagonal both are zeros)
+        for (int s = 0; s <= t; s += 2) {
             a = fmaf(QK[t * (DC_C + 1) + s], Rs[s * DC_LDM + lane], a);
-            a1 = fmaf(QK[t * (DC_C + 1) + s + 1], Rs[(s + 1) * DC_LDM + lane], a1);
+            if (s < t) a1 = fmaf(QK[t * (DC_C + 1) + s + 1], Rs[(s + 1) * DC_LDM + lane], a1);
         }
         Mg[t * DC_LDM + lane] = a + a1;
         Rg[t * DC_LDM + lane] = Rs[t * DC_LDM + lane];

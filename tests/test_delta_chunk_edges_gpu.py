@@ -48,3 +48,31 @@ def test_a_norm_beyond_float32_makes_a_row_of_zeros(dtype, monkeypatch):
     monkeypatch.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", 1 << 30)
     o1, s1 = call(*x, lens, H, G, dv)
     assert torch.isfinite(o).all() and (o - o1).abs().max() < 1e-5 and (s - s1).abs().max() < 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("what", ["key", "infinite key", "query", "decay", "write strength"])
+@pytest.mark.parametrize("place", [0, 7, 15, 16, 20, 25, 31, 32 + 5, 32 + 30, 64 + 9])
+def test_a_token_that_is_no_number_does_not_reach_back(dtype, what, place, monkeypatch):
+    from mini_sglang_b200 import ops
+    lens, H, G, dv = [40, 80, 33], 4, 2, 32
+    x = inputs(lens, H, G, dv, dtype)
+    clean, clean_s = call(*x, lens, H, G, dv)
+    t = lens[0] + place                                        # key and query head 1 and value head 2, which reads it, in the second request
+    if what in ("key", "infinite key", "query"):
+        x[0][t, (G + 1 if what != "query" else 1) * 128 + 5] = float("inf") if what == "infinite key" else float("nan")
+    else:
+        x[1][t, 2 if what == "decay" else H + 2] = float("nan")
+    o, s = call(*x, lens, H, G, dv)
+    heads = [2, 3] if what in ("key", "infinite key", "query") else [2]
+    o, clean = o.view(-1, H, dv), clean.view(-1, H, dv)
+    hit = torch.zeros_like(o, dtype=torch.bool)
+    hit[t:t + 1 if what == "query" else sum(lens[:2]), heads] = True
+    assert torch.equal(o[~hit], clean[~hit]) and not torch.isfinite(o[hit]).any()
+    kept = torch.ones_like(s, dtype=torch.bool)
+    if what != "query":
+        kept[1, heads] = False
+    assert torch.equal(s[kept], clean_s[kept]) and not torch.isfinite(s[~kept]).any()
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", 1 << 30)
+    o1, s1 = call(*x, lens, H, G, dv)
+    assert torch.equal(torch.isfinite(o1.view(-1, H, dv)), ~hit) and torch.equal(torch.isfinite(s1), kept)
