@@ -924,8 +924,9 @@ __global__ void causal_conv_act_kernel(const void* in_, long long stride, int of
 // The same with 16 bytes of channels a thread and TB tokens in turn (CV_TB in a long step, 1 in a short one, where the tokens
 // are better walked side by side), for up to 4 taps: the request's last three inputs stay in registers from token to token.  A tap that does not exist (fewer than 4) has weight 0 and is not read; the sum of a token is the
 // same sequence of multiply-adds as above.  The inputs of all TB tokens are asked for at the start: one after the other, each behind its request's
-// number, they made 1,411 tokens of 4,096 channels 15.1 us long; now 10.4, bound by
-// the instructions of the activation (20 an element).  Five blocks an SM: all of that step's blocks at once.
+// number, they made 1,411 tokens of 4,096 channels 15.6 us long; now 13.8 (512 tokens 12.1 -> 11.3, 8,000: 82 -> 62), bound by the instructions of the
+// activation.  An approximate division would take 11.5 of the 13.8, but round one result in 250,000 another way than the general kernel, and make those next to the smallest
+// normal numbers zero.  Five blocks an SM: all of that step's blocks at once.
 #define CV_TB 8
 template <typename T, int TB>
 __global__ void __launch_bounds__(128, 5)
@@ -987,7 +988,7 @@ causal_conv_act_vec_kernel(const void* in_, long long stride, int off, int C, in
             acc = fmaf(wv[1][i], win[1][i], acc);
             acc = fmaf(wv[2][i], win[2][i], acc);
             acc = fmaf(wv[3][i], cur[i], acc);
-            o[i] = act == 0 ? (V == 8 ? __fdividef(acc, 1.f + expf(-acc)) : siluf_(acc)) : acc;      // bfloat16: two units of the last of 24 bits, of which 8 stay
+            o[i] = act == 0 ? siluf_(acc) : acc;
             win[0][i] = win[1][i]; win[1][i] = win[2][i]; win[2][i] = cur[i];
         }
         VecOf<T>::store(out + (size_t)t * C, o);

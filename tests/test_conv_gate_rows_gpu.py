@@ -49,3 +49,19 @@ def test_head_norm_with_a_gate(dtype, T, heads, d, off, act):
     got = out.double().view(T, heads, d)
     # a sum of squares of d terms and four products in float32, then the rounding of the result
     assert ((got - want).abs() <= 1e-6 + (2.0 ** -8 if dtype == torch.bfloat16 else 2e-6) * want.abs()).all()
+
+
+def test_convolution_divides_as_the_general_kernel_does():
+    from mini_sglang_b200 import ops
+    T, C = 1024, 512
+    g = torch.Generator(device=DEV).manual_seed(3)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)      # noqa: E731
+    wide = torch.randn((T, C + 8), generator=g, device=DEV) * 4
+    wide[:, :C // 4] = torch.linspace(-89, -86, T * (C // 4), device=DEV).view(T, C // 4)         # silu down to the smallest normal numbers
+    taps = torch.randn((4, C), generator=g, device=DEV)
+    taps[:, :C // 4] = torch.tensor([0.0, 0.0, 0.0, 1.0], device=DEV)[:, None]
+    y = []
+    for x in (wide.bfloat16()[:, :C], torch.cat((wide[:, :1], wide), 1).bfloat16()[:, 1:C + 1]):         # rows on 16 bytes; rows that are not: the general kernel
+        y.append(ops.causal_conv_act(x, taps, None, state=torch.zeros((1, 3, C), dtype=torch.bfloat16, device=DEV), token_req=i32([0] * T), q_start=i32([0, T]),
+                                     slots=i32([0])))
+    assert (y[0][:, :C // 4] != 0).any() and torch.equal(y[0], y[1])
