@@ -63,3 +63,19 @@ def test_calls_that_stay_with_the_library():
             ops.linear(*odd[what])
     assert ops.linear(*odd["a gradient"]).requires_grad
     assert ops._gemm_f32(x, w, b) is not None
+
+
+def test_products_wanted_in_another_precision_stay_with_the_library():
+    from mini_sglang_b200 import ops
+    ops.set_true_fp32()
+    x, w, b = operands(32, 2048, 512)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert ops._gemm_f32(x, w, b) is None and ops.linear(x, w, b).dtype == torch.bfloat16
+    with torch.autocast("cpu", dtype=torch.bfloat16):
+        assert ops._gemm_f32(x, w, b) is not None
+    torch.backends.cuda.matmul.allow_tf32 = True
+    try:
+        assert ops._gemm_f32(x, w, b) is None
+    finally:
+        ops.set_true_fp32()
+    assert ops._gemm_f32(x, w, b) is not None
