@@ -837,7 +837,7 @@ def _f32_rule(rows: int, n_out: int, K: int) -> bool:
 
 def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     """x @ weight^T + bias in float32 on the tensor cores (csrc/gemm_f32.cu); None where the library's float32 product is to be called: few rows or
-    small weights, operands that do not lie as the kernel reads them, products that the caller wants in another precision (autocast, TF32),
+    small weights, operands that do not lie as the kernel reads them or on another device than the current one, products that the caller wants in another precision (autocast, TF32),
     and whatever a kernel called by address would slip past."""
     if not (x.dtype == torch.float32 and weight.dtype == torch.float32 and x.dim() == 2 and weight.dim() == 2
             and _f32_rule(x.shape[0], weight.shape[0], weight.shape[1]) and x.shape[1] == weight.shape[1] and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1]
@@ -846,6 +846,7 @@ def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
                                   and bias.get_device() == weight.get_device()))
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
             and not _observed(x, weight)
+            and x.get_device() == torch._C._cuda_getDevice()         # the launch goes to the current device's stream; the library changes the device
             and not torch.is_autocast_enabled("cuda") and torch._C._get_fp32_precision_getter("cuda", "matmul") != "tf32"):
         return None
     M, (N, K) = x.shape[0], weight.shape

@@ -79,3 +79,10 @@ def test_products_wanted_in_another_precision_stay_with_the_library():
     finally:
         ops.set_true_fp32()
     assert ops._gemm_f32(x, w, b) is not None
+
+
+def test_operands_on_another_device_than_the_current_one_stay_with_the_library(monkeypatch):
+    from mini_sglang_b200 import ops
+    x, w, b = operands(32, 2048, 512)
+    monkeypatch.setattr(ops.torch._C, "_cuda_getDevice", lambda: 1)
+    assert ops._gemm_f32(x, w, b) is None
