@@ -796,10 +796,10 @@ def tensor_maps() -> bool:
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
-def _observed(x: torch.Tensor, weight: torch.Tensor) -> bool:
+def _observed(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> bool:
     """Whether something looks on that a kernel called by address would slip past: tracing, a dispatch mode, vmap and its like, forward-mode
     derivatives, a tensor of another class."""
-    return (type(x) not in _PLAIN or type(weight) not in _PLAIN or torch._C._len_torch_dispatch_stack() > 0
+    return (type(x) not in _PLAIN or type(weight) not in _PLAIN or (bias is not None and type(bias) not in _PLAIN) or torch._C._len_torch_dispatch_stack() > 0
             or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0
             or torch._C._get_tracing_state() is not None)
 
@@ -809,7 +809,7 @@ def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     None where it cannot run."""
     if not (0 < x.shape[0] <= 256 and _product_ok(x, weight, bias)
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
-            and not _observed(x, weight)
+            and not _observed(x, weight, bias)
             and (x.stride(0) >= x.shape[1] or x.shape[0] == 1) and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and weight.shape[1] % 8 == 0):
         return None
     M, (N, K) = x.shape[0], weight.shape
@@ -845,7 +845,7 @@ def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
             and (bias is None or (bias.dtype == torch.float32 and bias.dim() == 1 and bias.shape[0] == weight.shape[0] and bias.is_contiguous()
                                   and bias.get_device() == weight.get_device()))
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
-            and not _observed(x, weight)
+            and not _observed(x, weight, bias)
             and x.get_device() == torch._C._cuda_getDevice()         # the launch goes to the current device's stream; the library changes the device
             and not torch.is_autocast_enabled("cuda") and torch._C._get_fp32_precision_getter("cuda", "matmul") != "tf32"):
         return None

@@ -86,3 +86,13 @@ def test_operands_on_another_device_than_the_current_one_stay_with_the_library(m
     x, w, b = operands(32, 2048, 512)
     monkeypatch.setattr(ops.torch._C, "_cuda_getDevice", lambda: 1)
     assert ops._gemm_f32(x, w, b) is None
+
+
+def test_a_bias_of_another_class_stays_with_the_library():
+    from mini_sglang_b200 import ops
+
+    class Other(torch.Tensor):
+        pass
+
+    x, w, b = operands(32, 2048, 512)
+    assert ops._gemm_f32(x, w, b.as_subclass(Other)) is None and isinstance(ops.linear(x, w, b.as_subclass(Other)), Other)
