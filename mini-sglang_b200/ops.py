@@ -339,6 +339,14 @@ def _status_tensor(device) -> torch.Tensor:
     return _status
 
 
+def _status_words(device) -> Optional[torch.Tensor]:
+    """The status words, or None in a stream capture that comes before they exist: made there they would lie in the graph's memory and be cleared
+    by every replay.  For calls that have another way."""
+    if _status is None and torch.cuda.is_current_stream_capturing():
+        return None
+    return _status_tensor(device)
+
+
 def poll_status() -> None:
     """Queue a copy of the kernels' status words to the host (no synchronisation).  Not inside a stream capture."""
     global _status_event
@@ -849,9 +857,12 @@ def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
             and x.get_device() == torch._C._cuda_getDevice()         # the launch goes to the current device's stream; the library changes the device
             and not torch.is_autocast_enabled("cuda") and torch._C._get_fp32_precision_getter("cuda", "matmul") != "tf32"):
         return None
+    status = _status_words(x.device)
+    if status is None:
+        return None
     M, (N, K) = x.shape[0], weight.shape
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    _check(_lib().msgl_gemm_f32(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), N, 0, _ptr(_status_tensor(x.device)), _stream()), "gemm_f32")
+    _check(_lib().msgl_gemm_f32(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), N, 0, _ptr(status), _stream()), "gemm_f32")
     return out
 
 
@@ -2070,6 +2081,9 @@ def delta_rule(qkv: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, heads: in
     # runs of tokens go in chunks, single tokens and short runs token by token: a matter of the request's own tokens in this step
     # and of the sizes, so a request's results do not depend on the requests beside it
     long_runs = [n for n in q_lens or () if n >= DELTA_CHUNK_MIN_TOKENS] if key_dim in DELTA_CHUNK_KEY_DIMS and value_dim % 16 == 0 else []
+    status = _status_words(qkv.device) if long_runs else None
+    if status is None:
+        long_runs = []
     n_chunks = sum(-(-n // DELTA_CHUNK) for n in long_runs)
     short = not long_runs or any(0 < n < DELTA_CHUNK_MIN_TOKENS for n in q_lens)
     if n_chunks and qkv.data_ptr() % 16:
@@ -2079,10 +2093,9 @@ def delta_rule(qkv: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, heads: in
     numel = lib.msgl_delta_rule_scratch(T, heads, kv_heads, key_dim, value_dim, n_chunks, short, dt)
     scratch = workspace.get("delta_rule_prep", numel, torch.float32) if workspace is not None else \
         torch.empty(numel, dtype=torch.float32, device=qkv.device)
-    status = (_status if _status is not None else _status_tensor(qkv.device)).data_ptr() if n_chunks else None
     code = lib.msgl_delta_rule(qkv.data_ptr(), a.data_ptr(), stride, 0, _col_off(b, a), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), q_start.data_ptr(),
                                slots.data_ptr(), out.data_ptr(), scratch.data_ptr(), heads, kv_heads, key_dim, value_dim, T, B, dt, n_chunks,
-                               DELTA_CHUNK_MIN_TOKENS, short, status, _stream())
+                               DELTA_CHUNK_MIN_TOKENS, short, _ptr(status), _stream())
     _check(code, f"delta_rule (key size {key_dim})")
     global LAUNCHES
     LAUNCHES += 1 + 2 * int(short and n_chunks > 0)

@@ -76,3 +76,19 @@ def test_a_token_that_is_no_number_does_not_reach_back(dtype, what, place, monke
     monkeypatch.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", 1 << 30)
     o1, s1 = call(*x, lens, H, G, dv)
     assert torch.equal(torch.isfinite(o1.view(-1, H, dv)), ~hit) and torch.equal(torch.isfinite(s1), kept)
+
+
+def test_a_capture_before_the_status_words_exist(monkeypatch):
+    from mini_sglang_b200 import ops
+    lens, H, G, dv = [40, 3], 2, 1, 16
+    x = inputs(lens, H, G, dv, torch.bfloat16)
+    want, want_s = call(*x, lens, H, G, dv)
+    monkeypatch.setattr(ops, "_status", None)
+    start, slots = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ([0, 40, 43], [0, 1]))
+    state, graph = x[4].clone(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        o = ops.delta_rule(x[0], x[1][:, :H], x[1][:, H:], heads=H, kv_heads=G, key_dim=128, value_dim=dv, a_log=x[2], dt_bias=x[3], state=state, q_start=start,
+                           slots=slots, q_lens=lens)
+    assert ops._status is None
+    graph.replay()
+    assert (o - want).abs().max() < 1e-5 and (state - want_s).abs().max() < 1e-5              # (token by token: the bound above)

@@ -96,3 +96,17 @@ def test_a_bias_of_another_class_stays_with_the_library():
 
     x, w, b = operands(32, 2048, 512)
     assert ops._gemm_f32(x, w, b.as_subclass(Other)) is None and isinstance(ops.linear(x, w, b.as_subclass(Other)), Other)
+
+
+def test_a_capture_before_the_status_words_exist(monkeypatch):
+    from mini_sglang_b200 import ops
+    ops.set_true_fp32()
+    x, w, b = operands(32, 2048, 512)
+    want = torch.nn.functional.linear(x, w, b)
+    monkeypatch.setattr(ops, "_status", None)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = ops.linear(x, w, b)
+    assert ops._status is None
+    graph.replay()
+    assert torch.allclose(y, want, rtol=1e-4, atol=1e-3)
