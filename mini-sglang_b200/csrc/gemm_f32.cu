@@ -130,11 +130,16 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
             buf[i][1] = in ? *reinterpret_cast<const float4*>(row[i] + k + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
         };
         unsigned rest = 0u;
+        // Before the wait the weights are only asked into L2 (a lane a 128-byte line of the first two slabs): the kernel before this one may be the one that writes them, as
+        // when one product's result is the next one's weight.
 #pragma unroll
-        for (int i = 0; i < NA; ++i) load(0, i);                 // weights depend on no kernel before this one
+        for (int i = 0; i < NA; ++i) {
+            const int s = c & 3, k = (k_begin + s) * 64 + 8 * (c & 4);
+            if (s < min(2, n_slabs) && ok[i] && k < p.K) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(row[i] + k));
+        }
         pdl_wait();
 #pragma unroll
-        for (int i = NA; i < NI; ++i) load(0, i);
+        for (int i = 0; i < NI; ++i) load(0, i);
         for (int s = 0; s < n_slabs; ++s) {
             const int st = s & 1;
             if (!tc_mbar_wait(bar_empty + 8u * st, ((s >> 1) & 1) ^ 1)) { fail = 1; break; }          // (passes at once the first time round)

@@ -110,3 +110,17 @@ def test_a_capture_before_the_status_words_exist(monkeypatch):
     assert ops._status is None
     graph.replay()
     assert torch.allclose(y, want, rtol=1e-4, atol=1e-3)
+
+
+def test_a_weight_that_the_kernel_before_writes(monkeypatch):
+    from mini_sglang_b200 import ops
+    ops.set_true_fp32()
+    monkeypatch.setattr(ops, "_f32_rule", lambda rows, n, k: True)
+    x, _, _ = operands(64, 1, 4096)
+    a, b, _ = operands(1024, 4096, 2048)
+    w = ops._gemm_f32(a, b, None)
+    torch.cuda.synchronize()
+    want = ops._gemm_f32(x, w, None)
+    for i in range(20):
+        w.fill_(float(i))
+        assert torch.equal(ops._gemm_f32(x, ops._gemm_f32(a, b, None), None), want)
