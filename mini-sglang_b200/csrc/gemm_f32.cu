@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
             sums[i] = (a[0] + a[1]) + (a[2] + a[3]);
         }
     }
+    __syncwarp();                                                // the aligned barrier wants whole warps
     if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     else __syncthreads();
     {   // the block's share of the tokens: range, range + splits, ..., SIDE at a time
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
             }
         }
     }
+    __syncwarp();                                                // the aligned barrier wants whole warps
     if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     const bool failed = __syncthreads_or(fail) != 0;
     if (failed && tid == 0) atomicExch(p.status + 2, 1);
