@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = tmem_base_s;
-    int fail = 0;
+    int fail = 0, issued = 0;                                    // slabs whose products are under way or done
     float acc[Z::COLS];                                          // adders: a weight row's sums, tokens col0 ..
     const int col0 = (warp >> 2) * Z::COLS;
 
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
         for (int i = 0; i < Z::COLS; ++i) acc[i] = 0.f;
         const unsigned src = tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)col0;
         for (int i = 0; i < n_slabs; ++i) {
-            if (!tc_mbar_wait(bar_acc + 8u * (i & 1), (i >> 1) & 1)) { fail = 1; break; }
+            if (!fail && !tc_mbar_wait(bar_acc + 8u * (i & 1), (i >> 1) & 1)) fail = 1;         // (goes on, without waiting: the lanes stay together)
             tc_fence_after();
 #pragma unroll
             for (int c = 0; c < Z::COLS; c += 16) {
@@ -142,7 +142,11 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
         for (int i = 0; i < NI; ++i) load(0, i);
         for (int s = 0; s < n_slabs; ++s) {
             const int st = s & 1;
-            if (!tc_mbar_wait(bar_empty + 8u * st, ((s >> 1) & 1) ^ 1)) { fail = 1; break; }          // (passes at once the first time round)
+            // (Passes at once the first time round.)  A warp gives up as one, or goes on without waiting, whichever the compiler schedules better around: [4096, 1024] with 9 rows and
+            // cold weights 10.2 / 10.8 us, with 600 rows 64 / 60.
+            if (BN < 64) {
+                if (!__all_sync(0xffffffffu, tc_mbar_wait(bar_empty + 8u * st, ((s >> 1) & 1) ^ 1))) { fail = 1; break; }
+            } else if (!fail && !tc_mbar_wait(bar_empty + 8u * st, ((s >> 1) & 1) ^ 1)) fail = 1;
             const unsigned base = ring + (unsigned)st * Z::STAGE;
 #pragma unroll
             for (int i = 0; i < NI; ++i) {
@@ -181,11 +185,18 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
                     tc_mma(d, da + (unsigned long long)(PA[q] * (Z::A >> 4) + 2 * kk), db + (unsigned long long)(PB[q] * (Z::B >> 4) + 2 * kk), idesc, (q > 0 || kk > 0) ? 1u : 0u);
             tc_commit(bar_empty + 8u * st);
             tc_commit(bar_acc + 8u * st);
+            ++issued;
         }
     }
     tc_fence_before();
     __syncwarp();
-    __syncthreads();                                             // every product is done: the stages become [token][weight row]
+    const bool failed = __syncthreads_or(fail) != 0;
+    if (failed) {                                                // somebody gave up waiting: no product may be under way when the stages and the tensor memory are let go
+        if (issued > 0) tc_mbar_wait(bar_acc + 8u * ((issued - 1) & 1), ((issued - 1) >> 1) & 1);
+        __syncwarp();
+        __syncthreads();
+    }
+    // every product is done: the stages become [token][weight row]
     tc_fence_after();
     if (warp < ADD_WARPS) {
 #pragma unroll
@@ -238,7 +249,7 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
     }
     __syncwarp();                                                // the aligned barrier wants whole warps
     if (splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-    const bool failed = __syncthreads_or(fail) != 0;
+    __syncthreads();
     if (failed && tid == 0) atomicExch(p.status + 2, 1);
     if (warp == LAST) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(Z::TMEM) : "memory");
 }
