@@ -15,8 +15,10 @@
 //     all         the blocks of a tile's ranges form a cluster: each sums its share of the tokens over the cluster's shared memories, in the order of
 //                 one tree, then bias and store
 //
-// Numbers that three bfloat16 parts do not hold (infinities, NaN, the last 2^-8 below the largest number, magnitudes below 2^-116 other than 0) are
-// seen on the way by what the split leaves; a block that meets one does its range again in plain multiply-adds, so they behave as in float32 arithmetic.
+// Numbers that three bfloat16 parts do not hold (infinities, NaN, the last 2^-8 below the largest number, and most of those below 2^-110 other than 0: bfloat16 ends at 2^-133)
+// are seen on the way by what the split leaves.  The block then does the sums of the tokens and weight rows that have one again in plain multiply-adds, so they behave as in float32
+// arithmetic, and all other sums keep their bits.  [4096, 1024], 247 tokens, such a number in none, one, every 64th, every token: 25, 40, 51, 208 us, in one weight row 39 (the
+// library 48); [1024, 2048], 64 tokens: 12.5, 21, 25, 75 and 18 (37).
 //
 // Bound by the split (11 instructions a pair of numbers) and the stores of the parts to shared memory.  Against the library's float32 product:
 // [4096, 1024] 247 tokens 45.1 -> 24.6 us (84 TFLOP/s of float32; multiply-adds give 74 at the most), 9 tokens 27.0 -> 10.1; [1024, 2048] 46.8 -> 16.6 and 19.5 -> 8.9.
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
     const unsigned ring = (smem_base + GF_HEAD_BYTES + 1023u) & ~1023u;
     float* sums = reinterpret_cast<float*>(gf_smem + (ring - smem_base));           // [BN][128], when the products are done
     unsigned& tmem_base_s = *reinterpret_cast<unsigned*>(gf_smem + 64);
-    int* odd_s = reinterpret_cast<int*>(gf_smem + 68);
+    unsigned* odd_s = reinterpret_cast<unsigned*>(gf_smem + 96);                    // a bit a weight row (four words) and a token (four): has a number that its parts do not hold
     const unsigned bar_full = smem_base, bar_empty = smem_base + 16u, bar_acc = smem_base + 32u, bar_free = smem_base + 48u;     // two of each
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int splits = p.splits, range = blockIdx.x % splits, tile = blockIdx.x / splits;
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
             tc_mbar_init(bar_full + 8u * i, GF_LOADERS / 32); tc_mbar_init(bar_empty + 8u * i, 1);
             tc_mbar_init(bar_acc + 8u * i, 1); tc_mbar_init(bar_free + 8u * i, ADD_WARPS);
         }
-        *odd_s = 0;
+        for (int i = 0; i < 8; ++i) odd_s[i] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     tc_fence_before();
@@ -167,7 +169,29 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
             __syncwarp();
             if (lane == 0) tc_mbar_arrive(bar_full + 8u * st);
         }
-        if (__any_sync(0xffffffffu, (rest & 0xffffu) != 0u) && lane == 0) atomicOr(odd_s, 1);
+        if ((rest & 0xffffu) != 0u) {                            // which of the thread's rows it was
+#pragma unroll 1
+            for (int i = 0; i < NI; ++i) {
+                const int rr = r + 32 * (i < NA ? i : i - NA);
+                if (i < NA ? n0 + rr >= p.N : rr >= n_tok) continue;
+                const float* src = i < NA ? p.W + (size_t)(n0 + rr) * p.K : p.X + (size_t)(m0 + rr) * p.ldx;
+                unsigned left = 0u;
+                const int k1 = min(p.K, (k_begin + n_slabs) * 64);
+                for (int k = k_begin * 64 + 8 * c; k < k1; k += 256) {
+                    float4 v[4][2];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        v[j >> 1][j & 1] = k + (j >> 1) * 64 < k1 ? *reinterpret_cast<const float4*>(src + k + (j >> 1) * 64 + (j & 1) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        float4& u = v[j >> 1][j & 1];
+                        gf_part(u.x, u.y); gf_part(u.x, u.y); gf_last(u.x, u.y, left);
+                        gf_part(u.z, u.w); gf_part(u.z, u.w); gf_last(u.z, u.w, left);
+                    }
+                }
+                if ((left & 0xffffu) != 0u) atomicOr(odd_s + (i < NA ? 0 : 4) + (rr >> 5), 1u << (rr & 31));
+            }
+        }
     } else if (lane == 0) {
         const unsigned idesc = tc_idesc(false, (unsigned)n16);
         const unsigned long long da0 = tc_desc(ring, 16, 1024), db0 = tc_desc(ring + 3u * Z::A, 16, 1024);
@@ -205,18 +229,35 @@ __global__ void __launch_bounds__(GfSizes<BN>::THREADS, 1) gemm_f32_kernel(const
     pdl_wait();                                                  // (all of x has been seen by the loaders; the others wait here before they write)
     pdl_late();
     __syncthreads();
-    if (*odd_s) {                                                // plain multiply-adds over the block's range
-        const int k0 = k_begin * 64, k1 = min(p.K, (k_begin + n_slabs) * 64);
-        for (int i = tid; i < n_tok * GF_ROWS; i += Z::THREADS) {
-            const int t = i / GF_ROWS, n = n0 + i % GF_ROWS;
-            if (n >= p.N) continue;
-            const float* w = p.W + (size_t)n * p.K;
-            const float* x = p.X + (size_t)(m0 + t) * p.ldx;
-            float a[4] = {};
-            for (int k = k0; k < k1; k += 4)
+    unsigned odd = 0u;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) a[j] = fmaf(w[k + j], x[k + j], a[j]);
-            sums[i] = (a[0] + a[1]) + (a[2] + a[3]);
+    for (int i = 0; i < 8; ++i) odd |= odd_s[i];
+    if (odd) {                                                   // plain multiply-adds over the block's range: a warp four tokens against four weight rows, its lanes along K
+        const int k1 = min(p.K, (k_begin + n_slabs) * 64);
+        for (int item = warp; item < ((n_tok + 3) >> 2) * (GF_ROWS / 4); item += Z::THREADS / 32) {
+            const int t0 = (item / (GF_ROWS / 4)) * 4, j0 = (item % (GF_ROWS / 4)) * 4;
+            const unsigned tokens = odd_s[4 + (t0 >> 5)] >> (t0 & 31) & 15u, rows = odd_s[j0 >> 5] >> (j0 & 31) & 15u;
+            if (!(tokens | rows) || n0 + j0 >= p.N) continue;
+            float a[4][4] = {};
+#pragma unroll 1
+            for (int k = k_begin * 64 + 4 * lane; k < k1; k += 128) {
+                float4 x[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(p.X + (size_t)(m0 + min(t0 + i, n_tok - 1)) * p.ldx + k);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 w = *reinterpret_cast<const float4*>(p.W + (size_t)min(n0 + j0 + j, p.N - 1) * p.K + k);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) a[i][j] = fmaf(w.w, x[i].w, fmaf(w.z, x[i].z, fmaf(w.y, x[i].y, fmaf(w.x, x[i].x, a[i][j]))));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float v = warp_sum(a[i][j]);
+                    if (lane == 0 && t0 + i < n_tok && ((tokens >> i | rows >> j) & 1u)) sums[(t0 + i) * GF_ROWS + j0 + j] = v;
+                }
         }
     }
     __syncwarp();                                                // the aligned barrier wants whole warps

@@ -124,3 +124,25 @@ def test_a_weight_that_the_kernel_before_writes(monkeypatch):
     for i in range(20):
         w.fill_(float(i))
         assert torch.equal(ops._gemm_f32(x, ops._gemm_f32(a, b, None), None), want)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), 2.0 ** -111 * 1.2345678, 1e-40])
+def test_a_number_that_three_parts_do_not_hold_stays_with_its_row(value, monkeypatch):
+    from mini_sglang_b200 import ops
+    ops.set_true_fp32()
+    monkeypatch.setattr(ops, "_f32_rule", lambda rows, n, k: True)
+    for M, N, K, t, n in ((70, 1000, 512, 60, 999), (9, 130, 2048, 0, 0), (130, 4096, 1024, 129, 64)):
+        x, w, _ = operands(M, N, K)
+        clean = ops._gemm_f32(x, w, None)
+        for rows, a, b in ((True, x.clone(), w), (False, x, w.clone())):
+            (a if rows else b)[t if rows else n, K - 3] = value
+            y, want = ops._gemm_f32(a, b, None), a.double() @ b.double().t()
+            same = torch.ones_like(y, dtype=torch.bool)
+            if rows:
+                same[t] = False
+            else:
+                same[:, n] = False
+            assert torch.equal(y[same], clean[same]) and torch.equal(torch.isfinite(y), torch.isfinite(want))
+            ok = torch.isfinite(want)
+            assert (y[ok].double() - want[ok]).abs().max() < 2.0 ** -20 * K ** 0.5
+    ops.check_kernel_status()
