@@ -314,34 +314,32 @@ static int gf_launch(const GemmF32Params& p, int blocks, cudaStream_t stream) {
     return msgl_check_launch();
 }
 
-// float32 operands; K and ldx multiples of 8 and 4, bases 16-byte aligned.  splits: ranges of K (1, 2, 4, 8), 0: chosen so that the launch has up to a block an
-// SM, of four slabs or more each.
-MSGL_API int msgl_gemm_f32(const float* W, const float* X, const float* bias, float* out, int M, int N, int K, long long ldx, long long ldo, int splits,
-                           void* status, cudaStream_t stream) {
+// float32 operands; K and ldx multiples of 8 and 4, bases 16-byte aligned.
+MSGL_API int msgl_gemm_f32(const float* W, const float* X, const float* bias, float* out, int M, int N, int K, long long ldx, long long ldo, void* status, cudaStream_t stream) {
     if (M <= 0) return MSGL_OK;
-    if (N <= 0 || K <= 0 || (K & 7) || (ldx & 3) || status == nullptr || splits < 0 || splits > GF_MAX_SPLITS || (splits & (splits - 1))) return MSGL_ERR_SIZE;
+    if (N <= 0 || K <= 0 || (K & 7) || (ldx & 3) || status == nullptr) return MSGL_ERR_SIZE;
     if (((uintptr_t)W | (uintptr_t)X) & 15) return MSGL_ERR_ALIGN;
     const int slabs = (K + 63) / 64;
     GemmF32Params p;
     p.W = W; p.X = X; p.bias = bias; p.out = out; p.ldx = ldx; p.ldo = ldo; p.M = M; p.N = N; p.K = K; p.status = (int*)status;
     p.n_tiles = (N + GF_ROWS - 1) / GF_ROWS;
     // Tokens a tile (up to 128 or up to 64, the tiles alike) and ranges of K: what takes least by a block's rows a slab, counted with those of 128 weights, and some 600
-    // rows for its start and end, as long as all blocks run at once (ranges are for launches that leave SMs idle).  Clusters of eight fill the chip's groups of SMs
+    // rows for its start and end, as long as all blocks run at once (ranges, of four slabs or more each, are for launches that leave SMs idle).  Clusters of eight fill the chip's groups of SMs
     // badly: no more than half of it.  [1024, 2048], 247 tokens: 64 a tile and 4 ranges 16 us, 128 and 4 ranges 20.5; [4096, 1024]: 64 and 1 range 25.8, 128 and 2 24.7.
-    const int sms = msgl_sm_count(), asked = splits;
+    const int sms = msgl_sm_count();
+    int splits = 1;
     long long tiles = 0;
     double best = 0.0;
     for (int cap = 128; cap >= 64; cap /= 2) {
         const int m_tiles = (M + cap - 1) / cap, rows = ((M + m_tiles - 1) / m_tiles + 15) & ~15;
         const long long t = (long long)p.n_tiles * ((M + rows - 1) / rows);
-        for (int sp = asked ? asked : 1; sp <= (asked ? asked : GF_MAX_SPLITS); sp *= 2) {
-            if (!asked && sp > 1 && (t * sp > (sp == 8 ? sms / 2 : sms) || slabs < 4 * sp)) break;
+        for (int sp = 1; sp <= GF_MAX_SPLITS; sp *= 2) {
+            if (sp > 1 && (t * sp > (sp == 8 ? sms / 2 : sms) || slabs < 4 * sp)) break;
             const double cost = (double)((t * sp + sms - 1) / sms) * (600.0 + (double)((slabs + sp - 1) / sp) * (GF_ROWS + rows));
             if (tiles == 0 || cost < best) { best = cost; tiles = t; splits = sp; p.rows = rows; }
         }
     }
     const int rows = p.rows;
-    while (splits > slabs) splits /= 2;
     if (tiles * splits > 0x7fffffff) return MSGL_ERR_SIZE;
     p.splits = splits;
     const int blocks = (int)(tiles * splits);

@@ -102,7 +102,7 @@ def _lib():
         lib.msgl_gemm_tc2_splits.restype = c_int
         lib.msgl_gemm_rows.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_int, c_float, c_int,
                                        c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
-        lib.msgl_gemm_f32.argtypes = [c_void_p] * 4 + [c_int] * 3 + [c_ll, c_ll, c_int, c_void_p, c_void_p]
+        lib.msgl_gemm_f32.argtypes = [c_void_p] * 4 + [c_int] * 3 + [c_ll, c_ll, c_void_p, c_void_p]
         lib.msgl_tensor_maps.argtypes = []
         lib.msgl_tensor_maps.restype = c_int
         lib.msgl_sample.argtypes = [c_void_p, c_int, c_int, c_ll, c_void_p, c_void_p, c_void_p, c_ull, c_void_p,
@@ -862,7 +862,7 @@ def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
         return None
     M, (N, K) = x.shape[0], weight.shape
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    _check(_lib().msgl_gemm_f32(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), N, 0, _ptr(status), _stream()), "gemm_f32")
+    _check(_lib().msgl_gemm_f32(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), N, _ptr(status), _stream()), "gemm_f32")
     return out
 
 
