@@ -1663,7 +1663,7 @@ __device__ __forceinline__ void route_rows(const T* __restrict__ h, long long h_
 }
 
 template <typename T, int ROWS /* 0: any sizes and places, an element at a time */, int TOK>
-__global__ void __launch_bounds__(TOK > 1 ? 320 : 1024, TOK > 1 ? 2 : 1) route_kernel(const T* __restrict__ h, long long h_stride, const T* __restrict__ W,
+__global__ void __maxnreg__(ROWS == 0 ? 40 : TOK == 1 ? 64 : 96) route_kernel(const T* __restrict__ h, long long h_stride, const T* __restrict__ W,
                                                     const float* __restrict__ correction, int H, int E, int n_groups, int keep,
                                                     int top, int* __restrict__ idx, float* __restrict__ wts, int T_, int score,
                                                     int group_max, int renorm, const T* __restrict__ gate_row,
@@ -1806,7 +1806,9 @@ MSGL_API int msgl_route(const void* h, long long h_stride, const void* W, const 
     if (gate_row && !gate_out) return MSGL_ERR_SIZE;
     const int rows = E + (gate_row ? 1 : 0), sms = msgl_sm_count();
     const int tok = !vec || T_ <= sms ? 1 : T_ <= 2 * sms ? 2 : 4;
-    const int each = !vec ? 1 : tok == 1 ? 2 : 4, most = tok == 1 ? 32 : 10;             // rows a warp takes at a time, warps
+    // rows a warp takes at a time; warps.  Rows that are read an element at a time, 32 of 2,048 bfloat16: 200 tokens 32 warps 13.7 us, 16: 11.6;  700 tokens 32: 29.5, 8: 24.3.
+    // (40 registers a thread there: six blocks an SM.  With the 62 that the compiler would take, 700 tokens of 8 rows of 256 are 7.1 us in place of 4.7.)
+    const int each = !vec ? 1 : tok == 1 ? 2 : 4, most = T_ <= sms ? 32 : vec ? 10 : T_ <= 2 * sms ? 16 : 8;
     const int warps = (rows + each - 1) / each < 4 ? 4 : (rows + each - 1) / each < most ? (rows + each - 1) / each : most;
     const int blocks = (T_ + tok - 1) / tok;
     // Up to a block an SM the blocks are set up while the kernel before this one finishes.  More of them would pile up on the SMs whose share of that
