@@ -1612,7 +1612,7 @@ MSGL_API int msgl_unary_act(const void* x, long long x_stride, void* out, long l
 // ---------------------------------------------------------------------------------------
 #define RT_MAX_EXPERTS 1024
 #define RT_MAX_GROUPS 64
-// A few tokens (a decode step): a block a token, a warp two router rows.  Many tokens: a block has TOK of them and a warp four rows, so that a row is read
+// A few tokens (a decode step): a block a token, a warp two router rows.  Many tokens: a block has TOK of them and a warp four rows (two where there are few), so that a row is read
 // and unpacked once for TOK tokens; two blocks fit an SM.  The sums of a logit are the
 // same in all (one lane's elements in turn, then over the lanes), so the choice does not depend on the batch.  A warp a token then chooses.
 // Against a warp a row at a time and a token a block (us, warm): 33 bfloat16 rows of 2,048, 8 tokens 6.2 -> 4.9, 296: 8.2 -> 5.9, 700: 12.6 -> 10.3, 2,000:
@@ -1805,10 +1805,14 @@ MSGL_API int msgl_route(const void* h, long long h_stride, const void* W, const 
                     ((uintptr_t)gate_row % 16) == 0;
     if (gate_row && !gate_out) return MSGL_ERR_SIZE;
     const int rows = E + (gate_row ? 1 : 0), sms = msgl_sm_count();
-    const int tok = !vec || T_ <= sms ? 1 : T_ <= 2 * sms ? 2 : 4;
-    // rows a warp takes at a time; warps.  Rows that are read an element at a time, 32 of 2,048 bfloat16: 200 tokens 32 warps 13.7 us, 16: 11.6;  700 tokens 32: 29.5, 8: 24.3.
+    // Tokens a block and rows a warp takes at a time.  Few rows are few warps with four a warp, so up to 12 go by twos, and a token a block for as long as that leaves an SM no more
+    // than five.  Before it had its own line, 8 float32 rows of 4,096 took 11.7 us for 500 tokens (8.6 now; a row a warp and a token a block 8.6), 1,500 tokens 12.7 (10.7; 24.8).
+    const bool few = rows <= 12;
+    const int tok = !vec || T_ <= (few ? 5 : 1) * sms ? 1 : !few && T_ <= 2 * sms ? 2 : 4;
+    const int each = !vec ? 1 : tok == 1 || few ? 2 : 4;
+    // Warps.  Rows that are read an element at a time, 32 of 2,048 bfloat16: 200 tokens 32 warps 13.7 us, 16: 11.6;  700 tokens 32: 29.5, 8: 24.3.
     // (40 registers a thread there: six blocks an SM.  With the 62 that the compiler would take, 700 tokens of 8 rows of 256 are 7.1 us in place of 4.7.)
-    const int each = !vec ? 1 : tok == 1 ? 2 : 4, most = T_ <= sms ? 32 : vec ? 10 : T_ <= 2 * sms ? 16 : 8;
+    const int most = T_ <= sms ? 32 : vec ? 10 : T_ <= 2 * sms ? 16 : 8;
     const int warps = (rows + each - 1) / each < 4 ? 4 : (rows + each - 1) / each < most ? (rows + each - 1) / each : most;
     const int blocks = (T_ + tok - 1) / tok;
     // Up to a block an SM the blocks are set up while the kernel before this one finishes.  More of them would pile up on the SMs whose share of that
@@ -1827,6 +1831,7 @@ MSGL_API int msgl_route(const void* h, long long h_stride, const void* W, const 
         if (!vec) ROUTE_GO(T, 0, 1); \
         else if (tok == 1) ROUTE_GO(T, 2, 1); \
         else if (tok == 2) ROUTE_GO(T, 4, 2); \
+        else if (few) ROUTE_GO(T, 2, 4); \
         else ROUTE_GO(T, 4, 4); \
     } while (0)
     if (dtype == MSGL_F32) ROUTE(float);
