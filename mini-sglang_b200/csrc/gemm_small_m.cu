@@ -33,7 +33,7 @@
 constexpr int GS_WARPS = MSGL_GS_WARPS;
 constexpr int GS_PF = MSGL_GS_PF;      // chunks in flight per warp (ring depth)
 constexpr unsigned GS_AHEAD_PIECE = 256u;
-constexpr long long GS_AHEAD_MAX = 8 << 20;
+constexpr long long GS_AHEAD_MAX = 6500000;
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
                                           unsigned b0, unsigned b1) {
@@ -191,8 +191,11 @@ __global__ void __launch_bounds__(GS_WARPS * 32) gemm_small_m_kernel(
 }
 
 // ahead: the weights of the product that comes next (gated modes; or null), which the blocks ask into L2 as they end, so that the memory has work while the last of them and
-// the next launch leave it idle.  Only where all blocks run at once and the weights are a few megabytes: feed-forward of 1,024 x 3,072 (384 blocks), 1 token, five in a
-// row 43.3 -> 40.4 us; with more blocks the first ones' requests are in the way of the others' streams (2,048 x 6,144, 768 blocks: 20.6 -> 22.4; 4,096 x 12,288: 53.9 -> 57.5).
+// the next launch leave it idle.  A feed-forward with weights that come from memory, with the request / without it, us.  1,024 x 3,072 (384 blocks): 1 token 7.8 / 8.5, 8: 7.9 / 8.6;
+// 1,024 x 2,432 (304 blocks) 6.9 / 7.4; 256 x 2,560 5.3 / 5.9; 4,096 x 3,072 with 512 outputs 14.5 / 15.3.  So where more than two blocks an SM come and all run at once (three).  With
+// fewer each asks for more at its end, and the product itself is short: 1,024 x 1,024 (128 blocks) 5.7 / 5.5, 2,048 x 768 7.1 / 6.3; with more the first ones' requests are in the way of
+// the others' streams: 2,048 x 6,144 (768 blocks) 22.4 / 20.6.  Not for weights of more than 6.5 MB or half of this product's own: 1,024 x 2,432 with 1,664 outputs (8 MB) 8.0 / 7.8,
+// 512 x 2,432 with 1,536 outputs 7.2 / 6.6.  (Where all weights are in L2 already it costs up to 8 %.)
 // mode: 0 = plain (out [M, N]), 1 / 2 = SwiGLU / ReGLU (W [2I, K], bias [2I], out [M, I], N = 2I).  out_f32: output type.
 MSGL_API int msgl_gemm_small_m(const void* W, const void* X, const void* bias, void* out, int M, int N, int K,
                                long long ldx, long long ldo, int mode, int out_f32, const void* ahead, long long ahead_bytes, cudaStream_t stream) {
@@ -224,7 +227,8 @@ MSGL_API int msgl_gemm_small_m(const void* W, const void* X, const void* bias, v
         if (I & 7) return MSGL_ERR_SIZE;
         const int grid = I / 8;
         if (out_f32) return MSGL_ERR_DTYPE;
-        if (ahead_bytes < 0 || ahead_bytes > GS_AHEAD_MAX || ((ahead_bytes | (long long)(uintptr_t)ahead) & 15) || ahead == nullptr || grid > 3 * msgl_sm_count()) ahead_bytes = 0;
+        if (ahead_bytes < 0 || ahead_bytes > GS_AHEAD_MAX || ((ahead_bytes | (long long)(uintptr_t)ahead) & 15) || ahead == nullptr || ahead_bytes > 2LL * I * K ||
+            grid <= 2 * msgl_sm_count() || grid > 3 * msgl_sm_count()) ahead_bytes = 0;
 #define SMALL_M_GLU(NB, GLU, SMEM) \
     msgl_launch_pdl(gemm_small_m_kernel<NB, GLU, __nv_bfloat16>, dim3(grid), dim3(threads), SMEM, stream, w, x, b, (__nv_bfloat16*)out, M, N, K, ldx, ldo, I, (const unsigned char*)ahead, (unsigned)ahead_bytes)
         if (mode == MSGL_GLU_SILU) { if (M <= 8) SMALL_M_GLU(1, 1, smem1); else SMALL_M_GLU(2, 1, smem2); }
