@@ -1880,9 +1880,10 @@ SINK_ATTENTION_MAX_HEAD_DIM = 512
 SINK_ATTENTION_SPLIT_KEYS = 256     # keys of a piece when a one-token step cuts a request's keys over several blocks
 DELTA_RULE_MAX_KEY_DIM = 512
 DELTA_CHUNK, DELTA_CHUNK_KEY_DIMS = 32, (128,)      # tokens of a chunk; key sizes whose runs of tokens are taken in chunks
-# Tokens of a request in one step from which they are taken in chunks; token by token / in chunks, 16 heads of 128 x 128 bfloat16 (us, all kernels): one
-# request of 16 tokens 11.0 / 10.9, 24: 14.5 / 10.9, 64: 28.8 / 13.2, 100: 42.7 / 16.0; 16 requests of 16: 45 / 42, of 24: 61 / 43, of 100: 208 / 101;
-# 64 of 16: 162 / 158, of 24: 228 / 159
+# Tokens of a request in one step from which they are taken in chunks; token by token / in chunks, 16 heads of 128 x 128 (us, all kernels).  Bfloat16: one
+# request of 16 tokens 11.9 / 11.1, 24: 14.6 / 11.5, 64: 29 / 13, 100: 42 / 16; 4 of 16: 16.5 / 17.2; 16 of 16: 46 / 43, of 24: 61 / 43, of 100: 208 / 102;
+# 64 of 16: 162 / 160, of 24: 229 / 161.  Float32, whose rows are three parts: one of 24 14.4 / 13.9, 4 of 32: 25 / 26, 16 of 33: 78 / 104, of 48: 106 / 104, of 64: 136 / 106, of
+# 65: 139 / 138; 64 of 33: 299 / 406, of 48: 402 / 410, of 64: 518 / 419, of 65: 529 / 532, of 100: 780 / 652.  So float32 activations wait for 8 / 3 as many, 64.
 DELTA_CHUNK_MIN_TOKENS = 24
 
 
@@ -2080,12 +2081,13 @@ def delta_rule(qkv: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, heads: in
     B = q_start.numel() - 1
     # runs of tokens go in chunks, single tokens and short runs token by token: a matter of the request's own tokens in this step
     # and of the sizes, so a request's results do not depend on the requests beside it
-    long_runs = [n for n in q_lens or () if n >= DELTA_CHUNK_MIN_TOKENS] if key_dim in DELTA_CHUNK_KEY_DIMS and value_dim % 16 == 0 else []
+    least = min(DELTA_CHUNK_MIN_TOKENS if qkv.dtype == torch.bfloat16 else DELTA_CHUNK_MIN_TOKENS * 8 // 3, 0x7fffffff)
+    long_runs = [n for n in q_lens or () if n >= least] if key_dim in DELTA_CHUNK_KEY_DIMS and value_dim % 16 == 0 else []
     status = _status_words(qkv.device) if long_runs else None
     if status is None:
         long_runs = []
     n_chunks = sum(-(-n // DELTA_CHUNK) for n in long_runs)
-    short = not long_runs or any(0 < n < DELTA_CHUNK_MIN_TOKENS for n in q_lens)
+    short = not long_runs or any(0 < n < least for n in q_lens)
     if n_chunks and qkv.data_ptr() % 16:
         qkv = qkv.clone()            # the chunks' rows are read by 16 bytes
     # what does not depend on the state (unit q and k, beta, g, and for chunks all that lies within one) is made for all tokens at once
@@ -2095,7 +2097,7 @@ def delta_rule(qkv: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, heads: in
         torch.empty(numel, dtype=torch.float32, device=qkv.device)
     code = lib.msgl_delta_rule(qkv.data_ptr(), a.data_ptr(), stride, 0, _col_off(b, a), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), q_start.data_ptr(),
                                slots.data_ptr(), out.data_ptr(), scratch.data_ptr(), heads, kv_heads, key_dim, value_dim, T, B, dt, n_chunks,
-                               DELTA_CHUNK_MIN_TOKENS, short, _ptr(status), _stream())
+                               least, short, _ptr(status), _stream())
     _check(code, f"delta_rule (key size {key_dim})")
     global LAUNCHES
     LAUNCHES += 1 + 2 * int(short and n_chunks > 0)

@@ -92,3 +92,19 @@ def test_a_capture_before_the_status_words_exist(monkeypatch):
     assert ops._status is None
     graph.replay()
     assert (o - want).abs().max() < 1e-5 and (state - want_s).abs().max() < 1e-5              # (token by token: the bound above)
+
+
+def test_float32_runs_go_in_chunks_from_64_tokens_on(monkeypatch):
+    from mini_sglang_b200 import ops
+    H, G, dv = 2, 1, 16
+    for lens in ([63], [64], [63, 64, 65, 1]):
+        x = inputs(lens, H, G, dv, torch.float32)
+        before = ops.LAUNCHES
+        o, s = call(*x, lens, H, G, dv)
+        launches = ops.LAUNCHES - before
+        assert launches == {1: 2, 4: 4}[len(lens)]             # two kernels token by token, two in chunks, both where the step has both
+        with monkeypatch.context() as m:
+            m.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", 1 << 30)
+            o1, s1 = call(*x, lens, H, G, dv)
+        assert (o - o1).abs().max() < 1e-5 and (s - s1).abs().max() < 1e-5
+        assert torch.equal(o, o1) == (lens == [63])            # (another order of sums in chunks)
