@@ -1269,6 +1269,22 @@ __device__ __forceinline__ void dc_find(const int* q_start, int B, int n_min, in
         left -= __shfl_sync(0xffffffffu, sum, 31);
     }
 }
+// the `nth` request with n_min tokens or more and the chunks of those before it (one warp); at < 0: there is none
+__device__ __forceinline__ void dc_nth(const int* q_start, int B, int n_min, int nth, int& at, int& before) {
+    const int lane = threadIdx.x & 31;
+    int sum = 0;
+    at = -1;
+    for (int r0 = 0; r0 < B && at < 0; r0 += 32) {
+        const int r = r0 + lane;
+        const int n = r < B ? q_start[r + 1] - q_start[r] : 0;
+        const unsigned hits = __ballot_sync(0xffffffffu, n >= n_min);
+        const unsigned own = __ballot_sync(0xffffffffu, n >= n_min && __popc(hits & ((1u << lane) - 1u)) == nth);
+        if (own) at = r0 + __ffs(own) - 1;
+        else nth -= __popc(hits);
+        if (n >= n_min && (at < 0 || r < at)) sum += (n + DC_C - 1) / DC_C;
+    }
+    before = __reduce_add_sync(0xffffffffu, sum);
+}
 }  // namespace
 
 template <typename T, int D> struct DcPrep {     // shared memory of delta_chunk_kernel, in bytes
@@ -1521,6 +1537,9 @@ constexpr int DC_WALKERS = 256, DC_READERS = 128;
 // a chunk, 121 us; tensor cores with W = R (beta P K) and U = R (beta v) from the first kernel in place of R, three times the copies and twice the
 // products, took 85.  Errors against 64 bits there: outputs 2.0e-7 (multiply-adds 2.4e-7), states 1.8e-7 (2.0e-7).
 //
+// A block a long request, not a request: the blocks of the others, a hundred kilobytes of shared memory each, cost more than they look (one of 24 tokens beside 63 single ones, 16 heads:
+// 73 -> 67 us, 32 heads: 148 -> 134).
+//
 // Named barriers (each side meets the other once a chunk, in turn): 1 the first chunk, 3 partial sums of K S, 4 u, 5 partial sums of Q S, 6 Q S read.
 template <typename T, int D>
 __global__ void __launch_bounds__(DC_WALKERS + DC_READERS, DcSizes<T, D>::PARTS == 1 ? 2 : 1) delta_chunk_scan_kernel(const DeltaChunkParams p) {
@@ -1532,29 +1551,26 @@ __global__ void __launch_bounds__(DC_WALKERS + DC_READERS, DcSizes<T, D>::PARTS 
     float* PK = reinterpret_cast<float*>(dc_smem + St::PK);                         // [C][LDP]: walker w's sums at 16 w
     float* PQ = reinterpret_cast<float*>(dc_smem + St::PQ);
     __nv_bfloat16* up = reinterpret_cast<__nv_bfloat16*>(dc_smem + St::UP);         // [3][C][LDU]
-    __shared__ int first_s;
-    const int h = blockIdx.x, c0 = blockIdx.y * DC_COLS, r = blockIdx.z;
+    __shared__ int where_s[2];
+    const int h = blockIdx.x, c0 = blockIdx.y * DC_COLS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int t0 = p.q_start[r], n = p.q_start[r + 1] - t0;
-    if (n < p.n_min) return;
     const int g = h / (p.heads / p.kv_heads), dv = p.dv;
     const unsigned bar = (unsigned)__cvta_generic_to_shared(dc_smem + St::BAR);     // a barrier a stage
-    if (warp == 0) {                                         // chunks of the requests before this one
-        int sum = 0;
-        for (int i = lane; i < r; i += 32) {
-            const int m = p.q_start[i + 1] - p.q_start[i];
-            sum += m >= p.n_min ? (m + DC_C - 1) / DC_C : 0;
-        }
-        sum = __reduce_add_sync(0xffffffffu, sum);
+    if (warp == 0) {
+        int at, before;
+        dc_nth(p.q_start, p.B, p.n_min, blockIdx.z, at, before);
         if (lane == 0) {
-            first_s = sum;
+            where_s[0] = at; where_s[1] = before;
             tc_mbar_init(bar, 1); tc_mbar_init(bar + 8u, 1);
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         }
     }
     __syncthreads();
-    const size_t first = (size_t)first_s;
-    const int n_chunks = min((n + DC_C - 1) / DC_C, p.n_chunks - first_s);         // (no more than the host's count has room for)
+    const int r = where_s[0];
+    if (r < 0) return;
+    const int t0 = p.q_start[r], n = p.q_start[r + 1] - t0;
+    const size_t first = (size_t)where_s[1];
+    const int n_chunks = min((n + DC_C - 1) / DC_C, p.n_chunks - where_s[1]);         // (no more than the host's count has room for)
     if (n_chunks <= 0) return;
     auto wait = [&](int c) {                                 // for the operands of chunk c: one thread, the others meet it at a barrier
         if (!tc_mbar_wait(bar + 8u * (c & 1), (unsigned)(c >> 1) & 1u)) atomicExch(p.status + 1, 1);
@@ -1777,7 +1793,7 @@ MSGL_API long long msgl_delta_rule_scratch(int T_, int heads, int kv_heads, int 
 }
 
 template <typename T, int D>
-static int delta_chunk_launch(DeltaChunkParams& p, unsigned char* scratch, int n_chunks, cudaStream_t stream) {
+static int delta_chunk_launch(DeltaChunkParams& p, unsigned char* scratch, int n_chunks, int n_long, cudaStream_t stream) {
     using Z = DcSizes<T, D>;
     constexpr int smem1 = DcPrep<T, D>::TOTAL, smem2 = DcStage<T, D>::TOTAL;
     static_assert(Z::PARTS > 1 || 2 * (smem2 + 1024 + 64) <= 228 * 1024, "two blocks of the walk an SM");
@@ -1794,18 +1810,18 @@ static int delta_chunk_launch(DeltaChunkParams& p, unsigned char* scratch, int n
     p.n_chunks = n_chunks;
     p.K = scratch; p.Q = p.K + cg * Z::KQ; p.R = p.Q + cg * Z::KQ; p.M = p.R + ch * Z::M;
     delta_chunk_kernel<T, D><<<dim3(n_chunks, p.heads), DC_THREADS, smem1, stream>>>(p);
-    delta_chunk_scan_kernel<T, D><<<dim3(p.heads, p.dv / DC_COLS, p.B), DC_WALKERS + DC_READERS, smem2, stream>>>(p);
+    delta_chunk_scan_kernel<T, D><<<dim3(p.heads, p.dv / DC_COLS, n_long), DC_WALKERS + DC_READERS, smem2, stream>>>(p);
     return msgl_check_launch();
 }
 
-// n_chunks, n_min: chunks of DC_C tokens of the requests with n_min tokens or more (host's count), which are taken in chunks; 0: none.
+// n_chunks, n_long, n_min: chunks of DC_C tokens and number of the requests with n_min tokens or more (host's count), which are taken in chunks; 0: none.
 // n_short: whether requests with fewer tokens are in the step.
 MSGL_API int msgl_delta_rule(const void* qkv, const void* proj, long long proj_stride, int a_off, int b_off, const float* a_log,
                              const float* dt_bias, float* state, const int* q_start, const int* slots, float* out, float* scratch,
-                             int heads, int kv_heads, int d, int dv, int T_, int B, int dtype, int n_chunks, int n_min, int n_short,
+                             int heads, int kv_heads, int d, int dv, int T_, int B, int dtype, int n_chunks, int n_long, int n_min, int n_short,
                              void* status, cudaStream_t stream) {
     if (B <= 0 || T_ <= 0) return MSGL_OK;
-    if (n_chunks > 0 && (!delta_chunks_ok(d, dv) || n_min < 1 || B > 65535 || heads > 65535 || dv / DC_COLS > 65535)) return MSGL_ERR_SIZE;
+    if (n_chunks > 0 && (!delta_chunks_ok(d, dv) || n_min < 1 || n_long < 1 || n_long > B || B > 65535 || heads > 65535 || dv / DC_COLS > 65535)) return MSGL_ERR_SIZE;
     if (n_chunks > 0 && (((uintptr_t)qkv & 15) != 0 || status == nullptr)) return MSGL_ERR_ALIGN;
     if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || d <= 0 || dv <= 0 || d > DR_PARTS * 64 || scratch == nullptr) return MSGL_ERR_SIZE;
     if (((uintptr_t)scratch & 15) != 0) return MSGL_ERR_ALIGN;
@@ -1830,8 +1846,8 @@ MSGL_API int msgl_delta_rule(const void* qkv, const void* proj, long long proj_s
         c.state = state; c.q_start = q_start; c.slots = slots; c.out = out; c.status = (int*)status;
         c.heads = heads; c.kv_heads = kv_heads; c.dv = dv; c.B = B; c.n_min = n_min;
         unsigned char* rest = reinterpret_cast<unsigned char*>(scratch + (n_short ? delta_prep_floats(T_, heads, kv_heads, d) : 0));
-        if (dtype == MSGL_F32) code = delta_chunk_launch<float, 128>(c, rest, n_chunks, stream);
-        else code = delta_chunk_launch<__nv_bfloat16, 128>(c, rest, n_chunks, stream);
+        if (dtype == MSGL_F32) code = delta_chunk_launch<float, 128>(c, rest, n_chunks, n_long, stream);
+        else code = delta_chunk_launch<__nv_bfloat16, 128>(c, rest, n_chunks, n_long, stream);
         if (code != MSGL_OK || !n_short) return code;
     }
     const int many_cols = DR_MANY_WARPS * DR_WCOLS;

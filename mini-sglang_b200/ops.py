@@ -1899,7 +1899,7 @@ def _delta_lib():
             [c_int] * 12 + [c_float, c_float, c_int, c_void_p, c_ll, c_int, c_void_p]
         lib.msgl_sink_attention_mma.argtypes = [c_void_p] * 6 + [c_int, c_int, c_int, c_void_p, c_void_p, c_ll, c_void_p, c_void_p] + \
             [c_int] * 10 + [c_float, c_float, c_void_p, c_ll, c_int, c_void_p]
-        lib.msgl_delta_rule.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_int] + [c_void_p] * 7 + [c_int] * 10 + [c_void_p] * 2
+        lib.msgl_delta_rule.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_int] + [c_void_p] * 7 + [c_int] * 11 + [c_void_p] * 2
         lib.msgl_delta_rule_scratch.argtypes = [c_int] * 8
         lib.msgl_delta_rule_scratch.restype = c_ll
         lib.msgl_side_gate_mul.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p]
@@ -2097,7 +2097,7 @@ def delta_rule(qkv: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, heads: in
         torch.empty(numel, dtype=torch.float32, device=qkv.device)
     code = lib.msgl_delta_rule(qkv.data_ptr(), a.data_ptr(), stride, 0, _col_off(b, a), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), q_start.data_ptr(),
                                slots.data_ptr(), out.data_ptr(), scratch.data_ptr(), heads, kv_heads, key_dim, value_dim, T, B, dt, n_chunks,
-                               least, short, _ptr(status), _stream())
+                               len(long_runs), least, short, _ptr(status), _stream())
     _check(code, f"delta_rule (key size {key_dim})")
     global LAUNCHES
     LAUNCHES += 1 + 2 * int(short and n_chunks > 0)

@@ -108,3 +108,17 @@ def test_float32_runs_go_in_chunks_from_64_tokens_on(monkeypatch):
             o1, s1 = call(*x, lens, H, G, dv)
         assert (o - o1).abs().max() < 1e-5 and (s - s1).abs().max() < 1e-5
         assert torch.equal(o, o1) == (lens == [63])            # (another order of sums in chunks)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_long_requests_anywhere_among_many_short_ones(dtype, monkeypatch):
+    from mini_sglang_b200 import ops
+    H, G, dv = 1, 1, 16
+    for long_ones in ((0,), (31, 32), (0, 30, 33, 63, 64, 69)):
+        lens = [64 + 33 * (i % 3) if i in long_ones else 1 + i % 5 for i in range(70)]
+        x = inputs(lens, H, G, dv, dtype)
+        o, s = call(*x, lens, H, G, dv)
+        with monkeypatch.context() as m:
+            m.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", 1 << 30)
+            o1, s1 = call(*x, lens, H, G, dv)
+        assert (o - o1).abs().max() < 1e-5 and (s - s1).abs().max() < 1e-5
