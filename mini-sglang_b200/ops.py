@@ -1880,11 +1880,12 @@ SINK_ATTENTION_MAX_HEAD_DIM = 512
 SINK_ATTENTION_SPLIT_KEYS = 256     # keys of a piece when a one-token step cuts a request's keys over several blocks
 DELTA_RULE_MAX_KEY_DIM = 512
 DELTA_CHUNK, DELTA_CHUNK_KEY_DIMS = 32, (128,)      # tokens of a chunk; key sizes whose runs of tokens are taken in chunks
-# Tokens of a request in one step from which they are taken in chunks; token by token / in chunks, 16 heads of 128 x 128 (us, all kernels).  Bfloat16: one
-# request of 16 tokens 11.9 / 11.1, 24: 14.6 / 11.5, 64: 29 / 13, 100: 42 / 16; 4 of 16: 16.5 / 17.2; 16 of 16: 46 / 43, of 24: 61 / 43, of 100: 208 / 102;
-# 64 of 16: 162 / 160, of 24: 229 / 161.  Float32, whose rows are three parts: one of 24 14.4 / 13.9, 4 of 32: 25 / 26, 16 of 33: 78 / 104, of 48: 106 / 104, of 64: 136 / 106, of
-# 65: 139 / 138; 64 of 33: 299 / 406, of 48: 402 / 410, of 64: 518 / 419, of 65: 529 / 532, of 100: 780 / 652.  So float32 activations wait for 8 / 3 as many, 64.
-DELTA_CHUNK_MIN_TOKENS = 24
+# Tokens of a request in one step from which they are taken in chunks: a whole chunk, and two of float32, whose rows are three parts.  Token by token / in chunks, us, all kernels,
+# heads of 128 x 128.  Bfloat16, 16 heads: one request of 24 14.6 / 11.5, 64: 29 / 13, 100: 42 / 16; 16 of 24: 61 / 43, of 100: 208 / 102; 64 of 24: 229 / 161.  One beside 63 single
+# tokens, which then take kernels of their own: 24 60 / 67, 32: 63 / 66, 48: 70 / 69, 64: 77 / 69; 32 heads 24: 128 / 134, 32: 130 / 135, 64: 137 / 138, 100: 159 / 143; beside one, 2 heads,
+# 24: 14.5 / 16.6.  Float32: one of 24 14.4 / 13.9; 16 of 33: 78 / 104, of 48: 106 / 104, of 64: 136 / 106, of 65: 139 / 138; 64 of 48: 402 / 410, of 64: 518 / 419, of 65: 529 / 532, of
+# 100: 780 / 652; 64 beside 63 single ones, 16 heads 77 / 72, 32: 138 / 147.
+DELTA_CHUNK_MIN_TOKENS = 32
 
 
 def _delta_lib():
@@ -2081,7 +2082,7 @@ def delta_rule(qkv: torch.Tensor, a: torch.Tensor, b: torch.Tensor, *, heads: in
     B = q_start.numel() - 1
     # runs of tokens go in chunks, single tokens and short runs token by token: a matter of the request's own tokens in this step
     # and of the sizes, so a request's results do not depend on the requests beside it
-    least = min(DELTA_CHUNK_MIN_TOKENS if qkv.dtype == torch.bfloat16 else DELTA_CHUNK_MIN_TOKENS * 8 // 3, 0x7fffffff)
+    least = min(DELTA_CHUNK_MIN_TOKENS if qkv.dtype == torch.bfloat16 else 2 * DELTA_CHUNK_MIN_TOKENS, 0x7fffffff)
     long_runs = [n for n in q_lens or () if n >= least] if key_dim in DELTA_CHUNK_KEY_DIMS and value_dim % 16 == 0 else []
     status = _status_words(qkv.device) if long_runs else None
     if status is None:

@@ -122,3 +122,16 @@ def test_long_requests_anywhere_among_many_short_ones(dtype, monkeypatch):
             m.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", 1 << 30)
             o1, s1 = call(*x, lens, H, G, dv)
         assert (o - o1).abs().max() < 1e-5 and (s - s1).abs().max() < 1e-5
+
+
+def test_bfloat16_runs_go_in_chunks_from_32_tokens_on():
+    from mini_sglang_b200 import ops
+    H, G, dv = 2, 1, 16
+    for lens, kernels in (([31], 2), ([32], 2), ([31, 32, 33, 1], 4)):
+        x = inputs(lens, H, G, dv, torch.bfloat16)
+        before = ops.LAUNCHES
+        o, s = call(*x, lens, H, G, dv)
+        assert ops.LAUNCHES - before == kernels
+        if lens[0] == 31:                                      # a request's results do not depend on those beside it
+            alone, end = call(x[0][:31].clone(), x[1][:31], x[2], x[3], x[4][:1], [31], H, G, dv)
+            assert torch.equal(alone, o[:31]) and torch.equal(end[0], s[0])
