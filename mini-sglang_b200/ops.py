@@ -855,7 +855,7 @@ def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
             and not _observed(x, weight, bias)
             and x.get_device() == torch._C._cuda_getDevice()         # the launch goes to the current device's stream; the library changes the device
-            and not torch.is_autocast_enabled("cuda") and torch._C._get_fp32_precision_getter("cuda", "matmul") != "tf32"):
+            and not torch.is_autocast_enabled() and torch._C._get_fp32_precision_getter("cuda", "matmul") != "tf32"):
         return None
     status = _status_words(x.device)
     if status is None:
