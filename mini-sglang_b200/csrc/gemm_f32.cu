@@ -21,8 +21,8 @@
 // library 48); [1024, 2048], 64 tokens: 12.5, 21, 25, 75 and 18 (37).
 //
 // Bound by the split (11 instructions a pair of numbers) and the stores of the parts to shared memory.  Against the library's float32 product:
-// [4096, 1024] 247 tokens 45.1 -> 24.6 us (84 TFLOP/s of float32; multiply-adds give 74 at the most), 9 tokens 27.0 -> 10.1; [1024, 2048] 46.8 -> 16.6 and 19.5 -> 8.9.
-// Errors against 64 bits 1e-7, the library's 2e-7 to 1e-6.
+// [4096, 1024] 247 tokens 45.1 -> 23.1 us (90 TFLOP/s of float32; multiply-adds give 74 at the most), 9 tokens 19.3 -> 9.8; [1024, 2048] 39.6 -> 17.1 and 19.6 -> 9.2.
+// Errors against 64 bits 1e-7 with terms of both signs (the library's 2e-7 to 1e-6) and 0.9e-7 with terms of one (0.7e-7 to 6e-7).
 #include "common.cuh"
 #include "tc_common.cuh"
 #include <math.h>

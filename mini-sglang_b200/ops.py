@@ -833,9 +833,10 @@ def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     return out
 
 
-# Float32 products on the tensor cores against the library's, us, library / kernel.  [4096, 1024] at 4 rows 13.7 / 10.1, 1: 5.7 / 9.9, 9: 27.0 / 10.1, 64: 27.4 / 12.7,
-# 247: 45.1 / 24.6, 600: 122.7 / 67.5; [1024, 2048] at 9: 19.5 / 8.9, 247: 46.8 / 16.6; [12288, 2048] at 600: 574 / 268; [512, 1024] at 9: 8.6 / 8.0; [2048, 512] at
-# 16: 10.7 / 8.6, 64: 11.0 / 11.3; [1024, 512] at 16: 7.1 / 8.6, 64: 10.9 / 11.3.  Errors against 64 bits, relative: 0.9e-7 to 1.3e-7, the library's 1.9e-7 to 1e-6.
+# Float32 products on the tensor cores against the library's, us, library / kernel.  [4096, 1024] at 4 rows 9.0 / 9.8, 9: 19.2 / 9.8, 64: 21.8 / 12.3, 256: 45.0 / 23.4,
+# 600: 121 / 63; [1024, 2048] at 9: 19.9 / 9.2, 256: 39.5 / 17.2; [5120, 5120] at 9: 88 / 48, 1,000: 1,031 / 409; [512, 1024] at 9: 9.1 / 8.4, 64: 16.6 / 10.7; [2048, 512] at 9: 11.1 / 8.7,
+# 64: 11.5 / 11.5, 128: 12.5 / 11.6; [1024, 512] at 16: 7.6 / 9.1, 128: 11.5 / 11.7.  With 4 rows the library is ahead on half of 17 sizes, with 6 on none that the rule has;
+# from 9, above the bfloat16 kernels for a few rows, the kernel is never behind.  Errors against 64 bits, relative: 0.9e-7 to 1.3e-7, the library's 1.9e-7 to 1e-6.
 F32_MIN_ROWS, F32_MIN_INNER, F32_LONG_INNER, F32_MIN_WEIGHT, F32_MIN_WEIGHT_LONG = 9, 512, 1024, 1_000_000, 500_000
 
 
