@@ -850,11 +850,12 @@ def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
     and whatever a kernel called by address would slip past."""
     if not (x.dtype == torch.float32 and weight.dtype == torch.float32 and x.dim() == 2 and weight.dim() == 2
             and _f32_rule(x.shape[0], weight.shape[0], weight.shape[1]) and x.shape[1] == weight.shape[1] and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1]
-            and weight.is_contiguous() and weight.shape[1] % 8 == 0 and x.get_device() == weight.get_device() and (x.data_ptr() | weight.data_ptr()) % 16 == 0
+            and weight.is_contiguous() and weight.shape[1] % 8 == 0 and x.get_device() == weight.get_device()
             and (bias is None or (bias.dtype == torch.float32 and bias.dim() == 1 and bias.shape[0] == weight.shape[0] and bias.is_contiguous()
                                   and bias.get_device() == weight.get_device()))
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
-            and not _observed(x, weight, bias)
+            and not _observed(x, weight, bias)                       # (before the addresses are asked for: some of these have none)
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0
             and x.get_device() == torch._C._cuda_getDevice()         # the launch goes to the current device's stream; the library changes the device
             and not torch.is_autocast_enabled() and torch._C._get_fp32_precision_getter("cuda", "matmul") != "tf32"):
         return None

@@ -72,3 +72,32 @@ def test_calls_that_are_traced_mapped_or_differentiated_stay_with_the_library():
         call(x)
     assert seen == [None] * 6
     assert not ops._observed(x, w) and not ops._observed(x, torch.nn.Parameter(w))
+
+
+def test_float32_calls_that_are_traced_mapped_or_differentiated_stay_with_the_library():
+    """The same of the float32 product, whose operands have no address while something maps over them or stands in for them."""
+    import torch.autograd.forward_ad as forward_ad
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils.flop_counter import FlopCounterMode
+
+    from mini_sglang_b200 import ops
+    x, w = torch.zeros((16, 512)), torch.zeros((2048, 512))
+    seen = []
+
+    def call(t):
+        seen.append(ops._gemm_f32(t, w, None))
+        return t + 1
+
+    torch.func.vmap(call)(x.expand(2, 16, 512).contiguous())
+    torch.func.jvp(call, (x,), (x,))
+    make_fx(call)(x)
+    make_fx(call, tracing_mode="fake")(x)
+    torch.jit.trace(call, x, check_trace=False)
+    with forward_ad.dual_level():
+        call(forward_ad.make_dual(x, x))
+    with FlopCounterMode(display=False):
+        call(x)
+    with FakeTensorMode() as fake:
+        assert ops._gemm_f32(fake.from_tensor(x), fake.from_tensor(w), None) is None
+    assert seen == [None] * 7
