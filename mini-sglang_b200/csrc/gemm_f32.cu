@@ -17,7 +17,7 @@
 //
 // Numbers that three bfloat16 parts do not hold (infinities, NaN, the last 2^-8 below the largest number, and most of those below 2^-110 other than 0: bfloat16 ends at 2^-133)
 // are seen on the way by what the split leaves.  The block then does the sums of the tokens and weight rows that have one again in plain multiply-adds, so they behave as in float32
-// arithmetic, and all other sums keep their bits.  [4096, 1024], 247 tokens, such a number in none, one, every 64th, every token: 25, 40, 51, 208 us, in one weight row 39 (the
+// arithmetic, and all other sums keep their bits.  (The parts of a product may lie up to 2^-8 above it: a sum that close to the largest number can come out infinite.)  [4096, 1024], 247 tokens, such a number in none, one, every 64th, every token: 25, 40, 51, 208 us, in one weight row 39 (the
 // library 48); [1024, 2048], 64 tokens: 12.5, 21, 25, 75 and 18 (37).
 //
 // Bound by the split (11 instructions a pair of numbers) and the stores of the parts to shared memory.  Against the library's float32 product:

@@ -805,9 +805,9 @@ _PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
 def _observed(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> bool:
-    """Whether something looks on that a kernel called by address would slip past: tracing, a dispatch mode, vmap and its like, forward-mode
+    """Whether something looks on that a kernel called by address would slip past: compiling, tracing, a dispatch mode, vmap and its like, forward-mode
     derivatives, a tensor of another class."""
-    return (type(x) not in _PLAIN or type(weight) not in _PLAIN or (bias is not None and type(bias) not in _PLAIN) or torch._C._len_torch_dispatch_stack() > 0
+    return (torch.compiler.is_compiling() or type(x) not in _PLAIN or type(weight) not in _PLAIN or (bias is not None and type(bias) not in _PLAIN) or torch._C._len_torch_dispatch_stack() > 0
             or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0
             or torch._C._get_tracing_state() is not None)
 

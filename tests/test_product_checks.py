@@ -101,3 +101,11 @@ def test_float32_calls_that_are_traced_mapped_or_differentiated_stay_with_the_li
     with FakeTensorMode() as fake:
         assert ops._gemm_f32(fake.from_tensor(x), fake.from_tensor(w), None) is None
     assert seen == [None] * 7
+
+
+def test_float32_calls_are_compiled_whole(monkeypatch):
+    from mini_sglang_b200 import ops
+    monkeypatch.setattr(ops, "_need_cuda", lambda *tensors: None)
+    x, w, b = torch.randn((16, 512)), torch.randn((2048, 512)), torch.randn(2048)
+    whole = torch.compile(lambda t: ops.linear(t, w, b), backend="eager", fullgraph=True)
+    assert torch.equal(whole(x), torch.nn.functional.linear(x, w, b))
