@@ -844,27 +844,39 @@ def _f32_rule(rows: int, n_out: int, K: int) -> bool:
     return rows >= F32_MIN_ROWS and K >= F32_MIN_INNER and n_out * K >= (F32_MIN_WEIGHT_LONG if K >= F32_LONG_INNER else F32_MIN_WEIGHT)
 
 
+def _tf32() -> bool:
+    """Whether the library's float32 products may use TF32.  The older question is five times as quick, but raises where the newer switches were used."""
+    try:
+        return torch._C._get_cublas_allow_tf32()
+    except RuntimeError:
+        return torch._C._get_fp32_precision_getter("cuda", "matmul") == "tf32"
+
+
 def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     """x @ weight^T + bias in float32 on the tensor cores (csrc/gemm_f32.cu); None where the library's float32 product is to be called: few rows or
     small weights, operands that do not lie as the kernel reads them or on another device than the current one, products that the caller wants in another precision (autocast, TF32),
     and whatever a kernel called by address would slip past."""
-    if not (x.dtype == torch.float32 and weight.dtype == torch.float32 and x.dim() == 2 and weight.dim() == 2
-            and _f32_rule(x.shape[0], weight.shape[0], weight.shape[1]) and x.shape[1] == weight.shape[1] and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.stride(0) >= x.shape[1]
-            and weight.is_contiguous() and weight.shape[1] % 8 == 0 and x.get_device() == weight.get_device()
-            and (bias is None or (bias.dtype == torch.float32 and bias.dim() == 1 and bias.shape[0] == weight.shape[0] and bias.is_contiguous()
-                                  and bias.get_device() == weight.get_device()))
+    if not (x.dtype == torch.float32 and weight.dtype == torch.float32 and x.dim() == 2 and weight.dim() == 2):
+        return None
+    (M, K), (N, k_weight) = x.shape, weight.shape
+    if K != k_weight or K % 8 or not _f32_rule(M, N, K):
+        return None
+    pitch, dev = x.stride(0), x.get_device()
+    if not (x.stride(1) == 1 and pitch % 4 == 0 and pitch >= K and weight.is_contiguous() and weight.get_device() == dev
+            and (bias is None or (bias.dtype == torch.float32 and bias.dim() == 1 and bias.shape[0] == N and bias.is_contiguous() and bias.get_device() == dev))
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
-            and not _observed(x, weight, bias)                       # (before the addresses are asked for: some of these have none)
-            and (x.data_ptr() | weight.data_ptr()) % 16 == 0
-            and x.get_device() == torch._C._cuda_getDevice()         # the launch goes to the current device's stream; the library changes the device
-            and not torch.is_autocast_enabled() and torch._C._get_fp32_precision_getter("cuda", "matmul") != "tf32"):
+            and not _observed(x, weight, bias)):                     # (before the addresses are asked for: some of these have none)
+        return None
+    x_at, w_at = x.data_ptr(), weight.data_ptr()
+    if (x_at | w_at) % 16 or dev != torch._C._cuda_getDevice():      # (the launch goes to the current device's stream; the library changes the device)
+        return None
+    if torch.is_autocast_enabled() or _tf32():
         return None
     status = _status_words(x.device)
     if status is None:
         return None
-    M, (N, K) = x.shape[0], weight.shape
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    _check(_lib().msgl_gemm_f32(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), N, _ptr(status), _stream()), "gemm_f32")
+    _check(_lib().msgl_gemm_f32(w_at, x_at, _ptr(bias), out.data_ptr(), M, N, K, pitch, N, status.data_ptr(), _stream()), "gemm_f32")
     return out
 
 

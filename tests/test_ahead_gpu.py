@@ -15,3 +15,18 @@ def test_results_do_not_change(M, I, K, rows):
     for a in (nxt, nxt[:, :I], nxt[:, :I].contiguous(), nxt.view(-1)[1:], nxt[:1, :3].contiguous(), nxt.cpu()):
         assert torch.equal(ops.linear_swiglu(x, w, a), want)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("blocks_an_sm", [2, 3])
+def test_at_the_edges_of_the_rule(M, blocks_an_sm):
+    from mini_sglang_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(M)
+    for blocks in (blocks_an_sm * ops.sm_count("cuda") + i for i in (0, 1)):
+        I, K = 8 * blocks, 96
+        x, w = (torch.randn(s, generator=g, device="cuda").bfloat16() for s in ((M, K), (2 * I, K)))
+        want, relu = ops.linear_swiglu(x, w), ops.linear_glu(x, w, None, ops.ACT_RELU)
+        for rows in (8, K, K + 8):                                # up to half of the product's own weights, and more
+            nxt = torch.randn((rows, I), generator=g, device="cuda").bfloat16()
+            assert torch.equal(ops.linear_swiglu(x, w, nxt), want) and torch.equal(ops.linear_glu(x, w, None, ops.ACT_RELU, nxt), relu)
+    torch.cuda.synchronize()

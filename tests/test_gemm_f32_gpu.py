@@ -78,6 +78,12 @@ def test_products_wanted_in_another_precision_stay_with_the_library():
         assert ops._gemm_f32(x, w, b) is None
     finally:
         ops.set_true_fp32()
+    torch.backends.cuda.matmul.fp32_precision = "tf32"         # the newer switch
+    try:
+        assert ops._gemm_f32(x, w, b) is None
+    finally:
+        torch.backends.cuda.matmul.fp32_precision = "ieee"
+        ops.set_true_fp32()
     assert ops._gemm_f32(x, w, b) is not None
 
 
