@@ -21,6 +21,7 @@
 //                               tensor cores with accumulators in tensor memory (attention_tc2.cuh, attention_tc.cuh)
 //   attn_mma_kernel<D>          bfloat16, the same runs at other head sizes (16..256 in steps of 16): mma.sync
 //                               m16n8k16, 64 rows per block, each warp owns 16 rows and walks all keys of a tile
+//   attn_decode_runs_kernel     bfloat16, head size 128, a step of single tokens: cuts up the keys by itself, one launch (attention_runs.cuh)
 //   attn_decode_t_kernel<D,...> bfloat16, short query runs (decode), head sizes in steps of 32: keys on the M
 //                               dimension of the mma, K straight from global memory into registers, kv splits
 //   attn_decode_even_kernel<D,...> the same arithmetic for a decode step whose keys the host has dealt out evenly over
@@ -1755,6 +1756,9 @@ __global__ void attn_combine_diff_kernel(const float* __restrict__ part_o, const
 #if MSGL_HEAD_DIM == 128
 #include "attention_tc.cuh"
 #include "attention_tc2.cuh"
+#if MSGL_HEAD_DIM == 128
+#include "attention_runs.cuh"
+#endif
 #endif
 
 // ---------------------------------------------------------------------------------------

@@ -61,8 +61,8 @@ def build_dir() -> str:
 
 
 # files a source pulls in with #include: an edit of any of them rebuilds the library
-INCLUDED = {"attention.cu": ["tc_common.cuh", "attention_tc.cuh", "attention_tc2.cuh"],
-            "attention_noalloc.cu": ["attention.cu", "tc_common.cuh", "attention_tc.cuh", "attention_tc2.cuh", "attention_noalloc.h"],
+INCLUDED = {"attention.cu": ["tc_common.cuh", "attention_tc.cuh", "attention_tc2.cuh", "attention_runs.cuh"],
+            "attention_noalloc.cu": ["attention.cu", "tc_common.cuh", "attention_tc.cuh", "attention_tc2.cuh", "attention_runs.cuh", "attention_noalloc.h"],
             "gemm_tc.cu": ["tc_common.cuh"], "gemm_rows.cu": ["tc_common.cuh"], "gemm_f32.cu": ["tc_common.cuh"], "mixers_delta.cu": ["tc_common.cuh"], "decode_step.cu": []}
 
 

@@ -125,6 +125,8 @@ def _attn_lib(head_dim: int):
         lib.msgl_attention_combine_diff.argtypes = [c_void_p] * 5 + [c_int, c_void_p] + [c_int] * 5 + [c_float, c_float, c_float, c_void_p]
         lib.msgl_attention_combine_range.argtypes = [c_void_p] * 4 + [c_int] * 9 + [c_void_p, c_void_p, c_ll, c_void_p]
         lib.msgl_attention_head_dim.restype = c_int
+        if hd == 128:
+            lib.msgl_attention_decode_runs.argtypes = [c_void_p] * 9 + [c_int] * 5 + [c_float, c_int, c_void_p]
         _attn[hd] = lib
     return lib
 
@@ -617,6 +619,33 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache
         max_split, float(scale), qlen_min, qlen_max, int(uniform_decode), variant, grid_x, _dt(q), _ptr(order), _ptr(even), int(even_nb),
         _ptr(null_log2), _ptr(gate), gate_stride, int(chunk), int(diff is not None), *(diff or (0.0, 0.0, 0.0)), _stream())
     _check(code, f"attention (head size {d}, variant {variant})")
+
+
+RUNS_MAX_REQUESTS, RUNS_MAX_BLOCKS, RUNS_COUNTERS = 256, 256, 4096
+
+
+def attention_decode_runs(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, *, kv_len: torch.Tensor,
+                          block_table: torch.Tensor, n_kv: int, page_size: int, scale: float, workspace) -> bool:
+    """Attention of a decode step (one new token a request, all of a request's keys) in one launch that deals the keys out over the SMs by
+    itself and merges its partial results (csrc/attention_runs.cuh).  -> False where it does not apply: bfloat16, head size 128, up to eight
+    query heads a kv head, pages of whole units of 16 keys, up to 256 requests; inside a stream capture only once its counters exist."""
+    B, n_q, d = q.shape
+    if (workspace is None or q.dtype != torch.bfloat16 or d != 128 or n_q > 8 * n_kv or page_size % 16 or not 0 < B <= RUNS_MAX_REQUESTS or kv_len.numel() != B
+            or B * n_kv * (block_table.shape[1] * (page_size // 16) + 1) >= 1 << 30):
+        return False
+    _need_cuda(q, out, k_cache, v_cache, kv_len, block_table)
+    count = workspace.counters("attn_runs_count", max(B * n_kv, RUNS_COUNTERS))
+    if count is None:
+        return False
+    assert q.is_contiguous() and out.is_contiguous() and block_table.dim() == 2 and block_table.stride(1) == 1
+    assert block_table.shape[0] == B and out.shape == q.shape
+    blocks = min(sm_count(q.device), RUNS_MAX_BLOCKS)
+    part = workspace.get("attn_runs_part", blocks * 2 * 8 * (d + 2), torch.float32)
+    code = _attn_lib(d).msgl_attention_decode_runs(
+        _ptr(q), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(kv_len), _ptr(block_table), _ptr(part), part.data_ptr() + blocks * 16 * d * 4,
+        _ptr(count), B, n_q, n_kv, page_size, block_table.stride(0), float(scale), blocks, _stream())
+    _check(code, f"attention of a decode step ({B} requests, {n_q} heads on {n_kv})")
+    return True
 
 
 def attention_combine(part_o: torch.Tensor, part_ml: torch.Tensor, token_req: Optional[torch.Tensor],

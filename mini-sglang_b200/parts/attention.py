@@ -126,6 +126,10 @@ def paged_attend(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KV
     extra = dict(joined, chunk=chunk, diff=diff) if plain else dict(keep_first=keep_first, bias_log2=bias_log2, **joined)
     g = cache.group
     G = n_q // n_kv
+    if (ctx.uniform_decode and use_mma and plain and not joined and window == 0 and not chunk and diff is None
+            and ops.attention_decode_runs(q, out, cache.k, cache.v, kv_len=ctx.kv_len, block_table=g.block_table, n_kv=n_kv,
+                                          page_size=cache.page_size, scale=scale, workspace=ctx.workspace)):
+        return
     max_split = g.max_split if g.nsplit is not None else 1
     part_o = part_ml = None
     qt_dec = ops.attention_tile_tokens(ops.VARIANT_MMA_DECODE, G, d) if use_mma else 0

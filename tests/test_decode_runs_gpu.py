@@ -1,0 +1,73 @@
+"""Decode attention that deals the keys out over the SMs by itself: against the plain softmax in 64 bits where segments have one, two and many
+pieces, at the edges of units, pages and groups, with rows of the pages behind the last key that hold no numbers."""
+import random
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda")
+D = 128
+CASES = [
+    ([1], 16, 8, 16), ([16], 8, 8, 16), ([17, 1, 500], 12, 4, 32), ([511], 3, 1, 64), ([512, 513], 10, 2, 48),      # every request in pieces of its own
+    ([4000], 16, 8, 16), ([0, 40, 0], 16, 8, 16),
+    ([60000], 4, 1, 64), ([20000, 33, 7000], 16, 2, 16),                                                            # one request over more than 32 blocks
+    ([700] * 9, 64, 8, 16), ([1500 + 13 * i for i in range(24)], 40, 8, 16),
+    (None, 16, 8, 16), (None, 8, 1, 32), ([5] * 256, 32, 8, 16),                                                   # many requests, a block holds several
+]
+
+
+@pytest.mark.parametrize("kv,n_q,n_kv,P", CASES)
+def test_decode_runs(kv, n_q, n_kv, P):
+    from mini_sglang_b200 import ops
+    from mini_sglang_b200.parts import Workspace
+    if kv is None:
+        r = random.Random(n_q)
+        kv = [r.choice((1, 15, 16, 97, 130, 3000)) + r.randrange(40) for _ in range(100)]
+    B, G = len(kv), n_q // n_kv
+    g = torch.Generator(device=DEV).manual_seed(B)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)      # noqa: E731
+    pages = [max(-(-k // P), 1) for k in kv]
+    ids = (torch.randperm(sum(pages), generator=torch.Generator().manual_seed(B)) + 1).tolist()
+    rows, at = [], 0
+    for n in pages:
+        rows.append(ids[at:at + n] + [0] * (max(pages) - n))
+        at += n
+    table = torch.tensor(rows, dtype=torch.int32, device=DEV)
+    k_c, v_c = (rnd(sum(pages) + 1, n_kv, P, D).bfloat16() for _ in range(2))
+    q = (2 * rnd(B, n_q, D)).bfloat16()
+    for r, k in enumerate(kv):
+        if k % P:
+            k_c[rows[r][k // P], :, k % P:] = float("nan")
+            v_c[rows[r][k // P], :, k % P:] = float("nan")
+    ws, lens = Workspace(DEV), torch.tensor(kv, dtype=torch.int32, device=DEV)
+    outs = []
+    for _ in range(2):
+        out = torch.full((B, n_q, D), 7.0, dtype=torch.bfloat16, device=DEV)
+        assert ops.attention_decode_runs(q, out, k_c, v_c, kv_len=lens, block_table=table, n_kv=n_kv, page_size=P, scale=D ** -0.5, workspace=ws)
+        outs.append(out)
+    assert torch.equal(*outs) and int(ws.counters("attn_runs_count", 1).abs().sum()) == 0
+    assert not ws._bufs["attn_runs_count"].any()
+    for r, k in enumerate(kv):
+        if k == 0:
+            assert not outs[0][r].any()
+            continue
+        pos = torch.arange(k, device=DEV)
+        kk, vv = (c[table[r].long()[pos // P], :, pos % P].double() for c in (k_c, v_c))
+        s = torch.einsum("hgd,khd->hgk", q[r].double().view(n_kv, G, D), kk) * D ** -0.5
+        want = torch.einsum("hgk,khd->hgd", s.softmax(-1), vv).reshape(n_q, D)
+        err = (outs[0][r].double() - want).abs()
+        # weights in bfloat16 (2^-9 each, random) and one rounding of the result
+        assert err.max() < 0.02 * want.abs().max() and err.pow(2).mean().sqrt() < 0.004 * want.pow(2).mean().sqrt() + 1e-4, r
+
+
+def test_counters_are_not_made_inside_a_capture(monkeypatch):
+    from mini_sglang_b200.parts import Workspace
+    ws = Workspace(DEV)
+    monkeypatch.setattr(ws, "_capturing", lambda: True)
+    assert ws.counters("n", 10) is None
+    monkeypatch.setattr(ws, "_capturing", lambda: False)
+    first = ws.counters("n", 10)
+    assert not first.any()
+    monkeypatch.setattr(ws, "_capturing", lambda: True)
+    assert ws.counters("n", 10).data_ptr() == first.data_ptr() and ws.counters("n", 11) is None
