@@ -63,7 +63,7 @@ def build_dir() -> str:
 # files a source pulls in with #include: an edit of any of them rebuilds the library
 INCLUDED = {"attention.cu": ["tc_common.cuh", "attention_tc.cuh", "attention_tc2.cuh", "attention_runs.cuh"],
             "attention_noalloc.cu": ["attention.cu", "tc_common.cuh", "attention_tc.cuh", "attention_tc2.cuh", "attention_runs.cuh", "attention_noalloc.h"],
-            "gemm_tc.cu": ["tc_common.cuh"], "gemm_rows.cu": ["tc_common.cuh"], "gemm_f32.cu": ["tc_common.cuh"], "mixers_delta.cu": ["tc_common.cuh"], "decode_step.cu": []}
+            "gemm_tc.cu": ["tc_common.cuh"], "gemm_rows.cu": ["tc_common.cuh"], "gemm_f32.cu": ["tc_common.cuh"], "gemm_stream.cu": ["tc_common.cuh"], "mixers_delta.cu": ["tc_common.cuh"], "decode_step.cu": []}
 
 
 def _digest(sources: Sequence[str], flags: Sequence[str]) -> str:
@@ -133,7 +133,7 @@ def load_library(name: str, sources: Sequence[str], defines: Optional[Dict[str, 
 
 # the libraries of the engine -----------------------------------------------------------
 
-COMMON_SOURCES = ["elementwise.cu", "sampling.cu", "gemm_small_m.cu", "gemm_tc.cu", "gemm_rows.cu", "gemm_f32.cu"]
+COMMON_SOURCES = ["elementwise.cu", "sampling.cu", "gemm_small_m.cu", "gemm_stream.cu", "gemm_tc.cu", "gemm_rows.cu", "gemm_f32.cu"]
 ATTENTION_SOURCES = ["attention.cu"]
 MIXER_SOURCES = ["mixers.cu"]
 GATED_MIXER_SOURCES = ["mixers_gated.cu"]

@@ -7,7 +7,7 @@ Matrix products with more than a few rows are the one exception to "hand-written
 the library GEMM that torch binds (cuBLAS), in bfloat16 with float32 accumulation or in true float32
 (TF32 off), as the reference does for every projection (F.linear in mini_sglang/layers/linear.py).  Float32 products of more than a few rows and
 of weights that are not small go to this engine's float32 kernel on the tensor cores.  Up to
-SMALL_M_MAX rows go to this engine's weight-streaming kernel, and the gated products and output heads of larger decode batches to
+SMALL_M_MAX rows go to this engine's weight-streaming kernels, and the gated products and output heads of larger decode batches to
 its decode-batch kernel.  The reference's own kernels for the
 other operations come from sgl_kernel / flash-attn (mini_sglang/layers/layernorm.py:39-50,
 mini_sglang/layers/rotary_embedding.py, mini_sglang/layers/attn/fa3_attn_backend.py).
@@ -93,6 +93,7 @@ def _lib():
         lib.msgl_cast_from_f32.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_void_p]
         lib.msgl_gemm_small_m.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int,
                                           c_int, c_void_p, c_ll, c_void_p]
+        lib.msgl_gemm_stream.argtypes = [c_void_p] * 4 + [c_int] * 3 + [c_ll, c_ll, c_int, c_int, c_void_p, c_void_p]
         lib.msgl_gemm_tc.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_void_p,
                                      c_void_p]
         lib.msgl_gemm_tc2.argtypes = lib.msgl_gemm_tc.argtypes
@@ -687,8 +688,19 @@ SMALL_M_MAX = int(os.environ.get("MSGL_SMALL_M_MAX", "8"))      # tokens up to w
 USE_SMALL_M = os.environ.get("MSGL_NO_SMALL_M", "") == ""
 
 
+# elements of a weight from which on the kernel of one block an SM is ahead; us a product of a chain, blocks of 16 rows / one an SM, one row: [1024, 1024] 1.63 / 1.86, [768, 2048] 2.40 /
+# 2.39, gated [1792, 1024] 2.23 / 2.14 and with 8 rows 2.33 / 2.39, [2048, 1024] 2.47 / 2.22, [1024, 3072] 4.02 / 3.08, [4096, 4096] 8.0 / 7.3, [5120, 25600] 54 / 41
+STREAM_MIN_WEIGHTS = 2_000_000
+
+
 def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> int:
-    """ahead: a weight that gated products are to ask into L2 for the product behind them (or None; one that lies elsewhere or in pieces is left alone)."""
+    """Weights of some size go through one block an SM (csrc/gemm_stream.cu), smaller ones, for which its barriers and tensor maps cost more than they bring, through
+    blocks of 16 rows (csrc/gemm_small_m.cu).  ahead: a weight that gated products of the second kind are to ask into L2 for the product behind them (or None; one that lies
+    elsewhere or in pieces is left alone); with the first the product behind has its own weights on their way by itself."""
+    if M <= 8 and N * K >= STREAM_MIN_WEIGHTS:
+        code = _lib().msgl_gemm_stream(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), ldo, mode, out_f32, _ptr(_status_words(x.device)), _stream())
+        if code != 2:             # (2: no tensor map of this layout)
+            return code
     if ahead is not None and (not ahead.is_contiguous() or ahead.get_device() != x.get_device()):
         ahead = None
     return _lib().msgl_gemm_small_m(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), ldo, mode, out_f32, _ptr(ahead), ahead.numel() * ahead.element_size() if ahead is not None else 0, _stream())
@@ -913,7 +925,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """y = x @ weight^T (+ bias); weight is [out, in] as stored in the checkpoint.
 
-    Up to SMALL_M_MAX bfloat16 rows go through this engine's weight-streaming kernel (csrc/gemm_small_m.cu), float32 results of
+    Up to SMALL_M_MAX bfloat16 rows go through this engine's weight-streaming kernels (csrc/gemm_stream.cu, csrc/gemm_small_m.cu), float32 results of
     very many columns for a decode batch through its decode-batch kernel (csrc/gemm_rows.cu, `_rows_f32`), float32 operands through the float32
     kernel of the tensor cores (csrc/gemm_f32.cu, `_f32_rule`); everything else is the
     library GEMM unless MSGL_TC_GEMM or MSGL_TC_MID ask for the tiled kernels."""
