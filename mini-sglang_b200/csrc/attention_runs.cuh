@@ -1,4 +1,4 @@
-// Decode attention (bfloat16, head size 128, one new token a request, up to eight query heads a kv head) in one launch: the keys
+// Decode attention (bfloat16, head size 128, one new token a request, up to eight query heads a kv head; MIXED: the requests of a step that bring one) in one launch: the keys
 // of all requests dealt out evenly over one block an SM, partial results merged by the block that comes last.
 //
 // A segment is one request under one kv head, cut into units of 16 keys (anchored at absolute positions; a page holds whole
@@ -24,7 +24,9 @@
 // before / with it, us (kernels of four warps with kv splits from the host and a merge of their own): 8B, 8 x 4,096 keys 58.7 / 51.8;
 // 4B, 40 of 64 ... 6,000 76.6 / 58.2; 8B, 64 x 2,000 133.6 / 113; 1.7B, one of 130 18.2 / 14.3, 16 x 512 32.9 / 25.2, 64 of 4 ... 64 23.2 / 22.5.
 // Rings of two units and of three are level but for 64 x 2,000 (113.0 / 114.8), and two leave room for a block of the product behind.  Without
-// RUN_HEAD the mixed case takes 70.6: the block that gets the short requests runs 49 us, the others 34.
+// RUN_HEAD the mixed case takes 70.6: the block that gets the short requests runs 49 us, the others 34.  Decoded tokens among prompt portions, launched behind the prefill tiles and
+// ahead of their merges, so that its blocks take the SMs that the last tiles leave free (8B, 1,500, 333, 65, 1, 1, 1 tokens behind 0, 700, 4,000, 2,047, 511, 37: the
+// layer 223.8 -> 213.7 us; before, 18 us of decode attention ahead of the tiles and a merge over all tokens of 9).
 #pragma once
 
 constexpr int RUN_NW = 8;            // warps of a block
@@ -48,12 +50,14 @@ struct RunParams {
     float* part_o;                   // [2 * blocks][8][128]
     float* part_ml;                  // [2 * blocks][8][2]
     int* count;                      // [B * n_kv], zero before and after
+    const int* q_start;              // MIXED: [B + 1]; the requests with one token are taken
+    int wait_last;                   // MIXED: q and the cache are written by kernels that are done when this one starts; it waits for the one before it at its end
     int B, n_q, n_kv, page_size, page_shift, bt_stride;
     float scale;
 };
 
 constexpr size_t run_smem_bytes() {
-    return (size_t)RUN_NW * RUN_ST * 2 * 16 * RUN_D * 2 + (size_t)RUN_NW * 8 * RUN_OLD * 4 + (size_t)RUN_NW * 8 * 2 * 4 + (RUN_MAX_B + 4) * 4;
+    return (size_t)RUN_NW * RUN_ST * 2 * 16 * RUN_D * 2 + (size_t)RUN_NW * 8 * RUN_OLD * 4 + (size_t)RUN_NW * 8 * 2 * 4 + (4 * RUN_MAX_B + 4) * 4;
 }
 
 static_assert(run_smem_bytes() + 256 <= 227 * 1024, "one block an SM");
@@ -63,6 +67,7 @@ struct RunCursor {
     int r, kvh, c0, u;               // request, kv head, first unit of the segment among all, units
 };
 
+template <bool MIXED>
 __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const RunParams p) {
     extern __shared__ __align__(128) unsigned char run_smem[];
     constexpr int UNIT_BYTES = 16 * RUN_D * 2;
@@ -79,9 +84,37 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
     const int g = lane >> 2, t = lane & 3;
     const int G = p.n_q / p.n_kv, NB = (int)gridDim.x, j = (int)blockIdx.x;
 
-    // ---- the requests' units and pieces and their sums, a request a thread (the lengths come from the step's fields, not from the kernel
-    // before this one)
-    const int my_u = tid < p.B ? max(p.kv_len[tid] + 15, 16) >> 4 : 0;
+    // ---- the requests that are taken (MIXED: numbered anew), their units and pieces and the sums, a request a thread (lengths and first tokens come from
+    // the step's fields, not from the kernel before this one)
+    int* lens = pre + RUN_MAX_B + 4;                     // MIXED: of request i here its length, its number in the step and its token
+    int* number = lens + RUN_MAX_B;
+    int* token = number + RUN_MAX_B;
+    int B = p.B, my_len = 0;
+    if (MIXED) {
+        __shared__ int sh_taken[RUN_NW];
+        const int first = tid < p.B ? p.q_start[tid] : 0, len = tid < p.B ? p.kv_len[tid] : 0;
+        const bool taken = tid < p.B && p.q_start[tid + 1] - first == 1;
+        const unsigned all = __ballot_sync(0xffffffffu, taken);
+        if (lane == 0) sh_taken[warp] = __popc(all);
+        __syncthreads();
+        int at = __popc(all & ((1u << lane) - 1u));
+        B = 0;
+#pragma unroll
+        for (int w = 0; w < RUN_NW; ++w) {
+            if (w < warp) at += sh_taken[w];
+            B += sh_taken[w];
+        }
+        if (taken) { lens[at] = len; number[at] = tid; token[at] = first; }
+        __syncthreads();
+        if (B == 0) { pdl_wait(); return; }
+        if (tid < B) my_len = lens[tid];
+    } else if (tid < p.B) {
+        my_len = p.kv_len[tid];
+    }
+    auto leave = [&]() { if (MIXED && p.wait_last) pdl_wait(); };      // (whoever waits for this kernel counts on the one before it as well)
+    auto len_of = [&](int r) { return MIXED ? lens[r] : p.kv_len[r]; };
+    auto token_of = [&](int r) { return MIXED ? token[r] : r; };
+    const int my_u = tid < B ? max(my_len + 15, 16) >> 4 : 0;
     int my_pre = my_u, my_pc = my_u > 0 ? max(1, my_u / RUN_UNITS) : 0, my_pcs = my_pc;                   // of the requests before this one, at last
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -102,13 +135,13 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
         pieces_all += v.y;
         longest = max(longest, v.z);
     }
-    if (tid < p.B) pre[tid] = my_pre;
-    if (tid == 0) pre[p.B] = U;
-    const int S = p.B * p.n_kv;                          // segments
+    if (tid < B) pre[tid] = my_pre;
+    if (tid == 0) pre[B] = U;
+    const int S = B * p.n_kv;                          // segments
     if (pieces_all * p.n_kv > NB && S <= NB && 3 * longest * NB <= 4 * U * p.n_kv) {      // a block a segment is nearly even, and nothing is left to merge
-        pieces_all = p.B;
+        pieces_all = B;
         my_pcs = tid;
-        my_pc = tid < p.B ? 1 : 0;
+        my_pc = tid < B ? 1 : 0;
     }
     const bool by_piece = pieces_all * p.n_kv <= NB;
     const bool by_warp = !by_piece && longest <= RUN_WARP_UNITS && (4 * longest + 6) * NB < 11 * S;
@@ -117,7 +150,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
     // ---- this block's run of units [lo, hi) of the segments laid end to end, and the segment it starts in
     const int V = U + RUN_HEAD * S, per = V / NB, rest = V - per * NB;      // with every segment's head ahead of its units
     if (by_piece) {
-        if (j >= pieces_all * p.n_kv) return;
+        if (j >= pieces_all * p.n_kv) { leave(); return; }
         const int in_r = j - my_pcs * p.n_kv;
         if (in_r >= 0 && in_r < my_pc * p.n_kv) {
             const int kvh = in_r / my_pc, piece = in_r - kvh * my_pc, c0 = my_pre * p.n_kv + kvh * my_u;
@@ -130,7 +163,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
         for (int e = 0; e < 2; ++e) {
             const int i = j + e, in_r = i * per + i * rest / NB - (my_pre + RUN_HEAD * tid) * p.n_kv;
             if (i == NB && tid == 0) sh_run.y = U;
-            if (tid < p.B && in_r >= 0 && in_r < (my_u + RUN_HEAD) * p.n_kv) {
+            if (tid < B && in_r >= 0 && in_r < (my_u + RUN_HEAD) * p.n_kv) {
                 const int kvh = in_r / (my_u + RUN_HEAD), off = in_r - kvh * (my_u + RUN_HEAD) - RUN_HEAD;
                 const int unit = off <= RUN_SNAP ? 0 : my_u - off <= RUN_SNAP ? my_u : off, x = my_pre * p.n_kv + kvh * my_u + unit;
                 if (e == 1) { sh_run.y = x; continue; }
@@ -145,7 +178,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
     RunCursor seg;
     if (by_warp) {                                       // segments [s0, s1) in order are this warp's
         const int idx = warp * NB + j, W = NB * RUN_NW, s0 = S * idx / W, s1 = S * (idx + 1) / W;
-        if (s0 >= s1) return;                            // (no barrier of the block lies behind)
+        if (s0 >= s1) { leave(); return; }                     // (no barrier of the block lies behind)
         seg.r = s0 / p.n_kv;
         seg.kvh = s0 - seg.r * p.n_kv;
         const int r1 = (s1 - 1) / p.n_kv;
@@ -153,7 +186,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
     } else {
         lo = sh_run.x; hi = sh_run.y;
         seg_pieces = sh_seg.z; piece = sh_seg.w;
-        if (lo >= hi) return;
+        if (lo >= hi) { leave(); return; }
         seg.r = sh_seg.x;
         seg.kvh = sh_seg.y;
     }
@@ -182,8 +215,8 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
         const int pi = p.page_shift >= 0 ? key >> p.page_shift : key / p.page_size;
         w.slot = key - pi * p.page_size;
         w.kvh = ld.kvh;
-        w.rows = p.kv_len[ld.r] - key;
-        w.page = w.rows > 0 ? p.block_table[(size_t)ld.r * p.bt_stride + pi] : 0;
+        w.rows = len_of(ld.r) - key;
+        w.page = w.rows > 0 ? p.block_table[(size_t)(MIXED ? number[ld.r] : ld.r) * p.bt_stride + pi] : 0;
         return w;
     };
     auto offset_of = [&](const Place& w) -> size_t { return (((size_t)w.page * p.n_kv + w.kvh) * p.page_size + w.slot) * RUN_D; };
@@ -213,8 +246,10 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
     for (int i = 0; i < RUN_ST; ++i) at[i] = place_of(i);
 #pragma unroll
     for (int i = 0; i < RUN_ST; ++i) ask_l2(at[i]);
-    pdl_wait();
-    pdl_after_wait();
+    if (!MIXED || !p.wait_last) {
+        pdl_wait();
+        pdl_after_wait();
+    }
 #pragma unroll
     for (int i = 0; i < RUN_ST - 1; ++i) {
         if (i < n_my) load(i, at[i]);
@@ -225,7 +260,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
     // Q as B operand: lane (g, t) holds Q[head g of the group][32 m + 8 t .. + 7]
     uint4 qf[4];
     auto load_q = [&](int r, int kvh) {
-        const __nv_bfloat16* src = p.q + ((size_t)r * p.n_q + (size_t)kvh * G + (g < G ? g : 0)) * RUN_D + 8 * t;
+        const __nv_bfloat16* src = p.q + ((size_t)token_of(r) * p.n_q + (size_t)kvh * G + (g < G ? g : 0)) * RUN_D + 8 * t;
 #pragma unroll
         for (int m = 0; m < 4; ++m) qf[m] = g < G ? *reinterpret_cast<const uint4*>(src + 32 * m) : make_uint4(0u, 0u, 0u, 0u);
     };
@@ -235,7 +270,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
     bool first_segment = true;
     for (int begin = lo; begin < hi;) {
         const int end = min(hi, seg.c0 + seg.u);
-        const int pos = p.kv_len[seg.r] - 1;
+        const int pos = len_of(seg.r) - 1;
         float o[8][4];
 #pragma unroll
         for (int mt = 0; mt < 8; ++mt) o[mt][0] = o[mt][1] = o[mt][2] = o[mt][3] = 0.f;
@@ -333,7 +368,7 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
                 Lm[warp * 8 + 2 * t + e] = l_c[e];
             }
         }
-        const size_t row0 = (size_t)seg.r * p.n_q + (size_t)seg.kvh * G;
+        const size_t row0 = (size_t)token_of(seg.r) * p.n_q + (size_t)seg.kvh * G;
         // pieces of this segment, this block's among them
         int pieces = seg_pieces, mine = piece;
         if (by_warp) {
@@ -429,11 +464,14 @@ __global__ void __launch_bounds__(RUN_THREADS, 1) attn_decode_runs_kernel(const 
         }
     }
     cp_async_wait<0>();
+    leave();
 }
 
+// q_start null: every request has one token, request r token r.  Else the requests with one token are taken, and with wait_last the kernel reads what it is given without waiting
+// for the one launched before it: for a launch behind the prefill kernels, whose launch waited for all that wrote it (and whose own rows nobody reads here).
 MSGL_API int msgl_attention_decode_runs(const void* q, void* out, const void* k_cache, const void* v_cache, const int* kv_len, const int* block_table,
-                                        float* part_o, float* part_ml, int* count, int B, int n_q, int n_kv, int page_size, int bt_stride, float scale,
-                                        int blocks, cudaStream_t stream) {
+                                        float* part_o, float* part_ml, int* count, const int* q_start, int wait_last, int B, int n_q, int n_kv, int page_size,
+                                        int bt_stride, float scale, int blocks, cudaStream_t stream) {
     if (B <= 0) return MSGL_OK;
     if (B > RUN_MAX_B || n_kv <= 0 || n_q % n_kv != 0 || n_q / n_kv > 8 || page_size <= 0 || page_size % 16 != 0 || bt_stride <= 0 || blocks <= 0 || blocks > 4096 ||
         (long long)B * n_kv * ((long long)bt_stride * (page_size / 16) + 1) > 0x7fffffffLL / 2)
@@ -442,15 +480,18 @@ MSGL_API int msgl_attention_decode_runs(const void* q, void* out, const void* k_
     if (part_o == nullptr || part_ml == nullptr || count == nullptr) return MSGL_ERR_SIZE;
     static MsglOncePerDevice attr_set;
     if (attr_set.due()) {
-        if (cudaFuncSetAttribute(attn_decode_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_smem_bytes()) != cudaSuccess) return msgl_check_launch();
+        if (cudaFuncSetAttribute(attn_decode_runs_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_smem_bytes()) != cudaSuccess ||
+            cudaFuncSetAttribute(attn_decode_runs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_smem_bytes()) != cudaSuccess)
+            return msgl_check_launch();
         attr_set.mark();
     }
     RunParams p;
     p.q = (const __nv_bfloat16*)q; p.out = (__nv_bfloat16*)out; p.k_cache = (const __nv_bfloat16*)k_cache; p.v_cache = (const __nv_bfloat16*)v_cache;
-    p.kv_len = kv_len; p.block_table = block_table; p.part_o = part_o; p.part_ml = part_ml; p.count = count;
+    p.kv_len = kv_len; p.block_table = block_table; p.part_o = part_o; p.part_ml = part_ml; p.count = count; p.q_start = q_start; p.wait_last = wait_last;
     p.B = B; p.n_q = n_q; p.n_kv = n_kv; p.page_size = page_size; p.bt_stride = bt_stride; p.scale = scale;
     p.page_shift = -1;
     if ((page_size & (page_size - 1)) == 0) { int sh = 0; while ((1 << sh) < page_size) ++sh; p.page_shift = sh; }
-    msgl_launch_pdl(attn_decode_runs_kernel, dim3(blocks), dim3(RUN_THREADS), run_smem_bytes(), stream, p);
+    if (q_start != nullptr) msgl_launch_pdl(attn_decode_runs_kernel<true>, dim3(blocks), dim3(RUN_THREADS), run_smem_bytes(), stream, p);
+    else msgl_launch_pdl(attn_decode_runs_kernel<false>, dim3(blocks), dim3(RUN_THREADS), run_smem_bytes(), stream, p);
     return msgl_check_launch();
 }

@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(TC2_THREADS, 1) attn_tc2_kernel(const AttnPara
     int* sh_tile = reinterpret_cast<int*>(tc_smem + 208);
     const unsigned smem_base = smem_u32(tc_smem);
     const unsigned smem0 = (smem_base + 256u + 1023u) & ~1023u;
+    pdl_small();             // decode rows beside the tiles start as these leave SMs free (attention_runs.cuh)
     if (status != nullptr && *reinterpret_cast<volatile int*>(status) != 0) return;      // an earlier block gave up: do not pile up
     if (smem0 + TC2_SMEM_BYTES > smem_base + TC2_SMEM_ALLOC) {            // allocation not aligned as assumed
         if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 2);

@@ -127,7 +127,7 @@ def _attn_lib(head_dim: int):
         lib.msgl_attention_combine_range.argtypes = [c_void_p] * 4 + [c_int] * 9 + [c_void_p, c_void_p, c_ll, c_void_p]
         lib.msgl_attention_head_dim.restype = c_int
         if hd == 128:
-            lib.msgl_attention_decode_runs.argtypes = [c_void_p] * 9 + [c_int] * 5 + [c_float, c_int, c_void_p]
+            lib.msgl_attention_decode_runs.argtypes = [c_void_p] * 10 + [c_int] * 6 + [c_float, c_int, c_void_p]
         _attn[hd] = lib
     return lib
 
@@ -398,13 +398,14 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
                  window: int, scale: float, qlen_min: int, qlen_max: int, q_lens: Sequence[int], keep_first: int = 0,
                  bias_log2: Optional[torch.Tensor] = None, null_log2: Optional[torch.Tensor] = None,
                  gate: Optional[torch.Tensor] = None, chunk: int = 0, diff: Optional[Tuple[float, float, float]] = None,
-                 kv_lens: Optional[Sequence[int]] = None, workspace=None) -> bool:
+                 kv_lens: Optional[Sequence[int]] = None, workspace=None, beside=None) -> bool:
     """Prefill attention on tcgen05 tensor cores for the requests with q_len in [qlen_min, qlen_max];
     q_lens: the host's copy of every request's number of query tokens (to size the grid).  keep_first, bias_log2: as in
     `attention`; they are taken by the kernel on pairs of query tiles only (TMA page sizes), and the call returns False,
     having launched nothing, where that kernel cannot run.  null_log2, gate, chunk: as in `attention`, taken by both kernels;
     diff: as there, by the kernel on pairs of query tiles only.  With kv_lens (the host's copy of kv_len) and a workspace
-    query tiles with far more keys than the launch's mean are cut into pieces (`plan_tc_pieces`) and merged here."""
+    query tiles with far more keys than the launch's mean are cut into pieces (`plan_tc_pieces`) and merged here.
+    beside: called behind the tiles' launch, ahead of the merges: for launches that run beside the tiles."""
     global _tc2_usable
     gate_stride = _attention_extras(q, null_log2, gate)
     _need_cuda(q, out, k_cache, v_cache, q_start, kv_len, block_table)
@@ -457,6 +458,8 @@ def attention_tc(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_ca
                 return False
             continue
         _check(code, "attention_tc")
+        if beside is not None:
+            beside()
         for tok0, n in cut[2] if cut is not None else ():
             _check(_attn_lib(d).msgl_attention_combine_range(_ptr(part_o), _ptr(part_ml), _ptr(tok_pieces), _ptr(out), T, lo, plane, tok0, n, n_q, d, cut[1],
                                                              _dt(out), _ptr(null_log2), _ptr(gate), gate_stride, _stream()), "attention_combine_range")
@@ -622,30 +625,45 @@ def attention(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache
     _check(code, f"attention (head size {d}, variant {variant})")
 
 
-RUNS_MAX_REQUESTS, RUNS_MAX_BLOCKS, RUNS_COUNTERS = 256, 256, 4096
+RUNS_MAX_REQUESTS, RUNS_MAX_BLOCKS = 256, 256
+
+
+def decode_runs_supported(q: torch.Tensor, B: int, n_kv: int, page_size: int, table_width: int, workspace) -> bool:
+    """Whether `attention_decode_runs` takes a step of B requests (but for a stream capture that comes before its counters)."""
+    return (workspace is not None and q.dtype == torch.bfloat16 and q.shape[2] == 128 and q.shape[1] <= 8 * n_kv and page_size % 16 == 0
+            and 0 < B <= RUNS_MAX_REQUESTS and B * n_kv * (table_width * (page_size // 16) + 1) < 1 << 30)
+
+
+def decode_runs_scratch(q: torch.Tensor, B: int, n_kv: int, workspace) -> Optional[torch.Tensor]:
+    """Counters (16 KB or a word a request and kv head), then partial results of two segments a block; None in a capture that comes before they exist."""
+    return workspace.counters("attn_runs", max(B * n_kv + 3 & ~3, 4096) + 2 * 8 * (128 + 2) * min(sm_count(q.device), RUNS_MAX_BLOCKS))
 
 
 def attention_decode_runs(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, *, kv_len: torch.Tensor,
-                          block_table: torch.Tensor, n_kv: int, page_size: int, scale: float, workspace) -> bool:
+                          block_table: torch.Tensor, n_kv: int, page_size: int, scale: float, workspace, q_start: Optional[torch.Tensor] = None,
+                          beside_tiles: bool = False, scratch: Optional[torch.Tensor] = None) -> bool:
     """Attention of a decode step (one new token a request, all of a request's keys) in one launch that deals the keys out over the SMs by
-    itself and merges its partial results (csrc/attention_runs.cuh).  -> False where it does not apply: bfloat16, head size 128, up to eight
-    query heads a kv head, pages of whole units of 16 keys, up to 256 requests; inside a stream capture only once its counters exist."""
-    B, n_q, d = q.shape
-    if (workspace is None or q.dtype != torch.bfloat16 or d != 128 or n_q > 8 * n_kv or page_size % 16 or not 0 < B <= RUNS_MAX_REQUESTS or kv_len.numel() != B
-            or B * n_kv * (block_table.shape[1] * (page_size // 16) + 1) >= 1 << 30):
-        return False
-    _need_cuda(q, out, k_cache, v_cache, kv_len, block_table)
-    count = workspace.counters("attn_runs_count", max(B * n_kv, RUNS_COUNTERS))
-    if count is None:
-        return False
-    assert q.is_contiguous() and out.is_contiguous() and block_table.dim() == 2 and block_table.stride(1) == 1
-    assert block_table.shape[0] == B and out.shape == q.shape
+    itself and merges its partial results (csrc/attention_runs.cuh).  With q_start, int32 [B + 1], of the requests of any step that bring one token, out's rows of the others
+    are left alone; beside_tiles: the launch before this one is the prefill kernel of the same step, beside which it may run; scratch: from `decode_runs_scratch`, asked for ahead of
+    that launch, with the sizes looked at.  -> False where it does not apply: bfloat16,
+    head size 128, up to eight query heads a kv head, pages of whole units of 16 keys, up to 256 requests; inside a stream capture only once its counters exist."""
+    (T, n_q, d), (B, width) = q.shape, block_table.shape
+    if scratch is None:
+        if (q_start is None and T != B) or not decode_runs_supported(q, B, n_kv, page_size, width, workspace):
+            return False
+        scratch = decode_runs_scratch(q, B, n_kv, workspace)
+        if scratch is None:
+            return False
+        _need_cuda(q, out, k_cache, v_cache, kv_len, block_table, q_start)
+        assert q.is_contiguous() and out.is_contiguous() and block_table.stride(1) == 1
+        assert kv_len.numel() == B and out.shape == q.shape and (q_start is None or q_start.numel() == B + 1)
     blocks = min(sm_count(q.device), RUNS_MAX_BLOCKS)
-    part = workspace.get("attn_runs_part", blocks * 2 * 8 * (d + 2), torch.float32)
+    count = scratch.data_ptr()
+    part = count + 4 * max(B * n_kv + 3 & ~3, 4096)
     code = _attn_lib(d).msgl_attention_decode_runs(
-        _ptr(q), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(kv_len), _ptr(block_table), _ptr(part), part.data_ptr() + blocks * 16 * d * 4,
-        _ptr(count), B, n_q, n_kv, page_size, block_table.stride(0), float(scale), blocks, _stream())
-    _check(code, f"attention of a decode step ({B} requests, {n_q} heads on {n_kv})")
+        q.data_ptr(), out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), kv_len.data_ptr(), block_table.data_ptr(), part, part + blocks * 16 * d * 4,
+        count, _ptr(q_start), int(beside_tiles), B, n_q, n_kv, page_size, block_table.stride(0), scale, blocks, _stream())
+    _check(code, "attention of a decode step")
     return True
 
 

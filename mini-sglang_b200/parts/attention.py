@@ -126,10 +126,13 @@ def paged_attend(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KV
     extra = dict(joined, chunk=chunk, diff=diff) if plain else dict(keep_first=keep_first, bias_log2=bias_log2, **joined)
     g = cache.group
     G = n_q // n_kv
-    if (ctx.uniform_decode and use_mma and plain and not joined and window == 0 and not chunk and diff is None
-            and ops.attention_decode_runs(q, out, cache.k, cache.v, kv_len=ctx.kv_len, block_table=g.block_table, n_kv=n_kv,
-                                          page_size=cache.page_size, scale=scale, workspace=ctx.workspace)):
-        return
+    if use_mma and plain and not joined and window == 0 and not chunk and diff is None:      # all of a request's keys, nothing beside them
+        if ctx.uniform_decode:
+            if ops.attention_decode_runs(q, out, cache.k, cache.v, kv_len=ctx.kv_len, block_table=g.block_table, n_kv=n_kv, page_size=cache.page_size, scale=scale,
+                                         workspace=ctx.workspace):
+                return
+        elif _beside_portions(q, out, ctx, cache, n_kv=n_kv, scale=scale):
+            return
     max_split = g.max_split if g.nsplit is not None else 1
     part_o = part_ml = None
     qt_dec = ops.attention_tile_tokens(ops.VARIANT_MMA_DECODE, G, d) if use_mma else 0
@@ -176,3 +179,25 @@ def paged_attend(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KV
                                    ctx.q_start, qt_dec, out, max_split, diff)
     elif merged:
         ops.attention_combine(part_o, part_ml, None if ctx.uniform_decode else ctx.token_req, g.nsplit, out, max_split, **joined)
+
+
+def _beside_portions(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KVCacheView, *, n_kv: int, scale: float) -> bool:
+    """A step of prompt portions with decoded tokens among them: the portions on the tcgen05 kernel, the single tokens by the launch that cuts its keys up by itself, beside
+    the tiles.  False, with nothing launched, where either does not apply or a run of a few tokens would go to the decode kernel."""
+    lens, table, P, ws = ctx.host_q_lens, cache.group.block_table, cache.page_size, ctx.workspace
+    G = q.shape[1] // n_kv
+    if 1 not in lens or not ops.decode_runs_supported(q, ctx.B, n_kv, P, table.shape[1], ws) or not ops.tc_supported(128, q.dtype, G):
+        return False
+    longer = [n for n in lens if n != 1]
+    if not longer or min(longer) <= 8 // G:
+        return False
+    scratch = ops.decode_runs_scratch(q, ctx.B, n_kv, ws)
+    if scratch is None:
+        return False
+
+    def single_tokens():                     # (attention_tc has looked at the same operands)
+        ops.attention_decode_runs(q, out, cache.k, cache.v, kv_len=ctx.kv_len, block_table=table, n_kv=n_kv, page_size=P, scale=scale, workspace=ws,
+                                  q_start=ctx.q_start, beside_tiles=True, scratch=scratch)
+
+    return ops.attention_tc(q, out, cache.k, cache.v, q_start=ctx.q_start, kv_len=ctx.kv_len, block_table=table, n_kv=n_kv, page_size=P, window=0, scale=scale,
+                            qlen_min=8 // G + 1, qlen_max=1 << 30, q_lens=lens, kv_lens=ctx.host_kv_lens, workspace=ws, beside=single_tokens)

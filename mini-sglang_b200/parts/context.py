@@ -82,14 +82,16 @@ class Workspace:
         return buf[:numel]
 
     def counters(self, name: str, numel: int) -> Optional[torch.Tensor]:
-        """int32 words that are zero when they are made, for kernels that leave them zero.  None where they would have to be made inside a stream
+        """At least numel int32 words that are zero when they are made, for kernels that leave zero what they count with.  None where they would have to be made inside a stream
         capture: their zeros would then be written by that graph's replays alone."""
         buf = self._bufs.get(name)
         if buf is None or buf.numel() < numel:
             if self._capturing():
                 return None
-            self.get(name, numel, torch.int32).zero_()
-        return self.get(name, numel, torch.int32)
+            return self.get(name, numel, torch.int32).zero_()
+        if name not in self._captured and self._capturing():
+            self._captured.add(name)
+        return buf
 
 
 @dataclasses.dataclass

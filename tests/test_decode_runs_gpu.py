@@ -46,8 +46,7 @@ def test_decode_runs(kv, n_q, n_kv, P):
         out = torch.full((B, n_q, D), 7.0, dtype=torch.bfloat16, device=DEV)
         assert ops.attention_decode_runs(q, out, k_c, v_c, kv_len=lens, block_table=table, n_kv=n_kv, page_size=P, scale=D ** -0.5, workspace=ws)
         outs.append(out)
-    assert torch.equal(*outs) and int(ws.counters("attn_runs_count", 1).abs().sum()) == 0
-    assert not ws._bufs["attn_runs_count"].any()
+    assert torch.equal(*outs) and not ws._bufs["attn_runs"][:max(B * n_kv, 4096)].any()
     for r, k in enumerate(kv):
         if k == 0:
             assert not outs[0][r].any()
@@ -58,6 +57,39 @@ def test_decode_runs(kv, n_q, n_kv, P):
         want = torch.einsum("hgk,khd->hgd", s.softmax(-1), vv).reshape(n_q, D)
         err = (outs[0][r].double() - want).abs()
         # weights in bfloat16 (2^-9 each, random) and one rounding of the result
+        assert err.max() < 0.02 * want.abs().max() and err.pow(2).mean().sqrt() < 0.004 * want.pow(2).mean().sqrt() + 1e-4, r
+
+
+@pytest.mark.parametrize("q_lens,kv", [([3, 1, 1, 40, 1], [700, 17, 4000, 40, 1]), ([1, 2], [333, 2]), ([5] * 7, [9] * 7), ([1 + r % 3 * 4 for r in range(200)], [r % 90 + 9 for r in range(200)]),
+                                       ([9] + [1] * 255, [9] + [1200] * 255)])
+@pytest.mark.parametrize("beside", [False, True])
+def test_single_tokens_among_portions(q_lens, kv, beside):
+    from mini_sglang_b200 import ops
+    from mini_sglang_b200.parts import Workspace
+    n_q, n_kv, P, B, T = 8, 2, 16, len(kv), sum(q_lens)
+    g = torch.Generator(device=DEV).manual_seed(B)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)      # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)      # noqa: E731
+    width = -(-max(kv) // P)
+    table = i32([[1 + (7 * r + 13 * i) % 500 for i in range(width)] for r in range(B)])      # (pages may be shared: nothing is written)
+    k_c, v_c, q = rnd(501, n_kv, P, D).bfloat16(), rnd(501, n_kv, P, D).bfloat16(), (2 * rnd(T, n_q, D)).bfloat16()
+    start = [0]
+    for n in q_lens:
+        start.append(start[-1] + n)
+    out = torch.full((T, n_q, D), 7.0, dtype=torch.bfloat16, device=DEV)
+    ws = Workspace(DEV)
+    assert ops.attention_decode_runs(q, out, k_c, v_c, kv_len=i32(kv), block_table=table, n_kv=n_kv, page_size=P, scale=D ** -0.5, workspace=ws, q_start=i32(start),
+                                     beside_tiles=beside)
+    assert not ws._bufs["attn_runs"][:4096].any()
+    for r, (n, k) in enumerate(zip(q_lens, kv)):
+        if n > 1:
+            assert (out[start[r]:start[r + 1]] == 7.0).all()
+            continue
+        pos = torch.arange(k, device=DEV)
+        kk, vv = (c[table[r].long()[pos // P], :, pos % P].double() for c in (k_c, v_c))
+        s = torch.einsum("hgd,khd->hgk", q[start[r]].double().view(n_kv, n_q // n_kv, D), kk) * D ** -0.5
+        want = torch.einsum("hgk,khd->hgd", s.softmax(-1), vv).reshape(n_q, D)
+        err = (out[start[r]].double() - want).abs()
         assert err.max() < 0.02 * want.abs().max() and err.pow(2).mean().sqrt() < 0.004 * want.pow(2).mean().sqrt() + 1e-4, r
 
 
