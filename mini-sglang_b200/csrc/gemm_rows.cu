@@ -38,6 +38,7 @@ struct GemmRowsParams {
     int up_off;                    // gated: how many rows of W an up row lies behind its gate row
     int expert_rows, experts;      // grouped: rows of W an expert has, how many there are
     const int* ends;               // grouped: [experts] running sum of the experts' rows in x
+    int apart;                     // grouped: the expert whose matrix is w2map's (one that all tokens use); -1: none
     int bn, stages, splits;        // tokens a pass (a multiple of 16), ring depth, blocks that share a tile's K
     int halves;                    // 2: a block has two ranges of K (splits is 1 then), an accumulator each
     unsigned tmem_cols;
@@ -135,7 +136,7 @@ __device__ __forceinline__ void gr_reduce(const GemmRowsParams& p, unsigned sums
 
 template <int MODE, typename OutT, bool GROUPED>
 __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
-                                                               const GemmRowsParams p) {
+                                                               const __grid_constant__ CUtensorMap w2map, const GemmRowsParams p) {
     constexpr bool GLU = MODE != GR_PLAIN;
     extern __shared__ __align__(16) unsigned char gr_smem[];
     const unsigned smem_base = tc_smem_u32(gr_smem);
@@ -225,17 +226,19 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
     }
     int fail = 0, g0 = 0, pass = 0;                    // g0: slabs that went through the ring before this run
     for (;;) {
-        const int w_row = expert * p.expert_rows + col0, n16 = (n_tok + 15) & ~15;      // n16: tokens that are multiplied
+        const bool other = GROUPED && expert == p.apart;
+        const CUtensorMap* wm = other ? &w2map : &wmap;
+        const int w_row = (other ? 0 : expert * p.expert_rows) + col0, n16 = (n_tok + 15) & ~15;      // n16: tokens that are multiplied
         const unsigned x_bytes = (GROUPED ? (unsigned)n16 : (unsigned)p.bn) * 128u;
         const bool last = !GROUPED || run + (int)gridDim.y >= n_runs;
         if (warp == 0) {
             if (lane == 0) {
                 auto load_w = [&](int k, unsigned a_s, unsigned bar) {
                     if (GLU) {
-                        tc_tma_load(a_s, &wmap, k * 64, w_row, bar);
-                        tc_tma_load(a_s + 64u * 128u, &wmap, k * 64, w_row + p.up_off, bar);
+                        tc_tma_load(a_s, wm, k * 64, w_row, bar);
+                        tc_tma_load(a_s + 64u * 128u, wm, k * 64, w_row + p.up_off, bar);
                     } else {
-                        tc_tma_load(a_s, &wmap, k * 64, w_row, bar);
+                        tc_tma_load(a_s, wm, k * 64, w_row, bar);
                     }
                 };
                 auto load_x = [&](int k, unsigned b_s, unsigned bar) {
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
 }
 
 template <int MODE, typename OutT, bool GROUPED>
-static int gr_launch(const CUtensorMap& xm, const CUtensorMap& wm, const GemmRowsParams& p, int tiles, int runs, size_t smem, cudaStream_t stream) {
+static int gr_launch(const CUtensorMap& xm, const CUtensorMap& wm, const CUtensorMap& w2m, const GemmRowsParams& p, int tiles, int runs, size_t smem, cudaStream_t stream) {
     auto* kernel = gemm_rows_kernel<MODE, OutT, GROUPED>;
     static MsglOncePerDevice attr_set;
     if (attr_set.due()) {      // first call on this device, never inside a stream capture
@@ -347,7 +350,7 @@ static int gr_launch(const CUtensorMap& xm, const CUtensorMap& wm, const GemmRow
     cfg.gridDim = dim3((unsigned)(tiles * p.splits), (unsigned)runs);
     cfg.blockDim = dim3(GR_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream; cfg.attrs = attr;
     cfg.numAttrs = msgl_pdl_enabled() ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xm, wm, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xm, wm, w2m, p);
     (void)e;
     return msgl_check_launch();
 }
@@ -395,19 +398,21 @@ MSGL_API int msgl_tensor_maps() { return tc_encoder() != nullptr; }
 // clamped form min(g, limit) * sigmoid(1.702 min(g, limit)) * (clamp(u, -limit, limit) + 1).
 // experts > 0: W is [experts][n_out or 2 n_out][K], x holds M rows in the order of their experts, ends [experts] their running sum on
 // the device; tokens: how many tokens brought the rows, M / tokens experts each.  Else M is at most 256.
+// W2 (grouped; or null): one more expert that all tokens use, its matrix apart from W; its rows lie behind the others' in x and out (M counts them not), ends is [experts + 1].
 // splits: ranges of K; 0 = chosen from the sizes, grouped: for steps that use all experts; -1 = grouped, for steps down to a single token.
 // per_sm: 0 = chosen by gr_plan.
 // bfloat16 operands; out bfloat16 or (mode 0) float32.  K, ldx multiples of 8, ldo even, bases 16-byte aligned.
-MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void* out, int M, int n_out, int K, long long ldx, long long ldo,
-                            int mode, int out_f32, float limit, int experts, const int* ends, int tokens, int splits, int per_sm,
-                            void* status, cudaStream_t stream) {
+MSGL_API int msgl_gemm_rows_apart(const void* W, const void* W2, const void* X, const void* bias, void* out, int M, int n_out, int K, long long ldx, long long ldo,
+                                  int mode, int out_f32, float limit, int experts, const int* ends, int tokens, int splits, int per_sm, void* status,
+                                  cudaStream_t stream) {
     if (M <= 0) return MSGL_OK;
     const bool glu = mode != GR_PLAIN, grouped = experts > 0;
     if (mode < 0 || mode > 3 || n_out <= 0 || K <= 0 || (K & 7) || (ldx & 7) || (ldo & 1) || status == nullptr || experts < 0 || experts > 65535 ||
         splits < -1 || (splits == -1 && !grouped) || splits > GR_MAX_SPLITS || (splits > 0 && (splits & (splits - 1))) || per_sm < 0 || per_sm > 3)
         return MSGL_ERR_SIZE;
     if (grouped ? (ends == nullptr || bias != nullptr || tokens <= 0) : M > 256) return MSGL_ERR_SIZE;
-    if (((uintptr_t)W | (uintptr_t)X | (uintptr_t)out) & 15) return MSGL_ERR_ALIGN;
+    if (W2 != nullptr && !grouped) return MSGL_ERR_SIZE;
+    if (((uintptr_t)W | (uintptr_t)W2 | (uintptr_t)X | (uintptr_t)out) & 15) return MSGL_ERR_ALIGN;
     long long w_rows = glu ? 2 * (long long)n_out : n_out;
     int bn = (M + 15) & ~15;
     double live = 1.0;
@@ -422,13 +427,17 @@ MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void
         if (bn > most) bn = most;
         live = experts * (1.0 - pow(1.0 - fmin(1.0, (double)M / tokens / experts), (double)tokens));       // experts that some token uses, in the mean
         if (live < 1.0) live = 1.0;
+        if (W2 != nullptr) live += 1.0;
         w_rows *= experts;
     }
-    CUtensorMap xm, wm;
-    if (!tc_matrix_map(X, M, K, ldx * 2, grouped ? 16 : bn, &xm) || !tc_matrix_map(W, w_rows, K, (long long)K * 2, glu ? 64 : 128, &wm)) return MSGL_ERR_SIZE;
+    CUtensorMap xm, wm, w2m;
+    const int apart_rows = W2 != nullptr ? tokens : 0;
+    if (!tc_matrix_map(X, (long long)M + apart_rows, K, ldx * 2, grouped ? 16 : bn, &xm) || !tc_matrix_map(W, w_rows, K, (long long)K * 2, glu ? 64 : 128, &wm)) return MSGL_ERR_SIZE;
+    if (W2 == nullptr) w2m = wm;
+    else if (!tc_matrix_map(W2, w_rows / experts, K, (long long)K * 2, glu ? 64 : 128, &w2m)) return MSGL_ERR_SIZE;
     GemmRowsParams p;
     p.bias = (const __nv_bfloat16*)bias; p.out = out; p.ldo = ldo; p.M = M; p.n_valid = n_out; p.K = K;
-    p.up_off = n_out; p.expert_rows = grouped ? (glu ? 2 * n_out : n_out) : 0; p.experts = experts; p.ends = ends; p.bn = bn; p.limit = limit; p.status = (int*)status;
+    p.up_off = n_out; p.expert_rows = grouped ? (glu ? 2 * n_out : n_out) : 0; p.experts = experts + (W2 != nullptr ? 1 : 0); p.apart = W2 != nullptr ? experts : -1; p.ends = ends; p.bn = bn; p.limit = limit; p.status = (int*)status;
     const int tiles = (n_out + (glu ? 63 : 127)) / (glu ? 64 : 128);
     const int slabs = (K + 63) / 64;
     p.halves = 1;
@@ -439,19 +448,24 @@ MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void
     // Blocks along y: no more than the runs of up to bn rows that the experts can have, and not many more than a random choice gives (one an
     // expert): blocks without a run are not free (128 experts, 8,192 rows: 73 rows of them added 12 us to 265).
     const long long most_runs = (long long)(M < experts ? M : experts) + M / bn, usual = experts + (experts > 128 ? experts / 16 : 8);
-    const long long runs = !grouped ? 1 : most_runs < usual ? most_runs : usual < 65535 ? usual : 65535;
+    const long long own_runs = !grouped ? 1 : most_runs < usual ? most_runs : usual < 65535 ? usual : 65535, runs = own_runs + (apart_rows + bn - 1) / bn;
     gr_plan((long long)(tiles * live), slabs, bn, p.splits, p.stages, splits, per_sm);
     p.tmem_cols = 32;
     while (p.tmem_cols < (unsigned)bn) p.tmem_cols *= 2;
     if (p.halves == 2) p.tmem_cols *= 2;
     const size_t smem = (size_t)p.stages * (GR_A_BYTES + (unsigned)bn * 128u) + GR_HEAD_BYTES + 1024u;
-#define GR_GO(MODE, T) (grouped ? gr_launch<MODE, T, true>(xm, wm, p, tiles, (int)runs, smem, stream) : gr_launch<MODE, T, false>(xm, wm, p, tiles, 1, smem, stream))
+#define GR_GO(MODE, T) (grouped ? gr_launch<MODE, T, true>(xm, wm, w2m, p, tiles, (int)runs, smem, stream) : gr_launch<MODE, T, false>(xm, wm, w2m, p, tiles, 1, smem, stream))
     if (out_f32) return mode == GR_PLAIN ? GR_GO(GR_PLAIN, float) : MSGL_ERR_DTYPE;
     switch (mode) {
         case GR_PLAIN: return GR_GO(GR_PLAIN, __nv_bfloat16);
         case GR_SILU: return GR_GO(GR_SILU, __nv_bfloat16);
-        case GR_RELU: return grouped ? MSGL_ERR_SIZE : gr_launch<GR_RELU, __nv_bfloat16, false>(xm, wm, p, tiles, 1, smem, stream);      // no experts with it
+        case GR_RELU: return grouped ? MSGL_ERR_SIZE : gr_launch<GR_RELU, __nv_bfloat16, false>(xm, wm, w2m, p, tiles, 1, smem, stream);      // no experts with it
         default: return GR_GO(GR_CLAMPED, __nv_bfloat16);
     }
 #undef GR_GO
+}
+
+MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void* out, int M, int n_out, int K, long long ldx, long long ldo,
+                            int mode, int out_f32, float limit, int experts, const int* ends, int tokens, int splits, int per_sm, void* status, cudaStream_t stream) {
+    return msgl_gemm_rows_apart(W, nullptr, X, bias, out, M, n_out, K, ldx, ldo, mode, out_f32, limit, experts, ends, tokens, splits, per_sm, status, stream);
 }

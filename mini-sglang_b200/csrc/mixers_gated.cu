@@ -2133,13 +2133,22 @@ MSGL_API int msgl_expert_combine_self(const void* y, int y_is_f32, const int* pl
 #define ER_MAX_PAIRS 8192
 template <typename T>
 __global__ void __launch_bounds__(128) expert_rows_kernel(const T* __restrict__ h, long long h_stride, const int* __restrict__ idx, int n_pairs, int top,
-                                                          int E, int H, T* __restrict__ rows, int* __restrict__ place, int* __restrict__ ends) {
+                                                          int E, int H, int shared, T* __restrict__ rows, int* __restrict__ place, int* __restrict__ ends) {
     __shared__ int count[RT_MAX_EXPERTS];
     __shared__ int at_sh[4];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, pair = blockIdx.x;
     pdl_wait();
     pdl_small();
+    constexpr int V = VecOf<T>::N;
+    if (pair > n_pairs) {                                // shared: every token once more behind the pairs, for an expert that all of them use
+        const int t = pair - n_pairs - 1;
+        const uint4* src = reinterpret_cast<const uint4*>(h + (size_t)t * h_stride);
+        uint4* dst = reinterpret_cast<uint4*>(rows + (size_t)(n_pairs + t) * H);
+        for (int i = tid; i < H / V; i += 128) dst[i] = src[i];
+        return;
+    }
     if (pair == n_pairs) {
+        if (shared > 0 && tid == 0) ends[E] = n_pairs + shared;
         for (int e = tid; e < E; e += 128) count[e] = 0;
         __syncthreads();
         for (int i = tid; i < n_pairs; i += 128) atomicAdd(&count[idx[i]], 1);
@@ -2165,24 +2174,23 @@ __global__ void __launch_bounds__(128) expert_rows_kernel(const T* __restrict__ 
     __syncthreads();
     const int at = at_sh[0] + at_sh[1] + at_sh[2] + at_sh[3];
     if (tid == 0) place[pair] = at;
-    constexpr int V = VecOf<T>::N;
     const uint4* src = reinterpret_cast<const uint4*>(h + (size_t)(pair / top) * h_stride);
     uint4* dst = reinterpret_cast<uint4*>(rows + (size_t)at * H);
     for (int i = tid; i < H / V; i += 128) dst[i] = src[i];
 }
 
 // idx [n_pairs] (every number below E) -> rows [n_pairs, H] in the order of the experts, place [n_pairs], ends [E].  H and h_stride in steps
-// of 16 bytes, bases 16-byte aligned.
-MSGL_API int msgl_expert_rows(const void* h, long long h_stride, const int* idx, int n_pairs, int top, int E, int H, void* rows, int* place,
+// of 16 bytes, bases 16-byte aligned.  shared > 0: that many tokens, all of h, stand once more behind the pairs (rows [n_pairs + shared, H], ends [E + 1]).
+MSGL_API int msgl_expert_rows(const void* h, long long h_stride, const int* idx, int n_pairs, int top, int E, int H, int shared, void* rows, int* place,
                               int* ends, int dtype, cudaStream_t stream) {
     if (n_pairs <= 0) return MSGL_OK;
     const int V = dtype == MSGL_F32 ? 4 : 8;
-    if (top < 1 || E < 1 || E > RT_MAX_EXPERTS || n_pairs > ER_MAX_PAIRS || H <= 0 || H % V || h_stride % V) return MSGL_ERR_SIZE;
+    if (top < 1 || E < 1 || E > RT_MAX_EXPERTS || n_pairs > ER_MAX_PAIRS || shared < 0 || shared > ER_MAX_PAIRS || H <= 0 || H % V || h_stride % V) return MSGL_ERR_SIZE;
     if (((uintptr_t)h | (uintptr_t)rows) & 15) return MSGL_ERR_ALIGN;
     if (dtype == MSGL_F32)
-        msgl_launch_pdl(expert_rows_kernel<float>, dim3(n_pairs + 1), dim3(128), 0, stream, (const float*)h, h_stride, idx, n_pairs, top, E, H, (float*)rows, place, ends);
+        msgl_launch_pdl(expert_rows_kernel<float>, dim3(n_pairs + 1 + shared), dim3(128), 0, stream, (const float*)h, h_stride, idx, n_pairs, top, E, H, shared, (float*)rows, place, ends);
     else if (dtype == MSGL_BF16)
-        msgl_launch_pdl(expert_rows_kernel<__nv_bfloat16>, dim3(n_pairs + 1), dim3(128), 0, stream, (const __nv_bfloat16*)h, h_stride, idx, n_pairs, top, E, H,
+        msgl_launch_pdl(expert_rows_kernel<__nv_bfloat16>, dim3(n_pairs + 1 + shared), dim3(128), 0, stream, (const __nv_bfloat16*)h, h_stride, idx, n_pairs, top, E, H, shared,
                         (__nv_bfloat16*)rows, place, ends);
     else return MSGL_ERR_DTYPE;
     return msgl_check_launch();

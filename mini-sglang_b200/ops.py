@@ -103,6 +103,7 @@ def _lib():
         lib.msgl_gemm_tc2_splits.restype = c_int
         lib.msgl_gemm_rows.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_int, c_float, c_int,
                                        c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
+        lib.msgl_gemm_rows_apart.argtypes = [c_void_p] + lib.msgl_gemm_rows.argtypes
         lib.msgl_gemm_f32.argtypes = [c_void_p] * 4 + [c_int] * 3 + [c_ll, c_ll, c_void_p, c_void_p]
         lib.msgl_tensor_maps.argtypes = []
         lib.msgl_tensor_maps.restype = c_int
@@ -1440,7 +1441,7 @@ def _gated_lib():
         lib.msgl_experts_few.argtypes = [c_void_p, c_ll] + [c_void_p] * 4 + [c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_int,
                                                                             c_float, c_void_p, c_void_p, c_void_p]
         lib.msgl_clamped_glu.argtypes = [c_void_p, c_ll, c_int, c_float, c_void_p, c_int, c_int, c_void_p]
-        lib.msgl_expert_rows.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
+        lib.msgl_expert_rows.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
         lib.msgl_expert_order.argtypes = [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]
         lib.msgl_expert_gather.argtypes = [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p]
         lib.msgl_expert_combine.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_void_p,
@@ -1812,6 +1813,26 @@ def experts_few(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx:
     return out
 
 
+def experts_few_shared(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, shared_gate_up: torch.Tensor,
+                       shared_down: torch.Tensor, shared_gate: torch.Tensor, limit: float) -> Optional[torch.Tensor]:
+    """`experts_few` with limit > 0 beside a shared expert of the experts' own sizes, shared_gate_up [2 F, H] and shared_down [H, F], whose output counts shared_gate [T] times: in the
+    same grouped launches, as one more expert that every token uses.  None where these do not apply or the tokens are more than a run of rows."""
+    T, H = h.shape
+    F, top = gate_up.shape[2], idx.shape[1]
+    if (T > SHARED_ROWS_MAX or limit <= 0 or not _experts_grouped(T * top, F * H) or tuple(shared_gate_up.shape) != (2 * F, H) or tuple(shared_down.shape) != (H, F)
+            or shared_gate_up.dtype != h.dtype or shared_down.dtype != h.dtype or not shared_gate_up.is_contiguous() or not shared_down.is_contiguous()
+            or (shared_gate_up.data_ptr() | shared_down.data_ptr()) % 16 or shared_gate.dtype != torch.float32 or shared_gate.numel() != T):
+        return None
+    _need_cuda(shared_gate_up, shared_down, shared_gate)
+    idx, wts = _expert_operands(h, gate_up, down, idx, wts, None, None)
+    return _experts_by_rows(h, gate_up, down, idx, wts, 1.0, limit, None, shared_gate, torch.float32, (shared_gate_up, shared_down))
+
+
+# us of the whole mixture (32 experts of [2 x 1536, 2048] + [2048, 1536], four a token), shared expert as launches of its own / in the grouped ones: 1 token 45.3 / 38.7, 8: 92.7 / 85.7, 16: 117.4 / 107.5,
+# 64: 132.0 / 124.0, 128: 135.3 / 127.6.  Beyond a decode batch the shared expert's tokens are several runs of rows, each of which reads its weights, and the library's products take them in one.
+SHARED_ROWS_MAX = 128
+
+
 # The chosen experts' products on the decode-batch kernel (csrc/gemm_rows.cu, grouped: an expert's weights are read once, whatever the
 # number of tokens that chose it) against the others, measured on B200: a feed-forward of 32 experts of [2 x 1536, 2048] + [2048, 1536], four
 # a token, beside a shared one.  Against a warp per row and (token, choice) pair: 1 token 82 -> 66 us, 8 tokens 224 -> 106, 24 tokens
@@ -1845,15 +1866,16 @@ def expert_rows(h: torch.Tensor, idx: torch.Tensor, n_experts: int) -> Optional[
     rows = torch.empty((T * top, H), dtype=h.dtype, device=h.device)
     place = torch.empty(T * top, dtype=torch.int32, device=h.device)
     ends = torch.empty(n_experts, dtype=torch.int32, device=h.device)
-    _check(_gated_lib().msgl_expert_rows(_ptr(h), h.stride(0), _ptr(idx), T * top, top, n_experts, H, _ptr(rows), _ptr(place), _ptr(ends), _dt(h),
+    _check(_gated_lib().msgl_expert_rows(_ptr(h), h.stride(0), _ptr(idx), T * top, top, n_experts, H, 0, _ptr(rows), _ptr(place), _ptr(ends), _dt(h),
                                          _stream()), "expert_rows")
     return rows, place, ends
 
 
 def _experts_by_rows(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, scale: float, limit: float,
-                     extra: Optional[torch.Tensor], extra_gate: Optional[torch.Tensor], y_dtype: torch.dtype) -> Optional[torch.Tensor]:
+                     extra: Optional[torch.Tensor], extra_gate: Optional[torch.Tensor], y_dtype: torch.dtype,
+                     shared: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> Optional[torch.Tensor]:
     """The chosen experts, gate_up [E, 2, F, H] and down [E, H, F], on the decode-batch kernel: `expert_rows`, both products with the activation
-    between them, `expert_combine`; None where that does not apply.  The operands have been through `_expert_operands`.  The ranges of K, and
+    between them, `expert_combine`; None where that does not apply.  shared = ([2 F, H], [H, F]) in place of extra, y_dtype float32: one more expert that every token uses.  The operands have been through `_expert_operands`.  The ranges of K, and
     with them the order of the sums, follow from the sizes: float32 outputs of the experts (decode steps) take those of a single token's
     step, so that a request's tokens are the same in every batch, rounded ones those of a step that uses all experts.  (One
     function and three scratch tensors for the four launches: small eager steps wait for the host.)"""
@@ -1864,21 +1886,23 @@ def _experts_by_rows(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor,
     if h.dtype != torch.bfloat16 or H % 8 or F % 8 or P > EXPERT_ROWS_MEAN_MAX * E or P > EXPERT_ROWS_MAX_PAIRS or E > ROUTE_MAX_EXPERTS or \
             h.stride(1) != 1 or h.stride(0) % 8 or (h.data_ptr() | gate_up.data_ptr() | down.data_ptr()) % 16 or not tensor_maps():
         return None
-    dev = h.device
-    numbers, buf = torch.empty(P + E, dtype=torch.int32, device=dev), torch.empty(P * (H + F), dtype=torch.bfloat16, device=dev)
-    y, out = torch.empty(P * H, dtype=y_dtype, device=dev), torch.empty((T, H), dtype=torch.float32, device=dev)
+    dev, R = h.device, P if shared is None else P + T          # R: rows of x and y
+    numbers, buf = torch.empty(P + E + 1, dtype=torch.int32, device=dev), torch.empty(R * (H + F), dtype=torch.bfloat16, device=dev)
+    y, out = torch.empty(R * H, dtype=y_dtype, device=dev), torch.empty((T, H), dtype=torch.float32, device=dev)
     place, rows, yp = numbers.data_ptr(), buf.data_ptr(), y.data_ptr()
-    ends, act = place + 4 * P, rows + 2 * P * H
+    ends, act = place + 4 * P, rows + 2 * R * H
+    gu_apart, down_apart = (None, None) if shared is None else (shared[0].data_ptr(), shared[1].data_ptr())
     f32, status, stream, lib, gated = int(y_dtype == torch.float32), _status_tensor(dev).data_ptr(), _stream(), _lib(), _gated_lib()
     ranges = -1 if f32 else 0
-    _check(gated.msgl_expert_rows(h.data_ptr(), h.stride(0), idx.data_ptr(), P, top, E, H, rows, place, ends, _DT[torch.bfloat16], stream), "expert_rows")
-    code = lib.msgl_gemm_rows(gate_up.data_ptr(), rows, None, act, P, F, H, H, F, 3 if limit > 0 else 1, 0, float(limit), E, ends, T, ranges, 0, status, stream)
+    _check(gated.msgl_expert_rows(h.data_ptr(), h.stride(0), idx.data_ptr(), P, top, E, H, R - P, rows, place, ends, _DT[torch.bfloat16], stream), "expert_rows")
+    code = lib.msgl_gemm_rows_apart(gate_up.data_ptr(), gu_apart, rows, None, act, P, F, H, H, F, 3 if limit > 0 else 1, 0, float(limit), E, ends, T, ranges, 0, status, stream)
     if code == 2:             # no tensor map of this layout
         return None
     _check(code, "gemm_rows (experts)")
-    _check(lib.msgl_gemm_rows(down.data_ptr(), act, None, yp, P, H, F, F, H, 0, f32, 0.0, E, ends, T, ranges, 0, status, stream), "gemm_rows (experts)")
-    _check(gated.msgl_expert_combine(yp, f32, place, wts.data_ptr(), top, H, float(scale), out.data_ptr(), T, _ptr(extra),
-                                     _ptr(extra_gate) if extra is not None else None, stream), "expert_combine")
+    _check(lib.msgl_gemm_rows_apart(down.data_ptr(), down_apart, act, None, yp, P, H, F, F, H, 0, f32, 0.0, E, ends, T, ranges, 0, status, stream), "gemm_rows (experts)")
+    more = _ptr(extra) if shared is None else yp + 4 * P * H
+    _check(gated.msgl_expert_combine(yp, f32, place, wts.data_ptr(), top, H, float(scale), out.data_ptr(), T, more,
+                                     _ptr(extra_gate) if more is not None else None, stream), "expert_combine")
     return out
 
 

@@ -108,7 +108,7 @@ class SoftmaxExperts(FeedForward):
     for every token and is added, times sigmoid(wsg . x), one number per token that the router kernel makes beside its logits.
 
     The launches are those of `routed_experts`: in bfloat16 one grouped product each way for the tokens in the order of their
-    experts, else the chosen experts' rows for a few (token, choice) pairs and a loop over the experts for many.
+    experts (in decode steps with the shared expert, where it has the others' sizes and limit, as one more of them), else the chosen experts' rows for a few (token, choice) pairs and a loop over the experts for many.
 
     params: hidden_size, intermediate_size, limit, num_experts, top, shared_size, shared_limit,
             names (router, expert (with {e}), gate, up, down, shared, shared_gate).
@@ -162,12 +162,17 @@ class SoftmaxExperts(FeedForward):
 
     def forward(self, x, ctx):
         idx, wts, sgate = ops.route(x, self.router, None, n_groups=1, keep=1, top=self.top, score="logits", gate_row=self.sh_gate)
+        T = x.shape[0]
+        few = ctx.uniform_decode or T * self.top <= ops.EXPERTS_FEW_PAIRS
+        if few and self.Fs == self.F and self.shared_limit == self.limit:
+            y = ops.experts_few_shared(x, self.gate_up, self.down, idx, wts, self.sh_gate_up, self.sh_down, sgate, self.limit)
+            if y is not None:
+                return y
         shared = None
         if self.Fs:
             a = ops.clamped_glu(ops.linear(x, self.sh_gate_up), self.shared_limit)
             shared = ops.linear(a, self.sh_down, out_dtype=torch.float32)
-        T = x.shape[0]
-        if ctx.uniform_decode or T * self.top <= ops.EXPERTS_FEW_PAIRS:
+        if few:
             return ops.experts_few(x, self.gate_up, self.down, idx, wts, limit=self.limit, extra=shared, extra_gate=sgate)
         y = ops.experts_many(x, self.gate_up, self.down, idx, wts, limit=self.limit, extra=shared, extra_gate=sgate)
         if y is not None:
