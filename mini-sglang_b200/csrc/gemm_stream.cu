@@ -1,4 +1,5 @@
-// Weight-streaming matrix product for decode: out[M, N] = x[M, K] . W[N, K]^T with M <= 8 tokens, for weights of some size (gemm_small_m.cu has the others).
+// Weight-streaming matrix product for decode: out[M, N] = x[M, K] . W[N, K]^T with M <= 32 tokens, for weights of some size (gemm_small_m.cu has the others
+// up to 8 tokens).
 //
 // With so few tokens the product is bound by reading W once from HBM, so the kernel is built around that stream:
 //   * one block an SM takes an equal share of the output columns (rows of W) and all of K, in passes of up to 16 MT rows;
@@ -6,9 +7,10 @@
 //     of 64 elements of every row, a chunk a warp.  With nine of them the rows of a chunk lie 1,152 bytes apart and change their place in the swizzle from row to row, so
 //     that ldmatrix meets no bank twice.  The rounds of all passes are one stream through a ring of stages; one thread of a tenth warp asks for
 //     a round as soon as the nine warps have read the stage's last one;
-//   * weights are nobody's output, so the ring's first rounds are on their way before the wait for the kernel before this one, and the next kernel may
+//   * up to 8 tokens weights are nobody's output, so the ring's first rounds are on their way before the wait for the kernel before this one (beyond, where products went to the
+//     library, they are asked into L2), and the next kernel may
 //     start behind that wait: of two products in a row the second has its first weights in shared memory when the first ends;
-//   * x comes beside them by cp.async, a chunk a warp, on the same barriers; both go to mma.sync m16n8k16 by ldmatrix, the tokens on its n dimension, fp32 accumulate;
+//   * x comes beside them by cp.async, a chunk a warp, on the same barriers; both go to mma.sync m16n8k16 by ldmatrix, the tokens on its n dimension (8 per n-block), fp32 accumulate;
 //   * the warps' partial sums are added in warp order through shared memory (a fixed order, so
 //     the result does not depend on timing), then bias / SwiGLU and one rounding to the output type.
 //
@@ -33,7 +35,7 @@ constexpr int GST_WARPS = 9, GST_THREADS = GST_WARPS * 32 + 32;      // a chunk 
 constexpr int GST_MAX_STAGES = 16;
 constexpr int GST_RING = 176 * 1024;      // bytes of a block's ring at most
 constexpr unsigned GST_ROW = GST_WARPS * 128u;
-constexpr int GST_MAX_TILES = 3;
+constexpr int GST_MAX_TILES = 3, GST_MAX_ROWS = 32;
 
 __device__ __forceinline__ void gst_mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -47,6 +49,9 @@ __device__ __forceinline__ void gst_ldmatrix(unsigned (&r)[4], unsigned addr) {
 __device__ __forceinline__ void gst_load3(unsigned dst, const CUtensorMap* map, int chunk, int row, unsigned bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
                  ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(0), "r"(chunk), "r"(row), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void gst_ask3(const CUtensorMap* map, int chunk, int row) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];\n" ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(0), "r"(chunk), "r"(row) : "memory");
 }
 __device__ __forceinline__ void gst_consumers_sync() { asm volatile("bar.sync 1, %0;\n" ::"n"(GST_WARPS * 32) : "memory"); }
 
@@ -63,18 +68,20 @@ struct StreamParams {
     int M, N, K;                 // N: output columns
     int share, per_pass, passes; // output columns of a block, of a pass (of the last ones maybe fewer), passes of a block
     int stages;
+    int bufs;                    // of the warps' sums
+    int asked;                   // weights are only asked into L2 ahead of the wait: the kernel before this one may be the one that writes them
     int ragged;                  // K is no multiple of 64: the map is [rows][K] with boxes of rows x 64, a copy a chunk; the rows of a chunk lie back to back
     unsigned half;               // bytes of a stage, gated: of its gate rows and of its up rows; a multiple of 1,024
 };
 
-// a pass has up to 16 MT output columns (gated: 8 MT)
-template <int MT, int GLU, typename OutT>
+// a pass has up to 16 MT output columns (gated: 8 MT); up to 8 NB tokens
+template <int NB, int MT, int GLU, typename OutT>
 __global__ void __launch_bounds__(GST_THREADS) gemm_stream_kernel(const __grid_constant__ CUtensorMap wmap, const StreamParams p) {
     extern __shared__ __align__(1024) unsigned char gs_smem[];
     constexpr int PITCH = 16 * MT + 4;
     const unsigned base = tc_smem_u32(gs_smem), ring = (base + 1023u) & ~1023u, stage_bytes = GLU ? 2u * p.half : p.half;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, S = p.stages;
-    const unsigned x_bytes = (unsigned)(GST_WARPS * p.M) * 128u, x_ring = ring + (unsigned)S * stage_bytes, bars = x_ring + (unsigned)S * x_bytes;
+    const unsigned x_bytes = ((unsigned)(GST_WARPS * p.M) * 128u + 1023u) & ~1023u, x_ring = ring + (unsigned)S * stage_bytes, bars = x_ring + (unsigned)S * x_bytes;
     auto bar_full = [&](int s) { return bars + 16u * (unsigned)s; };
     auto bar_empty = [&](int s) { return bars + 16u * (unsigned)s + 8u; };
     const int o_begin = p.share * (int)blockIdx.x, chunks = (p.K + 63) / 64, rounds = (chunks + GST_WARPS - 1) / GST_WARPS, total = p.passes * rounds;
@@ -102,11 +109,21 @@ __global__ void __launch_bounds__(GST_THREADS) gemm_stream_kernel(const __grid_c
         if (lane == 0) {
             for (int s = 0; s < S; ++s) { tc_mbar_init(bar_full(s), 1 + GST_WARPS * 32); tc_mbar_init(bar_empty(s), GST_WARPS); }
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-            for (int i = 0; i < first; ++i) load(i);
+            if (!p.asked) {
+                for (int i = 0; i < first; ++i) load(i);
+            } else if (!p.ragged) {
+                for (int i = 0, row = o_begin, r = 0; i < first; ++i) {
+                    gst_ask3(&wmap, r * GST_WARPS, row);
+                    if (GLU) gst_ask3(&wmap, r * GST_WARPS, p.N + row);
+                    if (++r == rounds) { r = 0; row += p.per_pass; }
+                }
+            }
         }
         __syncthreads();
         if (lane == 0) {
             pdl_wait();
+            if (p.asked)
+                for (int i = 0; i < first; ++i) load(i);
             pdl_small();    // (not ahead of the wait: a kernel may then take for finished what was launched before this one)
             for (int i = first, st = 0, phase = 0; i < total; ++i) {
                 if (!tc_mbar_wait(bar_empty(st), (unsigned)phase)) break;
@@ -116,7 +133,7 @@ __global__ void __launch_bounds__(GST_THREADS) gemm_stream_kernel(const __grid_c
         }
         return;
     }
-    float* red = reinterpret_cast<float*>(gs_smem + (bars - base) + GST_MAX_STAGES * 16);      // [2 (one pass: 1)][GST_WARPS][M][PITCH]
+    float* red = reinterpret_cast<float*>(gs_smem + (bars - base) + GST_MAX_STAGES * 16);      // [bufs][GST_WARPS][M][PITCH]
     const int g = lane >> 2, t = lane & 3, r8 = lane & 7;
     __syncthreads();                                 // the barriers are there
     pdl_wait();
@@ -129,7 +146,7 @@ __global__ void __launch_bounds__(GST_THREADS) gemm_stream_kernel(const __grid_c
         const int k = (x_round * GST_WARPS + warp) * 64 + x_col, n16 = k < p.K ? 16 : 0;
         const unsigned to = x_ring + (unsigned)st * x_bytes + (unsigned)(warp * p.M) * 128u;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < 2 * NB; ++q) {
             const int tok = 4 * q + (lane >> 3);
             const unsigned at = to + (unsigned)tok * 128u;
             if (tok < p.M)
@@ -144,28 +161,36 @@ __global__ void __launch_bounds__(GST_THREADS) gemm_stream_kernel(const __grid_c
     const unsigned up = (unsigned)((lane >> 3) & 1), piece = (unsigned)(lane >> 4);
     const unsigned pitch = p.ragged ? 128u : GST_ROW, tile = (GLU ? 8u : 16u) * pitch, first_row = (unsigned)(p.ragged ? warp * p.per_pass : warp);      // (row r in place first_row + r pitch / 128)
     const unsigned a_off = (unsigned)r8 * pitch + first_row * 128u + up * (GLU ? p.half : 8u * pitch) + ((piece ^ ((unsigned)r8 + first_row & 7u)) << 4);
-    const unsigned x_row = (unsigned)(warp * p.M + (r8 < p.M ? r8 : 0)) * 128u;
+    unsigned x_off[NB];                              // (tokens that are not there: the last one)
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+        const unsigned row = (unsigned)(warp * p.M + min(nb * 8 + r8, p.M - 1));
+        x_off[nb] = row * 128u + (((unsigned)(lane >> 3) ^ (row & 7u)) << 4);
+    }
     int stage = 0, phase = 0, done = 0, fail = 0;
     for (int ps = 0; ps < p.passes; ++ps) {
-        float c[MT][4];
+        float c[NB][MT][4];
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) c[mt][0] = c[mt][1] = c[mt][2] = c[mt][3] = 0.f;
+        for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) c[nb][mt][0] = c[nb][mt][1] = c[nb][mt][2] = c[nb][mt][3] = 0.f;
         for (int i = 0; i < rounds && !fail; ++i) {
             if (!__all_sync(0xffffffffu, tc_mbar_wait(bar_full(stage), (unsigned)phase))) { fail = 1; break; }
             if (i * GST_WARPS + warp < chunks) {
-                const unsigned at = ring + (unsigned)stage * stage_bytes + a_off, xr = x_ring + (unsigned)stage * x_bytes + x_row;
-                const unsigned xa = xr + (((unsigned)(lane >> 3) ^ (xr >> 7 & 7u)) << 4);
+                const unsigned at = ring + (unsigned)stage * stage_bytes + a_off, xt = x_ring + (unsigned)stage * x_bytes;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {        // 32 elements of K
-                    unsigned b[4];
-                    gst_ldmatrix(b, xa ^ (unsigned)(h << 6));
+                    unsigned b[NB][4];
+#pragma unroll
+                    for (int nb = 0; nb < NB; ++nb) gst_ldmatrix(b[nb], (xt + x_off[nb]) ^ (unsigned)(h << 6));
 #pragma unroll
                     for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
                         for (int mt = 0; mt < MT; ++mt) {
                             unsigned a[4];
                             gst_ldmatrix(a, (at + (unsigned)mt * tile) ^ (unsigned)((2 * h + kk) << 5));
-                            gst_mma(c[mt], a, b[2 * kk], b[2 * kk + 1]);
+#pragma unroll
+                            for (int nb = 0; nb < NB; ++nb) gst_mma(c[nb][mt], a, b[nb][2 * kk], b[nb][2 * kk + 1]);
                         }
                 }
             }
@@ -176,22 +201,26 @@ __global__ void __launch_bounds__(GST_THREADS) gemm_stream_kernel(const __grid_c
             if (++stage == S) { stage = 0; phase ^= 1; }
         }
         // the warps' sums -> shared memory, [token][row of the pass]; accumulator layout: c0, c1 = (row g, tokens 2t, 2t + 1), c2, c3 = row g + 8.  Two buffers in
-        // turn: a pass writes one when every thread has read it in the pass before the last
-        const int per_warp = p.M * PITCH;
-        float* mine = red + ((ps & 1) * GST_WARPS + warp) * per_warp;
+        // turn (a pass writes one when every thread has read it in the pass before the last), or one
+        const int per_warp = p.M * PITCH, buf = p.bufs == 2 ? ps & 1 : 0;
+        float* mine = red + (buf * GST_WARPS + warp) * per_warp;
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-            if (2 * t + e < p.M) {
+        for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    mine[(2 * t + e) * PITCH + mt * 16 + g] = c[mt][e];
-                    mine[(2 * t + e) * PITCH + mt * 16 + g + 8] = c[mt][2 + e];
+            for (int e = 0; e < 2; ++e) {
+                const int tok = nb * 8 + 2 * t + e;
+                if (tok < p.M) {
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) {
+                        mine[tok * PITCH + mt * 16 + g] = c[nb][mt][e];
+                        mine[tok * PITCH + mt * 16 + g + 8] = c[nb][mt][2 + e];
+                    }
                 }
             }
         gst_consumers_sync();
         constexpr int COLS = GLU ? 8 * MT : 16 * MT;
         const int o0 = ps * p.per_pass, n = min(min(p.per_pass, p.share - o0), p.N - o_begin - o0);
-        const float* sums = red + (ps & 1) * GST_WARPS * per_warp;
+        const float* sums = red + buf * GST_WARPS * per_warp;
         for (int idx = threadIdx.x; idx < p.M * COLS; idx += GST_WARPS * 32) {
             const int tok = idx / COLS, o = idx - tok * COLS, col = o_begin + o0 + o;
             if (o >= n) continue;
@@ -208,6 +237,7 @@ __global__ void __launch_bounds__(GST_THREADS) gemm_stream_kernel(const __grid_c
             }
             gst_store<OutT>(reinterpret_cast<OutT*>(p.out) + (size_t)tok * p.ldo + col, GLU ? glu_act<GLU>(acc) * gated : acc);
         }
+        if (p.bufs == 1 && ps + 1 < p.passes) gst_consumers_sync();
     }
     if (fail) {                                      // what is under way lands before the block lets go of its shared memory
         const int asked = min(total, done + S);
@@ -242,11 +272,11 @@ static bool gst_map(const void* W, long long rows, int K, int box_rows, CUtensor
     return true;
 }
 
-template <int MT, int GLU, typename OutT>
+template <int NB, int MT, int GLU, typename OutT>
 static int gst_launch(const void* W, StreamParams p, int grid, cudaStream_t stream) {
     constexpr int COLS = GLU ? 8 * MT : 16 * MT;
     constexpr size_t FIXED = 1024 + GST_MAX_STAGES * 16, RED = sizeof(float) * GST_WARPS * (16 * MT + 4);
-    auto* kernel = gemm_stream_kernel<MT, GLU, OutT>;
+    auto* kernel = gemm_stream_kernel<NB, MT, GLU, OutT>;
     static MsglOncePerDevice attr_set;
     if (attr_set.due()) {      // first call on this device, never inside a stream capture
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) return msgl_check_launch();
@@ -261,8 +291,10 @@ static int gst_launch(const void* W, StreamParams p, int grid, cudaStream_t stre
     const long long rows = GLU ? 2LL * p.N : p.N;
     if (!(p.ragged ? tc_matrix_map(W, rows, p.K, (long long)p.K * 2, p.per_pass, &wm) : gst_map(W, rows, p.K, p.per_pass, &wm))) return MSGL_ERR_SIZE;
     const int total = p.passes * (((p.K + 63) / 64 + GST_WARPS - 1) / GST_WARPS);
-    const size_t stage = (GLU ? 2 : 1) * (size_t)p.half, x_stage = (size_t)GST_WARPS * p.M * 128, sums = (p.passes > 1 ? 2 : 1) * RED * p.M;
-    p.stages = (int)(GST_RING / (stage + x_stage));
+    const size_t stage = (GLU ? 2 : 1) * (size_t)p.half, x_stage = ((size_t)GST_WARPS * p.M * 128 + 1023) / 1024 * 1024;
+    p.bufs = p.passes > 1 && p.M <= 8 ? 2 : 1;
+    const size_t sums = p.bufs * RED * p.M, room = 227 * 1024 - FIXED - sums;
+    p.stages = (int)((room < GST_RING ? room : GST_RING) / (stage + x_stage));
     if (p.stages > GST_MAX_STAGES) p.stages = GST_MAX_STAGES;
     if (p.stages < 2) p.stages = 2;
     if (p.stages > total) p.stages = total;
@@ -270,6 +302,7 @@ static int gst_launch(const void* W, StreamParams p, int grid, cudaStream_t stre
     const size_t reach = p.ragged ? (size_t)(GST_WARPS - 1) * p.per_pass * 128 + COLS * 128 : (size_t)COLS * GST_ROW, over = reach > p.half ? reach - p.half : 0;
     size_t smem = FIXED + p.stages * (stage + x_stage) + sums;
     if (smem < 1024 + p.stages * stage + over) smem = 1024 + p.stages * stage + over;
+    if (smem > 227 * 1024) return MSGL_ERR_SIZE;
     msgl_launch_pdl(kernel, dim3(grid), dim3(GST_THREADS), smem, stream, wm, p);
     return msgl_check_launch();
 }
@@ -278,7 +311,7 @@ static int gst_launch(const void* W, StreamParams p, int grid, cudaStream_t stre
 MSGL_API int msgl_gemm_stream(const void* W, const void* X, const void* bias, void* out, int M, int N, int K,
                                long long ldx, long long ldo, int mode, int out_f32, void* status, cudaStream_t stream) {
     if (M <= 0) return MSGL_OK;
-    if (M > 8 || K <= 0 || (K & 31) || N <= 0 || (N & 15)) return MSGL_ERR_SIZE;
+    if (M > GST_MAX_ROWS || K <= 0 || (K & 31) || N <= 0 || (N & 15)) return MSGL_ERR_SIZE;
     if (((uintptr_t)W | (uintptr_t)X) & 15) return MSGL_ERR_ALIGN;
     if ((ldx & 7) != 0) return MSGL_ERR_ALIGN;
     if (mode < 0 || mode > 2) return MSGL_ERR_SIZE;
@@ -286,17 +319,20 @@ MSGL_API int msgl_gemm_stream(const void* W, const void* X, const void* bias, vo
     if (glu && out_f32) return MSGL_ERR_DTYPE;
     StreamParams p = {};
     p.X = (const __nv_bfloat16*)X; p.ldx = ldx; p.bias = (const __nv_bfloat16*)bias; p.out = out; p.status = (int*)status; p.ldo = ldo;
-    p.M = M; p.N = glu ? N / 2 : N; p.K = K;
+    p.M = M; p.N = glu ? N / 2 : N; p.K = K; p.asked = M > 8;
     const int sms = msgl_sm_count();
     p.share = (p.N + sms - 1) / sms;
     if (p.share < 4) p.share = p.N < 4 ? p.N : 4;
     const int grid = (p.N + p.share - 1) / p.share;
     int tiles = (p.share + (glu ? 7 : 15)) / (glu ? 8 : 16);
     if (tiles > GST_MAX_TILES) tiles = GST_MAX_TILES;
-#define GST_GO(GLU, T) \
-    (tiles == 1 ? gst_launch<1, GLU, T>(W, p, grid, stream) : tiles == 2 ? gst_launch<2, GLU, T>(W, p, grid, stream) : gst_launch<3, GLU, T>(W, p, grid, stream))
-    if (mode == MSGL_GLU_SILU) return GST_GO(1, __nv_bfloat16);
-    if (mode == MSGL_GLU_RELU) return GST_GO(2, __nv_bfloat16);
-    return out_f32 ? GST_GO(0, float) : GST_GO(0, __nv_bfloat16);
+#define GST_MT(NB, GLU, T) \
+    (tiles == 1 ? gst_launch<NB, 1, GLU, T>(W, p, grid, stream) : tiles == 2 ? gst_launch<NB, 2, GLU, T>(W, p, grid, stream) : gst_launch<NB, 3, GLU, T>(W, p, grid, stream))
+#define GST_GO(GLU, T) (M <= 8 ? GST_MT(1, GLU, T) : M <= 16 ? GST_MT(2, GLU, T) : M <= 24 ? GST_MT(3, GLU, T) : GST_MT(4, GLU, T))
+    for (;; --tiles) {           // (fewer rows a pass where the sums of many tokens leave no room for two stages)
+        const int code = mode == MSGL_GLU_SILU ? GST_GO(1, __nv_bfloat16) : mode == MSGL_GLU_RELU ? GST_GO(2, __nv_bfloat16) : out_f32 ? GST_GO(0, float) : GST_GO(0, __nv_bfloat16);
+        if (code != MSGL_ERR_SIZE || tiles == 1) return code;
+    }
 #undef GST_GO
+#undef GST_MT
 }

@@ -725,6 +725,44 @@ def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> i
     return _lib().msgl_gemm_small_m(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), ldo, mode, out_f32, _ptr(ahead), ahead.numel() * ahead.element_size() if ahead is not None else 0, _stream())
 
 
+# Up to which rows the kernel of one block an SM is ahead of the library (plain products) and the decode-batch kernel (gated ones); us at 9 / 16 / 24 / 32 rows, other kernel then this one.
+# [4096, 1024] 4.8 4.8 4.9 4.9, 2.9 3.7 4.1 4.5; [1024, 3072] 8.5 8.5 7.6 7.5, 4.5 4.5 4.9 6.1; [2048, 6144] 10.5 10.5 10.5 10.6, 8.6 9.1 8.1 9.7; [4096, 2048] 6.2 6.3 6.4 6.4, 5.3 5.5 6.2 7.4;
+# [6144, 4096] 12.8 12.9 12.1 13.2, 11.8 12.0 13.3 24; [4096, 12288] 22.0 22.1 22.6 22.7, 18.5 19.2 23.4 32; [5120, 25600] 49.6 46.8 46.2 46.3, 43.2 43.4 55 69.  Gated: [6144, 1024] 6.4 6.4 6.7 6.9,
+# 4.4 4.7 5.1 7.0; [12288, 2048] 12.0 12.3 12.5 12.9, 11.9 12.3 13.5 16.7; [24576, 4096] 35.8 36.6 36.1 36.8, 37.7 38.9 41.6 54.  (Every SM reads all rows of x: what it costs grows with them.)
+STREAM_ROWS, STREAM_ROWS_SMALL, STREAM_SMALL_WEIGHTS, STREAM_FEW_COLUMNS = 16, 32, 4_500_000, 2_072
+STREAM_ROWS_GATED, STREAM_GATED_LEAST, STREAM_GATED_MOST = 24, 4_000_000, 16_000_000
+
+
+def _stream_rule(rows: int, N: int, K: int, gated: bool) -> bool:
+    """Whether a product of more rows than the weight-streaming kernels' own goes to the one of one block an SM all the same."""
+    if N * K < STREAM_MIN_WEIGHTS or N % 16 or K % 32:
+        return False
+    if gated:
+        return rows <= STREAM_ROWS_GATED and STREAM_GATED_LEAST <= N * K <= STREAM_GATED_MOST
+    return rows <= (STREAM_ROWS_SMALL if N * K <= STREAM_SMALL_WEIGHTS or N <= STREAM_FEW_COLUMNS else STREAM_ROWS)
+
+
+def _gemm_stream(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """x @ weight^T (mode 0) or its gated activation (1: SwiGLU, 2: ReGLU) of 9 rows and more by csrc/gemm_stream.cu; None where another kernel or the library is to be called: by
+    `_stream_rule`, operands that do not lie as the kernel reads them or on another device than the current one, autocast, and whatever a kernel called by address would slip past."""
+    if not (USE_SMALL_M and not MID_GEMM and x.dim() == 2 and weight.dim() == 2 and SMALL_M_MAX < x.shape[0] <= STREAM_ROWS_SMALL
+            and _stream_rule(x.shape[0], weight.shape[0], weight.shape[1], mode != 0) and (mode == 0 or weight.shape[0] // 2 % 8 == 0) and _product_ok(x, weight, bias)
+            and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
+            and not _observed(x, weight, bias)):                     # (before the addresses are asked for: some of these have none)
+        return None
+    if (x.data_ptr() | weight.data_ptr()) % 16 or x.get_device() != torch._C._cuda_getDevice() or torch.is_autocast_enabled():
+        return None
+    M, (N, K) = x.shape[0], weight.shape
+    n_out = N // 2 if mode else N
+    out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+    code = _lib().msgl_gemm_stream(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), n_out, mode, int(out_dtype == torch.float32), _ptr(_status_words(x.device)),
+                                   _stream())
+    if code == 2:             # no tensor map of this layout
+        return None
+    _check(code, "gemm_stream")
+    return out
+
+
 def _product_ok(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> bool:
     """Whether x [M, K] . weight [N, K]^T + bias [N] is a bfloat16 product whose operands lie as the kernels read them: rows of x one behind
     the other on 16-byte pitches, packed weights and bias, one device.  The kernels get addresses and sizes only, so whatever
@@ -944,7 +982,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """y = x @ weight^T (+ bias); weight is [out, in] as stored in the checkpoint.
 
-    Up to SMALL_M_MAX bfloat16 rows go through this engine's weight-streaming kernels (csrc/gemm_stream.cu, csrc/gemm_small_m.cu), float32 results of
+    Up to SMALL_M_MAX bfloat16 rows, and up to 16 or 32 by the weight's size (`_stream_rule`), go through this engine's weight-streaming kernels (csrc/gemm_stream.cu,
+    csrc/gemm_small_m.cu), float32 results of
     very many columns for a decode batch through its decode-batch kernel (csrc/gemm_rows.cu, `_rows_f32`), float32 operands through the float32
     kernel of the tensor cores (csrc/gemm_f32.cu, `_f32_rule`); everything else is the
     library GEMM unless MSGL_TC_GEMM or MSGL_TC_MID ask for the tiled kernels."""
@@ -960,6 +999,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         code = _small_m(weight, x, bias, out, M, N, K, N, 0, int(od == torch.float32))
         _check(code, "gemm_small_m")
         return out
+    if x.dtype == torch.bfloat16 and out_dtype in (None, torch.bfloat16, torch.float32):
+        y = _gemm_stream(x, weight, bias, 0, out_dtype or torch.bfloat16)
+        if y is not None:
+            return y
     if out_dtype in (None, torch.bfloat16):
         y = _tc_gemm(x, weight, bias, 0) if x.shape[0] >= TC_GEMM_MIN_M else _tc_gemm_mid(x, weight, bias, 0)
         if y is not None:
@@ -994,6 +1037,9 @@ def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tens
             code = _small_m(gate_up, x, bias, out, M, N, K, N // 2, mode, 0, ahead)
             _check(code, "gemm_small_m (gated)")
             return out
+        y = _gemm_stream(x, gate_up, bias, mode, torch.bfloat16)
+        if y is not None:
+            return y
         if x.dim() == 2 and not MID_GEMM and x.shape[0] <= _rows_glu_max(gate_up.numel()):
             y = _gemm_rows(x, gate_up, bias, mode, torch.bfloat16)
             if y is not None:

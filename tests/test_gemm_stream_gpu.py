@@ -7,10 +7,14 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("N,K", [(1024, 2048), (6144, 1024), (3056, 672), (2048, 1056), (24576, 96), (624, 3232), (16, 131072), (7168, 5120)])
-@pytest.mark.parametrize("M", [1, 2, 3, 5, 8])
-def test_products(N, K, M):
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9, 16, 17, 24, 32])
+def test_products(N, K, M, monkeypatch):
     from mini_sglang_b200 import ops
     assert N * K >= ops.STREAM_MIN_WEIGHTS
+    monkeypatch.setattr(ops, "_stream_rule", lambda rows, n, k, gated: True)
+    if M > 8:                                                 # nothing goes elsewhere
+        for name in ("_gemm_rows", "_tc_gemm", "_tc_gemm_mid", "swiglu"):
+            monkeypatch.setattr(ops, name, None)
     g = torch.Generator(device="cuda").manual_seed(N + M)
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda").bfloat16()      # noqa: E731
     w, b = rnd(N, K), rnd(N)
@@ -35,13 +39,13 @@ def test_products(N, K, M):
         assert ((y.double() - want).abs() <= slack + 2.0 ** -8 * want.abs() + 1e-6).all()
 
 
-@pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("M", [1, 8, 16])
 def test_rows_keep_to_themselves(M):
     from mini_sglang_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(M)
     x, w = (torch.randn(s, generator=g, device="cuda").bfloat16() for s in ((M, 2080), (1040, 2080)))
     want, gated = ops.linear(x, w), ops.linear_swiglu(x, w)
-    for i in range(M):                                        # a row's bits do not depend on the others
+    for i in range(M if M <= 8 else 0):                       # a row's bits do not depend on the others
         assert torch.equal(ops.linear(x[i:i + 1], w)[0], want[i]) and torch.equal(ops.linear_swiglu(x[i:i + 1], w)[0], gated[i])
     w[0, 5], w[1039, 2079] = float("nan"), float("inf")
     x[M - 1, 7] = float("nan")
@@ -49,3 +53,31 @@ def test_rows_keep_to_themselves(M):
     assert y[:, 0].isnan().all() and not y[:M - 1, 1039].isfinite().any() and y[M - 1].isnan().all()
     assert torch.equal(y[:M - 1, 1:1039], want[:M - 1, 1:1039])
     ops.check_kernel_status()
+
+
+def test_what_stays_with_the_library():
+    from mini_sglang_b200 import ops
+    x, w = torch.randn(12, 2048, device="cuda").bfloat16(), torch.randn(1024, 2048, device="cuda").bfloat16()
+    want = ops.linear(x, w)
+    assert ops._gemm_stream(x, w, None, 0, torch.bfloat16) is not None
+    assert ops.linear(x, w.clone().requires_grad_()).requires_grad
+    assert torch.func.vmap(lambda v: ops.linear(v, w))(x[None]).shape == (1, 12, 1024)
+    with torch.autocast("cuda", torch.float16):
+        assert ops.linear(x, w).dtype == torch.float16
+    for other in (x[:, ::2], x.float(), x.t()):
+        assert ops._gemm_stream(other, w, None, 0, torch.bfloat16) is None
+    big = torch.randn(2048, 2048, device="cuda").bfloat16()
+    for _ in range(3):                                        # weights that the launch ahead writes
+        made = ops.linear(big[:16], big).repeat(64, 1)
+        made2 = ops.rmsnorm(torch.ones(2048, device="cuda"), 1e-6, x=made, out_dtype=torch.bfloat16)
+        y = ops.linear(x, made2)
+        torch.cuda.synchronize()
+        assert torch.equal(y, ops.linear(x, made2.clone()))
+    assert torch.equal(ops.linear(x, w), want)
+
+
+def test_rule():
+    from mini_sglang_b200.ops import _stream_rule as rule
+    assert rule(16, 6144, 4096, False) and not rule(17, 6144, 4096, False) and rule(32, 2064, 6144, False) and not rule(32, 2080, 6144, False) and not rule(33, 1024, 3072, False)
+    assert rule(32, 4096, 1024, False) and not rule(9, 1024, 1024, False) and not rule(9, 2040, 2048, False) and not rule(9, 2048, 2056, False)
+    assert rule(24, 6144, 1024, True) and not rule(25, 6144, 1024, True) and not rule(9, 12288, 2048, True) and not rule(9, 2048, 1024, True)
