@@ -1556,6 +1556,8 @@ template <typename T, int R>
 __global__ void __launch_bounds__(128, 12) group_rms_gate_vec_kernel(const float* __restrict__ x, int heads, int d, const float* __restrict__ w, float eps,
                                                                  const T* __restrict__ gate, long long gate_stride, T* __restrict__ out,
                                                                  long long out_stride, float c, int act, int n_rows) {
+    pdl_wait();
+    pdl_small();
     const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R, lane = threadIdx.x & 31, e = 4 * lane;
     const bool ok = e < d;
     int t = row0 / heads, h = row0 - t * heads;
@@ -1594,7 +1596,7 @@ MSGL_API int msgl_group_rms_gate(const float* x, int heads, int d, const float* 
         // two rows a warp once that still leaves every SM four blocks or more
         const bool two = n_rows >= 2LL * 4 * warps * msgl_sm_count();
         const unsigned g = (unsigned)((n_rows + (two ? 2 : 1) * warps - 1) / ((two ? 2 : 1) * warps));
-#define GRG_VEC(T, R) group_rms_gate_vec_kernel<T, R><<<g, warps * 32, 0, stream>>>(x, heads, d, w, eps, (const T*)gate, gate_stride, (T*)out, out_stride, c, act, (int)n_rows)
+#define GRG_VEC(T, R) msgl_launch_pdl(group_rms_gate_vec_kernel<T, R>, dim3(g), dim3(warps * 32), 0, stream, x, heads, d, w, eps, (const T*)gate, gate_stride, (T*)out, out_stride, c, act, (int)n_rows)
         if (dtype == MSGL_F32) { if (two) GRG_VEC(float, 2); else GRG_VEC(float, 1); }
         else { if (two) GRG_VEC(__nv_bfloat16, 2); else GRG_VEC(__nv_bfloat16, 1); }
 #undef GRG_VEC

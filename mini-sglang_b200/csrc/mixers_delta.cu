@@ -1038,6 +1038,8 @@ struct DeltaParams {
 
 template <typename T>
 __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaParams p) {
+    pdl_wait();
+    pdl_small();
     const int t = blockIdx.x, lane = threadIdx.x & 31;
     const int g = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (g >= p.kv_heads) return;
@@ -1078,6 +1080,8 @@ __device__ __forceinline__ void cp_async16_(void* smem_dst, const void* gmem) {
 
 template <typename T, int RPT, bool EXACT /* d == RPT * DR_PARTS: no row of a thread lies beyond the state */>
 __global__ void __launch_bounds__(DR_MANY_WARPS * 32) delta_rule_kernel(const DeltaParams p) {
+    pdl_wait();
+    pdl_small();
     extern __shared__ __align__(16) unsigned char dr_smem[];
     const int d = p.d, dv = p.dv;
     const int warps = blockDim.x >> 5, cols = warps * DR_WCOLS;
@@ -1317,6 +1321,8 @@ __global__ void __launch_bounds__(DC_THREADS, 4) delta_chunk_kernel(const DeltaC
     float* tmp = reinterpret_cast<float*>(dc_smem + Sm::TMP);            // [16][17]
     __shared__ float beta_s[DC_C], g_s[DC_C], pre_s[DC_C], suf_s[DC_C], rk_s[DC_C], rq_s[DC_C];
     __shared__ int where_s[2];
+    pdl_wait();
+    pdl_small();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, per = p.heads / p.kv_heads, g = h / per;
     if (warp == 0) {
         int at, rest;
@@ -1556,6 +1562,8 @@ __global__ void __launch_bounds__(DC_WALKERS + DC_READERS, DcSizes<T, D>::PARTS 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = h / (p.heads / p.kv_heads), dv = p.dv;
     const unsigned bar = (unsigned)__cvta_generic_to_shared(dc_smem + St::BAR);     // a barrier a stage
+    pdl_wait();
+    pdl_small();
     if (warp == 0) {
         int at, before;
         dc_nth(p.q_start, p.B, p.n_min, blockIdx.z, at, before);
@@ -1809,8 +1817,8 @@ static int delta_chunk_launch(DeltaChunkParams& p, unsigned char* scratch, int n
     const size_t ch = (size_t)n_chunks * p.heads, cg = (size_t)n_chunks * p.kv_heads;
     p.n_chunks = n_chunks;
     p.K = scratch; p.Q = p.K + cg * Z::KQ; p.R = p.Q + cg * Z::KQ; p.M = p.R + ch * Z::M;
-    delta_chunk_kernel<T, D><<<dim3(n_chunks, p.heads), DC_THREADS, smem1, stream>>>(p);
-    delta_chunk_scan_kernel<T, D><<<dim3(p.heads, p.dv / DC_COLS, n_long), DC_WALKERS + DC_READERS, smem2, stream>>>(p);
+    msgl_launch_pdl(delta_chunk_kernel<T, D>, dim3(n_chunks, p.heads), dim3(DC_THREADS), smem1, stream, p);
+    msgl_launch_pdl(delta_chunk_scan_kernel<T, D>, dim3(p.heads, p.dv / DC_COLS, n_long), dim3(DC_WALKERS + DC_READERS), smem2, stream, p);
     return msgl_check_launch();
 }
 
@@ -1835,8 +1843,8 @@ MSGL_API int msgl_delta_rule(const void* qkv, const void* proj, long long proj_s
     int code;
     if (n_chunks <= 0 || n_short) {
         const dim3 g0(T_, (kv_heads + 3) / 4);
-        if (dtype == MSGL_F32) delta_prep_kernel<float><<<g0, 128, 0, stream>>>(p);
-        else delta_prep_kernel<__nv_bfloat16><<<g0, 128, 0, stream>>>(p);
+        if (dtype == MSGL_F32) msgl_launch_pdl(delta_prep_kernel<float>, g0, dim3(128), 0, stream, p);
+        else msgl_launch_pdl(delta_prep_kernel<__nv_bfloat16>, g0, dim3(128), 0, stream, p);
         code = msgl_check_launch();
         if (code != MSGL_OK) return code;
     }
@@ -1865,8 +1873,8 @@ MSGL_API int msgl_delta_rule(const void* qkv, const void* proj, long long proj_s
             cudaFuncSetAttribute(delta_rule_kernel<__nv_bfloat16, N, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); \
             once.mark();                                                                                                    \
         }                                                                                                                   \
-        if (dtype == MSGL_F32) delta_rule_kernel<float, N, E><<<grid, warps * 32, smem, stream>>>(p);                       \
-        else delta_rule_kernel<__nv_bfloat16, N, E><<<grid, warps * 32, smem, stream>>>(p);                                 \
+        if (dtype == MSGL_F32) msgl_launch_pdl(delta_rule_kernel<float, N, E>, grid, dim3(warps * 32), smem, stream, p);             \
+        else msgl_launch_pdl(delta_rule_kernel<__nv_bfloat16, N, E>, grid, dim3(warps * 32), smem, stream, p);                      \
     } while (0)
 #define DR_LAUNCH(N)                                                                                                        \
     do {                                                                                                                    \

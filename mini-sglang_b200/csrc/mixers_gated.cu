@@ -934,6 +934,8 @@ causal_conv_act_vec_kernel(const void* in_, long long stride, int off, int C, in
                            const void* state_, const int* __restrict__ token_req, const int* __restrict__ q_start,
                            const int* __restrict__ slots, void* out_, int act, int T_) {
     constexpr int V = VecOf<T>::N;
+    pdl_wait();
+    pdl_small();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (c >= C) return;
     const T* in = reinterpret_cast<const T*>(in_) + off + c;
@@ -998,6 +1000,8 @@ causal_conv_act_vec_kernel(const void* in_, long long stride, int off, int C, in
 template <typename T>
 __global__ void conv_state_shift_kernel(const void* in_, long long stride, int off, int C, int K, void* state_,
                                         const int* __restrict__ q_start, const int* __restrict__ slots) {
+    pdl_wait();
+    pdl_small();
     const int r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
@@ -1025,7 +1029,7 @@ MSGL_API int msgl_causal_conv_act(const void* in, long long stride, int off, int
     if (vec) {
         const bool turn = T_ >= 64 * CV_TB;
         const dim3 grid((C / V + threads - 1) / threads, turn ? (T_ + CV_TB - 1) / CV_TB : T_);
-#define CV_GO(T, TB) causal_conv_act_vec_kernel<T, TB><<<grid, threads, 0, stream>>>(in, stride, off, C, K, w, bias, state, token_req, q_start, slots, out, act, T_)
+#define CV_GO(T, TB) msgl_launch_pdl(causal_conv_act_vec_kernel<T, TB>, grid, dim3(threads), 0, stream, in, stride, off, C, K, w, bias, state, token_req, q_start, slots, out, act, T_)
         if (dtype == MSGL_F32) { if (turn) CV_GO(float, CV_TB); else CV_GO(float, 1); }
         else { if (turn) CV_GO(__nv_bfloat16, CV_TB); else CV_GO(__nv_bfloat16, 1); }
 #undef CV_GO
@@ -1037,8 +1041,8 @@ MSGL_API int msgl_causal_conv_act(const void* in, long long stride, int off, int
     int code = msgl_check_launch();
     if (code != MSGL_OK || K == 1) return code;
     const dim3 g2((C + threads - 1) / threads, B);
-    if (dtype == MSGL_F32) conv_state_shift_kernel<float><<<g2, threads, 0, stream>>>(in, stride, off, C, K, state, q_start, slots);
-    else conv_state_shift_kernel<__nv_bfloat16><<<g2, threads, 0, stream>>>(in, stride, off, C, K, state, q_start, slots);
+    if (dtype == MSGL_F32) msgl_launch_pdl(conv_state_shift_kernel<float>, g2, dim3(threads), 0, stream, in, stride, off, C, K, state, q_start, slots);
+    else msgl_launch_pdl(conv_state_shift_kernel<__nv_bfloat16>, g2, dim3(threads), 0, stream, in, stride, off, C, K, state, q_start, slots);
     return msgl_check_launch();
 }
 
