@@ -38,6 +38,7 @@ struct GemmRowsParams {
     int up_off;                    // gated: how many rows of W an up row lies behind its gate row
     int expert_rows, experts;      // grouped: rows of W an expert has, how many there are
     const int* ends;               // grouped: [experts] running sum of the experts' rows in x
+    int asked;                     // the kernel before this one may be the one that writes W: its first tiles are only asked into L2 ahead of the wait
     int apart;                     // grouped: the expert whose matrix is w2map's (one that all tokens use); -1: none
     int bn, stages, splits;        // tokens a pass (a multiple of 16), ring depth, blocks that share a tile's K
     int halves;                    // 2: a block has two ranges of K (splits is 1 then), an accumulator each
@@ -58,6 +59,10 @@ __device__ __forceinline__ float2 gr_peer_load(unsigned cluster_addr) {
 }
 __device__ __forceinline__ void gr_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+__device__ __forceinline__ void gr_ask(const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];\n" ::"l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y) : "memory");
 }
 
 template <int MODE> __device__ __forceinline__ float gr_act(float g, float u, float limit) {
@@ -251,11 +256,22 @@ __global__ void __launch_bounds__(GR_THREADS) gemm_rows_kernel(const __grid_cons
                 int first = 0;
                 if (!GROUPED) {                        // weights depend on no kernel: the ring's first round is under way before the wait
                     first = min(S, n_slabs);
-                    for (int i = 0; i < first; ++i) {
-                        tc_mbar_expect_tx(bar_full(i), GR_A_BYTES + x_bytes);
-                        load_w(k_begin + i, ring + (unsigned)i * stage_bytes, bar_full(i));
+                    auto first_w = [&]() {
+                        for (int i = 0; i < first; ++i) {
+                            tc_mbar_expect_tx(bar_full(i), GR_A_BYTES + x_bytes);
+                            load_w(k_begin + i, ring + (unsigned)i * stage_bytes, bar_full(i));
+                        }
+                    };
+                    if (!p.asked) {
+                        first_w();
+                    } else {
+                        for (int i = 0; i < first; ++i) {
+                            gr_ask(wm, (k_begin + i) * 64, w_row);
+                            if (GLU) gr_ask(wm, (k_begin + i) * 64, w_row + p.up_off);
+                        }
                     }
                     pdl_wait();
+                    if (p.asked) first_w();
                     for (int i = 0; i < first; ++i) load_x(k_begin + i, ring + (unsigned)i * stage_bytes + GR_A_BYTES, bar_full(i));
                 }
                 for (int i = first; i < n_slabs; ++i) {
@@ -402,9 +418,8 @@ MSGL_API int msgl_tensor_maps() { return tc_encoder() != nullptr; }
 // splits: ranges of K; 0 = chosen from the sizes, grouped: for steps that use all experts; -1 = grouped, for steps down to a single token.
 // per_sm: 0 = chosen by gr_plan.
 // bfloat16 operands; out bfloat16 or (mode 0) float32.  K, ldx multiples of 8, ldo even, bases 16-byte aligned.
-MSGL_API int msgl_gemm_rows_apart(const void* W, const void* W2, const void* X, const void* bias, void* out, int M, int n_out, int K, long long ldx, long long ldo,
-                                  int mode, int out_f32, float limit, int experts, const int* ends, int tokens, int splits, int per_sm, void* status,
-                                  cudaStream_t stream) {
+static int gr_product(const void* W, const void* W2, const void* X, const void* bias, void* out, int M, int n_out, int K, long long ldx, long long ldo,
+                      int mode, int out_f32, float limit, int experts, const int* ends, int tokens, int splits, int per_sm, bool asked, void* status, cudaStream_t stream) {
     if (M <= 0) return MSGL_OK;
     const bool glu = mode != GR_PLAIN, grouped = experts > 0;
     if (mode < 0 || mode > 3 || n_out <= 0 || K <= 0 || (K & 7) || (ldx & 7) || (ldo & 1) || status == nullptr || experts < 0 || experts > 65535 ||
@@ -436,6 +451,7 @@ MSGL_API int msgl_gemm_rows_apart(const void* W, const void* W2, const void* X, 
     if (W2 == nullptr) w2m = wm;
     else if (!tc_matrix_map(W2, w_rows / experts, K, (long long)K * 2, glu ? 64 : 128, &w2m)) return MSGL_ERR_SIZE;
     GemmRowsParams p;
+    p.asked = asked ? 1 : 0;
     p.bias = (const __nv_bfloat16*)bias; p.out = out; p.ldo = ldo; p.M = M; p.n_valid = n_out; p.K = K;
     p.up_off = n_out; p.expert_rows = grouped ? (glu ? 2 * n_out : n_out) : 0; p.experts = experts + (W2 != nullptr ? 1 : 0); p.apart = W2 != nullptr ? experts : -1; p.ends = ends; p.bn = bn; p.limit = limit; p.status = (int*)status;
     const int tiles = (n_out + (glu ? 63 : 127)) / (glu ? 64 : 128);
@@ -465,7 +481,16 @@ MSGL_API int msgl_gemm_rows_apart(const void* W, const void* W2, const void* X, 
 #undef GR_GO
 }
 
+MSGL_API int msgl_gemm_rows_apart(const void* W, const void* W2, const void* X, const void* bias, void* out, int M, int n_out, int K, long long ldx, long long ldo,
+                                  int mode, int out_f32, float limit, int experts, const int* ends, int tokens, int splits, int per_sm, void* status, cudaStream_t stream) {
+    return gr_product(W, W2, X, bias, out, M, n_out, K, ldx, ldo, mode, out_f32, limit, experts, ends, tokens, splits, per_sm, false, status, stream);
+}
 MSGL_API int msgl_gemm_rows(const void* W, const void* X, const void* bias, void* out, int M, int n_out, int K, long long ldx, long long ldo,
                             int mode, int out_f32, float limit, int experts, const int* ends, int tokens, int splits, int per_sm, void* status, cudaStream_t stream) {
-    return msgl_gemm_rows_apart(W, nullptr, X, bias, out, M, n_out, K, ldx, ldo, mode, out_f32, limit, experts, ends, tokens, splits, per_sm, status, stream);
+    return gr_product(W, nullptr, X, bias, out, M, n_out, K, ldx, ldo, mode, out_f32, limit, experts, ends, tokens, splits, per_sm, false, status, stream);
+}
+// the plain product with weights that the launch before this one may write
+MSGL_API int msgl_gemm_rows_plain(const void* W, const void* X, const void* bias, void* out, int M, int n_out, int K, long long ldx, long long ldo, int out_f32, void* status,
+                                  cudaStream_t stream) {
+    return gr_product(W, nullptr, X, bias, out, M, n_out, K, ldx, ldo, GR_PLAIN, out_f32, 0.f, 0, nullptr, 0, 0, 0, true, status, stream);
 }

@@ -104,6 +104,7 @@ def _lib():
         lib.msgl_gemm_rows.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_int, c_float, c_int,
                                        c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
         lib.msgl_gemm_rows_apart.argtypes = [c_void_p] + lib.msgl_gemm_rows.argtypes
+        lib.msgl_gemm_rows_plain.argtypes = [c_void_p] * 4 + [c_int] * 3 + [c_ll, c_ll, c_int, c_void_p, c_void_p]
         lib.msgl_gemm_f32.argtypes = [c_void_p] * 4 + [c_int] * 3 + [c_ll, c_ll, c_void_p, c_void_p]
         lib.msgl_tensor_maps.argtypes = []
         lib.msgl_tensor_maps.restype = c_int
@@ -729,7 +730,7 @@ def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> i
 # [4096, 1024] 4.8 4.8 4.9 4.9, 2.9 3.7 4.1 4.5; [1024, 3072] 8.5 8.5 7.6 7.5, 4.5 4.5 4.9 6.1; [2048, 6144] 10.5 10.5 10.5 10.6, 8.6 9.1 8.1 9.7; [4096, 2048] 6.2 6.3 6.4 6.4, 5.3 5.5 6.2 7.4;
 # [6144, 4096] 12.8 12.9 12.1 13.2, 11.8 12.0 13.3 24; [4096, 12288] 22.0 22.1 22.6 22.7, 18.5 19.2 23.4 32; [5120, 25600] 49.6 46.8 46.2 46.3, 43.2 43.4 55 69.  Gated: [6144, 1024] 6.4 6.4 6.7 6.9,
 # 4.4 4.7 5.1 7.0; [12288, 2048] 12.0 12.3 12.5 12.9, 11.9 12.3 13.5 16.7; [24576, 4096] 35.8 36.6 36.1 36.8, 37.7 38.9 41.6 54.  (Every SM reads all rows of x: what it costs grows with them.)
-STREAM_ROWS, STREAM_ROWS_SMALL, STREAM_SMALL_WEIGHTS, STREAM_FEW_COLUMNS = 16, 32, 4_500_000, 2_072
+STREAM_ROWS, STREAM_ROWS_FEW_COLUMNS, STREAM_ROWS_SMALL, STREAM_FEW_COLUMNS, STREAM_SMALL_WEIGHTS = 16, 24, 32, 2_072, 4_500_000
 STREAM_ROWS_GATED, STREAM_GATED_LEAST, STREAM_GATED_MOST = 24, 4_000_000, 16_000_000
 
 
@@ -739,7 +740,7 @@ def _stream_rule(rows: int, N: int, K: int, gated: bool) -> bool:
         return False
     if gated:
         return rows <= STREAM_ROWS_GATED and STREAM_GATED_LEAST <= N * K <= STREAM_GATED_MOST
-    return rows <= (STREAM_ROWS_SMALL if N * K <= STREAM_SMALL_WEIGHTS or N <= STREAM_FEW_COLUMNS else STREAM_ROWS)
+    return rows <= (STREAM_ROWS_SMALL if N * K <= STREAM_SMALL_WEIGHTS else STREAM_ROWS_FEW_COLUMNS if N <= STREAM_FEW_COLUMNS else STREAM_ROWS)
 
 
 def _gemm_stream(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
@@ -910,9 +911,19 @@ def _observed(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
             or torch._C._get_tracing_state() is not None)
 
 
-def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
+# Plain products of a decode batch with a long inner size (down projections) on the decode-batch kernel, whose ranges of K give them enough blocks; us, library / kernel, at 33 / 48 / 64 rows:
+# [1024, 3072] 6.8 / 6.1, 6.8 / 6.2, 6.7 / 6.4; [2048, 8192] 13.4 / 11.2, 13.3 / 11.6, 13.4 / 12.1; [2560, 9728] 15.7 / 13.9, 15.9 / 14.4, 15.6 / 14.6; [4096, 12288] 22.6 / 21.5, 22.5 / 21.9,
+# 22.6 / 22.4; [5120, 17408] 39.0 / 33.0, 41.0 / 34.0, 36.1 / 35.1; at 80 rows behind on half of them.  Shorter inner sizes: [5120, 8192] 18.2 / 18.9 at 33 rows, [4096, 4096] 10.3 / 10.7 at 48.
+ROWS_PLAIN_MAX, ROWS_PLAIN_INNER, ROWS_PLAIN_WEIGHTS = 64, 3, 3_000_000
+
+
+def _rows_plain(rows: int, N: int, K: int) -> bool:
+    return SMALL_M_MAX < rows <= ROWS_PLAIN_MAX and K >= ROWS_PLAIN_INNER * N and N * K >= ROWS_PLAIN_WEIGHTS and not MID_GEMM
+
+
+def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype, asked: bool = False) -> Optional[torch.Tensor]:
     """x @ weight^T (mode 0) or its gated activation (1: SwiGLU, 2: ReGLU; bias [2I]) for at most 256 rows by the decode-batch kernel;
-    None where it cannot run."""
+    None where it cannot run.  asked: a plain product that was the library's: weights that the launch before may write, autocast and the current device are heeded."""
     if not (0 < x.shape[0] <= 256 and _product_ok(x, weight, bias)
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
             and not _observed(x, weight, bias)
@@ -922,9 +933,15 @@ def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     n_out = N // 2 if mode else N
     if n_out % 2 or (mode and N % 2) or (mode and out_dtype != torch.bfloat16) or not tensor_maps():
         return None
+    if asked and (torch.is_autocast_enabled() or x.get_device() != torch._C._cuda_getDevice()):
+        return None
     out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
-    code = _lib().msgl_gemm_rows(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, n_out, K, x.stride(0), n_out, mode, int(out_dtype == torch.float32),
-                                 0.0, 0, None, 0, 0, 0, _ptr(_status_tensor(x.device)), _stream())
+    if asked:
+        code = _lib().msgl_gemm_rows_plain(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, n_out, K, x.stride(0), n_out, int(out_dtype == torch.float32),
+                                           _ptr(_status_tensor(x.device)), _stream())
+    else:
+        code = _lib().msgl_gemm_rows(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, n_out, K, x.stride(0), n_out, mode, int(out_dtype == torch.float32),
+                                     0.0, 0, None, 0, 0, 0, _ptr(_status_tensor(x.device)), _stream())
     if code == 2:             # no tensor map of this layout
         return None
     _check(code, "gemm_rows")
@@ -984,7 +1001,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
 
     Up to SMALL_M_MAX bfloat16 rows, and up to 16 or 32 by the weight's size (`_stream_rule`), go through this engine's weight-streaming kernels (csrc/gemm_stream.cu,
     csrc/gemm_small_m.cu), float32 results of
-    very many columns for a decode batch through its decode-batch kernel (csrc/gemm_rows.cu, `_rows_f32`), float32 operands through the float32
+    very many columns for a decode batch and plain products with long inner sizes through its decode-batch kernel (csrc/gemm_rows.cu, `_rows_f32`, `_rows_plain`), float32 operands through the float32
     kernel of the tensor cores (csrc/gemm_f32.cu, `_f32_rule`); everything else is the
     library GEMM unless MSGL_TC_GEMM or MSGL_TC_MID ask for the tiled kernels."""
     _need_cuda(x, weight, bias)
@@ -1001,6 +1018,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         return out
     if x.dtype == torch.bfloat16 and out_dtype in (None, torch.bfloat16, torch.float32):
         y = _gemm_stream(x, weight, bias, 0, out_dtype or torch.bfloat16)
+        if y is None and x.dim() == 2 and weight.dim() == 2 and _rows_plain(x.shape[0], *weight.shape):
+            y = _gemm_rows(x, weight, bias, 0, out_dtype or torch.bfloat16, True)
         if y is not None:
             return y
     if out_dtype in (None, torch.bfloat16):

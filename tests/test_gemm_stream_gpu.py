@@ -39,6 +39,30 @@ def test_products(N, K, M, monkeypatch):
         assert ((y.double() - want).abs() <= slack + 2.0 ** -8 * want.abs() + 1e-6).all()
 
 
+@pytest.mark.parametrize("N,K", [(1024, 3072), (2560, 9728), (1002, 3208)])
+@pytest.mark.parametrize("M", [25, 33, 48, 64, 65])
+def test_long_inner_sizes(N, K, M, monkeypatch):
+    from mini_sglang_b200 import ops
+    taken, rows = [], ops._gemm_rows
+    monkeypatch.setattr(ops, "_gemm_rows", lambda *a: taken.append(rows(*a)) or taken[-1])
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w, b = (torch.randn(s, generator=g, device="cuda").bfloat16() for s in ((M, K), (N, K), (N,)))
+    size = x.double().abs() @ w.double().abs().t()
+    for bias in (None, b):
+        want = x.double() @ w.double().t() + (0 if bias is None else bias.double())
+        f32, y = ops.linear(x, w, bias, out_dtype=torch.float32), ops.linear(x, w, bias)
+        assert len(taken) == (0 if M == 65 or (M == 25 and N == 1024) or K < 3 * N else 2)
+        taken.clear()
+        if M == 65:                                           # the library's, which rounds where it likes
+            continue
+        # as above
+        assert ((f32.double() - want).abs() <= (K / 16 + 20) * 2.0 ** -24 * size + 1e-6).all()
+        assert ((y.double() - want).abs() <= (K / 16 + 20) * 2.0 ** -24 * size + 2.0 ** -8 * want.abs() + 1e-6).all()
+    with torch.autocast("cuda", torch.float16):
+        assert ops.linear(x, w).dtype == torch.float16
+    ops.check_kernel_status()
+
+
 @pytest.mark.parametrize("M", [1, 8, 16])
 def test_rows_keep_to_themselves(M):
     from mini_sglang_b200 import ops
@@ -78,6 +102,6 @@ def test_what_stays_with_the_library():
 
 def test_rule():
     from mini_sglang_b200.ops import _stream_rule as rule
-    assert rule(16, 6144, 4096, False) and not rule(17, 6144, 4096, False) and rule(32, 2064, 6144, False) and not rule(32, 2080, 6144, False) and not rule(33, 1024, 3072, False)
+    assert rule(16, 6144, 4096, False) and not rule(17, 6144, 4096, False) and rule(24, 2064, 6144, False) and not rule(25, 2064, 6144, False) and not rule(17, 2080, 6144, False) and not rule(33, 1024, 3072, False)
     assert rule(32, 4096, 1024, False) and not rule(9, 1024, 1024, False) and not rule(9, 2040, 2048, False) and not rule(9, 2048, 2056, False)
     assert rule(24, 6144, 1024, True) and not rule(25, 6144, 1024, True) and not rule(9, 12288, 2048, True) and not rule(9, 2048, 1024, True)
