@@ -473,10 +473,12 @@ template <typename T, int L, int TOK>
 __global__ void __launch_bounds__(QKR_THREADS, TOK > 1 && sizeof(T) == 4 ? 3 : 4) qknorm_rope_kvwrite_vec_kernel(
     const T* __restrict__ qkv, int qkv_stride, const int* __restrict__ positions, const int* __restrict__ out_loc,
     const void* __restrict__ qw, const void* __restrict__ kw, int w_is_f32, float eps, const float* __restrict__ table, int max_pos,
-    T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache, int page_size, int n_q, int n_kv, int T_) {
+    T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache, int page_size, int n_q, int n_kv, int T_, int attention_next) {
     constexpr int d = 16 * L, half = 8 * L;
     using H8 = Half<T, sizeof(T) / 2>;
-    pdl_small();                // ahead of the wait: decode attention then cuts up its keys and asks for the first of them while this kernel and the product before it end (8 x 4,096 keys 53.6 -> 52.8 us a layer)
+    // attention_next: decode attention is launched next, which reads nothing ahead of its own wait that a kernel of this layer writes; released here it cuts up its keys and
+    // asks for the first of them while this kernel and the product before it end (8 x 4,096 keys 53.6 -> 52.8 us a layer).  Others wait for what is ahead of this kernel, too
+    if (attention_next) pdl_small();
     const int l8 = (threadIdx.x & (L - 1)) * 8;
     const int n_heads = n_q + 2 * n_kv;
     const long long row = (long long)blockIdx.x * (QKR_THREADS / L) + threadIdx.x / L;
@@ -510,6 +512,7 @@ __global__ void __launch_bounds__(QKR_THREADS, TOK > 1 && sizeof(T) == 4 ? 3 : 4
     if (AHEAD && rotates) angles(0, tab);
     pdl_wait();
     pdl_after_wait();
+    if (!attention_next) pdl_small();
     H8 lo[TOK], hi[TOK];
 #pragma unroll
     for (int i = 0; i < TOK; ++i) {
@@ -572,7 +575,7 @@ MSGL_API int msgl_qknorm_rope_kvwrite(const void* qkv, int qkv_stride, const int
                                       const void* qw, const void* kw, int w_is_f32, float eps,
                                       const float* table, int rot, int max_pos, void* q_out, void* k_cache,
                                       void* v_cache, int page_size, int n_q, int n_kv, int d, int T_, int dtype,
-                                      int interleaved, cudaStream_t stream) {
+                                      int interleaved, int attention_next, cudaStream_t stream) {
     if (T_ <= 0) return MSGL_OK;
     if (d <= 0 || d > 32 * QKR_MAX_PER_LANE || rot < 0 || rot > d || (rot & 1) || page_size <= 0) return MSGL_ERR_SIZE;
     const int n_heads = n_q + 2 * n_kv;
@@ -594,7 +597,7 @@ MSGL_API int msgl_qknorm_rope_kvwrite(const void* qkv, int qkv_stride, const int
 #define QKR_RUN(TT, LL, TOK)                                                                                         \
     msgl_launch_pdl(qknorm_rope_kvwrite_vec_kernel<TT, LL, TOK>, vgrid, dim3(QKR_THREADS), 0, stream,                \
         (const TT*)qkv, qkv_stride, positions, out_loc, qw, kw, w_is_f32, eps, table, max_pos, (TT*)q_out,           \
-        (TT*)k_cache, (TT*)v_cache, page_size, n_q, n_kv, T_)
+        (TT*)k_cache, (TT*)v_cache, page_size, n_q, n_kv, T_, attention_next)
 #define QKR_VEC(TT, LL) do { if (few) QKR_RUN(TT, LL, 1); else QKR_RUN(TT, LL, QKR_TOK); } while (0)
         if (dtype == MSGL_F32) {
             if (L == 2) QKR_VEC(float, 2); else if (L == 4) QKR_VEC(float, 4); else if (L == 8) QKR_VEC(float, 8); else QKR_VEC(float, 16);

@@ -94,7 +94,7 @@ class PagedAttention(Mixer):
             q_weight=self.q_norm, k_weight=self.k_norm, eps=self.qk_norm_eps, rope_table=table,
             out_loc=cache.group.out_loc if writes_cache else None,
             k_cache=cache.k if writes_cache else None, v_cache=cache.v if writes_cache else None,
-            page_size=cache.page_size, interleaved=bool(getattr(self.position, "interleaved", False)))
+            page_size=cache.page_size, interleaved=bool(getattr(self.position, "interleaved", False)), attention_next=ctx.uniform_decode)
         out = torch.empty_like(q)
         self.attend(q, out, ctx, cache)
         return ops.linear(out.view(ctx.T, self.n_q * self.d), self.o)
