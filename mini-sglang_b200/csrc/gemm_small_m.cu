@@ -1,4 +1,6 @@
-// Weight-streaming matrix product for decode: out[M, N] = x[M, K] . W[N, K]^T with M <= 16 tokens.
+// Weight-streaming matrix product for decode: out[M, N] = x[M, K] . W[N, K]^T with M <= 16 tokens.  Here come weights
+// of less than 2 million elements; for larger ones gemm_stream.cu is ahead (one row, us here / there: [1024, 1024] 1.63 / 1.86,
+// [2048, 1024] 2.47 / 2.22, [1024, 3072] 4.02 / 3.08).
 //
 // With so few tokens the product is bound by reading W once from HBM, so the kernel is built
 // around that stream:
@@ -191,8 +193,9 @@ __global__ void __launch_bounds__(GS_WARPS * 32) gemm_small_m_kernel(
 }
 
 // ahead: the weights of the product that comes next (gated modes; or null), which the blocks ask into L2 as they end, so that the memory has work while the last of them and
-// the next launch leave it idle.  A feed-forward with weights that come from memory, with the request / without it, us.  1,024 x 3,072 (384 blocks): 1 token 7.8 / 8.5, 8: 7.9 / 8.6;
-// 1,024 x 2,432 (304 blocks) 6.9 / 7.4; 256 x 2,560 5.3 / 5.9; 4,096 x 3,072 with 512 outputs 14.5 / 15.3.  So where more than two blocks an SM come and all run at once (three).  With
+// the next launch leave it idle.  A feed-forward with weights that come from memory, with the request / without it, us.  Of the sizes that come here (below 2 million elements of W):
+// 256 x 2,560 (320 blocks) 5.3 / 5.9.  The line was drawn with larger ones too, which have a kernel of their own since: 1,024 x 3,072 (384 blocks): 1 token 7.8 / 8.5, 8: 7.9 / 8.6;
+// 1,024 x 2,432 (304 blocks) 6.9 / 7.4; 4,096 x 3,072 with 512 outputs 14.5 / 15.3.  So where more than two blocks an SM come and all run at once (three).  With
 // fewer each asks for more at its end, and the product itself is short: 1,024 x 1,024 (128 blocks) 5.7 / 5.5, 2,048 x 768 7.1 / 6.3; with more the first ones' requests are in the way of
 // the others' streams: 2,048 x 6,144 (768 blocks) 22.4 / 20.6.  Not for weights of more than 6.5 MB or half of this product's own: 1,024 x 2,432 with 1,664 outputs (8 MB) 8.0 / 7.8,
 // 512 x 2,432 with 1,536 outputs 7.2 / 6.6.  (Where all weights are in L2 already it costs up to 8 %.)

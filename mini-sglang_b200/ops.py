@@ -1047,7 +1047,7 @@ def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tens
     """act(x @ gate^T + bg) * (x @ up^T + bu) with gate_up = [gate; up] packed row-wise ([2I, H]) and bias = [bg; bu] or None;
     act: one of the ACT_ numbers.  Where a kernel with the activation in its epilogue applies (silu and relu; a few rows, or
     many rows in bfloat16) the [T, 2I] intermediate never exists.  ahead: the weight of the product that takes the result, which the kernel for a few rows
-    asks into L2 as it ends."""
+    and a small weight asks into L2 as it ends."""
     _need_cuda(x, gate_up, bias)
     mode = GLU_MODES.get(act)
     if mode is not None:
