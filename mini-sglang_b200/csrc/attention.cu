@@ -1415,19 +1415,26 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_simt_kernel(const AttnParam
     }
 }
 
-// The same for float32 data at the library's own head size (a multiple of 16): 16 rows a block, key tiles of 32 in two stages (cp.async, 16 bytes a
-// lane, a tile's pages looked up once a warp), both products from registers.  A warp owns four rows: a lane takes four keys of them over a
+// The same for float32 data at the library's own head size (a multiple of 16): 16 rows a block, key tiles of 32 in two or three stages (cp.async,
+// 16 bytes a lane, a tile's pages looked up once a warp and a tile ahead), both products from registers.  Two groups of four warps take half of
+// every tile's keys each and are merged at the end.  A warp owns four rows: a lane takes two keys of them over a
 // quarter of the head's elements, the four lanes that share the keys then hand each other three quarters of their sums, so that a
-// lane is left with four scores of one row; for the second product it owns four elements of the head.  Weights pass through shared
+// lane is left with two scores of one row; for the second product it owns four elements of the head.  Weights pass through shared
 // memory within the warp, so the block meets once a key tile.  The kernel above takes 26 us a key tile (4-byte loads with a page
-// lookup each, one score a thread at a time), this one 4: 210 and 37 tokens, 16 heads on 8 of 128, 186 -> 28 us.
+// lookup each, one score a thread at a time).  Device us, 16 heads on 8 of 128, one group / two groups, two stages, two steps unrolled / as it is:
+// 210 and 37 tokens 27.9 / 26.2 / 25.6, 8 on 200 21.4 / 18.8 / 17.8, 700 tokens 133.6 / 121.7 / 115.2; four steps unrolled with two stages 25.5, 18.1, 119.0.
+// Bound by the reads of shared memory (q again for every key) and, where few blocks run, by a tile's chain of 1.8 us.  With q in registers
+// (239 of them, so one block an SM) the chain is 1.5 us, but 210 and 37 tokens take 28.6 and 700 116.5.
+constexpr int F32_GROUPS = 2, F32_THREADS = F32_GROUPS * SIMT_THREADS;
+static_assert(F32_GROUPS == 2, "the merge at the end is of two");
+__host__ __device__ constexpr int f32_stages(int d) { return d <= 128 ? 3 : 2; }     // (three of a larger head would leave no head size above 256)
 template <int D>
-__global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams p) {
-    constexpr int R = SIMT_R, KT = SIMT_KT, LD = D + 4, LDP = KT + 8, NV = (D + 127) / 128;
+__global__ void __launch_bounds__(F32_THREADS, D <= 128 ? 2 : 1) attn_f32_kernel(const AttnParams p) {
+    constexpr int R = SIMT_R, KT = SIMT_KT, LD = D + 4, LDP = KT + 8, NV = (D + 127) / 128, GK = KT / F32_GROUPS, J = GK / 8, ST = f32_stages(D);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* Qs = reinterpret_cast<float*>(smem_raw);          // [R][LD]
     float* Ps = Qs + R * LD;                                 // [R][LDP]
-    float* KV = Ps + R * LDP;                                // two stages of K [KT][LD], V [KT][LD]
+    float* KV = Ps + R * LDP;                                // stages of K [KT][LD], V [KT][LD]
     __shared__ int sh_tile[4];
     const int G = p.n_q / p.n_kv;
     const int Gc = G <= R ? G : R;
@@ -1445,7 +1452,7 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams
     int p_min, p_max, kt_begin, kt_end;
     key_tile_range(p, ti, KT, split, ns, p_min, p_max, kt_begin, kt_end);
     const int k_first = first_key(p, p_min);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, all_warp = tid >> 5, warp = all_warp & 3, part = GK * (all_warp >> 2);   // part: the group's first key of a tile
     const float* qg = reinterpret_cast<const float*>(p.q);
     const float* kc = reinterpret_cast<const float*>(p.k_cache);
     const float* vc = reinterpret_cast<const float*>(p.v_cache);
@@ -1455,13 +1462,15 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams
     auto row_token = [&](int r) { return (size_t)(ti.q_base + ti.t0 + r / Gc); };
     auto row_head = [&](int r) { return kvh * G + chunk * R + r % Gc; };
 
-    auto fetch = [&](int kt, int st) {                       // rows past the last key, before the window or the chunk arrive as zeros
-        float* Ks = KV + st * 2 * KT * LD;
+    auto look = [&](int kt) {                                // a lane's key of a tile: its page, or -1
         const int mine = kt * KT + lane;
-        const int pg_mine = (mine <= p_max && mine >= k_first) ? bt[page_index(p, mine)] : -1;
+        return kt < kt_end && mine <= p_max && mine >= k_first ? bt[page_index(p, mine)] : -1;
+    };
+    auto fetch = [&](int kt, int st, int pg_mine) {          // rows past the last key, before the window or the chunk arrive as zeros
+        float* Ks = KV + st * 2 * KT * LD;
 #pragma unroll
-        for (int i = 0; i < KT / 4; ++i) {
-            const int kl = warp * (KT / 4) + i, pg = __shfl_sync(0xffffffffu, pg_mine, kl);
+        for (int i = 0; i < KT / (4 * F32_GROUPS); ++i) {
+            const int kl = all_warp * (KT / (4 * F32_GROUPS)) + i, pg = __shfl_sync(0xffffffffu, pg_mine, kl);
             const size_t off = (((size_t)max(pg, 0) * p.n_kv + kvh) * p.page_size + (pg >= 0 ? page_slot(p, kt * KT + kl) : 0)) * D;
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
@@ -1473,9 +1482,15 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams
             }
         }
     };
-    if (kt_begin < kt_end) fetch(kt_begin, 0);
-    cp_async_commit();
-    for (int idx = tid; idx < R * (D / 4); idx += SIMT_THREADS) {
+    int pg_next = look(kt_begin);                            // a tile ahead: the copies do not wait for the table
+#pragma unroll
+    for (int st = 0; st < ST - 1; ++st) {
+        const int pg = pg_next;
+        pg_next = look(kt_begin + st + 1);
+        if (kt_begin + st < kt_end) fetch(kt_begin + st, st, pg);
+        cp_async_commit();
+    }
+    for (int idx = tid; idx < R * (D / 4); idx += F32_THREADS) {
         const int r = idx / (D / 4), e = 4 * (idx - r * (D / 4));
         *reinterpret_cast<float4*>(Qs + r * LD + e) =
             row_valid(r) ? *reinterpret_cast<const float4*>(qg + (row_token(r) * p.n_q + row_head(r)) * D + e) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1489,36 +1504,36 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams
     for (int v = 0; v < NV; ++v)
 #pragma unroll
         for (int r = 0; r < 4; ++r) o[v][r][0] = o[v][r][1] = o[v][r][2] = o[v][r][3] = 0.f;
-    for (int kt = kt_begin, st = 0; kt < kt_end; ++kt, st ^= 1) {
-        cp_async_wait<0>();
-        __syncthreads();                                     // the tile (and q) lie in shared memory; the other stage is free
-        if (kt + 1 < kt_end) fetch(kt + 1, st ^ 1);
+    for (int kt = kt_begin, st = 0; kt < kt_end; ++kt, st = st == ST - 1 ? 0 : st + 1) {
+        cp_async_wait<ST - 2>();
+        __syncthreads();                                     // the tile (and q) lie in shared memory; the stage before it is free
+        if (kt + ST - 1 < kt_end) fetch(kt + ST - 1, st == 0 ? ST - 1 : st - 1, pg_next);
         cp_async_commit();
+        pg_next = look(kt + ST);
         const float* Ks = KV + st * 2 * KT * LD;
         const float* Vs = Ks + KT * LD;
-        float s[4];
+        float s[J];
         {
-            float acc[4][4] = {};
+            float acc[4][J] = {};
             const float* qp = Qs + 4 * warp * LD + 4 * (lane >> 3);
-            const float* kp = Ks + kg * LD + 4 * (lane >> 3);
-#pragma unroll 2
+            const float* kp = Ks + (part + kg) * LD + 4 * (lane >> 3);
+#pragma unroll 4
             for (int e = 0; e < D; e += 16) {
-                float4 q4[4], k4[4];
+                float4 q4[4], k4[J];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    q4[i] = *reinterpret_cast<const float4*>(qp + i * LD + e);
-                    k4[i] = *reinterpret_cast<const float4*>(kp + 8 * i * LD + e);
-                }
+                for (int i = 0; i < 4; ++i) q4[i] = *reinterpret_cast<const float4*>(qp + i * LD + e);
+#pragma unroll
+                for (int j = 0; j < J; ++j) k4[j] = *reinterpret_cast<const float4*>(kp + 8 * j * LD + e);
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
+                    for (int j = 0; j < J; ++j) {
                         acc[i][j] = fmaf(q4[i].x, k4[j].x, acc[i][j]); acc[i][j] = fmaf(q4[i].y, k4[j].y, acc[i][j]);
                         acc[i][j] = fmaf(q4[i].z, k4[j].z, acc[i][j]); acc[i][j] = fmaf(q4[i].w, k4[j].w, acc[i][j]);
                     }
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < J; ++j) {
                 float v[2];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) v[i] = (b3 ? acc[2 + i][j] : acc[i][j]) + __shfl_xor_sync(0xffffffffu, b3 ? acc[i][j] : acc[2 + i][j], 8);
@@ -1527,8 +1542,8 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams
         }
         float mx = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int key = kt * KT + kg + 8 * j;
+        for (int j = 0; j < J; ++j) {
+            const int key = kt * KT + part + kg + 8 * j;
             s[j] = my_live && key <= my_pos && key >= my_first ? s[j] * sc : -INFINITY;
             mx = fmaxf(mx, s[j]);
         }
@@ -1538,10 +1553,10 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams
         m_run = m_new;
         l_run *= alpha;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < J; ++j) {
             const float w = exp2f(s[j] - mu);
             l_run += w;
-            Ps[my_row * LDP + kg + 8 * j] = w;
+            Ps[my_row * LDP + part + kg + 8 * j] = w;
         }
         __syncwarp();
 #pragma unroll
@@ -1550,8 +1565,8 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams
 #pragma unroll
             for (int v = 0; v < NV; ++v) { o[v][r][0] *= a; o[v][r][1] *= a; o[v][r][2] *= a; o[v][r][3] *= a; }
         }
-#pragma unroll 2
-        for (int kl = 0; kl < KT; kl += 4) {
+#pragma unroll 4
+        for (int kl = part; kl < part + GK; kl += 4) {
             float w[4][4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(w[r]) = *reinterpret_cast<const float4*>(Ps + (4 * warp + r) * LDP + kl);
@@ -1575,6 +1590,39 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams
     }
 #pragma unroll
     for (int x = 1; x < 8; x <<= 1) l_run += __shfl_xor_sync(0xffffffffu, l_run, x);
+    // the second group hands its sums over in the tiles' place, the first adds them to its own
+    float* Ox = KV;                                          // [R][D]
+    float* Mx = KV + R * D;                                  // [R][2]
+    __syncthreads();
+    if (part) {
+        if (kg == 0) { Mx[2 * my_row] = m_run; Mx[2 * my_row + 1] = l_run; }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const int e = 4 * (lane + 32 * v);
+                if (e < D) *reinterpret_cast<float4*>(Ox + (4 * warp + r) * D + e) = make_float4(o[v][r][0], o[v][r][1], o[v][r][2], o[v][r][3]);
+            }
+    }
+    __syncthreads();
+    if (part) return;
+    const float m_x = Mx[2 * my_row], m_all = fmaxf(m_run, m_x), m_at = (m_all == -INFINITY) ? 0.f : m_all;
+    const float f_own = exp2f(m_run - m_at), f_x = exp2f(m_x - m_at);
+    l_run = l_run * f_own + Mx[2 * my_row + 1] * f_x;
+    m_run = m_all;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int src = (r >> 1) * 8 + (r & 1) * 16;
+        const float fo = __shfl_sync(0xffffffffu, f_own, src), fx = __shfl_sync(0xffffffffu, f_x, src);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int e = 4 * (lane + 32 * v);
+            if (e >= D) continue;
+            const float4 x = *reinterpret_cast<const float4*>(Ox + (4 * warp + r) * D + e);
+            o[v][r][0] = o[v][r][0] * fo + x.x * fx; o[v][r][1] = o[v][r][1] * fo + x.y * fx;
+            o[v][r][2] = o[v][r][2] * fo + x.z * fx; o[v][r][3] = o[v][r][3] * fo + x.w * fx;
+        }
+    }
     float* og = reinterpret_cast<float*>(p.out);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -1600,7 +1648,7 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_f32_kernel(const AttnParams
     }
 }
 template <int D> static size_t f32_smem_bytes() {
-    return sizeof(float) * ((size_t)SIMT_R * (D + 4) + SIMT_R * (SIMT_KT + 8) + (size_t)4 * SIMT_KT * (D + 4));
+    return sizeof(float) * ((size_t)SIMT_R * (D + 4) + SIMT_R * (SIMT_KT + 8) + (size_t)2 * f32_stages(D) * SIMT_KT * (D + 4));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1896,7 +1944,7 @@ static int attention_launch(const void* q, void* out, const void* k_cache, const
                 cudaFuncSetAttribute(attn_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f32_smem_bytes<HD>());
                 f32_attr.mark();
             }
-            attn_f32_kernel<HD><<<grid, SIMT_THREADS, f32_smem_bytes<HD>(), stream>>>(p);
+            attn_f32_kernel<HD><<<grid, F32_THREADS, f32_smem_bytes<HD>(), stream>>>(p);
         } else if (dtype == MSGL_F32) {
             if (smem > 48 * 1024 && smem > granted[0]) {
                 cudaFuncSetAttribute(attn_simt_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
