@@ -747,18 +747,25 @@ def _stream_rule(rows: int, N: int, K: int, gated: bool) -> bool:
 def _gemm_stream(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
     """x @ weight^T (mode 0) or its gated activation (1: SwiGLU, 2: ReGLU) of 9 rows and more by csrc/gemm_stream.cu; None where another kernel or the library is to be called: by
     `_stream_rule`, operands that do not lie as the kernel reads them or on another device than the current one, autocast, and whatever a kernel called by address would slip past."""
-    if not (USE_SMALL_M and not MID_GEMM and x.dim() == 2 and weight.dim() == 2 and SMALL_M_MAX < x.shape[0] <= STREAM_ROWS_SMALL
-            and _stream_rule(x.shape[0], weight.shape[0], weight.shape[1], mode != 0) and (mode == 0 or weight.shape[0] // 2 % 8 == 0) and _product_ok(x, weight, bias)
+    # (a prompt step of a few tokens waits for the host: every size is asked for once, as `_gemm_f32` does)
+    if x.dim() != 2 or weight.dim() != 2:
+        return None
+    (M, K), (N, k_weight) = x.shape, weight.shape
+    if not SMALL_M_MAX < M <= STREAM_ROWS_SMALL or K != k_weight or not _stream_rule(M, N, K, mode != 0) or MID_GEMM or not USE_SMALL_M:
+        return None
+    pitch, dev = x.stride(0), x.get_device()
+    if not (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.stride(1) == 1 and pitch % 8 == 0 and weight.is_contiguous() and weight.get_device() == dev
+            and (bias is None or (bias.dtype == torch.bfloat16 and bias.dim() == 1 and bias.shape[0] == N and bias.is_contiguous() and bias.get_device() == dev))
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
             and not _observed(x, weight, bias)):                     # (before the addresses are asked for: some of these have none)
         return None
-    if (x.data_ptr() | weight.data_ptr()) % 16 or x.get_device() != torch._C._cuda_getDevice() or torch.is_autocast_enabled():
+    x_at, w_at = x.data_ptr(), weight.data_ptr()
+    if (x_at | w_at) % 16 or dev != torch._C._cuda_getDevice() or torch.is_autocast_enabled():
         return None
-    M, (N, K) = x.shape[0], weight.shape
-    n_out = N // 2 if mode else N
-    out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
-    code = _lib().msgl_gemm_stream(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), n_out, mode, int(out_dtype == torch.float32), _ptr(_status_words(x.device)),
-                                   _stream())
+    n_out, f32 = N // 2 if mode else N, out_dtype == torch.float32
+    out = x.new_empty((M, n_out), dtype=torch.float32) if f32 else x.new_empty((M, n_out))
+    status = _status_words(x.device) if _status is None else _status
+    code = _lib().msgl_gemm_stream(w_at, x_at, _ptr(bias), out.data_ptr(), M, N, K, pitch, n_out, mode, int(f32), _ptr(status), _stream())
     if code == 2:             # no tensor map of this layout
         return None
     _check(code, "gemm_stream")
@@ -927,22 +934,22 @@ def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     None where it cannot run.  asked: a plain product that was the library's: weights that the launch before may write, autocast and the current device are heeded."""
     if not (0 < x.shape[0] <= 256 and _product_ok(x, weight, bias)
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
-            and not _observed(x, weight, bias)
-            and (x.stride(0) >= x.shape[1] or x.shape[0] == 1) and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and weight.shape[1] % 8 == 0):
+            and not _observed(x, weight, bias)):
         return None
-    M, (N, K) = x.shape[0], weight.shape
-    n_out = N // 2 if mode else N
+    M, (N, K), pitch, x_at, w_at = x.shape[0], weight.shape, x.stride(0), x.data_ptr(), weight.data_ptr()
+    if (x_at | w_at) % 16 or K % 8 or (pitch < K and M != 1):
+        return None
+    n_out, f32 = N // 2 if mode else N, int(out_dtype == torch.float32)
     if n_out % 2 or (mode and N % 2) or (mode and out_dtype != torch.bfloat16) or not tensor_maps():
         return None
     if asked and (torch.is_autocast_enabled() or x.get_device() != torch._C._cuda_getDevice()):
         return None
-    out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+    out = x.new_empty((M, n_out), dtype=out_dtype)
+    status = _status_tensor(x.device).data_ptr()
     if asked:
-        code = _lib().msgl_gemm_rows_plain(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, n_out, K, x.stride(0), n_out, int(out_dtype == torch.float32),
-                                           _ptr(_status_tensor(x.device)), _stream())
+        code = _lib().msgl_gemm_rows_plain(w_at, x_at, _ptr(bias), out.data_ptr(), M, n_out, K, pitch, n_out, f32, status, _stream())
     else:
-        code = _lib().msgl_gemm_rows(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, n_out, K, x.stride(0), n_out, mode, int(out_dtype == torch.float32),
-                                     0.0, 0, None, 0, 0, 0, _ptr(_status_tensor(x.device)), _stream())
+        code = _lib().msgl_gemm_rows(w_at, x_at, _ptr(bias), out.data_ptr(), M, n_out, K, pitch, n_out, mode, f32, 0.0, 0, None, 0, 0, 0, status, _stream())
     if code == 2:             # no tensor map of this layout
         return None
     _check(code, "gemm_rows")
@@ -1010,21 +1017,22 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         y = _gemm_rows(x, weight, bias, 0, torch.float32)
         if y is not None:
             return y
-    if _small_m_ok(x, weight, bias) and out_dtype in (None, torch.bfloat16, torch.float32):
-        M, (N, K) = x.shape[0], weight.shape
+    rows = x.shape[0]
+    if rows <= SMALL_M_MAX and _small_m_ok(x, weight, bias) and out_dtype in (None, torch.bfloat16, torch.float32):
+        M, (N, K) = rows, weight.shape
         od = out_dtype or torch.bfloat16
         out = torch.empty((M, N), dtype=od, device=x.device)
         code = _small_m(weight, x, bias, out, M, N, K, N, 0, int(od == torch.float32))
         _check(code, "gemm_small_m")
         return out
-    if x.dtype == torch.bfloat16 and out_dtype in (None, torch.bfloat16, torch.float32):
-        y = _gemm_stream(x, weight, bias, 0, out_dtype or torch.bfloat16)
-        if y is None and x.dim() == 2 and weight.dim() == 2 and _rows_plain(x.shape[0], *weight.shape):
+    if SMALL_M_MAX < rows <= ROWS_PLAIN_MAX and x.dtype == torch.bfloat16 and out_dtype in (None, torch.bfloat16, torch.float32):
+        y = _gemm_stream(x, weight, bias, 0, out_dtype or torch.bfloat16) if rows <= STREAM_ROWS_SMALL else None
+        if y is None and x.dim() == 2 and weight.dim() == 2 and x.shape[1] >= ROWS_PLAIN_INNER * weight.shape[0] and _rows_plain(rows, *weight.shape):
             y = _gemm_rows(x, weight, bias, 0, out_dtype or torch.bfloat16, True)
         if y is not None:
             return y
-    if out_dtype in (None, torch.bfloat16):
-        y = _tc_gemm(x, weight, bias, 0) if x.shape[0] >= TC_GEMM_MIN_M else _tc_gemm_mid(x, weight, bias, 0)
+    if out_dtype in (None, torch.bfloat16) and (rows >= TC_GEMM_MIN_M or MID_GEMM):
+        y = _tc_gemm(x, weight, bias, 0) if rows >= TC_GEMM_MIN_M else _tc_gemm_mid(x, weight, bias, 0)
         if y is not None:
             return y
     if x.dtype == torch.float32 and out_dtype in (None, torch.float32):

@@ -131,7 +131,7 @@ def paged_attend(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KV
             if ops.attention_decode_runs(q, out, cache.k, cache.v, kv_len=ctx.kv_len, block_table=g.block_table, n_kv=n_kv, page_size=cache.page_size, scale=scale,
                                          workspace=ctx.workspace):
                 return
-        elif _beside_portions(q, out, ctx, cache, n_kv=n_kv, scale=scale):
+        elif 1 in ctx.host_q_lens and _beside_portions(q, out, ctx, cache, n_kv=n_kv, scale=scale):
             return
     max_split = g.max_split if g.nsplit is not None else 1
     part_o = part_ml = None
@@ -183,10 +183,10 @@ def paged_attend(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KV
 
 def _beside_portions(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KVCacheView, *, n_kv: int, scale: float) -> bool:
     """A step of prompt portions with decoded tokens among them: the portions on the tcgen05 kernel, the single tokens by the launch that cuts its keys up by itself, beside
-    the tiles.  False, with nothing launched, where either does not apply or a run of a few tokens would go to the decode kernel."""
+    the tiles.  (`paged_attend` asks where there are single tokens.)  False, with nothing launched, where either does not apply or a run of a few tokens would go to the decode kernel."""
     lens, table, P, ws = ctx.host_q_lens, cache.group.block_table, cache.page_size, ctx.workspace
     G = q.shape[1] // n_kv
-    if 1 not in lens or not ops.decode_runs_supported(q, ctx.B, n_kv, P, table.shape[1], ws) or not ops.tc_supported(128, q.dtype, G):
+    if not ops.decode_runs_supported(q, ctx.B, n_kv, P, table.shape[1], ws) or not ops.tc_supported(128, q.dtype, G):
         return False
     longer = [n for n in lens if n != 1]
     if not longer or min(longer) <= 8 // G:
