@@ -637,14 +637,18 @@ def decode_runs_supported(q: torch.Tensor, B: int, n_kv: int, page_size: int, ta
             and 0 < B <= RUNS_MAX_REQUESTS and B * n_kv * (table_width * (page_size // 16) + 1) < 1 << 30)
 
 
-def decode_runs_scratch(q: torch.Tensor, B: int, n_kv: int, workspace) -> Optional[torch.Tensor]:
-    """Counters (16 KB or a word a request and kv head), then partial results of two segments a block; None in a capture that comes before they exist."""
-    return workspace.counters("attn_runs", max(B * n_kv + 3 & ~3, 4096) + 2 * 8 * (128 + 2) * min(sm_count(q.device), RUNS_MAX_BLOCKS))
+def decode_runs_scratch(q: torch.Tensor, B: int, n_kv: int, workspace) -> Optional[Tuple[torch.Tensor, torch.Tensor]]:
+    """(counters, a word a request and kv head and zero between launches; float32 partial results of two segments a block), or None in a capture that comes before the counters exist.
+    Tensors of their own: a step's partial results must not reach words that a step of another size counts in.  Counters are made for the largest batch, so that no batch outgrows them."""
+    count = workspace.counters("attn_runs", max(RUNS_MAX_REQUESTS, B) * n_kv)
+    if count is None:
+        return None
+    return count, workspace.get("attn_runs_part", 2 * 8 * (128 + 2) * min(sm_count(q.device), RUNS_MAX_BLOCKS), torch.float32)
 
 
 def attention_decode_runs(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, *, kv_len: torch.Tensor,
                           block_table: torch.Tensor, n_kv: int, page_size: int, scale: float, workspace, q_start: Optional[torch.Tensor] = None,
-                          beside_tiles: bool = False, scratch: Optional[torch.Tensor] = None) -> bool:
+                          beside_tiles: bool = False, scratch: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> bool:
     """Attention of a decode step (one new token a request, all of a request's keys) in one launch that deals the keys out over the SMs by
     itself and merges its partial results (csrc/attention_runs.cuh).  With q_start, int32 [B + 1], of the requests of any step that bring one token, out's rows of the others
     are left alone; beside_tiles: the launch before this one is the prefill kernel of the same step, beside which it may run; scratch: from `decode_runs_scratch`, asked for ahead of
@@ -661,8 +665,7 @@ def attention_decode_runs(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Ten
         assert q.is_contiguous() and out.is_contiguous() and block_table.stride(1) == 1
         assert kv_len.numel() == B and out.shape == q.shape and (q_start is None or q_start.numel() == B + 1)
     blocks = min(sm_count(q.device), RUNS_MAX_BLOCKS)
-    count = scratch.data_ptr()
-    part = count + 4 * max(B * n_kv + 3 & ~3, 4096)
+    count, part = scratch[0].data_ptr(), scratch[1].data_ptr()
     code = _attn_lib(d).msgl_attention_decode_runs(
         q.data_ptr(), out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), kv_len.data_ptr(), block_table.data_ptr(), part, part + blocks * 16 * d * 4,
         count, _ptr(q_start), int(beside_tiles), B, n_q, n_kv, page_size, block_table.stride(0), scale, blocks, _stream())

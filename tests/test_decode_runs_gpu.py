@@ -93,6 +93,78 @@ def test_single_tokens_among_portions(q_lens, kv, beside):
         assert err.max() < 0.02 * want.abs().max() and err.pow(2).mean().sqrt() < 0.004 * want.pow(2).mean().sqrt() + 1e-4, r
 
 
+# (n_kv, requests and their keys, one call behind the other): counters of more than 16 KB, then calls that leave partial results, then the first again
+ONE_WORKSPACE = [(32, [(200, 2000), (64, 2000), (200, 2000)]), (64, [(96, 1500), (32, 1500), (96, 1500)]), (40, [(200, 300), (8, 4000), (200, 300), (256, 700), (3, 9000), (200, 300)]),
+                 (8, [(256, 900), (1, 9000), (256, 900)])]
+
+
+@pytest.mark.parametrize("n_kv,calls", ONE_WORKSPACE)
+@pytest.mark.parametrize("form", ["eager", "graphs", "mixed"])
+def test_one_workspace_for_steps_of_every_size(n_kv, calls, form):
+    from mini_sglang_b200 import ops
+    from mini_sglang_b200.parts import Workspace
+    P, pages = 16, 400
+    g = torch.Generator(device=DEV).manual_seed(n_kv)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)      # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)      # noqa: E731
+    k_c, v_c = (rnd(pages + 1, n_kv, P, D).bfloat16() for _ in range(2))
+    ws, steps, graphs = Workspace(DEV), {}, {}
+    for B, keys in calls:
+        if (B, keys) in steps:
+            continue
+        kv = [keys + 7 * i % 500 for i in range(B)]
+        width = -(-max(kv) // P)
+        table = i32([[1 + (7 * r + 13 * i) % pages for i in range(width)] for r in range(B)])      # (pages are shared: nothing is written)
+        q = (2 * rnd(B, n_kv, D)).bfloat16()
+        out = torch.empty_like(q)
+        kw = dict(kv_len=i32(kv), block_table=table, n_kv=n_kv, page_size=P, scale=D ** -0.5)
+        if form == "mixed":                   # (every request brings one token)
+            kw["q_start"] = torch.arange(B + 1, dtype=torch.int32, device=DEV)
+        want = torch.empty(B, n_kv, D, dtype=torch.float64, device=DEV)
+        for r, k in enumerate(kv):
+            pos = torch.arange(k, device=DEV)
+            kk, vv = (c[table[r].long()[pos // P], :, pos % P].double() for c in (k_c, v_c))
+            want[r] = torch.einsum("hk,khd->hd", (torch.einsum("hd,khd->hk", q[r].double(), kk) * D ** -0.5).softmax(-1), vv)
+        steps[B, keys] = q, out, kw, want
+
+    def call(step, ws):
+        assert ops.attention_decode_runs(step[0], step[1], k_c, v_c, workspace=ws, **step[2])
+
+    if form == "graphs":                      # as an engine captures them: the batch runs eagerly first
+        for key, step in steps.items():
+            call(step, ws)
+            graphs[key] = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graphs[key]):
+                call(step, ws)
+    for B, keys in calls:
+        q, out, _, want = step = steps[B, keys]
+        out.fill_(float("nan"))
+        if form == "graphs":
+            graphs[B, keys].replay()
+        else:
+            call(step, ws)
+        err = (out.double() - want).abs()
+        scale = want.abs().amax((1, 2), keepdim=True)
+        # as above
+        assert (err < 0.02 * scale).all() and err.pow(2).mean().sqrt() < 0.004 * want.pow(2).mean().sqrt() + 1e-4, (B, keys)
+        assert not ws._bufs["attn_runs"][:B * n_kv].any()
+
+
+def test_counters_keep_to_themselves(monkeypatch):
+    """Whatever the order of the sizes, a step's counters are words that no step's partial results are written to."""
+    from mini_sglang_b200 import ops
+    from mini_sglang_b200.parts import Workspace
+    ws = Workspace(DEV)
+    q = torch.empty(1, 1, D, dtype=torch.bfloat16, device=DEV)
+    for B, n_kv in ((200, 40), (8, 40), (256, 64), (3, 8), (200, 40), (256, 64), (256, 1)):
+        count, part = ops.decode_runs_scratch(q, B, n_kv, ws)
+        assert count.numel() >= B * n_kv and not count.any()
+        assert part.numel() >= 2 * 8 * (D + 2) * min(ops.sm_count(q.device), ops.RUNS_MAX_BLOCKS)
+        part.fill_(1.0)
+    monkeypatch.setattr(ws, "_capturing", lambda: True)
+    assert ops.decode_runs_scratch(q, 256, 65, ws) is None and ops.decode_runs_scratch(q, 200, 64, ws) is not None
+
+
 def test_counters_are_not_made_inside_a_capture(monkeypatch):
     from mini_sglang_b200.parts import Workspace
     ws = Workspace(DEV)
