@@ -747,28 +747,30 @@ def _stream_rule(rows: int, N: int, K: int, gated: bool) -> bool:
     return rows <= (STREAM_ROWS_SMALL if N * K <= STREAM_SMALL_WEIGHTS else STREAM_ROWS_FEW_COLUMNS if N <= STREAM_FEW_COLUMNS else STREAM_ROWS)
 
 
+def _by_address(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], N: int) -> bool:
+    """Whether operands of a product that was the library's, x [M, K] and weight [N, K], lie as a kernel called by address reads them, on the current device, and nothing looks on that
+    it would slip past: gradients, autocast, `_observed`."""
+    # (a prompt step of a few tokens waits for the host: one look at everything, each thing asked for once)
+    dev, (pitch, step) = x.get_device(), x.stride()
+    return (x.dtype is torch.bfloat16 and weight.dtype is torch.bfloat16 and step == 1 and pitch % 8 == 0 and weight.is_contiguous() and weight.get_device() == dev
+            and (bias is None or (bias.dtype == torch.bfloat16 and bias.dim() == 1 and bias.shape[0] == N and bias.is_contiguous() and bias.get_device() == dev))
+            and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
+            and not _observed(x, weight, bias)                       # (before the addresses are asked for: some of these have none)
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0 and dev == torch._C._cuda_getDevice() and not torch.is_autocast_enabled())
+
+
 def _gemm_stream(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
     """x @ weight^T (mode 0) or its gated activation (1: SwiGLU, 2: ReGLU) of 9 rows and more by csrc/gemm_stream.cu; None where another kernel or the library is to be called: by
-    `_stream_rule`, operands that do not lie as the kernel reads them or on another device than the current one, autocast, and whatever a kernel called by address would slip past."""
-    # (a prompt step of a few tokens waits for the host: every size is asked for once, as `_gemm_f32` does)
+    `_stream_rule` or `_by_address`."""
     if x.dim() != 2 or weight.dim() != 2:
         return None
     (M, K), (N, k_weight) = x.shape, weight.shape
-    if not SMALL_M_MAX < M <= STREAM_ROWS_SMALL or K != k_weight or not _stream_rule(M, N, K, mode != 0) or MID_GEMM or not USE_SMALL_M:
-        return None
-    pitch, dev = x.stride(0), x.get_device()
-    if not (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.stride(1) == 1 and pitch % 8 == 0 and weight.is_contiguous() and weight.get_device() == dev
-            and (bias is None or (bias.dtype == torch.bfloat16 and bias.dim() == 1 and bias.shape[0] == N and bias.is_contiguous() and bias.get_device() == dev))
-            and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
-            and not _observed(x, weight, bias)):                     # (before the addresses are asked for: some of these have none)
-        return None
-    x_at, w_at = x.data_ptr(), weight.data_ptr()
-    if (x_at | w_at) % 16 or dev != torch._C._cuda_getDevice() or torch.is_autocast_enabled():
+    if not SMALL_M_MAX < M <= STREAM_ROWS_SMALL or K != k_weight or not _stream_rule(M, N, K, mode != 0) or MID_GEMM or not USE_SMALL_M or not _by_address(x, weight, bias, N):
         return None
     n_out, f32 = N // 2 if mode else N, out_dtype == torch.float32
     out = x.new_empty((M, n_out), dtype=torch.float32) if f32 else x.new_empty((M, n_out))
     status = _status_words(x.device) if _status is None else _status
-    code = _lib().msgl_gemm_stream(w_at, x_at, _ptr(bias), out.data_ptr(), M, N, K, pitch, n_out, mode, int(f32), _ptr(status), _stream())
+    code = _lib().msgl_gemm_stream(weight.data_ptr(), x.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K, x.stride(0), n_out, mode, int(f32), _ptr(status), _stream())
     if code == 2:             # no tensor map of this layout
         return None
     _check(code, "gemm_stream")
@@ -932,9 +934,28 @@ def _rows_plain(rows: int, N: int, K: int) -> bool:
     return SMALL_M_MAX < rows <= ROWS_PLAIN_MAX and K >= ROWS_PLAIN_INNER * N and N * K >= ROWS_PLAIN_WEIGHTS and not MID_GEMM
 
 
-def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype, asked: bool = False) -> Optional[torch.Tensor]:
+def _gemm_rows_plain(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out_dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """x @ weight^T by the decode-batch kernel where it is ahead of the library (`_rows_plain`); None where the library is to be called: by that rule or `_by_address`, rows of x that
+    overlap, or a stream capture that comes before the status words, which the kernel cannot go without."""
+    if x.dim() != 2 or weight.dim() != 2:
+        return None
+    (M, K), (N, k_weight) = x.shape, weight.shape
+    if K != k_weight or not _rows_plain(M, N, K) or K % 8 or N % 2 or not _by_address(x, weight, bias, N):
+        return None
+    pitch, status, f32 = x.stride(0), _status_words(x.device) if _status is None else _status, out_dtype == torch.float32
+    if pitch < K or status is None:
+        return None
+    out = x.new_empty((M, N), dtype=torch.float32) if f32 else x.new_empty((M, N))
+    code = _lib().msgl_gemm_rows_plain(weight.data_ptr(), x.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K, pitch, N, int(f32), status.data_ptr(), _stream())
+    if code == 2:             # no tensor map of this layout
+        return None
+    _check(code, "gemm_rows")
+    return out
+
+
+def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], mode: int, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
     """x @ weight^T (mode 0) or its gated activation (1: SwiGLU, 2: ReGLU; bias [2I]) for at most 256 rows by the decode-batch kernel;
-    None where it cannot run.  asked: a plain product that was the library's: weights that the launch before may write, autocast and the current device are heeded."""
+    None where it cannot run."""
     if not (0 < x.shape[0] <= 256 and _product_ok(x, weight, bias)
             and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)))
             and not _observed(x, weight, bias)):
@@ -942,17 +963,12 @@ def _gemm_rows(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     M, (N, K), pitch, x_at, w_at = x.shape[0], weight.shape, x.stride(0), x.data_ptr(), weight.data_ptr()
     if (x_at | w_at) % 16 or K % 8 or (pitch < K and M != 1):
         return None
-    n_out, f32 = N // 2 if mode else N, int(out_dtype == torch.float32)
+    n_out = N // 2 if mode else N
     if n_out % 2 or (mode and N % 2) or (mode and out_dtype != torch.bfloat16) or not tensor_maps():
         return None
-    if asked and (torch.is_autocast_enabled() or x.get_device() != torch._C._cuda_getDevice()):
-        return None
     out = x.new_empty((M, n_out), dtype=out_dtype)
-    status = _status_tensor(x.device).data_ptr()
-    if asked:
-        code = _lib().msgl_gemm_rows_plain(w_at, x_at, _ptr(bias), out.data_ptr(), M, n_out, K, pitch, n_out, f32, status, _stream())
-    else:
-        code = _lib().msgl_gemm_rows(w_at, x_at, _ptr(bias), out.data_ptr(), M, n_out, K, pitch, n_out, mode, f32, 0.0, 0, None, 0, 0, 0, status, _stream())
+    code = _lib().msgl_gemm_rows(w_at, x_at, _ptr(bias), out.data_ptr(), M, n_out, K, pitch, n_out, mode, int(out_dtype == torch.float32),
+                                 0.0, 0, None, 0, 0, 0, _ptr(_status_tensor(x.device)), _stream())
     if code == 2:             # no tensor map of this layout
         return None
     _check(code, "gemm_rows")
@@ -1031,7 +1047,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if SMALL_M_MAX < rows <= ROWS_PLAIN_MAX and x.dtype == torch.bfloat16 and out_dtype in (None, torch.bfloat16, torch.float32):
         y = _gemm_stream(x, weight, bias, 0, out_dtype or torch.bfloat16) if rows <= STREAM_ROWS_SMALL else None
         if y is None and x.dim() == 2 and weight.dim() == 2 and x.shape[1] >= ROWS_PLAIN_INNER * weight.shape[0] and _rows_plain(rows, *weight.shape):
-            y = _gemm_rows(x, weight, bias, 0, out_dtype or torch.bfloat16, True)
+            y = _gemm_rows_plain(x, weight, bias, out_dtype or torch.bfloat16)
         if y is not None:
             return y
     if out_dtype in (None, torch.bfloat16) and (rows >= TC_GEMM_MIN_M or MID_GEMM):

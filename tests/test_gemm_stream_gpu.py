@@ -43,15 +43,15 @@ def test_products(N, K, M, monkeypatch):
 @pytest.mark.parametrize("M", [25, 33, 48, 64, 65])
 def test_long_inner_sizes(N, K, M, monkeypatch):
     from mini_sglang_b200 import ops
-    taken, rows = [], ops._gemm_rows
-    monkeypatch.setattr(ops, "_gemm_rows", lambda *a: taken.append(rows(*a)) or taken[-1])
+    taken, rows = [], ops._gemm_rows_plain
+    monkeypatch.setattr(ops, "_gemm_rows_plain", lambda *a: taken.append(rows(*a)) or taken[-1])
     g = torch.Generator(device="cuda").manual_seed(M)
     x, w, b = (torch.randn(s, generator=g, device="cuda").bfloat16() for s in ((M, K), (N, K), (N,)))
     size = x.double().abs() @ w.double().abs().t()
     for bias in (None, b):
         want = x.double() @ w.double().t() + (0 if bias is None else bias.double())
         f32, y = ops.linear(x, w, bias, out_dtype=torch.float32), ops.linear(x, w, bias)
-        assert len(taken) == (0 if M == 65 or (M == 25 and N == 1024) or K < 3 * N else 2)
+        assert len(taken) == (0 if M == 65 or (M == 25 and N == 1024) or K < 3 * N else 2) and all(t is not None for t in taken)      # (None: the library's after all)
         taken.clear()
         if M == 65:                                           # the library's, which rounds where it likes
             continue
@@ -61,6 +61,22 @@ def test_long_inner_sizes(N, K, M, monkeypatch):
     with torch.autocast("cuda", torch.float16):
         assert ops.linear(x, w).dtype == torch.float16
     ops.check_kernel_status()
+
+
+@pytest.mark.parametrize("N,K,M", [(1024, 3072, 48), (1024, 3072, 17), (1024, 2048, 12), (1024, 2048, 4)])
+def test_a_capture_before_the_status_words_exist(N, K, M, monkeypatch):
+    from mini_sglang_b200 import ops
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    want = ops.linear(x, w).clone()
+    monkeypatch.setattr(ops, "_status", None)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = ops.linear(x, w)
+    assert ops._status is None
+    graph.replay()
+    # two ways of summing K products, each rounded once to bfloat16
+    size = x.double().abs() @ w.double().abs().t()
+    assert ((y.double() - want.double()).abs() <= 2.0 ** -7 * want.double().abs() + (K / 8 + 40) * 2.0 ** -24 * size).all()
 
 
 @pytest.mark.parametrize("M", [1, 8, 16])
