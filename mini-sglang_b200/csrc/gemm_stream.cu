@@ -296,7 +296,9 @@ static int gst_launch(const void* W, StreamParams p, int grid, cudaStream_t stre
     const size_t sums = p.bufs * RED * p.M, room = 227 * 1024 - FIXED - sums;
     p.stages = (int)((room < GST_RING ? room : GST_RING) / (stage + x_stage));
     if (p.stages > GST_MAX_STAGES) p.stages = GST_MAX_STAGES;
-    if (p.stages < 2) p.stages = 2;
+    // full passes of five to eight tokens: with two stages a round is asked for when the one before it is read.  us at 8 rows, two / three, blocks of 16 rows: [20480, 2560] 21.3 / 19.4, 20.4;
+    // [32000, 2048] 25.1 / 23.3, 24.6; [65536, 2048] 46.7 / 44.3, 44.4
+    if (p.stages < 3) p.stages = 3 * (stage + x_stage) <= room ? 3 : 2;
     if (p.stages > total) p.stages = total;
     // fragments of rows that a pass does not have are read behind the last stage
     const size_t reach = p.ragged ? (size_t)(GST_WARPS - 1) * p.per_pass * 128 + COLS * 128 : (size_t)COLS * GST_ROW, over = reach > p.half ? reach - p.half : 0;

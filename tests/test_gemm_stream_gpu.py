@@ -39,6 +39,22 @@ def test_products(N, K, M, monkeypatch):
         assert ((y.double() - want).abs() <= slack + 2.0 ** -8 * want.abs() + 1e-6).all()
 
 
+@pytest.mark.parametrize("N,K", [(14208, 1216), (20480, 640), (21312, 544)])
+@pytest.mark.parametrize("M", [5, 8])
+def test_full_passes_of_a_few_rows(N, K, M):
+    """Passes of 47 and 48 columns: the ring's third stage lies beyond its usual size."""
+    from mini_sglang_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    x, w = (torch.randn(s, generator=g, device="cuda").bfloat16() for s in ((M, K), (N, K)))
+    out = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    status = ops._status_tensor(x.device)
+    assert ops._lib().msgl_gemm_stream(w.data_ptr(), x.data_ptr(), None, out.data_ptr(), M, N, K, K, N, 0, 1, status.data_ptr(), ops._stream()) == 0
+    size = x.double().abs() @ w.double().abs().t()
+    # as above
+    assert ((out.double() - x.double() @ w.double().t()).abs() <= (K / 16 + 20) * 2.0 ** -24 * size + 1e-6).all()
+    ops.check_kernel_status()
+
+
 @pytest.mark.parametrize("N,K", [(1024, 3072), (2560, 9728), (1002, 3208)])
 @pytest.mark.parametrize("M", [25, 33, 48, 64, 65])
 def test_long_inner_sizes(N, K, M, monkeypatch):
