@@ -721,7 +721,7 @@ def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> i
     """Weights of some size go through one block an SM (csrc/gemm_stream.cu), smaller ones, for which its barriers and tensor maps cost more than they bring, through
     blocks of 16 rows (csrc/gemm_small_m.cu).  ahead: a weight that gated products of the second kind are to ask into L2 for the product behind them (or None; one that lies
     elsewhere or in pieces is left alone); with the first the product behind has its own weights on their way by itself."""
-    if M <= 8 and N * K >= STREAM_MIN_WEIGHTS:
+    if M <= 8 and _stream_rule(M, N, K, mode != 0):
         code = _lib().msgl_gemm_stream(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), ldo, mode, out_f32, _ptr(_status_words(x.device)), _stream())
         if code != 2:             # (2: no tensor map of this layout)
             return code
@@ -730,20 +730,35 @@ def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> i
     return _lib().msgl_gemm_small_m(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), ldo, mode, out_f32, _ptr(ahead), ahead.numel() * ahead.element_size() if ahead is not None else 0, _stream())
 
 
-# Up to which rows the kernel of one block an SM is ahead of the library (plain products) and the decode-batch kernel (gated ones); us at 9 / 16 / 24 / 32 rows, other kernel then this one.
+# Where the kernel of one block an SM is ahead; us of a product with weights from memory, other kernel (blocks of 16 rows up to 8 rows, then the library and, gated, the decode-batch kernel) then
+# this one.  Lines in columns follow the B200's 148 SMs: 7,104 columns are 48 on each, the most of one pass, 2,072 are 14, 2,960 and (gated) 4,144 are 20.
+# Up to 8 rows: behind where a block has more than one pass of few rounds (576 elements of K each), by STREAM_SHORT's pairs of columns and K (the first for plain products alone).  8 rows of [7120, 768]
+# 4.2 5.1, [7120, 3072] 10.4 10.9, [7424, 2048] 8.4 8.4, [8192, 1024] 5.3 6.0, [8192, 4096] 16.0 14.2, [9216, 1024] 5.5 6.1, [9728, 1024] 6.0 6.1, [15936, 640] 6.5 7.2; gated [8192, 1024] 5.4 5.7,
+# [7424, 2048] 9.0 8.0.  An inner size that is no multiple of 64 is nine copies a round: [560, 8672] 7.5 11.2, [928, 2976] 3.8 4.4, gated 4.1 6.9, [7712, 1120] 5.5 6.2, but [3088, 1056] 3.6 2.9.
+# From 9 rows on every SM reads all rows of x, which costs more the more rows there are, and passes cost more: at 9 / 16 / 24 / 32 rows
 # [4096, 1024] 4.8 4.8 4.9 4.9, 2.9 3.7 4.1 4.5; [1024, 3072] 8.5 8.5 7.6 7.5, 4.5 4.5 4.9 6.1; [2048, 6144] 10.5 10.5 10.5 10.6, 8.6 9.1 8.1 9.7; [4096, 2048] 6.2 6.3 6.4 6.4, 5.3 5.5 6.2 7.4;
 # [6144, 4096] 12.8 12.9 12.1 13.2, 11.8 12.0 13.3 24; [4096, 12288] 22.0 22.1 22.6 22.7, 18.5 19.2 23.4 32; [5120, 25600] 49.6 46.8 46.2 46.3, 43.2 43.4 55 69.  Gated: [6144, 1024] 6.4 6.4 6.7 6.9,
-# 4.4 4.7 5.1 7.0; [12288, 2048] 12.0 12.3 12.5 12.9, 11.9 12.3 13.5 16.7; [24576, 4096] 35.8 36.6 36.1 36.8, 37.7 38.9 41.6 54.  (Every SM reads all rows of x: what it costs grows with them.)
+# 4.4 4.7 5.1 7.0; [12288, 2048] 12.0 12.3 12.5 12.9, 11.9 12.3 13.5 16.7; [24576, 4096] 35.8 36.6 36.1 36.8, 37.7 38.9 41.6 54.
+# More than one pass at 16 rows: [13776, 6144] 29.8 30.6, [14112, 192] 4.1 4.4, [64064, 448] 12.8 16.1, [116480, 128] 9.5 21.6; gated, two passes: [10240, 1024] 8.1 7.6 and [10240, 1536] 9.6 10.5 at 24 rows, seven:
+# [45984, 96] 4.9 11.2.  From K = 14,336 on the library cuts K up: [1024, 12288] x 16 27.0 15.9, [1024, 14336] 14.4 17.9, with more columns [2560, 25600] x 9 31.1 25.7.  No multiple of 64: [448, 6880] x 16 8.0 8.8,
+# [5872, 608] x 24 4.5 5.0, gated [1408, 5280] x 16 7.8 10.1, [4992, 2528] x 21 8.8 9.7.
 STREAM_ROWS, STREAM_ROWS_FEW_COLUMNS, STREAM_ROWS_SMALL, STREAM_FEW_COLUMNS, STREAM_SMALL_WEIGHTS = 16, 24, 32, 2_072, 4_500_000
-STREAM_ROWS_GATED, STREAM_GATED_LEAST, STREAM_GATED_MOST = 24, 4_000_000, 16_000_000
+STREAM_ROWS_GATED, STREAM_GATED_LEAST, STREAM_GATED_MOST = 24, 4_000_000, 16_000_000      # ([8192, 2048], 16.8 million, is ahead too, [10240, 2048] and [12288, 2048] are not)
+STREAM_ONE_PASS, STREAM_ROUND, STREAM_SHORT, STREAM_GATED_INNER = 7_104, 576, ((7_400, 3_600), (10_000, 1_300), (17_000, 800)), 1_100
+STREAM_LONG_INNER, STREAM_LONG_COLUMNS, STREAM_RAGGED, STREAM_RAGGED_GATED = 13_000, 2_560, 2_960, 4_144
 
 
 def _stream_rule(rows: int, N: int, K: int, gated: bool) -> bool:
-    """Whether a product of more rows than the weight-streaming kernels' own goes to the one of one block an SM all the same."""
-    if N * K < STREAM_MIN_WEIGHTS or N % 16 or K % 32:
+    """Whether a product goes to the kernel of one block an SM."""
+    if N * K < STREAM_MIN_WEIGHTS or N % 16 or K % 32 or (K % 64 and N < (STREAM_RAGGED_GATED if gated else STREAM_RAGGED)):
         return False
+    if rows <= 8:
+        return N <= STREAM_ONE_PASS or K <= STREAM_ROUND or not (K % 64 or any(N <= columns and K <= inner for columns, inner in STREAM_SHORT[gated:]))
     if gated:
-        return rows <= STREAM_ROWS_GATED and STREAM_GATED_LEAST <= N * K <= STREAM_GATED_MOST
+        return (rows <= (STREAM_ROWS if K % 64 else STREAM_ROWS_GATED) and STREAM_GATED_LEAST <= N * K <= STREAM_GATED_MOST
+                and (N <= STREAM_ONE_PASS or (N <= 2 * STREAM_ONE_PASS and (rows <= STREAM_ROWS or K <= STREAM_GATED_INNER))))
+    if N > STREAM_ONE_PASS or (K > STREAM_LONG_INNER and N < STREAM_LONG_COLUMNS) or (K % 64 and rows > STREAM_ROWS):
+        return False
     return rows <= (STREAM_ROWS_SMALL if N * K <= STREAM_SMALL_WEIGHTS else STREAM_ROWS_FEW_COLUMNS if N <= STREAM_FEW_COLUMNS else STREAM_ROWS)
 
 
