@@ -942,11 +942,15 @@ def _observed(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
 # Plain products of a decode batch with a long inner size (down projections) on the decode-batch kernel, whose ranges of K give them enough blocks; us, library / kernel, at 33 / 48 / 64 rows:
 # [1024, 3072] 6.8 / 6.1, 6.8 / 6.2, 6.7 / 6.4; [2048, 8192] 13.4 / 11.2, 13.3 / 11.6, 13.4 / 12.1; [2560, 9728] 15.7 / 13.9, 15.9 / 14.4, 15.6 / 14.6; [4096, 12288] 22.6 / 21.5, 22.5 / 21.9,
 # 22.6 / 22.4; [5120, 17408] 39.0 / 33.0, 41.0 / 34.0, 36.1 / 35.1; at 80 rows behind on half of them.  Shorter inner sizes: [5120, 8192] 18.2 / 18.9 at 33 rows, [4096, 4096] 10.3 / 10.7 at 48.
+# From K = 20,480 on the library cuts K of few columns up: at 48 rows [512, 18432] 16.5 / 16.0, [512, 20480] 13.9 / 17.4, at 64 [1536, 24576] 20.5 / 22.6, [3584, 32768] 45.2 / 44.2.  Between 4,096 and 5,120
+# columns eight ranges of K make 264 to 304 blocks in clusters of eight, and it is behind (256 blocks of 4,096 columns and 320 of 5,120 are not): at 48 rows [4096, 16384] 28.9 / 28.2, [4352, 16384] 29.0 / 39.9, [4736, 16128] 30.4 / 40.2, [5120, 16384] 38.9 / 32.1.
 ROWS_PLAIN_MAX, ROWS_PLAIN_INNER, ROWS_PLAIN_WEIGHTS = 64, 3, 3_000_000
+ROWS_PLAIN_LONGEST, ROWS_PLAIN_LONG_COLUMNS, ROWS_PLAIN_GAP = 18_432, 3_584, (4_096, 5_120)
 
 
 def _rows_plain(rows: int, N: int, K: int) -> bool:
-    return SMALL_M_MAX < rows <= ROWS_PLAIN_MAX and K >= ROWS_PLAIN_INNER * N and N * K >= ROWS_PLAIN_WEIGHTS and not MID_GEMM
+    return (SMALL_M_MAX < rows <= ROWS_PLAIN_MAX and K >= ROWS_PLAIN_INNER * N and N * K >= ROWS_PLAIN_WEIGHTS and (K <= ROWS_PLAIN_LONGEST or N >= ROWS_PLAIN_LONG_COLUMNS)
+            and not ROWS_PLAIN_GAP[0] < N < ROWS_PLAIN_GAP[1] and not MID_GEMM)
 
 
 def _gemm_rows_plain(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out_dtype: torch.dtype) -> Optional[torch.Tensor]:

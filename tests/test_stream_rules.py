@@ -14,3 +14,9 @@ GATED_BEHIND = [(8, 7168, 1024), (8, 8192, 768), (1, 1408, 2336), (8, 3424, 8224
 def test_one_block_an_sm(sizes, gated, wanted):
     from mini_sglang_b200 import ops
     assert [s for s in sizes if ops._stream_rule(*s, gated) != wanted] == []
+
+
+def test_long_inner_sizes():
+    from mini_sglang_b200.ops import _rows_plain as rule
+    assert all(rule(*s) for s in ((17, 1024, 3072), (33, 1002, 3208), (48, 4096, 12288), (64, 5120, 17408), (48, 512, 18432), (64, 3584, 32768), (64, 4096, 16384)))
+    assert not any(rule(*s) for s in ((65, 1024, 3072), (8, 1024, 3072), (48, 512, 20480), (33, 224, 27520), (64, 1536, 24576), (48, 4352, 16384), (17, 4736, 16128), (33, 5112, 16384), (48, 4096, 4096)))
