@@ -643,7 +643,7 @@ def decode_runs_scratch(q: torch.Tensor, B: int, n_kv: int, workspace) -> Option
     count = workspace.counters("attn_runs", max(RUNS_MAX_REQUESTS, B) * n_kv)
     if count is None:
         return None
-    return count, workspace.get("attn_runs_part", 2 * 8 * (128 + 2) * min(sm_count(q.device), RUNS_MAX_BLOCKS), torch.float32)
+    return count, workspace.whole("attn_runs_part", 2 * 8 * (128 + 2) * min(sm_count(q.device), RUNS_MAX_BLOCKS), torch.float32)
 
 
 def attention_decode_runs(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, *, kv_len: torch.Tensor,
@@ -722,7 +722,8 @@ def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> i
     blocks of 16 rows (csrc/gemm_small_m.cu).  ahead: a weight that gated products of the second kind are to ask into L2 for the product behind them (or None; one that lies
     elsewhere or in pieces is left alone); with the first the product behind has its own weights on their way by itself."""
     if M <= 8 and _stream_rule(M, N, K, mode != 0):
-        code = _lib().msgl_gemm_stream(_ptr(weight), _ptr(x), _ptr(bias), _ptr(out), M, N, K, x.stride(0), ldo, mode, out_f32, _ptr(_status_words(x.device)), _stream())
+        status = _status_words(x.device) if _status is None else _status
+        code = _lib().msgl_gemm_stream(weight.data_ptr(), x.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K, x.stride(0), ldo, mode, out_f32, _ptr(status), _stream())
         if code != 2:             # (2: no tensor map of this layout)
             return code
     if ahead is not None and (not ahead.is_contiguous() or ahead.get_device() != x.get_device()):
@@ -796,15 +797,17 @@ def _product_ok(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     """Whether x [M, K] . weight [N, K]^T + bias [N] is a bfloat16 product whose operands lie as the kernels read them: rows of x one behind
     the other on 16-byte pitches, packed weights and bias, one device.  The kernels get addresses and sizes only, so whatever
     does not fit goes to the library, which takes it or refuses it."""
-    return (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2 and weight.dim() == 2 and x.shape[1] == weight.shape[1]
-            and x.stride(1) == 1 and x.stride(0) % 8 == 0 and weight.is_contiguous() and x.get_device() == weight.get_device()
-            and (bias is None or (bias.dtype == torch.bfloat16 and bias.dim() == 1 and bias.shape[0] == weight.shape[0] and bias.is_contiguous()
+    return (x.dtype is torch.bfloat16 and weight.dtype is torch.bfloat16 and x.dim() == 2 and weight.dim() == 2 and x.shape[1] == (sizes := weight.shape)[1]
+            and (strides := x.stride())[1] == 1 and strides[0] % 8 == 0 and weight.is_contiguous() and x.get_device() == weight.get_device()
+            and (bias is None or (bias.dtype == torch.bfloat16 and bias.dim() == 1 and bias.shape[0] == sizes[0] and bias.is_contiguous()
                                   and bias.get_device() == weight.get_device())))
 
 
 def _small_m_ok(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> bool:
-    return (USE_SMALL_M and 0 < x.shape[0] <= SMALL_M_MAX and _product_ok(x, weight, bias)
-            and weight.shape[1] % 32 == 0 and weight.shape[0] % 16 == 0)
+    if not (USE_SMALL_M and 0 < x.shape[0] <= SMALL_M_MAX and _product_ok(x, weight, bias)):
+        return False
+    N, K = weight.shape
+    return K % 32 == 0 and N % 16 == 0
 
 
 # This engine's tcgen05 GEMM (csrc/gemm_tc.cu) against the library's, measured on B200 at Qwen3-8B's sizes.  With SwiGLU in
@@ -944,6 +947,7 @@ def _observed(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
 # 22.6 / 22.4; [5120, 17408] 39.0 / 33.0, 41.0 / 34.0, 36.1 / 35.1; at 80 rows behind on half of them.  Shorter inner sizes: [5120, 8192] 18.2 / 18.9 at 33 rows, [4096, 4096] 10.3 / 10.7 at 48.
 # From K = 20,480 on the library cuts K of few columns up: at 48 rows [512, 18432] 16.5 / 16.0, [512, 20480] 13.9 / 17.4, at 64 [1536, 24576] 20.5 / 22.6, [3584, 32768] 45.2 / 44.2.  Between 4,096 and 5,120
 # columns eight ranges of K make 264 to 304 blocks in clusters of eight, and it is behind (256 blocks of 4,096 columns and 320 of 5,120 are not): at 48 rows [4096, 16384] 28.9 / 28.2, [4352, 16384] 29.0 / 39.9, [4736, 16128] 30.4 / 40.2, [5120, 16384] 38.9 / 32.1.
+# (What the rule takes was measured at 533 sizes and rows: one of them, 64 rows of [4096, 14336], is 3 % behind.)
 ROWS_PLAIN_MAX, ROWS_PLAIN_INNER, ROWS_PLAIN_WEIGHTS = 64, 3, 3_000_000
 ROWS_PLAIN_LONGEST, ROWS_PLAIN_LONG_COLUMNS, ROWS_PLAIN_GAP = 18_432, 3_584, (4_096, 5_120)
 
@@ -1041,6 +1045,11 @@ def _gemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
     return out
 
 
+_PRODUCT_RESULTS = (None, torch.bfloat16, torch.float32)
+
+
+# Prompt steps of a few tokens wait for the host, so what stands ahead of a product's launch counts (us of host time a call on 9 to 64 bfloat16 rows: F.linear 10.2, this function ahead of it 0.8, on
+# the streaming kernel 10.5 in all, on the decode-batch kernel 10.5): a tensor's dtype and device are asked for at 50 ns, its shape at 130, a single size or stride at 220
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """y = x @ weight^T (+ bias); weight is [out, in] as stored in the checkpoint.
@@ -1050,26 +1059,27 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     very many columns for a decode batch and plain products with long inner sizes through its decode-batch kernel (csrc/gemm_rows.cu, `_rows_f32`, `_rows_plain`), float32 operands through the float32
     kernel of the tensor cores (csrc/gemm_f32.cu, `_f32_rule`); everything else is the
     library GEMM unless MSGL_TC_GEMM or MSGL_TC_MID ask for the tiled kernels."""
-    _need_cuda(x, weight, bias)
+    if not (x.is_cuda and weight.is_cuda and (bias is None or bias.is_cuda)):
+        _need_cuda(x, weight, bias)
     if out_dtype == torch.float32 and x.dim() == 2 and _rows_f32(x.shape[0], weight.shape[0], x.shape[1], x.device):
         y = _gemm_rows(x, weight, bias, 0, torch.float32)
         if y is not None:
             return y
     rows = x.shape[0]
-    if rows <= SMALL_M_MAX and _small_m_ok(x, weight, bias) and out_dtype in (None, torch.bfloat16, torch.float32):
+    if rows <= SMALL_M_MAX and _small_m_ok(x, weight, bias) and out_dtype in _PRODUCT_RESULTS:
         M, (N, K) = rows, weight.shape
         od = out_dtype or torch.bfloat16
         out = torch.empty((M, N), dtype=od, device=x.device)
         code = _small_m(weight, x, bias, out, M, N, K, N, 0, int(od == torch.float32))
         _check(code, "gemm_small_m")
         return out
-    if SMALL_M_MAX < rows <= ROWS_PLAIN_MAX and x.dtype == torch.bfloat16 and out_dtype in (None, torch.bfloat16, torch.float32):
+    if SMALL_M_MAX < rows <= ROWS_PLAIN_MAX and x.dtype is torch.bfloat16 and out_dtype in _PRODUCT_RESULTS:
         y = _gemm_stream(x, weight, bias, 0, out_dtype or torch.bfloat16) if rows <= STREAM_ROWS_SMALL else None
-        if y is None and x.dim() == 2 and weight.dim() == 2 and x.shape[1] >= ROWS_PLAIN_INNER * weight.shape[0] and _rows_plain(rows, *weight.shape):
+        if y is None and (sizes := weight.shape)[-1] >= ROWS_PLAIN_INNER * sizes[0]:
             y = _gemm_rows_plain(x, weight, bias, out_dtype or torch.bfloat16)
         if y is not None:
             return y
-    if out_dtype in (None, torch.bfloat16) and (rows >= TC_GEMM_MIN_M or MID_GEMM):
+    if (rows >= TC_GEMM_MIN_M or MID_GEMM) and out_dtype in (None, torch.bfloat16):
         y = _tc_gemm(x, weight, bias, 0) if rows >= TC_GEMM_MIN_M else _tc_gemm_mid(x, weight, bias, 0)
         if y is not None:
             return y

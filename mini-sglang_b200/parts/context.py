@@ -67,6 +67,10 @@ class Workspace:
         return self.device.type == "cuda" and torch.cuda.is_current_stream_capturing()
 
     def get(self, name: str, numel: int, dtype: torch.dtype) -> torch.Tensor:
+        return self.whole(name, numel, dtype)[:numel]
+
+    def whole(self, name: str, numel: int, dtype: torch.dtype) -> torch.Tensor:
+        """As `get`, with what the buffer holds beyond numel (a slice costs as much host time as all the rest)."""
         buf = self._bufs.get(name)
         if buf is None or buf.numel() < numel or buf.dtype != dtype:
             if name in self._captured or (buf is not None and self._capturing()):
@@ -79,7 +83,7 @@ class Workspace:
             self._bufs[name] = buf
         if name not in self._captured and self._capturing():
             self._captured.add(name)
-        return buf[:numel]
+        return buf
 
     def counters(self, name: str, numel: int) -> Optional[torch.Tensor]:
         """At least numel int32 words that are zero when they are made, for kernels that leave zero what they count with.  None where they would have to be made inside a stream
