@@ -1,6 +1,6 @@
 from __future__ import annotations
 
-from typing import Dict, Optional, Tuple
+from typing import Dict, Optional, Sequence, Tuple
 
 import torch
 
@@ -181,6 +181,16 @@ def paged_attend(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KV
         ops.attention_combine(part_o, part_ml, None if ctx.uniform_decode else ctx.token_req, g.nsplit, out, max_split, **joined)
 
 
+# Beside prefill tiles the launch that cuts its keys up by itself is behind the decode kernel where a block strings many short segments (a request under a kv head) together, us of the attention launches, decode
+# kernel / beside the tiles: 200 single tokens on 32 kv heads with 14,000 keys among them 112 / 124, on 64 with 65,000 465 / 555, 100 on 40 with 6,300 72 / 77.  Not with 100 on 32 (27,000 keys 143 / 137),
+# not where every request has up to 256 keys (a warp a segment: 200 on 64 147 / 56) and not with many keys a request (200 on 32 with 171,000 617 / 495).
+MANY_SEGMENTS, SHORT_SEGMENT, SEGMENT_MEAN = 3_600, 256, 720
+
+
+def _many_short_segments(keys: Sequence[int], n_kv: int) -> bool:
+    return len(keys) * n_kv > MANY_SEGMENTS and max(keys) > SHORT_SEGMENT and sum(keys) < SEGMENT_MEAN * len(keys)
+
+
 def _beside_portions(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache: KVCacheView, *, n_kv: int, scale: float) -> bool:
     """A step of prompt portions with decoded tokens among them: the portions on the tcgen05 kernel, the single tokens by the launch that cuts its keys up by itself, beside
     the tiles.  (`paged_attend` asks where there are single tokens.)  False, with nothing launched, where either does not apply or a run of a few tokens would go to the decode kernel."""
@@ -190,6 +200,8 @@ def _beside_portions(q: torch.Tensor, out: torch.Tensor, ctx: StepContext, cache
         return False
     longer = [n for n in lens if n != 1]
     if not longer or min(longer) <= 8 // G:
+        return False
+    if (ctx.B - len(longer)) * n_kv > MANY_SEGMENTS and _many_short_segments([k for n, k in zip(lens, ctx.host_kv_lens) if n == 1], n_kv):
         return False
     scratch = ops.decode_runs_scratch(q, ctx.B, n_kv, ws)
     if scratch is None:

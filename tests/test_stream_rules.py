@@ -20,3 +20,9 @@ def test_long_inner_sizes():
     from mini_sglang_b200.ops import _rows_plain as rule
     assert all(rule(*s) for s in ((17, 1024, 3072), (33, 1002, 3208), (48, 4096, 12288), (64, 5120, 17408), (48, 512, 18432), (64, 3584, 32768), (64, 4096, 16384)))
     assert not any(rule(*s) for s in ((65, 1024, 3072), (8, 1024, 3072), (48, 512, 20480), (33, 224, 27520), (64, 1536, 24576), (48, 4352, 16384), (17, 4736, 16128), (33, 5112, 16384), (48, 4096, 4096)))
+
+
+def test_single_tokens_among_portions():
+    from mini_sglang_b200.parts.attention import _many_short_segments as apart
+    assert apart([10] * 199 + [600], 32) and apart([300] * 100, 40) and apart([324] * 200, 64)
+    assert not apart([300] * 100, 32) and not apart([256] * 200, 64) and not apart([850] * 200, 32) and not apart([300] * 255, 8)
