@@ -719,7 +719,7 @@ STREAM_MIN_WEIGHTS = 2_000_000
 
 def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> int:
     """Weights of some size go through one block an SM (csrc/gemm_stream.cu), smaller ones, for which its barriers and tensor maps cost more than they bring, through
-    blocks of 16 rows (csrc/gemm_small_m.cu).  ahead: a weight that gated products of the second kind are to ask into L2 for the product behind them (or None; one that lies
+    blocks of 16 rows (csrc/gemm_small_m.cu).  ahead: a weight that gated products of the second kind, with inner sizes below 423, ask into L2 for the product behind them (or None; one that lies
     elsewhere or in pieces is left alone); with the first the product behind has its own weights on their way by itself."""
     if M <= 8 and _stream_rule(M, N, K, mode != 0):
         status = _status_words(x.device) if _status is None else _status
@@ -742,10 +742,10 @@ def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> i
 # 4.4 4.7 5.1 7.0; [12288, 2048] 12.0 12.3 12.5 12.9, 11.9 12.3 13.5 16.7; [24576, 4096] 35.8 36.6 36.1 36.8, 37.7 38.9 41.6 54.
 # More than one pass at 16 rows: [13776, 6144] 29.8 30.6, [14112, 192] 4.1 4.4, [64064, 448] 12.8 16.1, [116480, 128] 9.5 21.6; gated, two passes: [10240, 1024] 8.1 7.6 and [10240, 1536] 9.6 10.5 at 24 rows, seven:
 # [45984, 96] 4.9 11.2.  From K = 14,336 on the library cuts K up: [1024, 12288] x 16 27.0 15.9, [1024, 14336] 14.4 17.9, with more columns [2560, 25600] x 9 31.1 25.7.  No multiple of 64: [448, 6880] x 16 8.0 8.8,
-# [5872, 608] x 24 4.5 5.0, gated [1408, 5280] x 16 7.8 10.1, [4992, 2528] x 21 8.8 9.7.
+# [5872, 608] x 24 4.5 5.0, gated [1408, 5280] x 16 7.8 10.1, [4992, 2528] x 21 8.8 9.7, [8192, 1760] x 16 9.5 10.5.  Gated, long inner sizes, 24 rows: [1024, 8192] 9.5 10.0, [928, 11904] 11.9 13.2, [1184, 6848] 8.8 8.5.
 STREAM_ROWS, STREAM_ROWS_FEW_COLUMNS, STREAM_ROWS_SMALL, STREAM_FEW_COLUMNS, STREAM_SMALL_WEIGHTS = 16, 24, 32, 2_072, 4_500_000
 STREAM_ROWS_GATED, STREAM_GATED_LEAST, STREAM_GATED_MOST = 24, 4_000_000, 16_000_000      # ([8192, 2048], 16.8 million, is ahead too, [10240, 2048] and [12288, 2048] are not)
-STREAM_ONE_PASS, STREAM_ROUND, STREAM_SHORT, STREAM_GATED_INNER = 7_104, 576, ((7_400, 3_600), (10_000, 1_300), (17_000, 800)), 1_100
+STREAM_ONE_PASS, STREAM_ROUND, STREAM_SHORT, STREAM_GATED_INNER, STREAM_GATED_LONG = 7_104, 576, ((7_400, 3_600), (10_000, 1_300), (17_000, 800)), 1_100, 7_000
 STREAM_LONG_INNER, STREAM_LONG_COLUMNS, STREAM_RAGGED, STREAM_RAGGED_GATED = 13_000, 2_560, 2_960, 4_144
 
 
@@ -756,8 +756,8 @@ def _stream_rule(rows: int, N: int, K: int, gated: bool) -> bool:
     if rows <= 8:
         return N <= STREAM_ONE_PASS or K <= STREAM_ROUND or not (K % 64 or any(N <= columns and K <= inner for columns, inner in STREAM_SHORT[gated:]))
     if gated:
-        return (rows <= (STREAM_ROWS if K % 64 else STREAM_ROWS_GATED) and STREAM_GATED_LEAST <= N * K <= STREAM_GATED_MOST
-                and (N <= STREAM_ONE_PASS or (N <= 2 * STREAM_ONE_PASS and (rows <= STREAM_ROWS or K <= STREAM_GATED_INNER))))
+        return (rows <= (STREAM_ROWS if K % 64 or K > STREAM_GATED_LONG else STREAM_ROWS_GATED) and STREAM_GATED_LEAST <= N * K <= STREAM_GATED_MOST
+                and (N <= STREAM_ONE_PASS or (N <= 2 * STREAM_ONE_PASS and not K % 64 and (rows <= STREAM_ROWS or K <= STREAM_GATED_INNER))))
     if N > STREAM_ONE_PASS or (K > STREAM_LONG_INNER and N < STREAM_LONG_COLUMNS) or (K % 64 and rows > STREAM_ROWS):
         return False
     return rows <= (STREAM_ROWS_SMALL if N * K <= STREAM_SMALL_WEIGHTS else STREAM_ROWS_FEW_COLUMNS if N <= STREAM_FEW_COLUMNS else STREAM_ROWS)
@@ -1951,7 +1951,8 @@ def experts_few_shared(h: torch.Tensor, gate_up: torch.Tensor, down: torch.Tenso
 
 
 # us of the whole mixture (32 experts of [2 x 1536, 2048] + [2048, 1536], four a token), shared expert as launches of its own / in the grouped ones: 1 token 45.3 / 38.7, 8: 92.7 / 85.7, 16: 117.4 / 107.5,
-# 64: 132.0 / 124.0, 128: 135.3 / 127.6.  Beyond a decode batch the shared expert's tokens are several runs of rows, each of which reads its weights, and the library's products take them in one.
+# 64: 132.0 / 124.0, 128: 135.3 / 127.6.  Over nine mixtures (8 to 256 experts of 256 to 1,536, two to eight a token) at 1 to 128 tokens 1.13 times as fast in the mean, the worst 0.99.  The line is the largest batch
+# that is replayed as a graph, not where the gain ends: decode steps of 160 to 256 tokens were measured 1.00 to 1.31 times as fast but for one of 27 (8 experts, 256 tokens: 66.5 / 72.0).
 SHARED_ROWS_MAX = 128
 
 

@@ -7,7 +7,8 @@ AHEAD = [(1, 1024, 2048), (8, 6144, 4096), (8, 12288, 4096), (5, 65536, 2048), (
 BEHIND = [(8, 7120, 768), (1, 7168, 1024), (8, 8192, 1024), (8, 9216, 1024), (8, 15936, 640), (8, 7168, 3072), (4, 560, 8672), (1, 928, 2976), (8, 7712, 1120), (8, 352, 28128),
           (8, 21968, 2400), (16, 13776, 6144), (9, 14112, 192), (9, 79424, 64), (16, 64064, 448), (9, 1024, 14336), (16, 768, 12640), (24, 5872, 608), (32, 5872, 608), (25, 6144, 1024)]
 GATED_AHEAD = [(1, 6144, 1024), (8, 24576, 4096), (8, 7168, 2048), (8, 8192, 1536), (16, 6144, 2048), (24, 4096, 1024), (9, 10240, 1536), (24, 10240, 1024), (16, 3200 + 944, 1696)]
-GATED_BEHIND = [(8, 7168, 1024), (8, 8192, 768), (1, 1408, 2336), (8, 3424, 8224), (24, 10240, 1536), (16, 45984, 96), (9, 81440, 64), (16, 1408, 5280), (21, 4992, 2528), (9, 24576, 4096)]
+GATED_BEHIND = [(8, 7168, 1024), (8, 8192, 768), (1, 1408, 2336), (8, 3424, 8224), (24, 10240, 1536), (16, 45984, 96), (9, 81440, 64), (16, 1408, 5280), (21, 4992, 2528), (9, 24576, 4096), (16, 8192, 1760),
+                (24, 1024, 8192)]
 
 
 @pytest.mark.parametrize("sizes,gated,wanted", [(AHEAD, False, True), (BEHIND, False, False), (GATED_AHEAD, True, True), (GATED_BEHIND, True, False)])
