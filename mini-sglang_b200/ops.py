@@ -1104,23 +1104,26 @@ def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tens
     act: one of the ACT_ numbers.  Where a kernel with the activation in its epilogue applies (silu and relu; a few rows, or
     many rows in bfloat16) the [T, 2I] intermediate never exists.  ahead: the weight of the product that takes the result, which the kernel for a few rows
     and a small weight asks into L2 as it ends."""
-    _need_cuda(x, gate_up, bias)
+    if not (x.is_cuda and gate_up.is_cuda and (bias is None or bias.is_cuda)):
+        _need_cuda(x, gate_up, bias)
     mode = GLU_MODES.get(act)
     if mode is not None:
-        if _small_m_ok(x, gate_up, bias) and (gate_up.shape[0] // 2) % 8 == 0:
-            M, (N, K) = x.shape[0], gate_up.shape
+        rows = x.shape[0]
+        if rows <= SMALL_M_MAX and _small_m_ok(x, gate_up, bias) and (gate_up.shape[0] // 2) % 8 == 0:
+            M, (N, K) = rows, gate_up.shape
             out = torch.empty((M, N // 2), dtype=torch.bfloat16, device=x.device)
             code = _small_m(gate_up, x, bias, out, M, N, K, N // 2, mode, 0, ahead)
             _check(code, "gemm_small_m (gated)")
             return out
-        y = _gemm_stream(x, gate_up, bias, mode, torch.bfloat16)
-        if y is not None:
-            return y
-        if x.dim() == 2 and not MID_GEMM and x.shape[0] <= _rows_glu_max(gate_up.numel()):
+        if SMALL_M_MAX < rows <= STREAM_ROWS_GATED:
+            y = _gemm_stream(x, gate_up, bias, mode, torch.bfloat16)
+            if y is not None:
+                return y
+        if rows <= ROWS_GLU_MAX_LARGE and x.dim() == 2 and not MID_GEMM and rows <= _rows_glu_max(gate_up.numel()):
             y = _gemm_rows(x, gate_up, bias, mode, torch.bfloat16)
             if y is not None:
                 return y
-        y = _tc_gemm(x, gate_up, bias, mode) if x.shape[0] >= TC_GEMM_MIN_M else _tc_gemm_mid(x, gate_up, bias, mode)
+        y = _tc_gemm(x, gate_up, bias, mode) if rows >= TC_GEMM_MIN_M else _tc_gemm_mid(x, gate_up, bias, mode)
         if y is not None:
             return y
     gu = torch.nn.functional.linear(x, gate_up, bias)
