@@ -1115,7 +1115,7 @@ def linear_glu(x: torch.Tensor, gate_up: torch.Tensor, bias: Optional[torch.Tens
             code = _small_m(gate_up, x, bias, out, M, N, K, N // 2, mode, 0, ahead)
             _check(code, "gemm_small_m (gated)")
             return out
-        if SMALL_M_MAX < rows <= STREAM_ROWS_GATED:
+        if SMALL_M_MAX < rows <= STREAM_ROWS_SMALL:
             y = _gemm_stream(x, gate_up, bias, mode, torch.bfloat16)
             if y is not None:
                 return y
