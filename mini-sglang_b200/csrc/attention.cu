@@ -1423,6 +1423,8 @@ __global__ void __launch_bounds__(SIMT_THREADS) attn_simt_kernel(const AttnParam
 // memory within the warp, so the block meets once a key tile.  The kernel above takes 26 us a key tile (4-byte loads with a page
 // lookup each, one score a thread at a time).  Device us, 16 heads on 8 of 128, one group / two groups, two stages, two steps unrolled / as it is:
 // 210 and 37 tokens 27.9 / 26.2 / 25.6, 8 on 200 21.4 / 18.8 / 17.8, 700 tokens 133.6 / 121.7 / 115.2; four steps unrolled with two stages 25.5, 18.1, 119.0.
+// Over 88 steps at head sizes 16 to 128 1.18 times as fast as one group in the mean; behind are, at head size 64, 2,000 tokens of 16 heads on 4 (508 / 534: two blocks of eight warps an SM by registers, five of four
+// before) and 64 single tokens on 12 of 12 heads (65.7 / 67.3).  Three blocks an SM at head sizes up to 64 (80 registers) are 3 % slower in the mean.
 // Bound by the reads of shared memory (q again for every key) and, where few blocks run, by a tile's chain of 1.8 us.  With q in registers
 // (239 of them, so one block an SM) the chain is 1.5 us, but 210 and 37 tokens take 28.6 and 700 116.5.
 constexpr int F32_GROUPS = 2, F32_THREADS = F32_GROUPS * SIMT_THREADS;

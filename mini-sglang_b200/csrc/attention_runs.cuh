@@ -19,14 +19,16 @@
 // decode_t_run: keys on the M dimension of the mma with the head's elements permuted (16 bytes a lane), P through movmatrix, the
 // exponentials' reference moved only where a score lies DEC_LAZY above it.
 //
-// Bound by the stream of keys and values (8 requests of 4,096 keys, 134 MB: 18 us of the launch's 28 at 7.3 TB/s), then by the cut at its start
-// (1.3 us, under the kernels ahead of it as far as they last) and the exchange of partial results at its end (2 to 4 us).  An attention layer
+// Bound by the stream of keys and values (8 requests of 4,096 keys, 134 MB: 21 of the launch's 28 us from the first units asked for to the latest block's last one, 6.4 TB/s, part of them asked into L2 before that), then by
+// the cut at its start (1.3 us, under the kernels ahead of it as far as they last) and the exchange of partial results at its end (2 to 4 us).  An attention layer
 // before / with it, us (kernels of four warps with kv splits from the host and a merge of their own): 8B, 8 x 4,096 keys 58.7 / 51.8;
 // 4B, 40 of 64 ... 6,000 76.6 / 58.2; 8B, 64 x 2,000 133.6 / 113; 1.7B, one of 130 18.2 / 14.3, 16 x 512 32.9 / 25.2, 64 of 4 ... 64 23.2 / 22.5.
-// Rings of two units and of three are level but for 64 x 2,000 (113.0 / 114.8), and two leave room for a block of the product behind.  Without
+// Rings of two units and of three are level but for 64 x 2,000 (113.0 / 114.8), so it is two (58 KB of an SM are then free for a block behind: norms and small products, not a ring of gemm_stream.cu).  Without
 // RUN_HEAD the mixed case takes 70.6: the block that gets the short requests runs 49 us, the others 34.  Decoded tokens among prompt portions, launched behind the prefill tiles and
 // ahead of their merges, so that its blocks take the SMs that the last tiles leave free (8B, 1,500, 333, 65, 1, 1, 1 tokens behind 0, 700, 4,000, 2,047, 511, 37: the
 // layer 223.8 -> 213.7 us; before, 18 us of decode attention ahead of the tiles and a merge over all tokens of 9).
+// Against the kernels with kv splits over 837 steps (12 pairs of head counts, 1 to 256 requests, keys alike, spread and short, pages of 16): 1.58 times as fast in the mean, four behind by 4 to 6 % (64 x 128 keys on 7 of 7
+// heads 10.7 / 11.4, 5 x 128 on 64 of 64 8.8 / 9.3, 8 x 128 on 40 of 40 8.9 / 9.3, 17 x 600 on 32 of 32 35.6 / 36.9); pages of 48, 132 steps: 1.55, none behind.
 #pragma once
 
 constexpr int RUN_NW = 8;            // warps of a block

@@ -1,6 +1,6 @@
-// Weight-streaming matrix product for decode: out[M, N] = x[M, K] . W[N, K]^T with M <= 16 tokens.  Here come weights
-// of less than 2 million elements; for larger ones gemm_stream.cu is ahead (one row, us here / there: [1024, 1024] 1.63 / 1.86,
-// [2048, 1024] 2.47 / 2.22, [1024, 3072] 4.02 / 3.08).
+// Weight-streaming matrix product for decode: out[M, N] = x[M, K] . W[N, K]^T with M <= 16 tokens (the engine sends up to 8).  Here come weights
+// of less than 2 million elements and larger ones whose sizes suit gemm_stream.cu ill, which is ahead on the others (one row, us here / there:
+// [1024, 1024] 1.63 / 1.86, [2048, 1024] 2.47 / 2.22, [1024, 3072] 4.02 / 3.08; the rule and its figures stand in ops.py).
 //
 // With so few tokens the product is bound by reading W once from HBM, so the kernel is built
 // around that stream:
@@ -193,12 +193,10 @@ __global__ void __launch_bounds__(GS_WARPS * 32) gemm_small_m_kernel(
 }
 
 // ahead: the weights of the product that comes next (gated modes; or null), which the blocks ask into L2 as they end, so that the memory has work while the last of them and
-// the next launch leave it idle.  A feed-forward with weights that come from memory, with the request / without it, us.  Of the sizes that come here (below 2 million elements of W):
-// 256 x 2,560 (320 blocks) 5.3 / 5.9.  The line was drawn with larger ones too, which have a kernel of their own since: 1,024 x 3,072 (384 blocks): 1 token 7.8 / 8.5, 8: 7.9 / 8.6;
-// 1,024 x 2,432 (304 blocks) 6.9 / 7.4; 4,096 x 3,072 with 512 outputs 14.5 / 15.3.  So where more than two blocks an SM come and all run at once (three).  With
-// fewer each asks for more at its end, and the product itself is short: 1,024 x 1,024 (128 blocks) 5.7 / 5.5, 2,048 x 768 7.1 / 6.3; with more the first ones' requests are in the way of
-// the others' streams: 2,048 x 6,144 (768 blocks) 22.4 / 20.6.  Not for weights of more than 6.5 MB or half of this product's own: 1,024 x 2,432 with 1,664 outputs (8 MB) 8.0 / 7.8,
-// 512 x 2,432 with 1,536 outputs 7.2 / 6.6.  (Where all weights are in L2 already it costs up to 8 %.)
+// the next launch leave it idle.  Asked for where more than two blocks an SM come and all run at once (three), which of the sizes that come here are those with inner sizes
+// below 423 alone (more than 296 blocks of 16 rows in less than 2 million elements).  A feed-forward with weights that come from memory, with the request / without it, us:
+// 256 x 2,560 (320 blocks) 5.3 / 5.9.  With fewer blocks each asks for more at its end, and the product itself is short: 1,024 x 1,024 (128 blocks) 5.7 / 5.5.  Not for weights of more
+// than 6.5 MB or half of this product's own: 512 x 2,432 with 1,536 outputs 7.2 / 6.6.  (Where all weights are in L2 already it costs up to 8 %.)
 // mode: 0 = plain (out [M, N]), 1 / 2 = SwiGLU / ReGLU (W [2I, K], bias [2I], out [M, I], N = 2I).  out_f32: output type.
 MSGL_API int msgl_gemm_small_m(const void* W, const void* X, const void* bias, void* out, int M, int N, int K,
                                long long ldx, long long ldo, int mode, int out_f32, const void* ahead, long long ahead_bytes, cudaStream_t stream) {

@@ -18,6 +18,9 @@
 // 8 up rows that belong to them, which land in the two row halves of the accumulator fragment, so
 // out[M, I] = act(gate (+ bias)) * (up (+ bias)) is formed in registers and the [M, 2I] intermediate never exists.
 //
+// Which sizes come here is `_stream_rule` in ops.py, with the figures: not those where passes of few rounds, copies a chunk (K no multiple of 64) or, from 9 rows on, passes and the reads of x cost more
+// than the kernels that have the others.
+//
 // What bounds it: the stream of W (8B, 1 token: gate/up and down 302 MB in 48.4 us, 6.2 TB/s; before, in blocks of 16 rows by cp.async of 16 bytes, 53.5), and with small weights the
 // chain from the wait to the last store (0.6B feed-forward: 7.1 us a layer for 19 MB, before 8.2).  us of a product in a chain of them, before / now, 1 row: [4096, 4096] 8.0 / 7.3,
 // [5120, 5120] 12.6 / 10.0 (320 blocks on 148 SMs before), [4096, 12288] 19.4 / 17.4, gated [24576, 4096] 35.9 / 33.5, [51200, 5120] 81.7 / 77.3; 8 rows: 8.5 / 7.9, 13.4 / 10.8, 20.2 / 18.0, 36.9 / 34.0,
