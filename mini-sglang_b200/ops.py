@@ -732,33 +732,40 @@ def _small_m(weight, x, bias, out, M, N, K, ldo, mode, out_f32, ahead=None) -> i
 
 
 # Where the kernel of one block an SM is ahead; us of a product with weights from memory, other kernel (blocks of 16 rows up to 8 rows, then the library and, gated, the decode-batch kernel) then
-# this one.  Lines in columns follow the B200's 148 SMs: 7,104 columns are 48 on each, the most of one pass, 2,072 are 14, 2,960 and (gated) 4,144 are 20.
+# this one.  Lines in columns follow the B200's 148 SMs: 7,104 columns are 48 on each, the most of one pass, 2,072 are 14, 2,960 are 20, (gated) 5,328 are 36.
 # Up to 8 rows: behind where a block has more than one pass of few rounds (576 elements of K each), by STREAM_SHORT's pairs of columns and K (the first for plain products alone).  8 rows of [7120, 768]
 # 4.2 5.1, [7120, 3072] 10.4 10.9, [7424, 2048] 8.4 8.4, [8192, 1024] 5.3 6.0, [8192, 4096] 16.0 14.2, [9216, 1024] 5.5 6.1, [9728, 1024] 6.0 6.1, [15936, 640] 6.5 7.2; gated [8192, 1024] 5.4 5.7,
-# [7424, 2048] 9.0 8.0.  An inner size that is no multiple of 64 is nine copies a round: [560, 8672] 7.5 11.2, [928, 2976] 3.8 4.4, gated 4.1 6.9, [7712, 1120] 5.5 6.2, but [3088, 1056] 3.6 2.9.
+# [7424, 2048] 9.0 8.0.  Plain products of five rows and more with two passes or more also where the last of two or three rounds brings 160 elements of K at most: [14784, 1216] 8.8 9.5, [15376, 1280] 9.4 9.7,
+# [21344, 704] 8.4 9.0, but [14592, 1024] 7.9 7.8, [21344, 1536] 14.1 13.3.  An inner size that is no multiple of 64 is nine copies a round: [560, 8672] 7.5 11.2, [928, 2976] 3.8 4.4, gated 4.1 6.9, [7712, 1120] 5.5 6.2, gated [4480, 4960] 10.0 10.6, [14224, 288] 4.3 5.0, but [3088, 1056] 3.6 2.9.
 # From 9 rows on every SM reads all rows of x, which costs more the more rows there are, and passes cost more: at 9 / 16 / 24 / 32 rows
 # [4096, 1024] 4.8 4.8 4.9 4.9, 2.9 3.7 4.1 4.5; [1024, 3072] 8.5 8.5 7.6 7.5, 4.5 4.5 4.9 6.1; [2048, 6144] 10.5 10.5 10.5 10.6, 8.6 9.1 8.1 9.7; [4096, 2048] 6.2 6.3 6.4 6.4, 5.3 5.5 6.2 7.4;
 # [6144, 4096] 12.8 12.9 12.1 13.2, 11.8 12.0 13.3 24; [4096, 12288] 22.0 22.1 22.6 22.7, 18.5 19.2 23.4 32; [5120, 25600] 49.6 46.8 46.2 46.3, 43.2 43.4 55 69.  Gated: [6144, 1024] 6.4 6.4 6.7 6.9,
 # 4.4 4.7 5.1 7.0; [12288, 2048] 12.0 12.3 12.5 12.9, 11.9 12.3 13.5 16.7; [24576, 4096] 35.8 36.6 36.1 36.8, 37.7 38.9 41.6 54.
 # More than one pass at 16 rows: [13776, 6144] 29.8 30.6, [14112, 192] 4.1 4.4, [64064, 448] 12.8 16.1, [116480, 128] 9.5 21.6; gated, two passes: [10240, 1024] 8.1 7.6 and [10240, 1536] 9.6 10.5 at 24 rows, seven:
-# [45984, 96] 4.9 11.2.  From K = 14,336 on the library cuts K up: [1024, 12288] x 16 27.0 15.9, [1024, 14336] 14.4 17.9, with more columns [2560, 25600] x 9 31.1 25.7.  No multiple of 64: [448, 6880] x 16 8.0 8.8,
-# [5872, 608] x 24 4.5 5.0, gated [1408, 5280] x 16 7.8 10.1, [4992, 2528] x 21 8.8 9.7, [8192, 1760] x 16 9.5 10.5.  Gated, long inner sizes, 24 rows: [1024, 8192] 9.5 10.0, [928, 11904] 11.9 13.2, [1184, 6848] 8.8 8.5.
+# [45984, 96] 4.9 11.2.  From K of some 12,900 on the library cuts K up: [1024, 12288] x 16 27.0 15.9, [608, 12992] 13.2 15.7, [1024, 14336] 14.4 17.9, with more columns [2560, 25600] x 9 31.1 25.7.  No multiple of 64: [448, 6880] x 16 8.0 8.8,
+# [5872, 608] x 24 4.5 5.0, little in the last round: [3440, 1216] x 32 5.0 5.8, [6224, 704] 4.8 7.2, gated [1408, 5280] x 16 7.8 10.1, [4992, 2528] x 21 8.8 9.7, [8192, 1760] x 16 9.5 10.5.  Gated, long inner sizes, 24 rows: [1024, 8192] 9.5 10.0, [928, 11904] 11.9 13.2, [1184, 6848] 8.8 8.5.
 STREAM_ROWS, STREAM_ROWS_FEW_COLUMNS, STREAM_ROWS_SMALL, STREAM_FEW_COLUMNS, STREAM_SMALL_WEIGHTS = 16, 24, 32, 2_072, 4_500_000
 STREAM_ROWS_GATED, STREAM_GATED_LEAST, STREAM_GATED_MOST = 24, 4_000_000, 16_000_000      # ([8192, 2048], 16.8 million, is ahead too, [10240, 2048] and [12288, 2048] are not)
 STREAM_ONE_PASS, STREAM_ROUND, STREAM_SHORT, STREAM_GATED_INNER, STREAM_GATED_LONG = 7_104, 576, ((7_400, 3_600), (10_000, 1_300), (17_000, 800)), 1_100, 7_000
-STREAM_LONG_INNER, STREAM_LONG_COLUMNS, STREAM_RAGGED, STREAM_RAGGED_GATED = 13_000, 2_560, 2_960, 4_144
+STREAM_THIN_COLUMNS, STREAM_THIN_INNER, STREAM_THIN_ROUND = 23_000, 1_300, 160
+STREAM_LONG_INNER, STREAM_LONG_COLUMNS, STREAM_RAGGED, STREAM_RAGGED_GATED, STREAM_RAGGED_WIDE = 12_500, 2_560, 2_960, 5_328, 17_000
 
 
 def _stream_rule(rows: int, N: int, K: int, gated: bool) -> bool:
     """Whether a product goes to the kernel of one block an SM."""
     if N * K < STREAM_MIN_WEIGHTS or N % 16 or K % 32 or (K % 64 and N < (STREAM_RAGGED_GATED if gated else STREAM_RAGGED)):
         return False
+    thin = 0 < K % STREAM_ROUND <= STREAM_THIN_ROUND          # the last round brings little
     if rows <= 8:
-        return N <= STREAM_ONE_PASS or K <= STREAM_ROUND or not (K % 64 or any(N <= columns and K <= inner for columns, inner in STREAM_SHORT[gated:]))
+        if N <= STREAM_ONE_PASS or (K <= STREAM_ROUND and (N > STREAM_RAGGED_WIDE or not K % 64)):
+            return True
+        if K % 64 or any(N <= columns and K <= inner for columns, inner in STREAM_SHORT[gated:]):
+            return False
+        return gated or rows <= 4 or N > STREAM_THIN_COLUMNS or K > STREAM_THIN_INNER or not thin
     if gated:
         return (rows <= (STREAM_ROWS if K % 64 or K > STREAM_GATED_LONG else STREAM_ROWS_GATED) and STREAM_GATED_LEAST <= N * K <= STREAM_GATED_MOST
                 and (N <= STREAM_ONE_PASS or (N <= 2 * STREAM_ONE_PASS and not K % 64 and (rows <= STREAM_ROWS or K <= STREAM_GATED_INNER))))
-    if N > STREAM_ONE_PASS or (K > STREAM_LONG_INNER and N < STREAM_LONG_COLUMNS) or (K % 64 and rows > STREAM_ROWS):
+    if N > STREAM_ONE_PASS or (K > STREAM_LONG_INNER and N < STREAM_LONG_COLUMNS) or (rows > STREAM_ROWS and (K % 64 or (thin and N > STREAM_FEW_COLUMNS))):
         return False
     return rows <= (STREAM_ROWS_SMALL if N * K <= STREAM_SMALL_WEIGHTS else STREAM_ROWS_FEW_COLUMNS if N <= STREAM_FEW_COLUMNS else STREAM_ROWS)
 
@@ -945,16 +952,17 @@ def _observed(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor
 # Plain products of a decode batch with a long inner size (down projections) on the decode-batch kernel, whose ranges of K give them enough blocks; us, library / kernel, at 33 / 48 / 64 rows:
 # [1024, 3072] 6.8 / 6.1, 6.8 / 6.2, 6.7 / 6.4; [2048, 8192] 13.4 / 11.2, 13.3 / 11.6, 13.4 / 12.1; [2560, 9728] 15.7 / 13.9, 15.9 / 14.4, 15.6 / 14.6; [4096, 12288] 22.6 / 21.5, 22.5 / 21.9,
 # 22.6 / 22.4; [5120, 17408] 39.0 / 33.0, 41.0 / 34.0, 36.1 / 35.1; at 80 rows behind on half of them.  Shorter inner sizes: [5120, 8192] 18.2 / 18.9 at 33 rows, [4096, 4096] 10.3 / 10.7 at 48.
-# From K = 20,480 on the library cuts K of few columns up: at 48 rows [512, 18432] 16.5 / 16.0, [512, 20480] 13.9 / 17.4, at 64 [1536, 24576] 20.5 / 22.6, [3584, 32768] 45.2 / 44.2.  Between 4,096 and 5,120
-# columns eight ranges of K make 264 to 304 blocks in clusters of eight, and it is behind (256 blocks of 4,096 columns and 320 of 5,120 are not): at 48 rows [4096, 16384] 28.9 / 28.2, [4352, 16384] 29.0 / 39.9, [4736, 16128] 30.4 / 40.2, [5120, 16384] 38.9 / 32.1.
+# From K = 20,480 on the library cuts K of few columns up: at 48 rows [512, 18432] 16.5 / 16.0, [512, 20480] 13.9 / 17.4, at 64 [1536, 24576] 20.5 / 22.6, [3584, 32768] 45.2 / 44.2.  Eight ranges of K
+# are clusters of eight blocks, a tile of 128 columns each: behind with 33 to 39 tiles, planned two blocks an SM, and from 51 on, planned three, as if 32 and 48 clusters were all that run at once: at 48 rows
+# [4096, 16384] 28.9 / 28.2, [4352, 16384] 29.0 / 39.9, [4736, 16128] 30.4 / 40.2, [5120, 16384] 38.9 / 32.1, at 24 [6144, 20480] ahead by 4 to 8 %, [6480, 20352] 49.5 / 58.5.
 # (What the rule takes was measured at 533 sizes and rows: one of them, 64 rows of [4096, 14336], is 3 % behind.)
 ROWS_PLAIN_MAX, ROWS_PLAIN_INNER, ROWS_PLAIN_WEIGHTS = 64, 3, 3_000_000
-ROWS_PLAIN_LONGEST, ROWS_PLAIN_LONG_COLUMNS, ROWS_PLAIN_GAP = 18_432, 3_584, (4_096, 5_120)
+ROWS_PLAIN_LONGEST, ROWS_PLAIN_LONG_COLUMNS, ROWS_PLAIN_GAP, ROWS_PLAIN_COLUMNS = 18_432, 3_584, (4_096, 5_120), 6_144
 
 
 def _rows_plain(rows: int, N: int, K: int) -> bool:
     return (SMALL_M_MAX < rows <= ROWS_PLAIN_MAX and K >= ROWS_PLAIN_INNER * N and N * K >= ROWS_PLAIN_WEIGHTS and (K <= ROWS_PLAIN_LONGEST or N >= ROWS_PLAIN_LONG_COLUMNS)
-            and not ROWS_PLAIN_GAP[0] < N < ROWS_PLAIN_GAP[1] and not MID_GEMM)
+            and not ROWS_PLAIN_GAP[0] < N < ROWS_PLAIN_GAP[1] and N <= ROWS_PLAIN_COLUMNS and not MID_GEMM)
 
 
 def _gemm_rows_plain(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out_dtype: torch.dtype) -> Optional[torch.Tensor]:
